@@ -1106,7 +1106,12 @@ constexpr size_t smem_bytes() {
 // and face-adjacent sum F, and the node at z uses D(z), F(z-1), F(z+1), D(z-1), D(z+1).
 // FACES (coarse levels): nodes on the low domain faces use their 27-entry table row, which does
 // couple z-neighbours of the same class; those take the values from before the phase (new
-// values are written after a barrier), a Jacobi step along the column for those rows only.
+// values are written after a barrier), a Jacobi step along the column for those rows only.  On the
+// coarse levels these rows are a phase's critical path (few blocks, most of them on a face), so a
+// row is unrolled: its 26 tile and table loads (the table in shared memory) are in flight together
+// before the chain of its multiply-adds.  In a rolled loop with the table in global memory a launch
+// of the levels 16^3 to 64^3 took 29-31 us (115 us at 8 planes per thread); a depth-7 reconstruction
+// of 20,011 points went from 4.65 to 3.22 ms and a depth-9 one of 317,003 from 33.0 to 29.9 ms.
 namespace g16 {
 constexpr int CW = s16::CW;  // ZT, NT: as n16 (a node's relaxation is the same for every ZT)
 // Parity-split tile (u = local + 1 in 0..17 per axis): each row holds its even columns (u even)
@@ -1192,6 +1197,7 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
   T* tile = reinterpret_cast<T*>(smem_raw);  // TILE
   T* ctile = tile + TILE;                    // CW^3 (MODE 2)
   __shared__ uint32_t nb[27], cnb[27];
+  __shared__ T ftab[FACES ? 216 : 1];  // the face rows
   const int res = 1 << D;
   {
     const uint64_t nl = 1ull << (3 * D);
@@ -1214,6 +1220,9 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
   unmorton3(blk, bx, by, bz);
   const int ox = (int)bx * 16, oy = (int)by * 16, oz = (int)bz * 16;
   const int t = threadIdx.x;
+  const bool faces = FACES && (ox == 0 || oy == 0 || oz == 0);  // uniform in the block
+  if (faces)
+    for (int i = t; i < 216; i += NT) ftab[i] = table[i];  // read after the barriers below
   constexpr bool FROM_ZERO = MODE == 1 || MODE == 3;
   if (!FROM_ZERO) s16::neighbour_bases(nb, bx, by, bz, res >> 4);
   else if (t < 27) nb[t] = ~0u;  // zero halo
@@ -1291,7 +1300,6 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
     }
     __syncthreads();
   }
-  const bool faces = FACES && (ox == 0 || oy == 0 || oz == 0);
 #pragma unroll
   for (int ph = 0; ph < 4; ++ph) {
     const int cls = FWD ? ph : 3 - ph;
@@ -1306,17 +1314,19 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
       default: relax_column<T, 3, ZERO, ZT>(tile, x0, y0, z0, fv, v, ce, cc, c0inv, nv); break;
     }
     if (faces) {  // low-domain-face nodes of this column: their table rows, neighbours from the tile
+      const int cl = col(x), cm1 = col(x + 1), cr = col(x + 2);  // tile columns x-1, x, x+1
 #pragma unroll 1
       for (int k = 0; k < ZT; ++k) {
         const int z = z0 + k;
         const int mask = ((ox + x) == 0) | (((oy + y) == 0) << 1) | (((oz + z) == 0) << 2);
         if (!mask) continue;
-        const T* cm = table + 27 * mask;
+        const T* cm = ftab + 27 * mask;
+        const T* tb = tile + z * PS + y * RS;  // tile row y-1 of tile plane z-1
         T off = 0;
-#pragma unroll 1
+#pragma unroll
         for (int o = 0; o < 27; ++o) {
           if (o == 13) continue;
-          off += cm[o] * tile[nat(x + 1 + (o % 3 - 1), y + 1 + ((o / 3) % 3 - 1), z + 1 + (o / 9 - 1))];
+          off += cm[o] * tb[(o / 9) * PS + ((o / 3) % 3) * RS + (o % 3 == 0 ? cl : (o % 3 == 1 ? cm1 : cr))];
         }
         T fk = fv[0][cls];
 #pragma unroll
@@ -1327,8 +1337,8 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
         for (int kk = 0; kk < ZT; ++kk)
           if (kk == k) nv[kk] = nvk;
       }
+      __syncthreads();  // same-class column neighbours were read with their old values
     }
-    if (FACES) __syncthreads();  // same-class column neighbours were read with their old values
 #pragma unroll
     for (int k = 0; k < ZT; ++k) {
       v[k][cls] = nv[k];
@@ -1419,14 +1429,15 @@ void smooth_dispatch(cudaStream_t s, uint32_t D, const T* xi, T* xo, const T* f,
 // per thread, i.e. 512, 256 or 128 threads per 16^3 brick: more planes per thread read fewer halo
 // planes from shared memory per node but leave fewer threads to hide latency.  Every ZT computes
 // the same values (per-block sums in a fixed order), so the choice is free and made by timing: the
-// first FP32 launch of a (kernel family, level, launch size) key times each ZT (one warm-up and
+// first FP32 launch of a (kernel family, level, launch size, with or without face rows: the same
+// level is one solve's finest and another's coarse) key times each ZT (one warm-up and
 // three timed launches on the launch's own buffers; every candidate writes what the real launch
 // then overwrites) and keeps the fastest for the process.  FP64 launches and launches inside a
 // stream capture use ZT = 4.  PR_AUTOTUNE=0 fixes ZT = 4; PR_ZT=2|4|8 forces one.
 enum TuneFamily { kTuneSpmv = 0, kTuneResid = 1, kTuneSmooth = 2, kTuneSmoothPost = 3 };
 struct TuneTable {
   std::mutex mu;
-  std::map<std::tuple<int, int, int, int>, int> zt;  // (device, family, level, log2 blocks) -> ZT
+  std::map<std::tuple<int, int, int, int, bool>, int> zt;  // (device, family, level, log2 blocks, faces) -> ZT
   std::string log;
 };
 TuneTable& tune_table() {
@@ -1451,7 +1462,7 @@ int forced_zt(int family) {
 
 // Runs launch(zt) with the ZT of the key, timing the candidates first for a new key.
 template <typename L>
-void tuned_launch(cudaStream_t s, int family, uint32_t level, uint64_t blocks, bool tunable, L launch) {
+void tuned_launch(cudaStream_t s, int family, uint32_t level, uint64_t blocks, bool faces, bool tunable, L launch) {
   if (!tunable) {
     launch(4);
     return;
@@ -1464,7 +1475,7 @@ void tuned_launch(cudaStream_t s, int family, uint32_t level, uint64_t blocks, b
   PR_CUDA(cudaGetDevice(&dev));
   int bin = 0;
   while ((2ull << bin) <= blocks) ++bin;
-  const auto key = std::make_tuple(dev, family, (int)level, bin);
+  const auto key = std::make_tuple(dev, family, (int)level, bin, faces);
   TuneTable& tt = tune_table();
   {
     std::lock_guard<std::mutex> g(tt.mu);
@@ -1502,8 +1513,8 @@ void tuned_launch(cudaStream_t s, int family, uint32_t level, uint64_t blocks, b
     std::lock_guard<std::mutex> g(tt.mu);
     tt.zt[key] = cand[best];
     char line[200];
-    std::snprintf(line, sizeof(line), "%s level %u blocks 2^%d: ZT 2/4/8 = %.4f/%.4f/%.4f ms -> ZT %d\n",
-                  family_name(family), level, bin, ms[0] / 3, ms[1] / 3, ms[2] / 3, cand[best]);
+    std::snprintf(line, sizeof(line), "%s level %u%s blocks 2^%d: ZT 2/4/8 = %.4f/%.4f/%.4f ms -> ZT %d\n",
+                  family_name(family), level, faces ? " (faces)" : "", bin, ms[0] / 3, ms[1] / 3, ms[2] / 3, cand[best]);
     tt.log += line;
   }
   launch(cand[best]);
@@ -1521,7 +1532,7 @@ void launch_s16(cudaStream_t s, uint32_t D, const T* xi, T* xo, const T* f, cons
         D, xi, xo, f, ec, (T)(1.0 / L.c0), (T)L.ce, (T)L.cc, table, part, CgFuse<T>());
   };
   constexpr bool kTunable = std::is_same<T, float>::value && MODE != 0;
-  tuned_launch(s, MODE == 2 ? kTuneSmoothPost : kTuneSmooth, D, (uint64_t)grid.x * grid.y, kTunable, [&](int zt) {
+  tuned_launch(s, MODE == 2 ? kTuneSmoothPost : kTuneSmooth, D, (uint64_t)grid.x * grid.y, FACES, kTunable, [&](int zt) {
     if constexpr (kTunable) {
       if (zt == 2) return go(std::integral_constant<int, 2>());
       if (zt == 8) return go(std::integral_constant<int, 8>());
@@ -1668,7 +1679,7 @@ void mg_resid_restrict(cudaStream_t s, const LevelCoef& L, const T* table, const
       else go(z, std::false_type());
     };
     constexpr bool kTunable = std::is_same<T, float>::value;
-    tuned_launch(s, kTuneResid, D, (uint64_t)nb * clouds, kTunable, [&](int zt) {
+    tuned_launch(s, kTuneResid, D, (uint64_t)nb * clouds, L.has_faces, kTunable, [&](int zt) {
       if constexpr (kTunable) {
         if (zt == 2) return go_f(std::integral_constant<int, 2>());
         if (zt == 8) return go_f(std::integral_constant<int, 8>());
@@ -1709,7 +1720,7 @@ void mg_spmv(cudaStream_t s, const LevelCoef& L, const T* table, const T* z, con
       }
     };
     constexpr bool kTunable = std::is_same<T, float>::value;
-    tuned_launch(s, kTuneSpmv, D, (uint64_t)g.x * g.y, kTunable, [&](int zt) {
+    tuned_launch(s, kTuneSpmv, D, (uint64_t)g.x * g.y, false, kTunable, [&](int zt) {
       if constexpr (kTunable) {
         if (zt == 2) return go(std::integral_constant<int, 2>());
         if (zt == 8) return go(std::integral_constant<int, 8>());
