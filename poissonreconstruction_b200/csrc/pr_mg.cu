@@ -99,6 +99,59 @@ __device__ __forceinline__ T ldg_or0(const T* __restrict__ x, int gx, int gy, in
   return __ldg(x + morton3(gx, gy, gz));
 }
 
+// Gauss-Seidel value of one node of colour (cx, cy, cz) in a parity-split tile: `own` its sub-tile,
+// pos its index there, mask its low-face mask (0: the interior row, else its row of the table).
+template <typename T, int TB>
+__device__ __forceinline__ T relax_colour(const T* tile, int own, int cx, int cy, int cz, int pos, int mask, T fi, T c0,
+                                          T ce, T cc, const T* table) {
+  constexpr int H = Geo<TB>::H, H3 = Geo<TB>::H3;
+  T vals[27];
+#pragma unroll
+  for (int o = 0; o < 27; ++o) {
+    const int dx = o % 3 - 1, dy = (o / 3) % 3 - 1, dz = o / 9 - 1;
+    const int sub = own ^ ((dx != 0) | ((dy != 0) << 1) | ((dz != 0) << 2));
+    const int hx = dx == 0 ? 0 : (dx < 0 ? -cx : 1 - cx);
+    const int hy = dy == 0 ? 0 : (dy < 0 ? -cy : 1 - cy);
+    const int hz = dz == 0 ? 0 : (dz < 0 ? -cz : 1 - cz);
+    const int nzc = (dx != 0) + (dy != 0) + (dz != 0);
+    // faces are only read on the (rare) low-face path
+    vals[o] = (o == 13 || (nzc == 1 && mask == 0)) ? (T)0 : tile[sub * H3 + pos + (hz * H + hy) * H + hx];
+  }
+  T nv;
+  if (mask == 0) {
+    T se = 0, sc = 0;
+#pragma unroll
+    for (int o = 0; o < 27; ++o) {
+      const int nzc = (o % 3 != 1) + ((o / 3) % 3 != 1) + (o / 9 != 1);
+      if (nzc == 2) se += vals[o];
+      else if (nzc == 3) sc += vals[o];
+    }
+    nv = (fi - ce * se - cc * sc) / c0;
+  } else {
+    const T* cm = table + 27 * mask;
+    T off = 0;
+#pragma unroll
+    for (int o = 0; o < 27; ++o)
+      if (o != 13) off += cm[o] * vals[o];
+    nv = (fi - off) / cm[13];
+  }
+  return nv;
+}
+
+// P ec at fine node (gx, gy, gz) from a coarse tile of width CW whose entry 0 is coarse node (cox, coy, coz):
+// even -> coarse g/2 (w 1), odd -> (g-1)/2, (g+1)/2 (w 1/2 each)
+template <typename T, int CW>
+__device__ __forceinline__ T prolong_node(const T* ctile, int gx, int gy, int gz, int cox, int coy, int coz) {
+  const int ax = (gx >> 1) - cox, ay = (gy >> 1) - coy, az = (gz >> 1) - coz;
+  const int nx = 1 + (gx & 1), ny = 1 + (gy & 1), nz = 1 + (gz & 1);
+  T s = 0;
+  for (int a = 0; a < nz; ++a)
+    for (int b = 0; b < ny; ++b)
+      for (int c = 0; c < nx; ++c) s += ctile[((az + a) * CW + (ay + b)) * CW + (ax + c)];
+  const T w = (T)(((gx & 1) ? 0.5 : 1.0) * ((gy & 1) ? 0.5 : 1.0) * ((gz & 1) ? 0.5 : 1.0));
+  return w * s;
+}
+
 // ------------------------------------------------------------------ smoother
 // MODE 0: xo = sweep(xi); MODE 1: xo = sweep(0) (xi unused); MODE 2: xo = sweep(xi + P ec).
 // DOT: part[block] = sum_i f_i xo_i over the block.
@@ -140,17 +193,7 @@ __global__ void __launch_bounds__(Geo<TB>::THREADS) k_smooth(uint32_t D, const T
     }
     __syncthreads();
   }
-  // P ec at global (gx,gy,gz): even -> coarse g/2 (w 1), odd -> (g-1)/2, (g+1)/2 (w 1/2 each)
-  auto prolong = [&](int gx, int gy, int gz) -> T {
-    const int ax = (gx >> 1) - cox, ay = (gy >> 1) - coy, az = (gz >> 1) - coz;
-    const int nx = 1 + (gx & 1), ny = 1 + (gy & 1), nz = 1 + (gz & 1);
-    T s = 0;
-    for (int a = 0; a < nz; ++a)
-      for (int b = 0; b < ny; ++b)
-        for (int c = 0; c < nx; ++c) s += ctile[((az + a) * CW + (ay + b)) * CW + (ax + c)];
-    const T w = (T)(((gx & 1) ? 0.5 : 1.0) * ((gy & 1) ? 0.5 : 1.0) * ((gz & 1) ? 0.5 : 1.0));
-    return w * s;
-  };
+  auto prolong = [&](int gx, int gy, int gz) -> T { return prolong_node<T, CW>(ctile, gx, gy, gz, cox, coy, coz); };
   // interior + f
   for (int t = tid; t < N; t += G::THREADS) {
     uint32_t lx, ly, lz;
@@ -192,37 +235,7 @@ __global__ void __launch_bounds__(Geo<TB>::THREADS) k_smooth(uint32_t D, const T
     if (k.has_faces)
       mask = ((ox == 0 && cx == 0 && li == 0) ? 1 : 0) | ((oy == 0 && cy == 0 && lj == 0) ? 2 : 0) |
              ((oz == 0 && cz == 0 && lk == 0) ? 4 : 0);
-    T vals[27];
-#pragma unroll
-    for (int o = 0; o < 27; ++o) {
-      const int dx = o % 3 - 1, dy = (o / 3) % 3 - 1, dz = o / 9 - 1;
-      const int sub = own ^ ((dx != 0) | ((dy != 0) << 1) | ((dz != 0) << 2));
-      const int hx = dx == 0 ? 0 : (dx < 0 ? -cx : 1 - cx);
-      const int hy = dy == 0 ? 0 : (dy < 0 ? -cy : 1 - cy);
-      const int hz = dz == 0 ? 0 : (dz < 0 ? -cz : 1 - cz);
-      const int nzc = (dx != 0) + (dy != 0) + (dz != 0);
-      // faces are only read on the (rare) low-face path
-      vals[o] = (o == 13 || (nzc == 1 && mask == 0)) ? (T)0 : tile[sub * H3 + pos + (hz * H + hy) * H + hx];
-    }
-    const T fi = fs[col * C3 + tid];
-    T nv;
-    if (mask == 0) {
-      T se = 0, sc = 0;
-#pragma unroll
-      for (int o = 0; o < 27; ++o) {
-        const int nzc = (o % 3 != 1) + ((o / 3) % 3 != 1) + (o / 9 != 1);
-        if (nzc == 2) se += vals[o];
-        else if (nzc == 3) sc += vals[o];
-      }
-      nv = (fi - k.ce * se - k.cc * sc) / k.c0;
-    } else {
-      const T* cm = k.table + 27 * mask;
-      T off = 0;
-#pragma unroll
-      for (int o = 0; o < 27; ++o)
-        if (o != 13) off += cm[o] * vals[o];
-      nv = (fi - off) / cm[13];
-    }
+    const T nv = relax_colour<T, TB>(tile, own, cx, cy, cz, pos, mask, fs[col * C3 + tid], k.c0, k.ce, k.cc, k.table);
     tile[self] = nv;
     __syncthreads();
   }
@@ -374,6 +387,24 @@ __global__ void __launch_bounds__(Geo<TB>::THREADS) k_spmv(uint32_t D, const T* 
   if (tid == 0) part[blk] = s;
 }
 
+// restriction to coarse node (cx, cy, cz) of the block from a WR^3 residual tile whose entry 0 is the
+// fine node -1 per axis
+template <typename T, int WR>
+__device__ __forceinline__ T restrict_full(const T* rt, int cx, int cy, int cz) {
+  const int fx = 2 * cx + 1, fy = 2 * cy + 1, fz = 2 * cz + 1;  // tile coordinate of the fine centre
+  T s = 0;
+#pragma unroll
+  for (int dz = -1; dz <= 1; ++dz)
+#pragma unroll
+    for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+      for (int dx = -1; dx <= 1; ++dx) {
+        const T w = (T)((dx ? 0.5 : 1.0) * (dy ? 0.5 : 1.0) * (dz ? 0.5 : 1.0));
+        s += w * rt[((fz + dz) * WR + (fy + dy)) * WR + (fx + dx)];
+      }
+  return s;
+}
+
 // ------------------------------------------------------------------ residual + restriction
 // fc = P^T (f - A e) for the (TB/2)^3 coarse nodes whose fine centre lies in the block.
 // r is needed on local [-1, TB-1]^3: the block interior (z columns) plus its low shell.
@@ -464,18 +495,7 @@ __global__ void __launch_bounds__(Geo<TB>::THREADS) k_resid_restrict(uint32_t D,
   for (int t = tid; t < TC * TC * TC; t += G::THREADS) {
     uint32_t cx, cy, cz;
     unmorton3((uint32_t)t, cx, cy, cz);
-    const int fx = 2 * cx + 1, fy = 2 * cy + 1, fz = 2 * cz + 1;  // r tile coordinate of the fine centre
-    T s = 0;
-#pragma unroll
-    for (int dz = -1; dz <= 1; ++dz)
-#pragma unroll
-      for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-        for (int dx = -1; dx <= 1; ++dx) {
-          const T w = (T)((dx ? 0.5 : 1.0) * (dy ? 0.5 : 1.0) * (dz ? 0.5 : 1.0));
-          s += w * rt[((fz + dz) * WR + (fy + dy)) * WR + (fx + dx)];
-        }
-    fc[cbase + t] = s;
+    fc[cbase + t] = restrict_full<T, WR>(rt, (int)cx, (int)cy, (int)cz);
   }
 }
 
@@ -887,6 +907,48 @@ constexpr int N = 4096, FACE = 224;  // ZT, NT: as n16 (the residual is the same
 constexpr int RSR = 20, PSR = 16 * RSR + 8, RTILE = 16 * PSR;  // half-warps of the restriction on disjoint banks
 __device__ __forceinline__ int ridx(int x, int y, int z) { return z * PSR + y * RSR + x; }  // local coordinates
 
+// What the low-face row `cm` of a node changes in its residual: (interior row - face row) of A e, with
+// at(dx, dy, dz) the node's neighbours.
+template <typename T, typename At>
+__device__ __forceinline__ T face_change(At at, const T* cm, T c0, T ce, T cc) {
+  T yf = 0, se = 0, sc = 0;
+#pragma unroll
+  for (int o = 0; o < 27; ++o) {
+    const int dx = o % 3 - 1, dy = (o / 3) % 3 - 1, dz = o / 9 - 1;
+    const int nzc = (dx != 0) + (dy != 0) + (dz != 0);
+    const T v = at(dx, dy, dz);
+    yf += cm[o] * v;
+    if (nzc == 2) se += v;
+    else if (nzc == 3) sc += v;
+  }
+  const T yi = c0 * at(0, 0, 0) + ce * se + cc * sc;
+  return yi - yf;
+}
+
+// restriction of the block's residual tile to its coarse node ci (Morton) from its own fine nodes
+template <typename T>
+__device__ __forceinline__ T restrict_own(const T* rt, uint32_t ci) {
+  uint32_t cx, cy, cz;
+  unmorton3(ci, cx, cy, cz);
+  T s = 0;
+#pragma unroll
+  for (int dz = -1; dz <= 1; ++dz) {
+    const int fz = 2 * (int)cz + dz;
+    if (fz < 0) continue;
+#pragma unroll
+    for (int dy = -1; dy <= 1; ++dy) {
+      const int fy = 2 * (int)cy + dy;
+      if (fy < 0) continue;
+      const T wyz = (T)((dy == 0 ? 1.0 : 0.5) * (dz == 0 ? 1.0 : 0.5));
+      const T* row = rt + ridx(2 * cx, fy, fz);
+      const typename n16::Pair<T>::type pr = *reinterpret_cast<const typename n16::Pair<T>::type*>(row);
+      const T left = cx > 0 ? row[-1] : (T)0;
+      s += wyz * (pr.x + (T)0.5 * (pr.y + left));
+    }
+  }
+  return s;
+}
+
 template <typename T, bool FACES, int ZT>
 __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT / 4)
     k_resid16(uint32_t D, const T* __restrict__ e, const T* __restrict__ f, T* __restrict__ fc,
@@ -967,19 +1029,8 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
       const int mask = ((ox + (int)lx) == 0) | (((oy + (int)ly) == 0) << 1) | (((oz + (int)lz) == 0) << 2);
       if (!mask) continue;
       const int ei = n16::nat(lx + 1, ly + 1, lz + 1);
-      T yf = 0, se = 0, sc = 0;
-      const T* cm = table + 27 * mask;
-#pragma unroll
-      for (int o = 0; o < 27; ++o) {
-        const int dx = o % 3 - 1, dy = (o / 3) % 3 - 1, dz = o / 9 - 1;
-        const int nzc = (dx != 0) + (dy != 0) + (dz != 0);
-        const T v = et[ei + dx + n16::RS * dy + n16::PS * dz];
-        yf += cm[o] * v;
-        if (nzc == 2) se += v;
-        else if (nzc == 3) sc += v;
-      }
-      const T yi = c0 * et[ei] + ce * se + cc * sc;
-      rt[ridx(lx, ly, lz)] += yi - yf;
+      rt[ridx(lx, ly, lz)] += face_change<T>([&](int dx, int dy, int dz) { return et[ei + dx + n16::RS * dy + n16::PS * dz]; },
+                                             table + 27 * mask, c0, ce, cc);
     }
     __syncthreads();
   }
@@ -987,25 +1038,7 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
   const uint64_t cbase = (uint64_t)blk * 512;
 #pragma unroll
   for (int ci = t; ci < 512; ci += NT) {
-    uint32_t cx, cy, cz;
-    unmorton3((uint32_t)ci, cx, cy, cz);
-    T s = 0;
-#pragma unroll
-    for (int dz = -1; dz <= 1; ++dz) {
-      const int fz = 2 * (int)cz + dz;
-      if (fz < 0) continue;
-#pragma unroll
-      for (int dy = -1; dy <= 1; ++dy) {
-        const int fy = 2 * (int)cy + dy;
-        if (fy < 0) continue;
-        const T wyz = (T)((dy == 0 ? 1.0 : 0.5) * (dz == 0 ? 1.0 : 0.5));
-        const T* row = rt + ridx(2 * cx, fy, fz);
-        const typename n16::Pair<T>::type pr = *reinterpret_cast<const typename n16::Pair<T>::type*>(row);
-        const T left = cx > 0 ? row[-1] : (T)0;
-        s += wyz * (pr.x + (T)0.5 * (pr.y + left));
-      }
-    }
-    fc[cbase + ci] = s;
+    fc[cbase + ci] = restrict_own<T>(rt, (uint32_t)ci);
   }
   // restriction partials of the high faces, edges and corner
   {
@@ -1182,6 +1215,80 @@ __device__ __forceinline__ void relax_column(const T* tile, int x0, int y0, int 
   }
 }
 
+// One sweep of the tile: the four phases, each ended by a barrier.  faces: the block holds nodes on a
+// low domain face (uniform in the block), whose rows are in ftab.
+template <typename T, bool FWD, bool FROM_ZERO, bool FACES, int ZT>
+__device__ __forceinline__ void sweep(T* tile, const T* ftab, bool faces, int ox, int oy, int oz, int x0, int y0,
+                                      int z0, const T (&fv)[ZT][4], T (&v)[ZT][4], T ce, T cc, T c0inv) {
+#pragma unroll
+  for (int ph = 0; ph < 4; ++ph) {
+    const int cls = FWD ? ph : 3 - ph;
+    const int cx = cls & 1, cy = cls >> 1;
+    const int x = x0 + cx, y = y0 + cy;
+    T nv[ZT];
+    constexpr bool ZERO = FROM_ZERO && FWD;
+    switch (cls) {
+      case 0: relax_column<T, 0, ZERO, ZT>(tile, x0, y0, z0, fv, v, ce, cc, c0inv, nv); break;
+      case 1: relax_column<T, 1, ZERO, ZT>(tile, x0, y0, z0, fv, v, ce, cc, c0inv, nv); break;
+      case 2: relax_column<T, 2, ZERO, ZT>(tile, x0, y0, z0, fv, v, ce, cc, c0inv, nv); break;
+      default: relax_column<T, 3, ZERO, ZT>(tile, x0, y0, z0, fv, v, ce, cc, c0inv, nv); break;
+    }
+    if (faces) {  // low-domain-face nodes of this column: their table rows, neighbours from the tile
+      const int cl = col(x), cm1 = col(x + 1), cr = col(x + 2);  // tile columns x-1, x, x+1
+#pragma unroll 1
+      for (int k = 0; k < ZT; ++k) {
+        const int z = z0 + k;
+        const int mask = ((ox + x) == 0) | (((oy + y) == 0) << 1) | (((oz + z) == 0) << 2);
+        if (!mask) continue;
+        const T* cm = ftab + 27 * mask;
+        const T* tb = tile + z * PS + y * RS;  // tile row y-1 of tile plane z-1
+        T off = 0;
+#pragma unroll
+        for (int o = 0; o < 27; ++o) {
+          if (o == 13) continue;
+          off += cm[o] * tb[(o / 9) * PS + ((o / 3) % 3) * RS + (o % 3 == 0 ? cl : (o % 3 == 1 ? cm1 : cr))];
+        }
+        T fk = fv[0][cls];
+#pragma unroll
+        for (int kk = 1; kk < ZT; ++kk)
+          if (kk == k) fk = fv[kk][cls];
+        const T nvk = (fk - off) / cm[13];
+#pragma unroll
+        for (int kk = 0; kk < ZT; ++kk)
+          if (kk == k) nv[kk] = nvk;
+      }
+      __syncthreads();  // same-class column neighbours were read with their old values
+    }
+#pragma unroll
+    for (int k = 0; k < ZT; ++k) {
+      v[k][cls] = nv[k];
+      tile[nat(x + 1, y + 1, z0 + k + 1)] = nv[k];
+    }
+    __syncthreads();
+  }
+}
+
+// v += P ec on the quad column: coarse (cx, cx+1) x (cy, cy+1) at the coarse planes z0/2 .. z0/2+ZT/2
+// (z0 even: planes z0, z0+2 lie on a coarse plane, z0+1, z0+3 halfway between two)
+template <typename T, int ZT>
+__device__ __forceinline__ void prolong_quads(const T* ctile, int x0, int y0, int z0, T (&v)[ZT][4]) {
+  const int ax = x0 / 2 + 1, ay = y0 / 2 + 1, az = z0 / 2 + 1;
+  T pl[ZT / 2 + 1][4];
+#pragma unroll
+  for (int w = 0; w <= ZT / 2; ++w) {
+    const T* c = ctile + ((az + w) * CW + ay) * CW + ax;
+    const T c00 = c[0], c10 = c[1], c01 = c[CW], c11 = c[CW + 1];
+    pl[w][0] = c00;
+    pl[w][1] = (T)0.5 * (c00 + c10);
+    pl[w][2] = (T)0.5 * (c00 + c01);
+    pl[w][3] = (T)0.25 * ((c00 + c10) + (c01 + c11));
+  }
+#pragma unroll
+  for (int k = 0; k < ZT; ++k)  // even planes on a coarse plane, odd halfway between two
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[k][e] += (k & 1) ? (T)0.5 * (pl[k / 2][e] + pl[k / 2 + 1][e]) : pl[k / 2][e];
+}
+
 // MODE 0: xo = sweep(xi); 1: xo = sweep(0); 2: xo = sweep(xi + P ec).  DOT: part = f.xo
 // MODE 3 (finest level, forward): first the CG update x += alpha d, r -= alpha q in place
 // (pointwise), then xo = sweep(0) with f = the new r; part = per-block sums of r^2.  A sweep
@@ -1260,25 +1367,7 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
       v[k][0] = xq.x; v[k][1] = xq.y; v[k][2] = xq.z; v[k][3] = xq.w;
     }
   }
-  if (MODE == 2) {
-    // P ec on the quad column: coarse (cx, cx+1) x (cy, cy+1) at the coarse planes z0/2 .. z0/2+2
-    // (z0 even: planes z0, z0+2 lie on a coarse plane, z0+1, z0+3 halfway between two)
-    const int ax = x0 / 2 + 1, ay = y0 / 2 + 1, az = z0 / 2 + 1;
-    T pl[ZT / 2 + 1][4];
-#pragma unroll
-    for (int w = 0; w <= ZT / 2; ++w) {
-      const T* c = ctile + ((az + w) * CW + ay) * CW + ax;
-      const T c00 = c[0], c10 = c[1], c01 = c[CW], c11 = c[CW + 1];
-      pl[w][0] = c00;
-      pl[w][1] = (T)0.5 * (c00 + c10);
-      pl[w][2] = (T)0.5 * (c00 + c01);
-      pl[w][3] = (T)0.25 * ((c00 + c10) + (c01 + c11));
-    }
-#pragma unroll
-    for (int k = 0; k < ZT; ++k)  // even planes on a coarse plane, odd halfway between two
-#pragma unroll
-      for (int e = 0; e < 4; ++e) v[k][e] += (k & 1) ? (T)0.5 * (pl[k / 2][e] + pl[k / 2 + 1][e]) : pl[k / 2][e];
-  }
+  if (MODE == 2) prolong_quads<T, ZT>(ctile, x0, y0, z0, v);
 #pragma unroll
   for (int k = 0; k < ZT; ++k) {
     T* p0 = tile + nat(0, y0 + 1, z0 + k + 1);
@@ -1300,52 +1389,7 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
     }
     __syncthreads();
   }
-#pragma unroll
-  for (int ph = 0; ph < 4; ++ph) {
-    const int cls = FWD ? ph : 3 - ph;
-    const int cx = cls & 1, cy = cls >> 1;
-    const int x = x0 + cx, y = y0 + cy;
-    T nv[ZT];
-    constexpr bool ZERO = FROM_ZERO && FWD;
-    switch (cls) {
-      case 0: relax_column<T, 0, ZERO, ZT>(tile, x0, y0, z0, fv, v, ce, cc, c0inv, nv); break;
-      case 1: relax_column<T, 1, ZERO, ZT>(tile, x0, y0, z0, fv, v, ce, cc, c0inv, nv); break;
-      case 2: relax_column<T, 2, ZERO, ZT>(tile, x0, y0, z0, fv, v, ce, cc, c0inv, nv); break;
-      default: relax_column<T, 3, ZERO, ZT>(tile, x0, y0, z0, fv, v, ce, cc, c0inv, nv); break;
-    }
-    if (faces) {  // low-domain-face nodes of this column: their table rows, neighbours from the tile
-      const int cl = col(x), cm1 = col(x + 1), cr = col(x + 2);  // tile columns x-1, x, x+1
-#pragma unroll 1
-      for (int k = 0; k < ZT; ++k) {
-        const int z = z0 + k;
-        const int mask = ((ox + x) == 0) | (((oy + y) == 0) << 1) | (((oz + z) == 0) << 2);
-        if (!mask) continue;
-        const T* cm = ftab + 27 * mask;
-        const T* tb = tile + z * PS + y * RS;  // tile row y-1 of tile plane z-1
-        T off = 0;
-#pragma unroll
-        for (int o = 0; o < 27; ++o) {
-          if (o == 13) continue;
-          off += cm[o] * tb[(o / 9) * PS + ((o / 3) % 3) * RS + (o % 3 == 0 ? cl : (o % 3 == 1 ? cm1 : cr))];
-        }
-        T fk = fv[0][cls];
-#pragma unroll
-        for (int kk = 1; kk < ZT; ++kk)
-          if (kk == k) fk = fv[kk][cls];
-        const T nvk = (fk - off) / cm[13];
-#pragma unroll
-        for (int kk = 0; kk < ZT; ++kk)
-          if (kk == k) nv[kk] = nvk;
-      }
-      __syncthreads();  // same-class column neighbours were read with their old values
-    }
-#pragma unroll
-    for (int k = 0; k < ZT; ++k) {
-      v[k][cls] = nv[k];
-      tile[nat(x + 1, y + 1, z0 + k + 1)] = nv[k];
-    }
-    __syncthreads();
-  }
+  sweep<T, FWD, FROM_ZERO, FACES, ZT>(tile, ftab, faces, ox, oy, oz, x0, y0, z0, fv, v, ce, cc, c0inv);
   double acc[ZT];  // DOT: per plane, the quad's f.x
 #pragma unroll
   for (int k = 0; k < ZT; ++k) {
@@ -1372,6 +1416,208 @@ constexpr size_t smem_bytes(int mode) {
   return sizeof(T) * (TILE + (mode == 2 ? CW * CW * CW : 0));
 }
 }  // namespace g16
+
+// ------------------------------------------------------------------ the coarsest levels in one block
+// V-cycle of the levels 16^3, 8^3 and 4^3 (each a single block of its kernel) in one CTA per cloud:
+// eight launches of one or a few warps' work each, whose time was launch and memory latency.  The
+// level vectors, the face rows and the dense inverse stay in shared memory between the steps; every
+// step is the arithmetic of its own kernel (k_smooth16, k_resid16, k_smooth, k_resid_restrict,
+// k_dense_solve), so the result is the same, bit for bit.  512 threads: thread = one 2x2 quad column
+// over 2 planes of the 16^3 level, or one node of the 8^3 level; the 64 nodes of an 8^3 colour and of
+// the 4^3 level are two warps' work.
+namespace t4 {
+constexpr int NT = 512, ZT = 2;
+constexpr int kInvStride = 65;  // the dense inverse's rows on disjoint banks
+constexpr int WE = 11, WR = 9;  // the 8^3 level's natural tiles: e over local [-2, 8], r over [-1, 7]
+constexpr int CW3 = 6;          // the 4^3 level with a zero border
+template <typename T>
+struct Coefs {  // of the 16^3 and the 8^3 level
+  T c0inv4, c04, ce4, cc4, c03, ce3, cc3;
+  const T *table4, *table3;  // face rows, 216 each
+  const T* inv;              // 64 x 64
+};
+constexpr int kWords = g16::TILE + r16::RTILE + 1000 + 1000 + 512 + WE * WE * WE + WR * WR * WR + 64 +
+                       CW3 * CW3 * CW3 + 64 * kInvStride + 432;
+
+// the 8 colours of an 8^3 sweep by threads 0..63 (two warps, their own barrier)
+template <typename T, bool FWD>
+__device__ __forceinline__ void sweep8(T* tile, const T* fs, const T* ftab, T c0, T ce, T cc, int t) {
+  using G = Geo<8>;
+  constexpr int H = G::H, H3 = G::H3, C = G::C, C3 = G::C3, LOGC = G::LOGC;
+  const int li = t & (C - 1), lj = (t >> LOGC) & (C - 1), lk = t >> (2 * LOGC);
+#pragma unroll
+  for (int step = 0; step < 8; ++step) {
+    const int col = FWD ? step : 7 - step;
+    const int cx = col & 1, cy = (col >> 1) & 1, cz = col >> 2;
+    const int own = (1 - cx) | ((1 - cy) << 1) | ((1 - cz) << 2);
+    const int pos = ((lk + cz) * H + (lj + cy)) * H + (li + cx);
+    const int mask = ((cx == 0 && li == 0) ? 1 : 0) | ((cy == 0 && lj == 0) ? 2 : 0) | ((cz == 0 && lk == 0) ? 4 : 0);
+    const T nv = relax_colour<T, 8>(tile, own, cx, cy, cz, pos, mask, fs[col * C3 + t], c0, ce, cc, ftab);
+    tile[own * H3 + pos] = nv;
+    asm volatile("bar.sync 1, 64;" ::: "memory");
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(NT, 1) k_coarse_tail(const T* __restrict__ f, T* __restrict__ e, Coefs<T> k) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* tile = reinterpret_cast<T*>(smem_raw);  // 16^3 level: parity-split tile
+  T* rt = tile + g16::TILE;                  // its residual
+  T* ctile = rt + r16::RTILE;                // the 8^3 level with a one-node border, natural
+  T* tile3 = ctile + 1000;                   // 8^3 level: parity-split tile
+  T* fs3 = tile3 + 1000;                     // its right-hand side, colour-major
+  T* et3 = fs3 + 512;                        // natural tiles of its residual
+  T* rt3 = et3 + WE * WE * WE;
+  T* f2 = rt3 + WR * WR * WR;                // 4^3 level: right-hand side
+  T* ctile3 = f2 + 64;                       // and solution with a zero border
+  T* inv = ctile3 + CW3 * CW3 * CW3;
+  T* tab4 = inv + 64 * kInvStride;
+  T* tab3 = tab4 + 216;
+  f = cloud_slice(f, 4096);
+  e = cloud_slice(e, 4096);
+  const int t = threadIdx.x;
+  const int qi = t & 63, zs = t >> 6;
+  const int x0 = 2 * (qi & 7), y0 = 2 * (qi >> 3), z0 = ZT * zs;
+  const uint32_t mq = s16::sp4(x0) | (s16::sp4(y0) << 1);
+  T fv[ZT][4], v[ZT][4];
+#pragma unroll
+  for (int p = 0; p < ZT; ++p) {
+    const typename s16::Vec4<T>::type q = s16::ld4(f + (mq | (s16::sp4(z0 + p) << 2)));
+    fv[p][0] = q.x; fv[p][1] = q.y; fv[p][2] = q.z; fv[p][3] = q.w;
+    v[p][0] = v[p][1] = v[p][2] = v[p][3] = (T)0;
+  }
+  for (int i = t; i < 64 * 64; i += NT) inv[(i >> 6) * kInvStride + (i & 63)] = k.inv[i];
+  for (int i = t; i < 216; i += NT) {
+    tab4[i] = k.table4[i];
+    tab3[i] = k.table3[i];
+  }
+  // everything outside the domain is zero, and the sweeps start from zero
+  for (int i = t; i < g16::TILE; i += NT) tile[i] = 0;
+  for (int i = t; i < 1000; i += NT) ctile[i] = tile3[i] = 0;
+  for (int i = t; i < WE * WE * WE; i += NT) et3[i] = 0;
+  for (int i = t; i < WR * WR * WR; i += NT) rt3[i] = 0;
+  for (int i = t; i < CW3 * CW3 * CW3; i += NT) ctile3[i] = 0;
+  __syncthreads();
+
+  // 16^3: pre-smoothing from zero
+  g16::sweep<T, true, true, true, ZT>(tile, tab4, true, 0, 0, 0, x0, y0, z0, fv, v, k.ce4, k.cc4, k.c0inv4);
+  {  // r = f - A a on quad columns
+    T cur[4] = {0, 0, 0, 0}, nxt[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int p = 0; p < ZT + 2; ++p) {  // local plane z0 + p - 1
+      T r[4][4], tz[4], own[4], ctr[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const T* row = tile + (z0 + p) * g16::PS + (y0 + j) * g16::RS + (x0 >> 1);
+        r[j][0] = row[0];
+        r[j][1] = row[g16::HS];
+        r[j][2] = row[1];
+        r[j][3] = row[g16::HS + 1];
+      }
+      n16::plane_terms<T>(r, k.c04, k.ce4, k.cc4, tz, own, ctr);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        cur[i] += tz[i];
+        nxt[i] += own[i];
+      }
+      if (p >= 2) {
+        T* q0 = rt + r16::ridx(x0, y0, z0 + p - 2);
+        q0[0] = fv[p - 2][0] - cur[0];
+        q0[1] = fv[p - 2][1] - cur[1];
+        q0[r16::RSR] = fv[p - 2][2] - cur[2];
+        q0[r16::RSR + 1] = fv[p - 2][3] - cur[3];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        cur[i] = nxt[i];
+        nxt[i] = tz[i];
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = t; i < 721; i += NT) {  // the low-face nodes: x = 0, then y = 0 < x, then z = 0 < x, y
+    int lx, ly, lz;
+    if (i < 256) { lx = 0; ly = i & 15; lz = i >> 4; }
+    else if (i < 496) { lx = 1 + (i - 256) % 15; ly = 0; lz = (i - 256) / 15; }
+    else { lx = 1 + (i - 496) % 15; ly = 1 + (i - 496) / 15; lz = 0; }
+    const int mask = (lx == 0) | ((ly == 0) << 1) | ((lz == 0) << 2);
+    rt[r16::ridx(lx, ly, lz)] += r16::face_change<T>(
+        [&](int dx, int dy, int dz) { return tile[g16::nat(lx + 1 + dx, ly + 1 + dy, lz + 1 + dz)]; },
+        tab4 + 27 * mask, k.c04, k.ce4, k.cc4);
+  }
+  __syncthreads();
+  uint32_t nx, ny, nz;  // this thread's 8^3 node (Morton t)
+  unmorton3((uint32_t)t, nx, ny, nz);
+  const int ux = (int)nx + 1, uy = (int)ny + 1, uz = (int)nz + 1;
+  {
+    const T s = r16::restrict_own<T>(rt, (uint32_t)t);
+    const int col = (nx & 1) | ((ny & 1) << 1) | ((nz & 1) << 2);
+    fs3[col * 64 + ((nx >> 1) | ((ny >> 1) << 2) | ((nz >> 1) << 4))] = s;
+    rt3[(uz * WR + uy) * WR + ux] = s;  // f first, r = f - A a below
+  }
+  __syncthreads();
+
+  // 8^3: pre-smoothing from zero, residual, restriction
+  if (t < 64) sweep8<T, true>(tile3, fs3, tab3, k.c03, k.ce3, k.cc3, t);
+  __syncthreads();
+  const int self3 = ps_index<8>(ux, uy, uz);
+  const T a3 = tile3[self3];
+  et3[((uz + 1) * WE + (uy + 1)) * WE + (ux + 1)] = a3;
+  __syncthreads();
+  {
+    const int ei = ((uz + 1) * WE + (uy + 1)) * WE + (ux + 1), ri = (uz * WR + uy) * WR + ux;
+    column_apply<T, WE, 1>(et3, ux + 1, uy + 1, uz + 1, k.c03, k.ce3, k.cc3, [&](int, T, T y) { rt3[ri] -= y; });
+    const int mask = (nx == 0) | ((ny == 0) << 1) | ((nz == 0) << 2);
+    if (mask) {
+      const T yi = row_interior<T, WE>(et3, ei, k.c03, k.ce3, k.cc3);
+      const T yf = row_general<T, WE>(et3, ei, tab3 + 27 * mask);
+      rt3[ri] += yi - yf;
+    }
+  }
+  __syncthreads();
+  if (t < 64) {
+    uint32_t cx, cy, cz;
+    unmorton3((uint32_t)t, cx, cy, cz);
+    f2[t] = restrict_full<T, WR>(rt3, (int)cx, (int)cy, (int)cz);
+    asm volatile("bar.sync 1, 64;" ::: "memory");
+    // 4^3: the dense inverse
+    double s = 0.0;
+#pragma unroll 16
+    for (int j = 0; j < 64; ++j) s += (double)inv[t * kInvStride + j] * (double)f2[j];
+    ctile3[((cz + 1) * CW3 + (cy + 1)) * CW3 + (cx + 1)] = (T)s;
+  }
+  __syncthreads();
+
+  // 8^3: post-smoothing on a + P e
+  T v3 = a3;
+  v3 += prolong_node<T, CW3>(ctile3, (int)nx, (int)ny, (int)nz, -1, -1, -1);
+  tile3[self3] = v3;
+  __syncthreads();
+  if (t < 64) sweep8<T, false>(tile3, fs3, tab3, k.c03, k.ce3, k.cc3, t);
+  __syncthreads();
+  ctile[(uz * s16::CW + uy) * s16::CW + ux] = tile3[self3];
+  __syncthreads();
+
+  // 16^3: post-smoothing on a + P e
+  g16::prolong_quads<T, ZT>(ctile, x0, y0, z0, v);
+#pragma unroll
+  for (int p = 0; p < ZT; ++p) {
+    T* p0 = tile + g16::nat(0, y0 + 1, z0 + p + 1);
+    p0[g16::col(x0 + 1)] = v[p][0];
+    p0[g16::col(x0 + 2)] = v[p][1];
+    p0[g16::RS + g16::col(x0 + 1)] = v[p][2];
+    p0[g16::RS + g16::col(x0 + 2)] = v[p][3];
+  }
+  __syncthreads();
+  g16::sweep<T, false, false, true, ZT>(tile, tab4, true, 0, 0, 0, x0, y0, z0, fv, v, k.ce4, k.cc4, k.c0inv4);
+#pragma unroll
+  for (int p = 0; p < ZT; ++p) {
+    typename s16::Vec4<T>::type o;
+    o.x = v[p][0]; o.y = v[p][1]; o.z = v[p][2]; o.w = v[p][3];
+    s16::st4(e + (mq | (s16::sp4(z0 + p) << 2)), o);
+  }
+}
+}  // namespace t4
 
 template <typename T>
 DevCoef<T> dev_coef(const LevelCoef& L, const T* table) {
@@ -1696,6 +1942,28 @@ void mg_resid_restrict(cudaStream_t s, const LevelCoef& L, const T* table, const
   PR_CHECK_LAUNCH();
 }
 
+template <typename T>
+void mg_coarse_tail(cudaStream_t s, const LevelCoef& L4, const LevelCoef& L3, const T* table4, const T* table3,
+                    const T* inv, const T* f, T* e, uint32_t clouds) {
+  if (L4.depth != 4 || L3.depth != 3 || !L4.has_faces || !L3.has_faces)
+    throw Error(PR_ERR_INTERNAL, "the coarse tail starts at a coarse 16^3 level");
+  t4::Coefs<T> k;
+  k.c0inv4 = (T)(1.0 / L4.c0);
+  k.c04 = (T)L4.c0;
+  k.ce4 = (T)L4.ce;
+  k.cc4 = (T)L4.cc;
+  k.c03 = (T)L3.c0;
+  k.ce3 = (T)L3.ce;
+  k.cc3 = (T)L3.cc;
+  k.table4 = table4;
+  k.table3 = table3;
+  k.inv = inv;
+  const size_t sm = t4::kWords * sizeof(T);
+  allow_smem(t4::k_coarse_tail<T>, sm);
+  t4::k_coarse_tail<T><<<dim3(1, clouds), t4::NT, sm, s>>>(f, e, k);
+  PR_CHECK_LAUNCH();
+}
+
 size_t mg_face_entries(uint32_t D) { return D >= 4 ? (size_t)r16::FACE << (3 * (D - 4)) : 0; }
 
 template <typename T>
@@ -1866,6 +2134,8 @@ double kernel_bench(pr_context* c, int kid, uint32_t D, int precision, int reps,
 #define PR_INST(T)                                                                                                 \
   template void mg_smooth<T>(cudaStream_t, const LevelCoef&, const T*, const T*, T*, const T*, const T*, int, bool, \
                              double*, uint32_t);                                                                  \
+  template void mg_coarse_tail<T>(cudaStream_t, const LevelCoef&, const LevelCoef&, const T*, const T*, const T*,   \
+                                  const T*, T*, uint32_t);                                                        \
   template void mg_resid_restrict<T>(cudaStream_t, const LevelCoef&, const T*, const T*, const T*, T*, T*,        \
                                      uint32_t);                                                                   \
   template void mg_cg_update_presmooth<T>(cudaStream_t, const LevelCoef&, const T*, const CgFuse<T>&, T*, double*, \

@@ -49,6 +49,11 @@ template <typename T>
 void mg_resid_restrict(cudaStream_t s, const LevelCoef& L, const T* table, const T* e, const T* f, T* fc, T* face,
                        uint32_t clouds = 1);
 size_t mg_face_entries(uint32_t depth);
+// e = V(f) from the coarse 16^3 level down (one sweep before and after on the 16^3 and 8^3 levels, the
+// dense inverse of the 4^3 one): one launch.  table4, table3: the levels' face rows.
+template <typename T>
+void mg_coarse_tail(cudaStream_t s, const LevelCoef& L4, const LevelCoef& L3, const T* table4, const T* table3,
+                    const T* inv, const T* f, T* e, uint32_t clouds = 1);
 // finest level only.  xpby: dn = z + beta d, q = A dn; else q = A d.  Stencil part only;
 // per-block (dn or d).q into part.  beta_dev (packed, nullable): per-cloud beta.
 template <typename T>

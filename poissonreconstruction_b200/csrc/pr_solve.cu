@@ -186,6 +186,11 @@ struct Multigrid {
       dense_solve<T>(s, nc, inv, fl, el, clouds);
       return;
     }
+    // the coarse levels that fit one block; with more sweeps, and on grids up to 16^3, level by level
+    if (l == 4 && l < D && sweeps == 1) {
+      mg_coarse_tail<T>(s, L[4], L[3], table(4), table(3), inv, fl, el, clouds);
+      return;
+    }
     // pre-smoothing (forward) from zero; result in a_l
     T* cur = a[l];
     if (!presmoothed) mg_smooth<T>(s, L[l], table(l), nullptr, cur, fl, nullptr, 1, true, nullptr, clouds);

@@ -1,0 +1,25 @@
+"""Kernels that serve part of the size range, at the sizes where one hands over to another."""
+import numpy as np
+import pytest
+
+import oracle
+import poissonreconstruction_b200 as prb
+from poissonreconstruction_b200 import synthetic
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("precision", [prb.PR_PRECISION_FP64, prb.PR_PRECISION_MIXED])
+@pytest.mark.parametrize("depth,sweeps", [(4, 1), (5, 1), (5, 2), (6, 1)])
+def test_coarse_levels_of_the_degree1_vcycle(ctx, depth, sweeps, precision):
+    """Depth 4 and two sweeps run the coarse levels one by one, the others in one launch: the solution
+    meets the oracle's, and the preconditioner keeps its convergence (a factor of about ten per
+    iteration, so at most 15 iterations to 1e-10)."""
+    pts = synthetic.torus(3000, seed=40 + depth)
+    st = ctx.solve(pts, prb.ReconstructParams(depth=depth, point_weight=4.0, precision=precision,
+                                              smooth_sweeps=sweeps, target_rel_residual=1e-10))
+    assert st.converged == 1 and st.pcg_iterations <= 15, st
+    unit, _ = oracle.to_unit(pts)
+    x_ref, _, _ = oracle.Tree(depth, unit).solve_converged(4.0, tol=1e-13, maxit=200000)
+    x = ctx.coefficients()
+    assert np.linalg.norm(x - x_ref) <= 1e-6 * np.linalg.norm(x_ref)
