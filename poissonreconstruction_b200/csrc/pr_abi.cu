@@ -823,6 +823,7 @@ int pr_context_create(int device, void* stream, pr_context** out_ctx) {
       c->own_stream = true;
     }
     PR_CUDA(cudaMallocHost(&c->h_scalars, 64 * sizeof(double)));
+    PR_CUDA(cudaMallocHost(&c->h_flag, sizeof(int)));
     {
       std::lock_guard<std::mutex> g(pr::spare_mutex());
       pr::context_registry().insert(c.get());
@@ -857,6 +858,8 @@ int pr_context_destroy(pr_context* c) {
     }
     if (c->h_scalars) cudaFreeHost(c->h_scalars);
     if (c->h_pack) cudaFreeHost(c->h_pack);
+    if (c->h_ring) cudaFreeHost(c->h_ring);
+    if (c->h_flag) cudaFreeHost(c->h_flag);
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;

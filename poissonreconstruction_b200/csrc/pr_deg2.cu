@@ -1914,8 +1914,7 @@ struct System2 {
       auto upload = [&](const Band& b, const std::string& nm) {
         std::vector<T> tb(b.begin(), b.end());
         T* p = c->buf<T>("d2_" + nm + sfx, tb.size());
-        PR_CUDA(cudaMemcpyAsync(p, tb.data(), tb.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
-        c->sync();
+        c->upload(p, tb.data(), tb.size() * sizeof(T));
         return p;
       };
       q.tM = upload(M, "tM");
@@ -1957,7 +1956,7 @@ struct System2 {
     }
   }
 
-  // dense inverse of the coarsest operator (Cholesky on the host, FP64)
+  // dense inverse of the coarsest operator
   void build_dense(const Band& M, const Band& S, int r, double wg, double H) {
     nc = r * r * r;
     std::vector<double> A((size_t)nc * nc, 0.0);
@@ -1970,36 +1969,8 @@ struct System2 {
         if (i == j) v += wg;
         A[(size_t)i * nc + j] = v;
       }
-    std::vector<double> Lc((size_t)nc * nc, 0.0);
-    for (int i = 0; i < nc; ++i)
-      for (int j = 0; j <= i; ++j) {
-        double s = A[(size_t)i * nc + j];
-        for (int k = 0; k < j; ++k) s -= Lc[(size_t)i * nc + k] * Lc[(size_t)j * nc + k];
-        if (i == j) {
-          PR_REQUIRE(s > 0.0, PR_ERR_INTERNAL, "degree-2 coarsest operator is not positive definite");
-          Lc[(size_t)i * nc + i] = std::sqrt(s);
-        } else {
-          Lc[(size_t)i * nc + j] = s / Lc[(size_t)j * nc + j];
-        }
-      }
-    std::vector<T> invt((size_t)nc * nc);
-    std::vector<double> y(nc), col(nc);
-    for (int cc = 0; cc < nc; ++cc) {
-      for (int i = 0; i < nc; ++i) {
-        double s = (i == cc) ? 1.0 : 0.0;
-        for (int k = 0; k < i; ++k) s -= Lc[(size_t)i * nc + k] * y[k];
-        y[i] = s / Lc[(size_t)i * nc + i];
-      }
-      for (int i = nc - 1; i >= 0; --i) {
-        double s = y[i];
-        for (int k = i + 1; k < nc; ++k) s -= Lc[(size_t)k * nc + i] * col[k];
-        col[i] = s / Lc[(size_t)i * nc + i];
-      }
-      for (int i = 0; i < nc; ++i) invt[(size_t)i * nc + cc] = (T)col[i];
-    }
-    inv = c->buf<T>(std::string("d2_inv_") + tn2<T>(), invt.size());
-    PR_CUDA(cudaMemcpyAsync(inv, invt.data(), invt.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
-    c->sync();
+    inv = c->buf<T>(std::string("d2_inv_") + tn2<T>(), (size_t)nc * nc);
+    spd_inverse<T>(c, nc, A.data(), inv);
   }
 
   void set_screen(const T* phi) {
@@ -2289,6 +2260,7 @@ int pcg2(pr_context* c, System2<T>& sys, T* r, T* x, double tol_abs, int maxit, 
   if (!fused) {
     sys.vcycle(0, r, z);
     double rz = dot<T>(c, r, z, n);
+    spd_check(c, "degree-2 coarsest operator");
     PR_CUDA(cudaMemcpyAsync(d, z, n * sizeof(T), cudaMemcpyDeviceToDevice, s));
     sys.bytes += 4.0 * n * sizeof(T);
     while (it < maxit) {
@@ -2326,6 +2298,7 @@ int pcg2(pr_context* c, System2<T>& sys, T* r, T* x, double tol_abs, int maxit, 
     return sys.sum_parts(sys.rz_np, 0, 0.0);
   };
   double rz = precondition();
+  spd_check(c, "degree-2 coarsest operator");
   double alpha = 0.0, alpha_prev = 0.0, beta = 0.0;
   bool pending = false;  // x += alpha dcur not applied yet
   bool x_def = false;    // x written (until then it is zero and never read)

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <chrono>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <set>
@@ -152,6 +153,31 @@ struct pr_context {
     }
     return h_pack;
   }
+  // Pinned ring for small host -> device tables: the bytes are copied into it and from there to the
+  // device on `stream`, so the caller's buffer is free at once and the host does not wait.  When the
+  // ring is full the stream is waited for, after which none of it is in flight.
+  unsigned char* h_ring = nullptr;
+  size_t h_ring_cap = 0, h_ring_used = 0;
+  void upload(void* dst, const void* src, size_t bytes) {
+    if (bytes == 0) return;
+    const size_t need = (bytes + 255) & ~size_t(255);
+    if (h_ring_used + need > h_ring_cap) {
+      PR_CUDA(cudaStreamSynchronize(stream));
+      h_ring_used = 0;
+      if (need > h_ring_cap) {
+        if (h_ring) PR_CUDA(cudaFreeHost(h_ring));
+        h_ring = nullptr;
+        h_ring_cap = 0;
+        const size_t cap = need > (size_t(1) << 20) ? need : (size_t(1) << 20);
+        PR_CUDA(cudaMallocHost(&h_ring, cap));
+        h_ring_cap = cap;
+      }
+    }
+    std::memcpy(h_ring + h_ring_used, src, bytes);
+    PR_CUDA(cudaMemcpyAsync(dst, h_ring + h_ring_used, bytes, cudaMemcpyHostToDevice, stream));
+    h_ring_used += need;
+  }
+  int* h_flag = nullptr;  // pinned: the status of the last spd_inverse (pr_operator.cu)
   // pinned staging for device->host mesh copies (grown on demand)
   unsigned char* h_stage = nullptr;
   size_t h_stage_cap = 0;

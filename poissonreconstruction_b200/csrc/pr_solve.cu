@@ -29,8 +29,8 @@ namespace {
 
 constexpr uint32_t kCoarseDepth = 2;
 
-// Dense inverse of a level's Galerkin operator (depth Dc <= 2, Morton order), FP64 Cholesky.
-std::vector<double> dense_inverse(const LevelCoef& L) {
+// A level's Galerkin operator as a dense matrix (depth Dc <= 2, Morton order), FP64.
+std::vector<double> dense_operator(const LevelCoef& L) {
   const uint32_t Dc = L.depth;
   const int res = 1 << Dc;
   const int n = res * res * res;
@@ -46,32 +46,7 @@ std::vector<double> dense_inverse(const LevelCoef& L) {
       A[(size_t)i * n + morton3(jx, jy, jz)] = L.table[mask][o];
     }
   }
-  for (int j = 0; j < n; ++j) {
-    double d = A[(size_t)j * n + j];
-    for (int k = 0; k < j; ++k) d -= A[(size_t)j * n + k] * A[(size_t)j * n + k];
-    if (!(d > 0.0)) throw Error(PR_ERR_INTERNAL, "coarse operator is not positive definite");
-    d = std::sqrt(d);
-    A[(size_t)j * n + j] = d;
-    for (int i = j + 1; i < n; ++i) {
-      double s = A[(size_t)i * n + j];
-      for (int k = 0; k < j; ++k) s -= A[(size_t)i * n + k] * A[(size_t)j * n + k];
-      A[(size_t)i * n + j] = s / d;
-    }
-  }
-  std::vector<double> inv((size_t)n * n), y(n);
-  for (int col = 0; col < n; ++col) {
-    for (int i = 0; i < n; ++i) {
-      double s = (i == col) ? 1.0 : 0.0;
-      for (int k = 0; k < i; ++k) s -= A[(size_t)i * n + k] * y[k];
-      y[i] = s / A[(size_t)i * n + i];
-    }
-    for (int i = n - 1; i >= 0; --i) {
-      double s = y[i];
-      for (int k = i + 1; k < n; ++k) s -= A[(size_t)k * n + i] * inv[(size_t)k * n + col];
-      inv[(size_t)i * n + col] = s / A[(size_t)i * n + i];
-    }
-  }
-  return inv;
+  return A;
 }
 
 // ------------------------------------------------------------------ packed systems
@@ -169,12 +144,9 @@ struct Multigrid {
     }
     tables = c->buf<T>(std::string("mg_tab_") + tname<T>(), tab.size());
     nc = 1u << (3 * Dc);
-    std::vector<double> invd = dense_inverse(L[Dc]);
-    std::vector<T> invt(invd.begin(), invd.end());
-    inv = c->buf<T>(std::string("mg_inv_") + tname<T>(), invt.size());
-    PR_CUDA(cudaMemcpyAsync(tables, tab.data(), tab.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
-    PR_CUDA(cudaMemcpyAsync(inv, invt.data(), invt.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
-    c->sync();  // host temporaries
+    inv = c->buf<T>(std::string("mg_inv_") + tname<T>(), (size_t)nc * nc);
+    c->upload(tables, tab.data(), tab.size() * sizeof(T));
+    spd_inverse<T>(c, (int)nc, dense_operator(L[Dc]).data(), inv);
   }
   const T* table(uint32_t l) const { return tables + (size_t)l * 216; }
 
@@ -235,7 +207,9 @@ struct Multigrid {
       dense_solve<T>(c->stream, nc, inv, r, z, clouds);
       double* part = c->buf<double>("pk_dot_part", (size_t)kDotBlocks * clouds);
       dots_pk<T>(c->stream, r, z, n, clouds, part, pk->ds(Pack::kOut));
-      return pk->fetch();
+      const std::vector<double> rz = pk->fetch();
+      if (applies++ == 0) spd_check(c, "coarse operator");
+      return rz;
     }
     double* part = c->buf<double>("mg_part", (size_t)mg_blocks(D) * clouds);
     auto body = [&] {
@@ -243,9 +217,12 @@ struct Multigrid {
       sum_parts(c->stream, part, (int)mg_blocks(D), 0.0, part, 0, pk->ds(Pack::kOut), clouds);
     };
     const char* gr = std::getenv("PR_GRAPHS");
-    if (applies++ == 0 || (gr && std::atoi(gr) == 0)) body();
+    const bool first = applies++ == 0;
+    if (first || (gr && std::atoi(gr) == 0)) body();
     else c->run_graph(graph_key(r, z, part, presmoothed), body);
-    return pk->fetch();
+    const std::vector<double> rz = pk->fetch();
+    if (first) spd_check(c, "coarse operator");
+    return rz;
   }
   int applies = 0;
   // everything a captured V-cycle depends on: sizes, the shift (kernel arguments), every buffer
@@ -298,8 +275,7 @@ struct CgOperator {
     for (int m = 0; m < 8; ++m)
       for (int o = 0; o < 27; ++o) tab[27 * m + o] = (T)Lf.table[m][o];
     table = c->buf<T>(std::string("cg_tab_") + tname<T>(), 216);
-    PR_CUDA(cudaMemcpyAsync(table, tab.data(), 216 * sizeof(T), cudaMemcpyHostToDevice, c->stream));
-    c->sync();
+    c->upload(table, tab.data(), 216 * sizeof(T));
   }
   const FineOp<T>& small_op() const;
   // xpby: dn = z + beta d, q = A dn; else q = A d (dn unused).  Returns (dn or d).q per cloud
@@ -544,6 +520,10 @@ void solve_pack(Pack& pk, const pr_params& p, const double* b, double* xA, std::
         rn[k] = rn_new[k];
       }
     }
+    if (M.applies == 0) {  // nothing to solve: the setup's check alone
+      c->sync();
+      spd_check(c, "coarse operator");
+    }
   };
   if (mixed) round(float());
   else round(double());
@@ -605,8 +585,7 @@ void make_pack(Pack& pk, pr_context* sc, const std::vector<pr_context*>& cl) {
     pk.scr.maxS = std::max<uint64_t>(pk.scr.maxS, desc.back().S);
   }
   ScreenDesc* dd = sc->buf<ScreenDesc>("pk_screen", desc.size());
-  PR_CUDA(cudaMemcpyAsync(dd, desc.data(), desc.size() * sizeof(ScreenDesc), cudaMemcpyHostToDevice, sc->stream));
-  sc->sync();  // host descriptors
+  sc->upload(dd, desc.data(), desc.size() * sizeof(ScreenDesc));
   pk.scr.desc = dd;
   pk.scr.clouds = pk.clouds;
   pk.scr.sentinel = 1u << (3 * pk.D);
