@@ -238,6 +238,11 @@ struct pr_context {
   void run_graph(const std::string& key, F body) {
     auto it = graphs.find(key);
     if (it == graphs.end()) {
+      if (graphs.size() >= 64) {  // keyed by buffers that were replaced since, most likely
+        PR_CUDA(cudaStreamSynchronize(stream));
+        for (auto& kv : graphs) cudaGraphExecDestroy(kv.second.exec);
+        graphs.clear();
+      }
       cudaGraph_t g = nullptr;
       const uint64_t l0 = pr::thread_launch_count(0), p0 = pr::thread_launch_count(1);
       PR_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));

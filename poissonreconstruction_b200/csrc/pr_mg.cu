@@ -499,13 +499,11 @@ __global__ void __launch_bounds__(Geo<TB>::THREADS) k_resid_restrict(uint32_t D,
   }
 }
 
-// fixed-order sum of two partial arrays: out = sum(part) + scale2 * sum(part2)
-__global__ void __launch_bounds__(1024) k_sum_parts(const double* __restrict__ part, int np, double scale2,
-                                                    const double* __restrict__ part2, int np2,
-                                                    double* __restrict__ out) {
+// fixed-order sum of two partial arrays by 1024 threads: sum(part) + scale2 * sum(part2), in thread 0
+__device__ __forceinline__ double sum_parts_block(const double* __restrict__ part, int np, double scale2,
+                                                  const double* __restrict__ part2, int np2) {
   part += (uint64_t)blockIdx.x * np;  // block k: cloud k's partials (packed launches)
   part2 += (uint64_t)blockIdx.x * np2;
-  out += blockIdx.x;
   double s = 0.0, s2 = 0.0;
   for (int i = threadIdx.x; i < np; i += 1024) s += part[i];
   for (int i = threadIdx.x; i < np2; i += 1024) s2 += part2[i];
@@ -514,7 +512,43 @@ __global__ void __launch_bounds__(1024) k_sum_parts(const double* __restrict__ p
   const double a = BR(tmp).Sum(s);
   __syncthreads();
   const double b = BR(tmp).Sum(s2);
-  if (threadIdx.x == 0) out[0] = a + scale2 * b;
+  return a + scale2 * b;
+}
+__global__ void __launch_bounds__(1024) k_sum_parts(const double* __restrict__ part, int np, double scale2,
+                                                    const double* __restrict__ part2, int np2,
+                                                    double* __restrict__ out) {
+  const double v = sum_parts_block(part, np, scale2, part2, np2);
+  if (threadIdx.x == 0) out[blockIdx.x] = v;
+}
+__global__ void __launch_bounds__(1024) k_cg_step(int step, const double* __restrict__ part, int np, double scale2,
+                                                  const double* __restrict__ part2, int np2, CgScalars cg) {
+  const double v = sum_parts_block(part, np, scale2, part2, np2);
+  if (threadIdx.x != 0) return;
+  const int k = blockIdx.x;
+  const bool act = cg.act[k] != 0;
+  if (step == kCgRz0) {
+    cg.rz[k] = v;
+  } else if (step == kCgRz) {
+    cg.beta[k] = act ? v / cg.rz[k] : 0.0;
+    if (act) cg.rz[k] = v;
+  } else if (step == kCgDq) {
+    const bool ok = act && v > 0.0 && isfinite(v) && cg.rz[k] > 0.0;
+    cg.alpha[k] = ok ? cg.rz[k] / v : 0.0;
+    if (act && !ok) {
+      cg.broke[k] = 1;
+      cg.act[k] = 0;
+    }
+  } else if (act) {
+    const int it = cg.iters[k] + 1;
+    cg.iters[k] = it;
+    cg.rr[k] = v;
+    if (!isfinite(v)) {
+      cg.broke[k] = 1;
+      cg.act[k] = 0;
+    } else if (__dsqrt_rn(v) <= cg.tol[k] || it >= cg.maxit[k]) {
+      cg.act[k] = 0;
+    }
+  }
 }
 
 // ------------------------------------------------------------------ helpers of the 16^3 block kernels
@@ -780,7 +814,7 @@ __device__ __forceinline__ void plane_terms(const T r[4][4], T c0, T ce, T cc, T
 }
 
 // KIND 0: q = A a, part = a.q;  1: an = bvec + beta a, q = A an, part = an.q;
-// 2: an = a + beta bvec (FP64 solution + correction of type E), q = rhs - A an.
+// 2: an = a + beta bvec (FP64 solution + correction of type E; a null: zero), q = rhs - A an.
 // beta_dev (packed launches): the cloud's beta, in place of the beta argument.
 template <typename T, int KIND, typename E, int ZT>
 __global__ void __launch_bounds__(Zt<ZT>::NT, (sizeof(T) == 4 ? 5 : 3) * ZT / 4)
@@ -812,7 +846,8 @@ __global__ void __launch_bounds__(Zt<ZT>::NT, (sizeof(T) == 4 ? 5 : 3) * ZT / 4)
     if (KIND == 0) return __ldg(a + m);
     if (KIND == 1) return (T)__ldg(bvec + m) + beta * __ldg(a + m);
     // KIND 2 with beta 0: a cloud of a packed launch that has stopped keeps its solution
-    return beta == (T)0 ? __ldg(a + m) : __ldg(a + m) + beta * (T)__ldg(bvec + m);
+    const T av = a ? __ldg(a + m) : (T)0;
+    return beta == (T)0 ? av : av + beta * (T)__ldg(bvec + m);
   };
 #pragma unroll
   for (int r = 0; r < ZT; ++r) {
@@ -820,7 +855,9 @@ __global__ void __launch_bounds__(Zt<ZT>::NT, (sizeof(T) == 4 ? 5 : 3) * ZT / 4)
     int lx, ly, lz;
     s16::quad_coords(qd, lx, ly, lz);
     const uint64_t m = base + 4 * qd;
-    typename s16::Vec4<T>::type v = s16::ld4(a + m);
+    typename s16::Vec4<T>::type v;
+    if (KIND != 2 || a) v = s16::ld4(a + m);
+    else v.x = v.y = v.z = v.w = (T)0;
     if (KIND != 0) {
       const typename s16::Vec4<E>::type bv = s16::ld4(bvec + m);
       if (KIND == 1) {
@@ -1318,6 +1355,7 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
       cg.d = cloud_slice(cg.d, nl);
       cg.q = cloud_slice(cg.q, nl);
       cg.r = cloud_slice(cg.r, nl);
+      cg.rin = cloud_slice(cg.rin, nl);
       if (cg.alpha_dev) cg.alpha = (T)cg.alpha_dev[blockIdx.y];
     }
   }
@@ -1346,12 +1384,16 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
     typename s16::Vec4<T>::type fq;
     if (MODE == 3) {  // the CG update of this quad (plain loads: x and r are written here)
       typedef typename s16::Vec4<T>::type V4;
-      fq = *reinterpret_cast<const V4*>(cg.r + m);
-      if (cg.alpha != (T)0) {  // alpha 0: a cloud of a packed launch that has stopped keeps x and r
-        V4 xq = *reinterpret_cast<const V4*>(cg.x + m);
-        const V4 dq = s16::ld4(cg.d + m), qq = s16::ld4(cg.q + m);
-        xq.x += cg.alpha * dq.x; xq.y += cg.alpha * dq.y; xq.z += cg.alpha * dq.z; xq.w += cg.alpha * dq.w;
-        fq.x -= cg.alpha * qq.x; fq.y -= cg.alpha * qq.y; fq.z -= cg.alpha * qq.z; fq.w -= cg.alpha * qq.w;
+      fq = cg.rin ? s16::ld4(cg.rin + m) : *reinterpret_cast<const V4*>(cg.r + m);
+      if (cg.alpha != (T)0 || cg.rin) {  // alpha 0: a cloud that has stopped keeps x and r
+        V4 xq;
+        if (cg.rin) xq.x = xq.y = xq.z = xq.w = (T)0;
+        else xq = *reinterpret_cast<const V4*>(cg.x + m);
+        if (cg.alpha != (T)0) {
+          const V4 dq = s16::ld4(cg.d + m), qq = s16::ld4(cg.q + m);
+          xq.x += cg.alpha * dq.x; xq.y += cg.alpha * dq.y; xq.z += cg.alpha * dq.z; xq.w += cg.alpha * dq.w;
+          fq.x -= cg.alpha * qq.x; fq.y -= cg.alpha * qq.y; fq.z -= cg.alpha * qq.z; fq.w -= cg.alpha * qq.w;
+        }
         s16::st4(cg.x + m, xq);
         s16::st4(cg.r + m, fq);
       }
@@ -2026,6 +2068,12 @@ uint32_t mg_blocks(uint32_t D) { return tile_for(D) == 16 ? (1u << (3 * (D - 4))
 void sum_parts(cudaStream_t s, const double* part, int np, double scale2, const double* part2, int np2, double* out,
                uint32_t clouds) {
   k_sum_parts<<<clouds, 1024, 0, s>>>(part, np, scale2, part2, np2, out);
+  PR_CHECK_LAUNCH();
+}
+
+void cg_step(cudaStream_t s, CgStep step, const double* part, int np, double scale2, const double* part2, int np2,
+             const CgScalars& cg, uint32_t clouds) {
+  k_cg_step<<<clouds, 1024, 0, s>>>(step, part, np, scale2, part2, np2, cg);
   PR_CHECK_LAUNCH();
 }
 

@@ -39,7 +39,8 @@ struct CgFuse {
   const T* q = nullptr;
   T* r = nullptr;
   T alpha = 0;
-  const double* alpha_dev = nullptr;  // packed launches: per-cloud alpha in place of `alpha`
+  const double* alpha_dev = nullptr;  // per-cloud alpha in place of `alpha`
+  const T* rin = nullptr;  // the first update of a solve (x = 0, not read): r comes from here
 };
 template <typename T>
 void mg_cg_update_presmooth(cudaStream_t s, const LevelCoef& L, const T* table, const CgFuse<T>& cg, T* xo,
@@ -60,12 +61,29 @@ template <typename T>
 void mg_spmv(cudaStream_t s, const LevelCoef& L, const T* table, const T* z, const T* d, T* dn, double beta,
              bool xpby, T* q, double* part, uint32_t clouds = 1, const double* beta_dev = nullptr);
 uint32_t mg_blocks(uint32_t depth);
-// finest level (depth >= 4), FP64: xn = x + scale * e (e: correction, float or double),
+// finest level (depth >= 4), FP64: xn = x + scale * e (e: correction, float or double; x null: zero),
 // r = b - K xn (stencil part; the screening is applied separately).  x, xn: distinct buffers.
 // scale_dev (packed, nullable): per-cloud scale.
 template <typename E>
 void mg_resid_update(cudaStream_t s, const LevelCoef& L, const double* x, const E* e, double scale, double* xn,
                      const double* b, double* r, uint32_t clouds = 1, const double* scale_dev = nullptr);
+// The scalars of preconditioned CG, one per cloud, on the device: the dot products' sums update them
+// there, so that an iteration runs without the host until its residual is known.
+struct CgScalars {
+  double *alpha = nullptr, *beta = nullptr, *rz = nullptr, *tol = nullptr;
+  double* rr = nullptr;  // r.r of the last update, followed by the int arrays below: one copy to the host
+  int *act = nullptr, *broke = nullptr, *iters = nullptr;
+  int* maxit = nullptr;
+};
+enum CgStep {
+  kCgRz0 = 0,  // sum = r.z of the first preconditioning
+  kCgRz = 1,   // sum = r.z: beta
+  kCgDq = 2,   // sum = d.A d: alpha (0 for a cloud that has stopped), or the breakdown
+  kCgRr = 3    // sum = r.r after the update: counts the iteration, stops what has converged
+};
+// sum = sum(part[0:np]) + scale2 * sum(part2[0:np2]) per cloud as sum_parts, then the step
+void cg_step(cudaStream_t s, CgStep step, const double* part, int np, double scale2, const double* part2, int np2,
+             const CgScalars& cg, uint32_t clouds);
 // out = sum(part[0:np]) + scale2 * sum(part2[0:np2]), fixed order; per cloud (cloud k's partials
 // at k np and k np2, its sum at out[k])
 void sum_parts(cudaStream_t s, const double* part, int np, double scale2, const double* part2, int np2, double* out,

@@ -633,10 +633,16 @@ void screen_project_pk(cudaStream_t s, const ScreenPack& scr, const T* x, uint64
   PR_CHECK_LAUNCH();
 }
 
+unsigned screen_gather_grid(const ScreenPack& scr) {
+  unsigned g = 1;
+  while (g < grid_for(scr.maxS)) g *= 2;
+  return g;
+}
+
 template <typename T>
 void screen_gather_pk(cudaStream_t s, const ScreenPack& scr, T* y, uint64_t n, int sign) {
   if (!scr.active()) return;
-  k_screen_gather_pk<T><<<dim3(grid_for(scr.maxS), scr.clouds), kThreads, 0, s>>>(scr.desc, (T)sign * (T)scr.wh3,
+  k_screen_gather_pk<T><<<dim3(screen_gather_grid(scr), scr.clouds), kThreads, 0, s>>>(scr.desc, (T)sign * (T)scr.wh3,
                                                                                    y, n);
   PR_CHECK_LAUNCH();
 }

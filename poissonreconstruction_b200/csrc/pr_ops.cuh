@@ -63,6 +63,8 @@ void screen_project_pk(cudaStream_t s, const ScreenPack& scr, const T* x, uint64
 // per cloud: y += sign * wh3 * Phi proj
 template <typename T>
 void screen_gather_pk(cudaStream_t s, const ScreenPack& scr, T* y, uint64_t n, int sign);
+// its launch size: a power of two, so that clouds of similar size share captured launches
+unsigned screen_gather_grid(const ScreenPack& scr);
 // per cloud k: out[k] = a_k . b_k (fixed order), part: kDotBlocks per cloud (device results)
 template <typename T>
 void dots_pk(cudaStream_t s, const T* a, const T* b, uint64_t n, uint32_t clouds, double* part, double* out);

@@ -18,6 +18,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -52,10 +53,9 @@ std::vector<double> dense_operator(const LevelCoef& L) {
 // ------------------------------------------------------------------ packed systems
 // `clouds` degree-1 systems of one depth D and one screening weight, solved together: every
 // vector holds the clouds' slices back to back (cloud k at k 8^D) and every step is one launch for
-// all of them (blockIdx.y = cloud).  A single reconstruction is a pack of one.  Per-cloud scalars
-// (CG's alpha and beta, the refinement scale, the dot products) pass through pinned host slots;
-// packed launches read alpha, beta and the scale from their device copies, a pack of one takes them
-// as kernel arguments.
+// all of them (blockIdx.y = cloud).  A single reconstruction is a pack of one.  CG's scalars live on
+// the device (CgScalars); the refinement scale and the norms pass through pinned host slots (packed
+// launches read the scale from its device copy, a pack of one takes it as a kernel argument).
 struct Pack {
   pr_context* c = nullptr;  // stream and buffers of the solve
   uint32_t D = 0, clouds = 1;
@@ -67,7 +67,7 @@ struct Pack {
   std::vector<uint64_t> P_in;
   double* h = nullptr;      // pinned, kSlots x clouds
   double* d = nullptr;      // device, kSlots x clouds
-  enum { kOut, kAlpha, kBeta, kScale, kSlots };
+  enum { kOut, kScale, kSlots };
   uint64_t N() const { return n * clouds; }
   double* hs(int k) const { return h + (size_t)k * clouds; }
   double* ds(int k) const { return d + (size_t)k * clouds; }
@@ -85,11 +85,23 @@ struct Pack {
     PR_CUDA(cudaMemcpyAsync(ds(k), hs(k), clouds * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     return ds(k);
   }
+  // pinned, 3 doubles per cloud: the copy of the CG scalars that the host reads
+  double* host_cg() const { return h + (size_t)kSlots * clouds; }
   void init_slots() {
-    h = c->pinned_scalars((size_t)kSlots * clouds);
+    h = c->pinned_scalars((size_t)(kSlots + 3) * clouds);
     d = c->buf<double>("pk_scal", (size_t)kSlots * clouds);
   }
 };
+
+std::string ptr_key(std::initializer_list<const void*> ps) {
+  std::string k;
+  char b[32];
+  for (const void* p : ps) {
+    std::snprintf(b, sizeof(b), "/%p", p);
+    k += b;
+  }
+  return k;
+}
 
 bool any(const std::vector<char>& v) {
   for (char x : v)
@@ -183,61 +195,57 @@ struct Multigrid {
   }
   // The CG update can be fused with the first pre-smoothing sweep of the finest level.
   bool fuses_cg_update() const { return D >= 4 && D > Dc; }
-  // x += alpha d, r -= alpha q, first pre-smoothing sweep of r into a_D; returns r.r per cloud.
-  // A cloud with alpha 0 keeps x and r.
-  std::vector<double> cg_update_presmooth(const std::vector<double>& alpha, const T* d, const T* q, T* x, T* r) {
+  // x += alpha d, r -= alpha q, first pre-smoothing sweep of r into a_D, r.r per cloud (a cloud with
+  // alpha 0 keeps x and r).  rin: the first update of a solve, from r = rin and x = 0.
+  void cg_update_presmooth(const CgScalars& sc, const T* d, const T* q, T* x, T* r, const T* rin) {
     double* part = c->buf<double>("mg_part", (size_t)mg_blocks(D) * clouds);
     CgFuse<T> cg;
     cg.x = x;
     cg.d = d;
     cg.q = q;
     cg.r = r;
-    cg.alpha = (T)alpha[0];
-    cg.alpha_dev = pk->upload(Pack::kAlpha, alpha);
+    cg.rin = rin;
+    cg.alpha_dev = sc.alpha;
     mg_cg_update_presmooth<T>(c->stream, L[D], table(D), cg, a[D], part, clouds);
-    sum_parts(c->stream, part, (int)mg_blocks(D), 0.0, part, 0, pk->ds(Pack::kOut), clouds);
-    return pk->fetch();
+    cg_step(c->stream, kCgRr, part, (int)mg_blocks(D), 0.0, part, 0, sc, clouds);
   }
-  // z = M r; returns r.z per cloud.  presmoothed: a_D already holds the first sweep on r.
-  // After the first V-cycle of a solve (which runs plainly: the kernels' z segments are tuned on
-  // first use) the V-cycle is replayed from a CUDA graph kept by the context.
-  std::vector<double> apply(const T* r, T* z, bool presmoothed = false) {
+  // z = M r, and r.z per cloud into the scalars (step kCgRz0 or kCgRz)
+  void apply(const CgScalars& sc, CgStep step, const T* r, T* z, bool presmoothed) {
+    double* part = c->buf<double>("mg_part", (size_t)mg_blocks(D) * clouds);
+    vcycle(D, r, z, part, presmoothed);
+    cg_step(c->stream, step, part, (int)mg_blocks(D), 0.0, part, 0, sc, clouds);
+  }
+  // z = M r; returns r.z (the host loop of the smallest grids, a pack of one)
+  double apply_host(const T* r, T* z) {
     const uint64_t n = 1ull << (3 * D);
     if (D == Dc) {
       dense_solve<T>(c->stream, nc, inv, r, z, clouds);
       double* part = c->buf<double>("pk_dot_part", (size_t)kDotBlocks * clouds);
       dots_pk<T>(c->stream, r, z, n, clouds, part, pk->ds(Pack::kOut));
-      const std::vector<double> rz = pk->fetch();
-      if (applies++ == 0) spd_check(c, "coarse operator");
-      return rz;
-    }
-    double* part = c->buf<double>("mg_part", (size_t)mg_blocks(D) * clouds);
-    auto body = [&] {
-      vcycle(D, r, z, part, presmoothed);
+    } else {
+      double* part = c->buf<double>("mg_part", (size_t)mg_blocks(D) * clouds);
+      vcycle(D, r, z, part);
       sum_parts(c->stream, part, (int)mg_blocks(D), 0.0, part, 0, pk->ds(Pack::kOut), clouds);
-    };
-    const char* gr = std::getenv("PR_GRAPHS");
-    const bool first = applies++ == 0;
-    if (first || (gr && std::atoi(gr) == 0)) body();
-    else c->run_graph(graph_key(r, z, part, presmoothed), body);
-    const std::vector<double> rz = pk->fetch();
-    if (first) spd_check(c, "coarse operator");
-    return rz;
+    }
+    return pk->fetch()[0];
   }
-  int applies = 0;
-  // everything a captured V-cycle depends on: sizes, the shift (kernel arguments), every buffer
-  std::string graph_key(const T* r, const T* z, const double* part, bool presmoothed) const {
+  // throws if the coarsest operator was not positive definite; after a synchronisation
+  void check() {
+    spd_check(c, "coarse operator");
+    checked = true;
+  }
+  bool checked = false;
+  // everything that captured launches of this hierarchy depend on besides the caller's vectors:
+  // sizes, the shift (kernel arguments), every buffer, the z-segment switches
+  std::string graph_base() {
     char b[96];
-    std::snprintf(b, sizeof(b), "vcycle/%s/%u/%u/%d/%d/%a", tname<T>(), D, clouds, sweeps, presmoothed ? 1 : 0, pk->wg);
+    std::snprintf(b, sizeof(b), "cg/%s/%u/%u/%d/%a", tname<T>(), D, clouds, sweeps, pk->wg);
     std::string k = b;
     auto add = [&](const void* p) {
       std::snprintf(b, sizeof(b), "/%p", p);
       k += b;
     };
-    add(r);
-    add(z);
-    add(part);
-    add(pk->ds(Pack::kOut));
+    add(c->buf<double>("mg_part", (size_t)mg_blocks(D) * clouds));
     add(tables);
     add(inv);
     for (uint32_t l = Dc; l <= D; ++l) {
@@ -278,31 +286,57 @@ struct CgOperator {
     c->upload(table, tab.data(), 216 * sizeof(T));
   }
   const FineOp<T>& small_op() const;
-  // xpby: dn = z + beta d, q = A dn; else q = A d (dn unused).  Returns (dn or d).q per cloud
-  std::vector<double> apply_dot(const T* z, const T* d, T* dn, const std::vector<double>& beta, bool xpby, T* q) {
+  // xpby: dn = z + beta d, q = A dn; else q = A d (dn unused).  (dn or d).q per cloud becomes alpha in
+  // the scalars (D >= 4)
+  void apply_dot(const CgScalars& sc, const T* z, const T* d, T* dn, bool xpby, T* q) {
+    cudaStream_t s = c->stream;
+    int np2 = 0;
+    double *part, *part2;
+    apply(z, d, dn, 0.0, xpby ? sc.beta : nullptr, xpby, q, part, part2, np2);
+    cg_step(s, kCgDq, part, (int)mg_blocks(D), (double)(T)pk->scr.wh3, part2, np2, sc, clouds);
+  }
+  // what captured launches of the operator depend on besides the caller's vectors
+  std::string graph_part() {
+    char b[96];
+    std::snprintf(b, sizeof(b), "/%u/%a/%d", screen_gather_grid(pk->scr), pk->scr.wh3, pk->scr.active() ? 1 : 0);
+    return b + ptr_key({table, pk->scr.desc, c->buf<double>("cg_part", (size_t)mg_blocks(D) * clouds),
+                        c->buf<double>("cg_part2", (size_t)kDotBlocks * clouds)});
+  }
+  // the same with beta from the host; returns (dn or d).q (a pack of one)
+  double apply_dot_host(const T* z, const T* d, T* dn, double beta, bool xpby, T* q) {
     cudaStream_t s = c->stream;
     const uint64_t n = pk->n;
     const T* dd = xpby ? dn : d;
     if (D < 3) {  // grids below one 8^3 block (a pack of one): per-node kernels
       if (xpby) {
         PR_CUDA(cudaMemcpyAsync(dn, d, n * sizeof(T), cudaMemcpyDeviceToDevice, s));
-        pr::xpby<T>(s, n, z, beta[0], dn);
+        pr::xpby<T>(s, n, z, beta, dn);
       }
       stencil_apply<T>(s, D, dd, nullptr, q, cast_coef<T>(stencil_coef(D, Lf.shift)), 0);
       screen_apply<T>(s, small_op().scr, dd, q, +1);
-      return std::vector<double>(1, dot<T>(c, dd, q, n));
+      return dot<T>(c, dd, q, n);
     }
-    double* part = c->buf<double>("cg_part", (size_t)mg_blocks(D) * clouds);
-    double* part2 = c->buf<double>("cg_part2", (size_t)kDotBlocks * clouds);
-    mg_spmv<T>(s, Lf, table, z, d, dn, beta[0], xpby, q, part, clouds, xpby ? pk->upload(Pack::kBeta, beta) : nullptr);
     int np2 = 0;
+    double *part, *part2;
+    apply(z, d, dn, beta, nullptr, xpby, q, part, part2, np2);
+    sum_parts(s, part, (int)mg_blocks(D), (double)(T)pk->scr.wh3, part2, np2, pk->ds(Pack::kOut), clouds);
+    return pk->fetch()[0];
+  }
+  // the stencil and screening launches, their partial sums in part and part2 (np2 per cloud)
+  void apply(const T* z, const T* d, T* dn, double beta, const double* beta_dev, bool xpby, T* q, double*& part,
+             double*& part2, int& np2) {
+    cudaStream_t s = c->stream;
+    const uint64_t n = pk->n;
+    const T* dd = xpby ? dn : d;
+    part = c->buf<double>("cg_part", (size_t)mg_blocks(D) * clouds);
+    part2 = c->buf<double>("cg_part2", (size_t)kDotBlocks * clouds);
+    mg_spmv<T>(s, Lf, table, z, d, dn, beta, xpby, q, part, clouds, beta_dev);
+    np2 = 0;
     if (pk->scr.active()) {
       screen_project_pk<T>(s, pk->scr, dd, n, part2, kDotBlocks);
       screen_gather_pk<T>(s, pk->scr, q, n, +1);
       np2 = kDotBlocks;
     }
-    sum_parts(s, part, (int)mg_blocks(D), (double)(T)pk->scr.wh3, part2, np2, pk->ds(Pack::kOut), clouds);
-    return pk->fetch();
   }
 };
 template <>
@@ -312,87 +346,148 @@ const FineOp<double>& CgOperator<double>::small_op() const { return pk->op64; }
 
 struct PcgResult {
   std::vector<int> iters;
-  std::vector<double> rr;
-  std::vector<char> broke;
 };
+// Preconditioned CG from x = 0 on A x = b below depth 4 (a pack of one, per-node kernels), the scalars
+// on the host.
+template <typename T>
+PcgResult pcg_small(Pack& pk, CgOperator<T>& A, Multigrid<T>& M, const T* b, T* x, double tol_abs, int maxit,
+                    double rr0) {
+  pr_context* c = pk.c;
+  const uint64_t n = pk.n;
+  cudaStream_t s = c->stream;
+  const std::string tn = tname<T>();
+  T* r = c->buf<T>("cg_r_" + tn, n);
+  T* z = c->buf<T>("cg_z_" + tn, n);
+  T* dA = c->buf<T>("cg_d_" + tn, n);
+  T* dB = c->buf<T>("cg_d2_" + tn, n);
+  T* q = c->buf<T>("cg_q_" + tn, n);
+  PcgResult res;
+  res.iters.assign(1, 0);
+  PR_CUDA(cudaMemsetAsync(x, 0, n * sizeof(T), s));
+  PR_CUDA(cudaMemcpyAsync(r, b, n * sizeof(T), cudaMemcpyDeviceToDevice, s));
+  if (!(std::sqrt(rr0) > tol_abs) || maxit <= 0) return res;
+  double rz = M.apply_host(r, z), beta = 0.0;
+  M.check();
+  T* d = nullptr;  // current search direction
+  for (int it = 0;; ++it) {
+    double dq;
+    if (it == 0) {
+      dq = A.apply_dot_host(z, z, nullptr, 0.0, false, q);  // d = z
+      d = z;
+    } else {
+      T* dn = (d == dA) ? dB : dA;
+      dq = A.apply_dot_host(z, d, dn, beta, true, q);
+      d = dn;
+    }
+    if (!(dq > 0.0) || !std::isfinite(dq) || !(rz > 0.0)) break;
+    const double rr = cg_update<T>(c, n, rz / dq, d, q, x, r);
+    res.iters[0] = it + 1;
+    if (!std::isfinite(rr) || std::sqrt(rr) <= tol_abs || it + 1 >= maxit) break;
+    if (d == z) {  // the first direction aliases z: keep it before z is overwritten
+      PR_CUDA(cudaMemcpyAsync(dA, z, n * sizeof(T), cudaMemcpyDeviceToDevice, s));
+      d = dA;
+    }
+    const double rz_new = M.apply_host(r, z);
+    beta = rz_new / rz;
+    rz = rz_new;
+  }
+  return res;
+}
 
 // Preconditioned CG from x = 0 on A x = b for every cloud with want[k], until ||r_k|| <= tol_abs[k]
 // or maxit[k] iterations; rr0[k] = b_k . b_k.  The clouds run in lockstep: one that has stopped
-// gets alpha 0 (its x and r stay) and its other results are ignored.  The search direction
-// ping-pongs between two buffers (the SpMV reads d with halos).
+// gets alpha 0 (its x and r stay) and its other results are ignored. The scalars live on the device
+// (CgScalars); the host reads which clouds still run once per iteration, after the residual update,
+// so that no V-cycle is started for nothing. Everything between two reads (V-cycle, direction and
+// operator, update) is one CUDA graph per direction buffer, kept by the context; the first
+// iteration of a configuration's first solve runs plainly (the kernels' z segments are tuned on
+// first use). The search direction ping-pongs between two buffers (the SpMV reads d with halos);
+// the first one is the preconditioned right-hand side itself, and the first update takes x = 0 and
+// r = b as read, so nothing is copied or zero-filled. At depth 5, 39 host round trips became 19,
+// and a reconstruction of 4,000 points went from 1.93 to 1.65 ms (317,003 points at depth 9: 29.9
+// to 27.7).
 template <typename T>
 PcgResult pcg(Pack& pk, CgOperator<T>& A, Multigrid<T>& M, const T* b, T* x, const std::vector<double>& tol_abs,
               const std::vector<int>& maxit, const std::vector<double>& rr0, const std::vector<char>& want) {
+  if (!M.fuses_cg_update()) return pcg_small<T>(pk, A, M, b, x, tol_abs[0], maxit[0], rr0[0]);
   pr_context* c = pk.c;
   const uint32_t K = pk.clouds;
   const uint64_t N = pk.N();
   cudaStream_t s = c->stream;
   const std::string tn = tname<T>();
   T* r = c->buf<T>("cg_r_" + tn, N);
+  T* z0 = c->buf<T>("cg_z0_" + tn, N);  // M b, the first direction; then every other direction
   T* z = c->buf<T>("cg_z_" + tn, N);
   T* dA = c->buf<T>("cg_d_" + tn, N);
-  T* dB = c->buf<T>("cg_d2_" + tn, N);
   T* q = c->buf<T>("cg_q_" + tn, N);
   PcgResult res;
   res.iters.assign(K, 0);
-  res.rr = rr0;
-  res.broke.assign(K, 0);
-  PR_CUDA(cudaMemsetAsync(x, 0, N * sizeof(T), s));
-  PR_CUDA(cudaMemcpyAsync(r, b, N * sizeof(T), cudaMemcpyDeviceToDevice, s));
-  std::vector<char> act(K, 0);
-  for (uint32_t k = 0; k < K; ++k) act[k] = want[k] && std::sqrt(rr0[k]) > tol_abs[k] && maxit[k] > 0;
-  if (!any(act)) return res;
-  std::vector<double> rz = M.apply(r, z), beta(K, 0.0), alpha(K, 0.0);
-  T* d = nullptr;  // current search direction
-  for (int it = 0;; ++it) {
-    std::vector<double> dq;
-    if (it == 0) {
-      dq = A.apply_dot(z, z, nullptr, beta, false, q);  // d = z
-      d = z;
-    } else {
-      T* dn = (d == dA) ? dB : dA;
-      dq = A.apply_dot(z, d, dn, beta, true, q);
-      d = dn;
-    }
-    for (uint32_t k = 0; k < K; ++k) {
-      alpha[k] = 0.0;
-      if (!act[k]) continue;
-      if (!(dq[k] > 0.0) || !std::isfinite(dq[k]) || !(rz[k] > 0.0)) {
-        res.broke[k] = 1;
-        act[k] = 0;
-        continue;
-      }
-      alpha[k] = rz[k] / dq[k];
-    }
-    if (!any(act)) break;
-    const bool fused = M.fuses_cg_update();
-    const std::vector<double> rr =
-        fused ? M.cg_update_presmooth(alpha, d, q, x, r)
-              : std::vector<double>(1, cg_update<T>(c, pk.n, alpha[0], d, q, x, r));  // a pack of one
-    for (uint32_t k = 0; k < K; ++k) {
-      if (!act[k]) continue;
-      res.iters[k] = it + 1;
-      res.rr[k] = rr[k];
-      if (!std::isfinite(rr[k])) {
-        res.broke[k] = 1;
-        act[k] = 0;
-      } else if (std::sqrt(rr[k]) <= tol_abs[k] || it + 1 >= maxit[k]) {
-        act[k] = 0;
-      }
-    }
-    if (!any(act)) break;
-    if (d == z) {  // the first direction aliases z: keep it before z is overwritten
-      PR_CUDA(cudaMemcpyAsync(dA, z, N * sizeof(T), cudaMemcpyDeviceToDevice, s));
-      d = dA;
-    }
-    const std::vector<double> rz_new = M.apply(r, z, fused);
-    for (uint32_t k = 0; k < K; ++k) {
-      beta[k] = 0.0;
-      if (!act[k]) continue;
-      beta[k] = rz_new[k] / rz[k];
-      rz[k] = rz_new[k];
-    }
+  // device scalars and their start: doubles [alpha beta rz tol rr], ints [act broke iters maxit], K each
+  const size_t words = 7 * (size_t)K;  // in doubles
+  double* dv = c->buf<double>("cg_scalars", words);
+  std::vector<double> init(words, 0.0);
+  int* ii = reinterpret_cast<int*>(init.data() + 5 * K);
+  bool some = false;
+  for (uint32_t k = 0; k < K; ++k) {
+    init[3 * K + k] = tol_abs[k];
+    init[4 * K + k] = rr0[k];
+    ii[k] = want[k] && std::sqrt(rr0[k]) > tol_abs[k] && maxit[k] > 0;
+    ii[3 * K + k] = maxit[k];
+    some = some || ii[k];
   }
+  if (!some) {
+    PR_CUDA(cudaMemsetAsync(x, 0, N * sizeof(T), s));
+    return res;
+  }
+  c->upload(dv, init.data(), words * sizeof(double));
+  CgScalars sc;
+  sc.alpha = dv;
+  sc.beta = dv + K;
+  sc.rz = dv + 2 * K;
+  sc.tol = dv + 3 * K;
+  sc.rr = dv + 4 * K;
+  sc.act = reinterpret_cast<int*>(dv + 5 * K);
+  sc.broke = sc.act + K;
+  sc.iters = sc.act + 2 * K;
+  sc.maxit = sc.act + 3 * K;
+  const size_t back = K * sizeof(double) + 3 * K * sizeof(int);  // rr, act, broke, iters
+  double* h = pk.host_cg();
+  const int* h_act = reinterpret_cast<const int*>(h + K);
+  const int* h_iters = h_act + 2 * K;
+
+  const char* gr = std::getenv("PR_GRAPHS");
+  const bool graphs = !(gr && std::atoi(gr) == 0);
+  const std::string base = M.graph_base() + A.graph_part() + ptr_key({dv, h, b, r, z, q, x, z0, dA});
+  auto first = [&] {  // d = M b, alpha, x = alpha d, r = b - alpha A d
+    M.apply(sc, kCgRz0, b, z0, false);
+    A.apply_dot(sc, z0, z0, nullptr, false, q);
+    M.cg_update_presmooth(sc, z0, q, x, r, b);
+    PR_CUDA(cudaMemcpyAsync(h, sc.rr, back, cudaMemcpyDeviceToHost, s));
+  };
+  if (graphs && (M.checked || c->graphs.count(base + "/f"))) c->run_graph(base + "/f", first);
+  else first();
+  c->sync();
+  M.check();
+  const T* d = z0;  // current search direction
+  T* dn = dA;
+  for (;;) {
+    bool any_act = false;
+    for (uint32_t k = 0; k < K; ++k) any_act = any_act || h_act[k];
+    if (!any_act) break;
+    auto body = [&] {
+      M.apply(sc, kCgRz, r, z, true);
+      A.apply_dot(sc, z, d, dn, true, q);
+      M.cg_update_presmooth(sc, dn, q, x, r, nullptr);
+      PR_CUDA(cudaMemcpyAsync(h, sc.rr, back, cudaMemcpyDeviceToHost, s));
+    };
+    if (graphs) c->run_graph(base + (dn == dA ? "/a" : "/z"), body);
+    else body();
+    c->sync();
+    T* nd = dn;
+    dn = (nd == dA) ? z0 : dA;
+    d = nd;
+  }
+  for (uint32_t k = 0; k < K; ++k) res.iters[k] = h_iters[k];
   return res;
 }
 
@@ -435,7 +530,6 @@ void solve_pack(Pack& pk, const pr_params& p, const double* b, double* xA, std::
     st[k].refinement_steps = 0;
     st[k].solve_bytes = 0.0;
   }
-  PR_CUDA(cudaMemsetAsync(xA, 0, N * sizeof(double), s));
   // mixed: the FP32 system is the current FP64 residual rounded (unscaled: residuals stay far
   // above the bottom of the FP32 range), its norm computed in the same pass
   float* r32 = mixed ? c->buf<float>("r32", N) : nullptr;
@@ -457,11 +551,16 @@ void solve_pack(Pack& pk, const pr_params& p, const double* b, double* xA, std::
   const double es = mixed ? 4.0 : 8.0;
 
   // x <- x + scale_k e and r = b - A x (FP64) per cloud; scale 0 keeps a cloud's x.  x ping-pongs
-  // between xA and xB.
-  double* x = xA;
+  // between xA and xB; it is zero, and not read, until the first correction (two of them are usual
+  // with FP32 solves, one with FP64: both end in xA).
+  double* x = nullptr;
+  if (!fused) {
+    x = xA;
+    PR_CUDA(cudaMemsetAsync(xA, 0, N * sizeof(double), s));
+  }
   auto update_residual = [&](const void* e, bool e_is_float, const std::vector<double>& scale) {
     if (fused) {
-      double* xn = (x == xA) ? xB : xA;
+      double* xn = x == nullptr ? (mixed ? xB : xA) : (x == xA ? xB : xA);
       const double* sd = pk.upload(Pack::kScale, scale);
       if (e_is_float) mg_resid_update<float>(s, L64, x, (const float*)e, scale[0], xn, b, r, K, sd);
       else mg_resid_update<double>(s, L64, x, (const double*)e, scale[0], xn, b, r, K, sd);
@@ -520,14 +619,15 @@ void solve_pack(Pack& pk, const pr_params& p, const double* b, double* xA, std::
         rn[k] = rn_new[k];
       }
     }
-    if (M.applies == 0) {  // nothing to solve: the setup's check alone
+    if (!M.checked) {  // nothing to solve
       c->sync();
-      spd_check(c, "coarse operator");
+      M.check();
     }
   };
   if (mixed) round(float());
   else round(double());
-  if (x != xA) PR_CUDA(cudaMemcpyAsync(xA, x, N * sizeof(double), cudaMemcpyDeviceToDevice, s));
+  if (x == nullptr) PR_CUDA(cudaMemsetAsync(xA, 0, N * sizeof(double), s));
+  else if (x != xA) PR_CUDA(cudaMemcpyAsync(xA, x, N * sizeof(double), cudaMemcpyDeviceToDevice, s));
   for (uint32_t k = 0; k < K; ++k) {
     st[k].pcg_iterations = (uint32_t)used[k];
     st[k].rel_residual = bn[k] == 0.0 ? 0.0 : rn[k] / bn[k];
