@@ -813,7 +813,23 @@ __device__ __forceinline__ void plane_terms(const T r[4][4], T c0, T ce, T cc, T
     }
 }
 
+// in-plane sums of the quad's 4 nodes by themselves: the 4 face neighbours and the 4 diagonal ones
+template <typename T>
+__device__ __forceinline__ void plane_sums(const T r[4][4], T f[4], T d[4], T ctr[4]) {
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int e = 2 * j + i, R = j + 1, Cc = i + 1;
+      f[e] = (r[R][Cc - 1] + r[R][Cc + 1]) + (r[R - 1][Cc] + r[R + 1][Cc]);
+      d[e] = (r[R - 1][Cc - 1] + r[R - 1][Cc + 1]) + (r[R + 1][Cc - 1] + r[R + 1][Cc + 1]);
+      ctr[e] = r[R][Cc];
+    }
+}
+
 // KIND 0: q = A a, part = a.q;  1: an = bvec + beta a, q = A an, part = an.q;
+// 3: q = A a for a caller's vector: a node's 12 edge and 8 corner neighbours are summed before they
+// meet their coefficients, as in the per-node stencil, which rounds less than the solver's order;
 // 2: an = a + beta bvec (FP64 solution + correction of type E; a null: zero), q = rhs - A an.
 // beta_dev (packed launches): the cloud's beta, in place of the beta argument.
 template <typename T, int KIND, typename E, int ZT>
@@ -843,7 +859,7 @@ __global__ void __launch_bounds__(Zt<ZT>::NT, (sizeof(T) == 4 ? 5 : 3) * ZT / 4)
   const int t = threadIdx.x;
   s16::neighbour_bases(nb, bx, by, bz, res >> 4);
   auto val = [&](uint32_t m) -> T {
-    if (KIND == 0) return __ldg(a + m);
+    if (KIND == 0 || KIND == 3) return __ldg(a + m);
     if (KIND == 1) return (T)__ldg(bvec + m) + beta * __ldg(a + m);
     // KIND 2 with beta 0: a cloud of a packed launch that has stopped keeps its solution
     const T av = a ? __ldg(a + m) : (T)0;
@@ -858,7 +874,7 @@ __global__ void __launch_bounds__(Zt<ZT>::NT, (sizeof(T) == 4 ? 5 : 3) * ZT / 4)
     typename s16::Vec4<T>::type v;
     if (KIND != 2 || a) v = s16::ld4(a + m);
     else v.x = v.y = v.z = v.w = (T)0;
-    if (KIND != 0) {
+    if (KIND == 1 || KIND == 2) {
       const typename s16::Vec4<E>::type bv = s16::ld4(bvec + m);
       if (KIND == 1) {
         v.x = (T)bv.x + beta * v.x; v.y = (T)bv.y + beta * v.y; v.z = (T)bv.z + beta * v.z; v.w = (T)bv.w + beta * v.w;
@@ -879,6 +895,32 @@ __global__ void __launch_bounds__(Zt<ZT>::NT, (sizeof(T) == 4 ? 5 : 3) * ZT / 4)
   const int qi = t & 63, zs = t >> 6;
   const int x0 = 2 * (qi & 7), y0 = 2 * (qi >> 3), z0 = ZT * zs;
   const uint32_t mq = s16::sp4(x0) | (s16::sp4(y0) << 1);
+  if constexpr (KIND == 3) {
+    T fm[4], dm[4], f0[4], d0[4], c0v[4], fp[4], dp[4], cp[4];  // planes p - 2, p - 1 and p
+#pragma unroll
+    for (int p = 0; p < ZT + 2; ++p) {  // tile plane z0 + p = local z0 + p - 1
+      T r[4][4];
+      patch<T, RS>(tile, nat(x0, y0, z0 + p), r);
+      plane_sums<T>(r, fp, dp, cp);
+      if (p >= 2) {
+        T y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = c0 * c0v[e] + ce * (d0[e] + (fm[e] + fp[e])) + cc * (dm[e] + dp[e]);
+        typename s16::Vec4<T>::type o;
+        o.x = y[0]; o.y = y[1]; o.z = y[2]; o.w = y[3];
+        s16::st4(q + base + (mq | (s16::sp4(z0 + p - 2) << 2)), o);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        fm[e] = f0[e];
+        dm[e] = d0[e];
+        f0[e] = fp[e];
+        d0[e] = dp[e];
+        c0v[e] = cp[e];
+      }
+    }
+    return;
+  }
   T cur[4] = {0, 0, 0, 0}, nxt[4] = {0, 0, 0, 0}, cprev[4] = {0, 0, 0, 0};
   double pv[ZT];  // per plane: the quad's four products of the dot
 #pragma unroll
@@ -913,7 +955,7 @@ __global__ void __launch_bounds__(Zt<ZT>::NT, (sizeof(T) == 4 ? 5 : 3) * ZT / 4)
       cprev[e] = ctr[e];
     }
   }
-  if (KIND != 2) {
+  if (KIND < 2) {
     __syncthreads();  // the tile's last reads: its memory takes the per-plane sums
     double* red = reinterpret_cast<double*>(smem_raw);
 #pragma unroll
@@ -2047,6 +2089,17 @@ void mg_spmv(cudaStream_t s, const LevelCoef& L, const T* table, const T* z, con
   PR_CHECK_LAUNCH();
 }
 
+template <typename T>
+void mg_apply(cudaStream_t s, const LevelCoef& L, const T* x, T* y) {
+  const uint32_t D = L.depth;
+  if (D < 4 || L.has_faces) throw Error(PR_ERR_INTERNAL, "mg_apply needs the finest level, depth >= 4");
+  const size_t sm = n16::smem_bytes<T>();
+  allow_smem(n16::k_spmv16<T, 3, T, 4>, sm);
+  n16::k_spmv16<T, 3, T, 4><<<1u << (3 * (D - 4)), n16::Zt<4>::NT, sm, s>>>(
+      D, x, nullptr, nullptr, (T)0, y, (T)L.c0, (T)L.ce, (T)L.cc, nullptr, nullptr, nullptr);
+  PR_CHECK_LAUNCH();
+}
+
 template <typename E>
 void mg_resid_update(cudaStream_t s, const LevelCoef& L, const double* x, const E* e, double scale, double* xn,
                      const double* b, double* r, uint32_t clouds, const double* scale_dev) {
@@ -2182,6 +2235,7 @@ double kernel_bench(pr_context* c, int kid, uint32_t D, int precision, int reps,
 #define PR_INST(T)                                                                                                 \
   template void mg_smooth<T>(cudaStream_t, const LevelCoef&, const T*, const T*, T*, const T*, const T*, int, bool, \
                              double*, uint32_t);                                                                  \
+  template void mg_apply<T>(cudaStream_t, const LevelCoef&, const T*, T*);                                        \
   template void mg_coarse_tail<T>(cudaStream_t, const LevelCoef&, const LevelCoef&, const T*, const T*, const T*,   \
                                   const T*, T*, uint32_t);                                                        \
   template void mg_resid_restrict<T>(cudaStream_t, const LevelCoef&, const T*, const T*, const T*, T*, T*,        \

@@ -61,6 +61,9 @@ template <typename T>
 void mg_spmv(cudaStream_t s, const LevelCoef& L, const T* table, const T* z, const T* d, T* dn, double beta,
              bool xpby, T* q, double* part, uint32_t clouds = 1, const double* beta_dev = nullptr);
 uint32_t mg_blocks(uint32_t depth);
+// finest level (depth >= 4): y = A x, stencil part, for a caller's 16-byte aligned vectors
+template <typename T>
+void mg_apply(cudaStream_t s, const LevelCoef& L, const T* x, T* y);
 // finest level (depth >= 4), FP64: xn = x + scale * e (e: correction, float or double; x null: zero),
 // r = b - K xn (stencil part; the screening is applied separately).  x, xn: distinct buffers.
 // scale_dev (packed, nullable): per-cloud scale.

@@ -23,3 +23,26 @@ def test_coarse_levels_of_the_degree1_vcycle(ctx, depth, sweeps, precision):
     x_ref, _, _ = oracle.Tree(depth, unit).solve_converged(4.0, tol=1e-13, maxit=200000)
     x = ctx.coefficients()
     assert np.linalg.norm(x - x_ref) <= 1e-6 * np.linalg.norm(x_ref)
+
+
+@pytest.mark.parametrize("precision", [prb.PR_PRECISION_FP64, prb.PR_PRECISION_MIXED])
+@pytest.mark.parametrize("depth,offset", [(3, 0), (4, 0), (4, 1), (5, 0), (5, 1), (5, 2)])
+def test_operator_on_device_vectors(ctx, depth, offset, precision):
+    """The tiled operator (depth >= 4, 16-byte aligned vectors) and the per-node one against the oracle;
+    offset: the vectors start that many elements past an aligned address."""
+    import torch
+    pts = synthetic.sphere(2500, seed=50 + depth)
+    ctx.solve(pts, prb.ReconstructParams(depth=depth, point_weight=4.0))
+    unit, _ = oracle.to_unit(pts)
+    t = oracle.Tree(depth, unit)
+    t.assemble(4.0)
+    dtype = torch.float64 if precision == prb.PR_PRECISION_FP64 else torch.float32
+    x = torch.randn(t.n + offset, dtype=dtype, generator=torch.Generator().manual_seed(depth)).cuda()[offset:]
+    y = torch.full((t.n + offset,), float("nan"), dtype=dtype, device="cuda")[offset:]
+    torch.cuda.synchronize()
+    ctx.apply_operator_device(x.data_ptr(), y.data_ptr(), precision)
+    ctx.synchronize()
+    y_ref = t.spmv(x.double().cpu().numpy())
+    err = np.abs(y.double().cpu().numpy() - y_ref).max()
+    # 21 products of at most max|A| max|x| each, rounded to 24 or 53 bits
+    assert err <= (1e-13 if dtype == torch.float64 else 1e-5) * np.abs(y_ref).max()
