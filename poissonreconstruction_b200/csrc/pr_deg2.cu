@@ -46,11 +46,25 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int TX = 32, TY = 8;           // output columns of a CTA
 constexpr int SW = TX + 4, SH = TY + 4;  // staged input plane (halo 2)
-constexpr int kZChunk = 64;              // output planes per CTA (k_op2)
 constexpr int kZChunk3 = 76;             // output planes per CTA (k_op3): 80 staged planes = 16 x 5
 constexpr int kChebSteps = 3;            // Chebyshev degree of one smoothing
 constexpr double kLamMax = 2.1;          // bound of the spectrum of D^-1 (K + wg I) on every level
 constexpr double kLamRatio = 15.0;       // smoothed interval [kLamMax / kLamRatio, kLamMax]
+
+// Planes per CTA on the small levels.  A CTA takes its planes one after the other, about 0.4 us each
+// (k_op3, k_op3r) or 0.3 us (k_op2), so a level of few tiles is cut into short runs that fill the
+// 148 SMs, down to where the four halo planes a run reads besides its own cost as much as they save:
+// k_op2, whose levels have one to four tiles, 2 planes; k_op3 and k_op3r 6 planes at 64^3 (88 CTAs)
+// and 16 at 128^3 (256), with the halo a multiple of the five stages; larger levels keep 76.  A node's
+// value does not depend on the run.  FP32 passes at 64^3 took 29 us in 8 CTAs, k_op2 12 us.
+constexpr int kZChunk2 = 2;
+// dots: the pass leaves partial sums whose total enters the solution (FP64 solves keep their order)
+inline int z_chunk3(int L, bool keep_order) {
+  if (keep_order || L > 7) return kZChunk3;
+  return L == 6 ? 6 : 16;
+}
+// coarse planes per CTA of the grid transfers to and from a fine level
+inline int z_chunk_transfer(int Lf, int full) { return Lf == 6 ? 2 : (Lf == 7 ? 4 : full); }
 
 inline unsigned grid_for(uint64_t n, uint64_t cap = 1u << 22) {
   uint64_t g = (n + kThreads - 1) / kThreads;
@@ -145,14 +159,14 @@ struct LevelView {
 
 enum { kOpApply = 0, kOpResid = 1, kOpCheb = 2 };
 
-// One pass of the level operator over a CTA's 32 x 8 columns and up to kZChunk planes.
+// One pass of the level operator over a CTA's 32 x 8 columns and up to zc planes.
 //   kOpApply: out = A x
 //   kOpResid: out = f - A x
 //   kOpCheb:  out = x + ca (x - xp) + cb D^-1 (f - A x)   (xp null: previous iterate 0); out may
 //             alias xp (each element is read before it is written by the same thread), never x.
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kThreads) k_op2(const T* __restrict__ x, const T* __restrict__ f, const T* xp,
-                                                  T* out, LevelView<T> lv, T ca, T cb) {
+                                                  T* out, LevelView<T> lv, T ca, T cb, int zc) {
   __shared__ T s_in[SH][SW];
   __shared__ T s_um[SH][TX];
   __shared__ T s_us[SH][TX];
@@ -160,7 +174,7 @@ __global__ void __launch_bounds__(kThreads) k_op2(const T* __restrict__ x, const
   const int64_t plane = (int64_t)res * res;
   const int t = threadIdx.x, tx = t & 31, ty = t >> 5;
   const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
-  const int z0 = blockIdx.z * kZChunk, z1 = min(z0 + kZChunk, res);
+  const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, res);
   const int gx = x0 + tx, gy = y0 + ty;
   const bool own = gx < res && gy < res;
   T cmx[5], csx[5], cmy[5], csy[5];
@@ -367,6 +381,7 @@ struct Op3Args {
   int all;         // EDGE: the grid enumerates every tile, not only the face tiles
   int ox, oy;      // interior: tile of block (i, j) is (i + ox, j + oy)
   int oz;          // interior: z run of block k is k + oz
+  int zc;          // output planes of a z run
   int* err;
   double* dot;     // optional per-CTA partials: kOpApply x . out, kOpCheb f . out, kOpApplyD d . out
   int dot_base;    // index of this launch's first partial
@@ -453,7 +468,7 @@ __global__ void __launch_bounds__(kThreads) k_op3(const __grid_constant__ CUtens
     by = blockIdx.y + A.oy;
   }
   const int x0 = bx * TXP, y0 = by * TY;
-  const int z0 = (blockIdx.z + A.oz) * kZChunk3, z1 = min(z0 + kZChunk3, res);
+  const int z0 = (blockIdx.z + A.oz) * A.zc, z1 = min(z0 + A.zc, res);
   const int gx = x0 + 2 * p, gy = y0 + ty;  // res >= 64: every column is inside the grid
   const int nplanes = z1 - z0 + 4;
   const int ngroups = (nplanes + NS - 1) / NS;  // planes past z1 + 1 read zeros and emit nothing
@@ -813,7 +828,7 @@ __global__ void __launch_bounds__(kThreadsR) k_op3r(const __grid_constant__ CUte
   const int64_t plane = (int64_t)res * res;
   const int t = threadIdx.x, p = t & 31, ry = RY * (t >> 5);  // tile rows ry, ry + 1; staged ry .. ry + 5
   const int x0 = (blockIdx.x + A.ox) * TXP, y0 = (blockIdx.y + A.oy) * TY;
-  const int z0 = (blockIdx.z + A.oz) * kZChunk3, z1 = min(z0 + kZChunk3, res);
+  const int z0 = (blockIdx.z + A.oz) * A.zc, z1 = min(z0 + A.zc, res);
   const int gx = x0 + 2 * p;
   const int nplanes = z1 - z0 + 4;
   const int ngroups = (nplanes + NS - 1) / NS;
@@ -1157,7 +1172,7 @@ struct GeoRs {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kThreadsR) k_restrict3(const __grid_constant__ CUtensorMap mr, int Lf,
+__global__ void __launch_bounds__(kThreadsR) k_restrict3(const __grid_constant__ CUtensorMap mr, int Lf, int czn,
                                                          T* __restrict__ fc, int* __restrict__ err) {
   typedef GeoRs<T> G;
   typedef typename Vec2<T>::type V2;
@@ -1170,7 +1185,7 @@ __global__ void __launch_bounds__(kThreadsR) k_restrict3(const __grid_constant__
   const int64_t pc = (int64_t)rc * rc;
   const int t = threadIdx.x, tx = t & 15, ty = t >> 4;  // coarse pair tx, coarse row ty of the tile
   const int x0 = blockIdx.x * 64, y0 = blockIdx.y * 16;
-  const int cz0 = blockIdx.z * kRestrictCZ, cz1 = min(cz0 + kRestrictCZ, rc);
+  const int cz0 = blockIdx.z * czn, cz1 = min(cz0 + czn, rc);
   const int nplanes = 2 * (cz1 - cz0) + 2;  // fine 2 cz0 - 1 .. 2 cz1
   if (t == 0) {
     for (int q = 0; q < NS; ++q) mbar_init(&bar[q], 1);
@@ -1263,7 +1278,7 @@ struct GeoPr {
 
 template <typename T>
 __global__ void __launch_bounds__(kThreadsR) k_prolong3(const __grid_constant__ CUtensorMap mc, const T* __restrict__ xf,
-                                                        int Lf, T* __restrict__ out, int* __restrict__ err) {
+                                                        int Lf, int czn, T* __restrict__ out, int* __restrict__ err) {
   typedef GeoPr<T> G;
   typedef typename Vec2<T>::type V2;
   constexpr int NS = G::NS, XO = G::XO, CW = G::CW;
@@ -1275,7 +1290,7 @@ __global__ void __launch_bounds__(kThreadsR) k_prolong3(const __grid_constant__ 
   const int64_t pf = (int64_t)rf * rf;
   const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
   const int x0 = blockIdx.x * 64, y0 = blockIdx.y * 16, cx0 = x0 / 2, cy0 = y0 / 2;
-  const int cz0 = blockIdx.z * kProlongCZ, cz1 = min(cz0 + kProlongCZ, rc);
+  const int cz0 = blockIdx.z * czn, cz1 = min(cz0 + czn, rc);
   const int nplanes = cz1 - cz0 + 2;  // coarse cz0 - 1 .. cz1
   if (t == 0) {
     for (int q = 0; q < NS; ++q) mbar_init(&bar[q], 1);
@@ -1778,9 +1793,9 @@ int launch_op3(pr_context* c, cudaStream_t s, const CUtensorMap& mx, const CUten
       int zlo = nz, zhi = nz;
       if (a.edge <= 6 && nz >= 5) {
         zlo = 0;
-        while (zlo < nz && zlo * kZChunk3 - 2 < a.edge) ++zlo;
+        while (zlo < nz && zlo * a.zc - 2 < a.edge) ++zlo;
         zhi = zlo;
-        while (zhi < nz && std::min((zhi + 1) * kZChunk3, res) + 2 <= res - a.edge) ++zhi;
+        while (zhi < nz && std::min((zhi + 1) * a.zc, res) + 2 <= res - a.edge) ++zhi;
       }
       const int ni = (nbx - 2) * (nby - 2);
       auto run = [&](int z_begin, int z_end, bool regs) {
@@ -1823,8 +1838,9 @@ void launch_prolong(cudaStream_t s, const T* xf, const T* ec, int Lf, T* out, in
     typedef GeoPr<T> G;
     const int rf = 1 << Lf, rc = rf >> 1;
     const CUtensorMap m = plane_map<T>(ec, Lf - 1, G::CW, G::CR);
-    const dim3 grid(rf / 64, rf / 16, (rc + kProlongCZ - 1) / kProlongCZ);
-    k_prolong3<T><<<grid, kThreadsR, G::BYTES, s>>>(m, xf, Lf, out, err);
+    const int czn = z_chunk_transfer(Lf, kProlongCZ);
+    const dim3 grid(rf / 64, rf / 16, (rc + czn - 1) / czn);
+    k_prolong3<T><<<grid, kThreadsR, G::BYTES, s>>>(m, xf, Lf, czn, out, err);
   } else {
     k_prolong4<T><<<grid_for(1ull << (3 * (Lf - 1) - 1)), kThreads, 0, s>>>(xf, ec, Lf, out);
   }
@@ -1838,8 +1854,9 @@ void launch_restrict(cudaStream_t s, const T* rf, int Lf, T* fc, int* err) {
     typedef GeoRs<T> G;
     const int res = 1 << Lf, rc = res >> 1;
     const CUtensorMap m = plane_map<T>(rf, Lf, G::BW, G::SR);
-    const dim3 grid(res / 64, res / 16, (rc + kRestrictCZ - 1) / kRestrictCZ);
-    k_restrict3<T><<<grid, kThreadsR, G::BYTES, s>>>(m, Lf, fc, err);
+    const int czn = z_chunk_transfer(Lf, kRestrictCZ);
+    const dim3 grid(res / 64, res / 16, (rc + czn - 1) / czn);
+    k_restrict3<T><<<grid, kThreadsR, G::BYTES, s>>>(m, Lf, czn, fc, err);
   } else {
     k_restrict4<T><<<grid_for(1ull << (3 * (Lf - 1) - 1)), kThreads, 0, s>>>(rf, Lf, fc);
   }
@@ -2051,7 +2068,8 @@ struct System2 {
   bool fused_dots() const { return !lv.empty() && lv[0].L >= kTmaMinLevel; }
   void alloc_parts() {
     const int res = 1 << lv[0].L;
-    const size_t tiles = (size_t)(res / Geo3<T>::TXP) * (res / TY) * ((res + kZChunk3 - 1) / kZChunk3);
+    const int zc = z_chunk3(lv[0].L, false);  // the shortest runs of any pass
+    const size_t tiles = (size_t)(res / Geo3<T>::TXP) * (res / TY) * ((res + zc - 1) / zc);
     parts_a = c->buf<double>(std::string("d2_parts_a_") + tn2<T>(), tiles);
     parts_b = c->buf<double>(std::string("d2_parts_b_") + tn2<T>(), 1u << 20);
     sums = c->buf<double>(std::string("d2_sums_") + tn2<T>(), 2);
@@ -2121,7 +2139,8 @@ struct System2 {
       A.out2 = (two || refine) ? fu->out2 : nullptr;
       A.xacc = two ? fu->xacc : nullptr;
       A.xmode = two ? fu->xmode : 0;
-      const int nz = (res + kZChunk3 - 1) / kZChunk3;
+      A.zc = z_chunk3(q.L, sizeof(T) == 8 && dot && (mode == kOpApplyD || mode == kOpCheb || mode == kOpApply));
+      const int nz = (res + A.zc - 1) / A.zc;
       const CUtensorMap mx = plane_map<T>(x, q.L, G::BW, SH);
       const CUtensorMap mf = f ? (two ? plane_map<T>(f, q.L, G::BW, SH) : plane_map<T>(f, q.L, G::TXP, TY)) : mx;
       const CUtensorMap mp = refine ? plane_map<float>(fu->e32, q.L, 72, SH)
@@ -2140,10 +2159,10 @@ struct System2 {
     } else {
       PR_REQUIRE(mode <= kOpCheb, PR_ERR_INTERNAL, "fused Chebyshev modes need the TMA operator");
       PR_REQUIRE(dot == nullptr, PR_ERR_INTERNAL, "fused dot products need the TMA operator");
-      dim3 grid((res + TX - 1) / TX, (res + TY - 1) / TY, (res + kZChunk - 1) / kZChunk);
-      if (mode == kOpApply) k_op2<T, kOpApply><<<grid, kThreads, 0, s>>>(x, f, xp, out, v, (T)a, (T)b);
-      else if (mode == kOpResid) k_op2<T, kOpResid><<<grid, kThreads, 0, s>>>(x, f, xp, out, v, (T)a, (T)b);
-      else k_op2<T, kOpCheb><<<grid, kThreads, 0, s>>>(x, f, xp, out, v, (T)a, (T)b);
+      dim3 grid((res + TX - 1) / TX, (res + TY - 1) / TY, (res + kZChunk2 - 1) / kZChunk2);
+      if (mode == kOpApply) k_op2<T, kOpApply><<<grid, kThreads, 0, s>>>(x, f, xp, out, v, (T)a, (T)b, kZChunk2);
+      else if (mode == kOpResid) k_op2<T, kOpResid><<<grid, kThreads, 0, s>>>(x, f, xp, out, v, (T)a, (T)b, kZChunk2);
+      else k_op2<T, kOpCheb><<<grid, kThreads, 0, s>>>(x, f, xp, out, v, (T)a, (T)b, kZChunk2);
       PR_CHECK_LAUNCH();
     }
     // vectors moved (reads + writes)

@@ -46,3 +46,18 @@ def test_operator_on_device_vectors(ctx, depth, offset, precision):
     err = np.abs(y.double().cpu().numpy() - y_ref).max()
     # 21 products of at most max|A| max|x| each, rounded to 24 or 53 bits
     assert err <= (1e-13 if dtype == torch.float64 else 1e-5) * np.abs(y_ref).max()
+
+
+@pytest.mark.parametrize("precision", [prb.PR_PRECISION_FP64, prb.PR_PRECISION_MIXED])
+@pytest.mark.parametrize("depth", [5, 6, 7])
+def test_degree2_short_plane_runs(ctx, depth, precision):
+    """The levels up to 128^3 run in short runs of planes: the solution satisfies the oracle's equations
+    to the requested residual (1e-10, times ten for the two operators' own rounding)."""
+    pts = synthetic.torus(4000, seed=60 + depth)
+    st = ctx.solve(pts, prb.ReconstructParams(depth=depth, degree=2, point_weight=4.0, precision=precision,
+                                              target_rel_residual=1e-10))
+    assert st.converged == 1 and st.pcg_iterations <= 11, st
+    unit, _ = oracle.to_unit(pts)
+    t = oracle.Tree2(depth, unit, 4.0)
+    b = t.rhs()
+    assert np.linalg.norm(b - t.apply(ctx.coefficients())) <= 1e-9 * np.linalg.norm(b)
