@@ -33,6 +33,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdio>
+#include <cstdlib>
 #include <string>
 #include <vector>
 
@@ -385,7 +387,8 @@ struct Op3Args {
   int* err;
   double* dot;     // optional per-CTA partials: kOpApply x . out, kOpCheb f . out, kOpApplyD d . out
   int dot_base;    // index of this launch's first partial
-  T s1, s2;        // kOpApplyD: beta, alpha of the previous step
+  const double* s1;  // kOpApplyD: beta on the device (null: 0)
+  const double* s2;  // kOpApplyD: alpha of the previous step on the device (unless xmode is 0)
   T* out2;         // kOpApplyD: d
   T* xacc;         // kOpApplyD: the CG iterate
   int xmode;       // kOpApplyD: 0 leave xacc alone, 1 xacc = s2 dold (not read), 2 xacc += s2 dold
@@ -561,7 +564,8 @@ __global__ void __launch_bounds__(kThreads) k_op3(const __grid_constant__ CUtens
   V2 wa[NS], wb[NS], wc[NS], wo[NS];  // wo: kOpApplyD, the centres of dold
 #pragma unroll
   for (int k = 0; k < NS; ++k) wa[k] = wb[k] = wc[k] = wo[k] = V2{T(0), T(0)};
-  const V2 pbeta = p_bc<V2>(A.s1);
+  const V2 pbeta = p_bc<V2>(two && A.s1 ? (T)*A.s1 : T(0));
+  const V2 palpha = p_bc<V2>(two && A.xmode ? (T)*A.s2 : T(0));
   T* op = out + (int64_t)gx + (int64_t)res * gy + plane * (z0 - 4);  // output row of plane zo = z0 - 4 + it
   const bool want_dot = A.dot != nullptr;
   double dacc = 0.0;  // A.dot: this thread's share of the product
@@ -766,7 +770,7 @@ __global__ void __launch_bounds__(kThreads) k_op3(const __grid_constant__ CUtens
         *reinterpret_cast<V2*>(op) = res2;
         if (two) {
           *reinterpret_cast<V2*>(A.out2 + (op - out)) = wc[(k + 3) % NS];
-          if (A.xmode) *reinterpret_cast<V2*>(A.xacc + (op - out)) = p_fma(p_bc<V2>(A.s2), wo[(k + 3) % NS], xold);
+          if (A.xmode) *reinterpret_cast<V2*>(A.xacc + (op - out)) = p_fma(palpha, wo[(k + 3) % NS], xold);
         }
         if ((MODE == kOpApply || MODE == kOpApplyD) && want_dot) {
           const V2 cc = wc[(k + 3) % NS];
@@ -886,7 +890,8 @@ __global__ void __launch_bounds__(kThreadsR) k_op3r(const __grid_constant__ CUte
   for (int j = 0; j < RY; ++j)
 #pragma unroll
     for (int k = 0; k < NS; ++k) acc[j][k] = wc[j][k] = V2{T(0), T(0)};
-  const V2 pbeta = p_bc<V2>(A.s1);
+  const V2 pbeta = p_bc<V2>(two && A.s1 ? (T)*A.s1 : T(0));
+  const V2 palpha = p_bc<V2>(two && A.xmode ? (T)*A.s2 : T(0));
   T* op = out + (int64_t)gx + (int64_t)res * (y0 + ry) + plane * (z0 - 4);  // row ry of plane z0 - 4 + it
   const bool want_dot = A.dot != nullptr;
   double dacc = 0.0;
@@ -944,7 +949,7 @@ __global__ void __launch_bounds__(kThreadsR) k_op3r(const __grid_constant__ CUte
         }
         if (upd && (r == 2 || r == 3))  // centre columns 2p, 2p + 1 of dold
           *reinterpret_cast<V2*>(A.xacc + (op - out) + 2 * plane + (int64_t)(r - 2) * res) =
-              p_fma(p_bc<V2>(A.s2), v1, xold[r - 2]);
+              p_fma(palpha, v1, xold[r - 2]);
         if (two) {
           const T* zr = &s_z[k][ry + r][2 * p + XOFF];
           v0 = p_fma(pbeta, v0, *reinterpret_cast<const V2*>(zr));
@@ -1018,13 +1023,67 @@ __global__ void __launch_bounds__(kThreadsR) k_op3r(const __grid_constant__ CUte
   }
 }
 
-// one warp sums np partials in a fixed order
-__global__ void k_sum_parts(const double* __restrict__ part, int np, double* __restrict__ out) {
+// one warp sums np partials in a fixed order (lane 0 returns the sum); the loads run ahead of the
+// chain of additions
+__device__ __forceinline__ double warp_sum_parts(const double* __restrict__ part, int np) {
   double s = 0.0;
-  for (int i = threadIdx.x; i < np; i += 32) s += part[i];
+  int i = threadIdx.x & 31;
+  for (; i + 15 * 32 < np; i += 16 * 32) {
+    double v[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = part[i + 32 * k];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) s += v[k];
+  }
+  for (; i < np; i += 32) s += part[i];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  return s;
+}
+__global__ void k_sum_parts(const double* __restrict__ part, int np, double* __restrict__ out) {
+  const double s = warp_sum_parts(part, np);
   if (threadIdx.x == 0) out[0] = s;
+}
+
+// The scalars of preconditioned CG on the device: a dot product's sum updates them there, so that an
+// iteration runs without the host until its residual is known.
+struct Cg2 {
+  double alpha, beta, rz, tol, rr;
+  int act, broke, iters, maxit;
+};
+enum Cg2Step {
+  kCg2Rz0 = 0,  // sum = r.z of the first preconditioning
+  kCg2Rz = 1,   // sum = r.z: beta
+  kCg2Dq = 2,   // sum = d.A d: alpha, or the breakdown (alpha 0)
+  kCg2Rr = 3    // sum = r.r after the update: counts the iteration, decides whether it was the last
+};
+// sum of na partials of pa + w * (nb partials of pb), a warp each, then the step
+__global__ void __launch_bounds__(64) k_cg2_step(int step, const double* __restrict__ pa, int na,
+                                                 const double* __restrict__ pb, int nb, double w, Cg2* __restrict__ st) {
+  __shared__ double s_b;
+  const double s = threadIdx.x < 32 ? warp_sum_parts(pa, na) : warp_sum_parts(pb, nb);
+  if (threadIdx.x == 32) s_b = s;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  const double v = nb > 0 ? xadd(s, xmul(w, s_b)) : s;
+  const bool act = st->act != 0;
+  if (step == kCg2Rz0) {
+    st->rz = v;
+  } else if (step == kCg2Rz) {
+    st->beta = xdiv(v, st->rz);
+    st->rz = v;
+  } else if (step == kCg2Dq) {
+    const bool ok = act && v > 0.0 && st->rz > 0.0;
+    st->alpha = ok ? xdiv(st->rz, v) : 0.0;
+    if (act && !ok) {
+      st->broke = 1;
+      st->act = 0;
+    }
+  } else if (act) {
+    st->iters += 1;
+    st->rr = v;
+    if (!isfinite(v) || __dsqrt_rn(v) <= st->tol || st->iters >= st->maxit) st->act = 0;
+  }
 }
 
 // first Chebyshev step from x = 0: out = cb D^-1 f
@@ -1907,6 +1966,8 @@ struct System2 {
   Screen2<T> scr;
   double bytes = 0.0;         // algorithmic HBM bytes of the launched kernels
   int* err = nullptr;         // set by a TMA wait that ran out
+  std::string graph_base;     // vcycle_graph: what the V-cycle's launches depend on
+  bool plain_done = false;    // vcycle_graph: a V-cycle has run without a graph
 
   // levels D (finest) down to the dense 4^3 level; `multigrid` false: the finest level only
   void init(pr_context* ctx, uint32_t depth, double pw, bool multigrid) {
@@ -2094,7 +2155,7 @@ struct System2 {
   struct Fuse {
     T* out2 = nullptr;
     T* xacc = nullptr;
-    double s1 = 0.0, s2 = 0.0;
+    const double *s1 = nullptr, *s2 = nullptr;
     int xmode = 2;               // see Op3Args::xmode
     const float* e32 = nullptr;  // kOpRefine: the correction
     float* r32 = nullptr;        // kOpRefine: the residual in FP32
@@ -2134,8 +2195,8 @@ struct System2 {
                  "fused refinement without its operands");
       A.r32 = refine ? fu->r32 : nullptr;
       A.xzero = refine && fu->xzero ? 1 : 0;
-      A.s1 = two ? (T)fu->s1 : T(0);
-      A.s2 = two ? (T)fu->s2 : T(0);
+      A.s1 = two ? fu->s1 : nullptr;
+      A.s2 = two ? fu->s2 : nullptr;
       A.out2 = (two || refine) ? fu->out2 : nullptr;
       A.xacc = two ? fu->xacc : nullptr;
       A.xmode = two ? fu->xmode : 0;
@@ -2248,6 +2309,47 @@ struct System2 {
   }
 };
 
+// X = V(f) on the finest level: from the second use of the same buffers on, the V-cycle's launches
+// (9 per level) are replayed from a CUDA graph kept by the context
+template <typename T>
+void vcycle_graph(pr_context* c, System2<T>& sys, const T* f, T* X) {
+  const char* gr = std::getenv("PR_GRAPHS");
+  if (sys.lv.size() < 2 || (gr && std::atoi(gr) == 0)) {
+    sys.vcycle(0, f, X);
+    return;
+  }
+  if (sys.graph_base.empty()) {
+    char b[64];
+    std::snprintf(b, sizeof(b), "d2v/%s/%u/%a", tn2<T>(), sys.D, sys.lv[0].wg);
+    sys.graph_base = b;
+    auto add = [&](const void* p) {
+      std::snprintf(b, sizeof(b), "/%p", p);
+      sys.graph_base += b;
+    };
+    for (const auto& q : sys.lv)
+      for (const void* p : {(const void*)q.tM, (const void*)q.tS, (const void*)q.f, (const void*)q.x, (const void*)q.y}) add(p);
+    add(sys.inv);
+    add(sys.err);
+  }
+  char b[96];
+  std::snprintf(b, sizeof(b), "/%p/%p/%p", (const void*)f, (const void*)X, (const void*)sys.rz_parts);
+  const std::string key = sys.graph_base + b;
+  if (!sys.plain_done && !c->graphs.count(key)) {
+    sys.vcycle(0, f, X);
+    sys.plain_done = true;
+    return;
+  }
+  const double before = sys.bytes;
+  pr_context::Graph& g = c->run_graph(key, [&] { sys.vcycle(0, f, X); });
+  if (sys.bytes != before) {  // captured now: what the launches move and how many partials they leave
+    g.bytes = sys.bytes - before;
+    g.parts = sys.rz_np;
+  } else {
+    sys.bytes += g.bytes;
+    sys.rz_np = g.parts;
+  }
+}
+
 // preconditioned CG on the finest level from x = 0 to ||r|| <= tol_abs; r holds b on entry and is
 // overwritten with the recursively updated residual; rr0 = r . r on entry when the caller knows it
 // (else negative).  On the TMA operator (res >= 64) the vector
@@ -2277,7 +2379,7 @@ int pcg2(pr_context* c, System2<T>& sys, T* r, T* x, double tol_abs, int maxit, 
   }
   int it = 0;
   if (!fused) {
-    sys.vcycle(0, r, z);
+    vcycle_graph(c, sys, r, z);
     double rz = dot<T>(c, r, z, n);
     spd_check(c, "degree-2 coarsest operator");
     PR_CUDA(cudaMemcpyAsync(d, z, n * sizeof(T), cudaMemcpyDeviceToDevice, s));
@@ -2293,7 +2395,7 @@ int pcg2(pr_context* c, System2<T>& sys, T* r, T* x, double tol_abs, int maxit, 
       sys.bytes += 6.0 * n * sizeof(T);
       ++it;
       if (!std::isfinite(rr) || std::sqrt(rr) <= tol_abs) break;
-      sys.vcycle(0, r, z);
+      vcycle_graph(c, sys, r, z);
       const double rz_new = dot<T>(c, r, z, n);
       const double beta = rz_new / rz;
       rz = rz_new;
@@ -2304,56 +2406,65 @@ int pcg2(pr_context* c, System2<T>& sys, T* r, T* x, double tol_abs, int maxit, 
   }
   sys.alloc_parts();
   T* d2 = c->buf<T>("d2cg_d2_" + tn, n);
+  double* rparts = c->buf<double>("dot_part", kDotBlocks);
+  Cg2* st = c->buf<Cg2>("d2cg_scalars", 1);
+  Cg2* h = reinterpret_cast<Cg2*>(c->h_scalars);  // pinned copy of the scalars
+  static_assert(sizeof(Cg2) <= 64 * sizeof(double), "the scalars fit the pinned staging");
+  Cg2 init{};
+  init.tol = tol_abs;
+  init.rr = rr;
+  init.act = maxit > 0 ? 1 : 0;
+  init.maxit = maxit;
+  c->upload(st, &init, sizeof(init));
+  if (maxit <= 0) {
+    PR_CUDA(cudaMemsetAsync(x, 0, n * sizeof(T), s));
+    return 0;
+  }
+  auto step = [&](Cg2Step k, const double* pa, int na, int nb, double w) {
+    k_cg2_step<<<1, 64, 0, s>>>(k, pa, na, sys.parts_b, nb, w, st);
+    PR_CHECK_LAUNCH();
+  };
   T* dcur = d;
   T* dalt = d2;
-  const T* dprev = nullptr;
-  // z = M r, r . z
-  auto precondition = [&]() {
+  // one iteration: z = M r, r . z; d = z + beta dprev (d = z at first), q = A d (+ screening), d . q,
+  // x += alpha dprev (the previous step's, pending until here); r -= alpha q with r . r.  The host
+  // reads the scalars after that, once, so that convergence is known before the next V-cycle.
+  for (int k = 0;; ++k) {
+    const T* dprev = k > 0 ? dalt : nullptr;
     sys.rz_parts = sys.parts_a;
     sys.rz_np = 0;
-    sys.vcycle(0, r, z);
+    vcycle_graph(c, sys, r, z);
     sys.rz_parts = nullptr;
     PR_REQUIRE(sys.rz_np > 0, PR_ERR_INTERNAL, "fused r.z was not produced");
-    return sys.sum_parts(sys.rz_np, 0, 0.0);
-  };
-  double rz = precondition();
-  spd_check(c, "degree-2 coarsest operator");
-  double alpha = 0.0, alpha_prev = 0.0, beta = 0.0;
-  bool pending = false;  // x += alpha dcur not applied yet
-  bool x_def = false;    // x written (until then it is zero and never read)
-  while (it < maxit) {
-    // d = z + beta dprev (d = z at first), q = A d (+ screening), d . q, x += alpha_prev dprev
+    step(k == 0 ? kCg2Rz0 : kCg2Rz, sys.parts_a, sys.rz_np, 0, 0.0);
     typename System2<T>::Fuse fu;
     fu.out2 = dcur;
     fu.xacc = x;
-    fu.s1 = dprev ? beta : 0.0;
-    fu.s2 = dprev ? alpha_prev : 0.0;
-    fu.xmode = dprev ? (x_def ? 2 : 1) : 0;
+    fu.s1 = dprev ? &st->beta : nullptr;
+    fu.s2 = &st->alpha;
+    fu.xmode = std::min(k, 2);  // x is written by the second pass (x = alpha d, not read), then added to
     const int na = sys.op(0, kOpApplyD, dprev ? dprev : z, z, nullptr, q, 0.0, 0.0, -1, 0.0, sys.parts_a, &fu);
-    if (dprev) x_def = true;
-    pending = false;
     const int nb = sys.screen(dcur, q, +1, sys.parts_b);
-    const double dq = sys.sum_parts(na, nb, sys.scr.wh3);
-    if (!(dq > 0.0) || !(rz > 0.0)) break;
-    alpha = rz / dq;
-    pending = true;
-    ++it;
-    rr = r_update<T>(c, n, alpha, q, r);
+    step(kCg2Dq, sys.parts_a, na, nb, sys.scr.wh3);
+    r_update_dev<T>(s, n, &st->alpha, q, r, rparts);
+    step(kCg2Rr, rparts, kDotBlocks, 0, 0.0);
     sys.bytes += 3.0 * n * sizeof(T);
-    if (!std::isfinite(rr) || std::sqrt(rr) <= tol_abs) break;
-    const double rz_new = precondition();
-    beta = rz_new / rz;
-    rz = rz_new;
-    alpha_prev = alpha;
-    dprev = dcur;
+    PR_CUDA(cudaMemcpyAsync(h, st, sizeof(Cg2), cudaMemcpyDeviceToHost, s));
+    c->sync();
+    if (k == 0) spd_check(c, "degree-2 coarsest operator");
+    if (!h->act) break;
     std::swap(dcur, dalt);
   }
-  if (pending && x_def) {
-    axpy<T, T>(s, n, alpha, dcur, x);
-    sys.bytes += 3.0 * n * sizeof(T);
-  } else if (pending) {
-    scale_convert<T, T>(s, n, alpha, dcur, x);
-    sys.bytes += 2.0 * n * sizeof(T);
+  it = h->iters;
+  const bool x_def = it + h->broke >= 2;  // a second direction pass has run
+  if (h->broke == 0) {                    // x += alpha d of the last step
+    if (x_def) {
+      axpy<T, T>(s, n, h->alpha, dcur, x);
+      sys.bytes += 3.0 * n * sizeof(T);
+    } else {
+      scale_convert<T, T>(s, n, h->alpha, dcur, x);
+      sys.bytes += 2.0 * n * sizeof(T);
+    }
   } else if (!x_def) {
     PR_CUDA(cudaMemsetAsync(x, 0, n * sizeof(T), s));
   }
@@ -2664,8 +2775,11 @@ double bench2(pr_context* c, int kid, uint32_t D, int reps, double* bytes) {
   if (kid == 10) {
     fu.out2 = p;
     fu.xacc = xa;
-    fu.s1 = 0.3;
-    fu.s2 = 0.2;
+    const double ab[2] = {0.3, 0.2};
+    double* dab = c->buf<double>("kb_ab", 2);
+    c->upload(dab, ab, sizeof(ab));
+    fu.s1 = dab;
+    fu.s2 = dab + 1;
     fu.xmode = 2;
   } else if (kid == 11) {
     fu.out2 = xa;

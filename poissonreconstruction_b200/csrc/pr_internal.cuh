@@ -231,11 +231,13 @@ struct pr_context {
   struct Graph {
     cudaGraphExec_t exec = nullptr;
     uint64_t launches = 0, primitives = 0;
+    double bytes = 0.0;  // noted by the capturing caller: algorithmic bytes of the launches
+    int parts = 0;       // and the partial sums that they leave
   };
   std::map<std::string, Graph> graphs;
   // Runs body() through the graph of `key`, capturing it on first use.
   template <typename F>
-  void run_graph(const std::string& key, F body) {
+  Graph& run_graph(const std::string& key, F body) {
     auto it = graphs.find(key);
     if (it == graphs.end()) {
       if (graphs.size() >= 64) {  // keyed by buffers that were replaced since, most likely
@@ -263,12 +265,12 @@ struct pr_context {
       gr.launches = l1 - l0;
       gr.primitives = p1 - p0;
       PR_CUDA(cudaGraphLaunch(gr.exec, stream));  // counted by the capture
-      graphs.emplace(key, gr);
-      return;
+      return graphs.emplace(key, gr).first->second;
     }
     PR_CUDA(cudaGraphLaunch(it->second.exec, stream));
     for (uint64_t k = 0; k < it->second.launches; ++k) pr::pr_count_launch_(0);
     for (uint64_t k = 0; k < it->second.primitives; ++k) pr::pr_count_launch_(1);
+    return it->second;
   }
 
   template <typename T>

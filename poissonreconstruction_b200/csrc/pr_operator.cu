@@ -241,8 +241,9 @@ __global__ void k_cg_update4(uint64_t n, T alpha, const T* __restrict__ d, const
 
 // r -= alpha q with per-block sums of r^2 (the CG residual update when x is updated elsewhere)
 template <typename T>
-__global__ void k_r_update4(uint64_t n, T alpha, const T* __restrict__ q, T* __restrict__ r,
-                            double* __restrict__ part) {
+__global__ void k_r_update4(uint64_t n, const double* __restrict__ alpha_dev, const T* __restrict__ q,
+                            T* __restrict__ r, double* __restrict__ part) {
+  const T alpha = (T)*alpha_dev;
   double s = 0.0;
   const uint64_t n4 = n / 4, stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n4; i += stride) {
@@ -250,13 +251,13 @@ __global__ void k_r_update4(uint64_t n, T alpha, const T* __restrict__ q, T* __r
     Q4<T> rv = ld4(r, i);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      rv.v[k] = rv.v[k] - alpha * qv.v[k];
+      if (alpha != (T)0) rv.v[k] = rv.v[k] - alpha * qv.v[k];
       s += (double)rv.v[k] * (double)rv.v[k];
     }
     st4(r, i, rv);
   }
   for (uint64_t i = 4 * n4 + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-    const T ri = r[i] - alpha * q[i];
+    const T ri = alpha != (T)0 ? r[i] - alpha * q[i] : r[i];
     r[i] = ri;
     s += (double)ri * (double)ri;
   }
@@ -681,17 +682,10 @@ double cg_update(pr_context* c, uint64_t n, double alpha, const T* d, const T* q
 }
 
 template <typename T>
-double r_update(pr_context* c, uint64_t n, double alpha, const T* q, T* r) {
-  PR_REQUIRE(aligned16(q) && aligned16(r), PR_ERR_INTERNAL, "r_update needs 16-byte aligned vectors");
-  double* part = c->buf<double>("dot_part", kDotBlocks);
-  double* out = c->buf<double>("dot_out", 1);
-  k_r_update4<T><<<kDotBlocks, kThreads, 0, c->stream>>>(n, (T)alpha, q, r, part);
+void r_update_dev(cudaStream_t s, uint64_t n, const double* alpha, const T* q, T* r, double* part) {
+  PR_REQUIRE(aligned16(q) && aligned16(r), PR_ERR_INTERNAL, "r_update_dev needs 16-byte aligned vectors");
+  k_r_update4<T><<<kDotBlocks, kThreads, 0, s>>>(n, alpha, q, r, part);
   PR_CHECK_LAUNCH();
-  k_sum_final<<<1, 32, 0, c->stream>>>(part, kDotBlocks, out);
-  PR_CHECK_LAUNCH();
-  PR_CUDA(cudaMemcpyAsync(c->h_scalars, out, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  c->sync();
-  return c->h_scalars[0];
 }
 
 double convert_norm(pr_context* c, const double* x, float* y, uint64_t n) {
@@ -790,7 +784,7 @@ void spd_check(pr_context* c, const char* what) {
   template void screen_gather<T>(cudaStream_t, const Screen<T>&, T*, int);                            \
   template double dot<T>(pr_context*, const T*, const T*, uint64_t);                                  \
   template double cg_update<T>(pr_context*, uint64_t, double, const T*, const T*, T*, T*);            \
-  template double r_update<T>(pr_context*, uint64_t, double, const T*, T*);                           \
+  template void r_update_dev<T>(cudaStream_t, uint64_t, const double*, const T*, T*, double*);                             \
   template void xpby<T>(cudaStream_t, uint64_t, const T*, double, T*);                                \
   template void gs_sweep<T>(cudaStream_t, uint32_t, T*, const T*, Coef<T>, bool);                     \
   template void restrict_to_coarse<T>(cudaStream_t, uint32_t, const T*, T*);                          \
