@@ -553,12 +553,12 @@ __global__ void __launch_bounds__(1024) k_cg_step(int step, const double* __rest
 
 // ------------------------------------------------------------------ helpers of the 16^3 block kernels
 namespace s16 {
-constexpr int CW = 10;  // coarse tile width
-
 // spread the 4 low bits of v to bit positions 0,3,6,9
 __device__ __forceinline__ uint32_t sp4(uint32_t v) {
   return (v & 1u) | ((v & 2u) << 2) | ((v & 4u) << 4) | ((v & 8u) << 6);
 }
+// spread the 3 low bits of v to bit positions 0,2,4
+__device__ __forceinline__ uint32_t sp2(uint32_t v) { return (v & 1u) | ((v & 2u) << 1) | ((v & 4u) << 2); }
 template <typename T>
 struct Vec4;
 template <>
@@ -581,88 +581,6 @@ __device__ __forceinline__ void st4(double* p, const double4& v) {
   reinterpret_cast<double2*>(p)[1] = make_double2(v.z, v.w);
 }
 
-// local coordinates of element 4q of a 16^3 Morton block (q = quad index), x0 = y0 = 0
-__device__ __forceinline__ void quad_coords(int q, int& lx, int& ly, int& lz) {
-  lx = ((q >> 1) & 1) << 1 | ((q >> 4) & 1) << 2 | ((q >> 7) & 1) << 3;
-  ly = ((q >> 2) & 1) << 1 | ((q >> 5) & 1) << 2 | ((q >> 8) & 1) << 3;
-  lz = (q & 1) | ((q >> 3) & 1) << 1 | ((q >> 6) & 1) << 2 | ((q >> 9) & 1) << 3;
-}
-
-// Load the one-node halo of the block into a tile (idx: tile index of tile coordinates).
-// nb[27]: Morton base of the neighbour block (dx+1)+3(dy+1)+9(dz+1), or ~0u if outside.
-// NT: threads of the CTA.
-template <int NT, typename T, typename Idx, typename Xf>
-__device__ __forceinline__ void load_halo(T* tile, const T* __restrict__ x, const uint32_t* nb, Idx idx, Xf xf) {
-#pragma unroll
-  for (int i = threadIdx.x; i < 256; i += NT) {  // faces: (a, b) = in-face coordinates of position i
-    const int a = i & 15, b = i >> 4;
-    const uint32_t sa = sp4(a), sb = sp4(b);
-#pragma unroll
-    for (int f = 0; f < 6; ++f) {
-      const int axis = f >> 1, hi = f & 1;
-      const int nbi = axis == 0 ? (hi ? 14 : 12) : (axis == 1 ? (hi ? 16 : 10) : (hi ? 22 : 4));
-      const uint32_t side = hi ? 0u : 0x249u;  // neighbour-local coordinate 0 or 15, spread
-      uint32_t m;
-      int ux, uy, uz;
-      const int s = hi ? 17 : 0;
-      if (axis == 0) { m = side | (sa << 1) | (sb << 2); ux = s; uy = a + 1; uz = b + 1; }
-      else if (axis == 1) { m = sa | (side << 1) | (sb << 2); ux = a + 1; uy = s; uz = b + 1; }
-      else { m = sa | (sb << 1) | (side << 2); ux = a + 1; uy = b + 1; uz = s; }
-      const uint32_t base = nb[nbi];
-      tile[idx(ux, uy, uz)] = base != ~0u ? xf(base + m) : (T)0;
-    }
-  }
-#pragma unroll
-  for (int i = threadIdx.x; i < 200; i += NT) {
-    if (i >= 192) {  // corners
-      const int c = i - 192;
-      const int sx = c & 1, sy = (c >> 1) & 1, sz = (c >> 2) & 1;
-      const uint32_t m = (sx ? 0u : 0x249u) | ((sy ? 0u : 0x249u) << 1) | ((sz ? 0u : 0x249u) << 2);
-      const int nbi = (sx ? 2 : 0) + 3 * (sy ? 2 : 0) + 9 * (sz ? 2 : 0);
-      const uint32_t base = nb[nbi];
-      tile[idx(sx ? 17 : 0, sy ? 17 : 0, sz ? 17 : 0)] = base != ~0u ? xf(base + m) : (T)0;
-      continue;
-    }
-    // edges: 4 per axis, 16 nodes each
-    const int e = i >> 4, a = i & 15, axis = e >> 2, s1 = e & 1, s2 = (e >> 1) & 1;
-    const uint32_t sa = sp4(a);
-    const uint32_t c1 = s1 ? 0u : 0x249u, c2 = s2 ? 0u : 0x249u;
-    const int d1 = s1 ? 1 : -1, d2 = s2 ? 1 : -1;
-    const int u1 = s1 ? 17 : 0, u2 = s2 ? 17 : 0;
-    uint32_t m;
-    int ux, uy, uz, nbi;
-    if (axis == 0) { m = sa | (c1 << 1) | (c2 << 2); ux = a + 1; uy = u1; uz = u2; nbi = 1 + 3 * (d1 + 1) + 9 * (d2 + 1); }
-    else if (axis == 1) { m = c1 | (sa << 1) | (c2 << 2); ux = u1; uy = a + 1; uz = u2; nbi = (d1 + 1) + 3 + 9 * (d2 + 1); }
-    else { m = c1 | (c2 << 1) | (sa << 2); ux = u1; uy = u2; uz = a + 1; nbi = (d1 + 1) + 3 * (d2 + 1) + 9; }
-    const uint32_t base = nb[nbi];
-    tile[idx(ux, uy, uz)] = base != ~0u ? xf(base + m) : (T)0;
-  }
-}
-
-// The sum over a 16^3 block of one value per (quad column q, plane z), in an order fixed by the
-// block whatever the launch shape: each column's planes in z order, then the 64 column sums by a
-// fixed tree.  red: 1024 doubles of shared memory holding the value of (q, z) at [z 64 + q] (the
-// caller writes it after a barrier that ends every other use of that memory).  Every thread calls
-// this (it has barriers); thread 0 returns the sum.
-__device__ __forceinline__ double block_sum_fixed(double* red) {
-  __syncthreads();
-  const int t = threadIdx.x;
-  double s = 0.0;
-  if (t < 64) {
-#pragma unroll
-    for (int z = 0; z < 16; ++z) s += red[z * 64 + t];
-  }
-  __syncthreads();
-  if (t < 64) red[t] = s;
-  __syncthreads();
-  if (t < 32) {
-    s = red[t] + red[t + 32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  }
-  return s;
-}
-
 __device__ __forceinline__ void neighbour_bases(uint32_t* nb, uint32_t bx, uint32_t by, uint32_t bz, int nblk_axis) {
   const int t = threadIdx.x;
   if (t < 27) {
@@ -674,128 +592,10 @@ __device__ __forceinline__ void neighbour_bases(uint32_t* nb, uint32_t bx, uint3
   }
 }
 
-// Coarse tile for the prolongation: coarse block (8^3, Morton-contiguous) with a one-node
-// halo, natural layout 10^3, coordinate = coarse local + 1.  Ends with a barrier.
-template <int NT, typename T>
-__device__ __forceinline__ void load_coarse_tile(T* ctile, const T* __restrict__ ec, uint32_t blk, uint32_t bx,
-                                                 uint32_t by, uint32_t bz, int nblk_axis, uint32_t* cnb) {
-  const int t = threadIdx.x;
-  // interior: 512 contiguous coarse values
-  for (int i = t; i < 512; i += NT) {
-    uint32_t cx, cy, cz;
-    unmorton3((uint32_t)i, cx, cy, cz);
-    ctile[((cz + 1) * CW + (cy + 1)) * CW + (cx + 1)] = __ldg(ec + (uint64_t)blk * 512 + i);
-  }
-  // halo (488 positions): faces of 8x8 from the neighbour coarse blocks, then edges, corners
-  if (t < 27) {
-    const int dx = t % 3 - 1, dy = (t / 3) % 3 - 1, dz = t / 9 - 1;
-    const int x = (int)bx + dx, y = (int)by + dy, z = (int)bz + dz;
-    cnb[t] = (x < 0 || y < 0 || z < 0 || x >= nblk_axis || y >= nblk_axis || z >= nblk_axis)
-                 ? ~0u
-                 : (morton3((uint32_t)x, (uint32_t)y, (uint32_t)z) << 9);
-  }
-  __syncthreads();
-  auto sp3 = [](uint32_t v) { return (v & 1u) | ((v & 2u) << 2) | ((v & 4u) << 4); };
-  for (int i = t; i < 488; i += NT) {
-    int ux, uy, uz;
-    uint32_t mloc;
-    int nbi;
-    if (i < 384) {  // faces: 6 x 64
-      const int f = i >> 6, a = i & 7, b = (i >> 3) & 7, axis = f >> 1, hi = f & 1;
-      const uint32_t side = hi ? 0u : 0x49u;  // local 0 or 7, spread
-      const int s = hi ? 9 : 0;
-      if (axis == 0) { mloc = side | (sp3(a) << 1) | (sp3(b) << 2); ux = s; uy = a + 1; uz = b + 1; nbi = (hi ? 2 : 0) + 3 + 9; }
-      else if (axis == 1) { mloc = sp3(a) | (side << 1) | (sp3(b) << 2); ux = a + 1; uy = s; uz = b + 1; nbi = 1 + 3 * (hi ? 2 : 0) + 9; }
-      else { mloc = sp3(a) | (sp3(b) << 1) | (side << 2); ux = a + 1; uy = b + 1; uz = s; nbi = 1 + 3 + 9 * (hi ? 2 : 0); }
-    } else if (i < 480) {  // edges: 12 x 8
-      const int e = (i - 384) >> 3, a = (i - 384) & 7, axis = e >> 2, s1 = e & 1, s2 = (e >> 1) & 1;
-      const uint32_t c1 = s1 ? 0u : 0x49u, c2 = s2 ? 0u : 0x49u;
-      const int u1 = s1 ? 9 : 0, u2 = s2 ? 9 : 0, d1 = s1 ? 2 : 0, d2 = s2 ? 2 : 0;
-      if (axis == 0) { mloc = sp3(a) | (c1 << 1) | (c2 << 2); ux = a + 1; uy = u1; uz = u2; nbi = 1 + 3 * d1 + 9 * d2; }
-      else if (axis == 1) { mloc = c1 | (sp3(a) << 1) | (c2 << 2); ux = u1; uy = a + 1; uz = u2; nbi = d1 + 3 + 9 * d2; }
-      else { mloc = c1 | (c2 << 1) | (sp3(a) << 2); ux = u1; uy = u2; uz = a + 1; nbi = d1 + 3 * d2 + 9; }
-    } else {  // corners
-      const int c = i - 480, sx = c & 1, sy = (c >> 1) & 1, sz = (c >> 2) & 1;
-      mloc = (sx ? 0u : 0x49u) | ((sy ? 0u : 0x49u) << 1) | ((sz ? 0u : 0x49u) << 2);
-      ux = sx ? 9 : 0; uy = sy ? 9 : 0; uz = sz ? 9 : 0;
-      nbi = (sx ? 2 : 0) + 3 * (sy ? 2 : 0) + 9 * (sz ? 2 : 0);
-    }
-    const uint32_t b0 = cnb[nbi];
-    ctile[(uz * CW + uy) * CW + ux] = b0 != ~0u ? __ldg(ec + b0 + mloc) : (T)0;
-  }
-  __syncthreads();  // the caller reads halo entries written by other threads
-}
-
-// P ec at fine tile coordinate (ux,uy,uz) (fine local + 1); ctile coordinate = coarse local + 1.
-// Even fine local coordinate l -> coarse l/2 (w 1); odd -> (l-1)/2, (l+1)/2 (w 1/2 each).
-template <typename T>
-__device__ __forceinline__ T prolong_at(const T* ctile, int ux, int uy, int uz) {
-  const int lx = ux - 1, ly = uy - 1, lz = uz - 1;
-  const int ax = (lx >> 1) + 1, ay = (ly >> 1) + 1, az = (lz >> 1) + 1;  // floor(l/2) + 1
-  const int ox = lx & 1, oy = ly & 1, oz = lz & 1;
-  const T* c = ctile + (az * CW + ay) * CW + ax;
-  // the +1 neighbours exist (index <= CW-1) exactly when the coordinate is odd
-  T v00 = c[0];
-  T v01 = oy ? c[CW] : (T)0;
-  T v10 = oz ? c[CW * CW] : (T)0;
-  T v11 = (oy && oz) ? c[CW * CW + CW] : (T)0;
-  if (ox) {
-    v00 = (T)0.5 * (v00 + c[1]);
-    if (oy) v01 = (T)0.5 * (v01 + c[CW + 1]);
-    if (oz) v10 = (T)0.5 * (v10 + c[CW * CW + 1]);
-    if (oy && oz) v11 = (T)0.5 * (v11 + c[CW * CW + CW + 1]);
-  }
-  const T y0 = oy ? (T)0.5 * (v00 + v01) : v00;
-  const T y1 = oy ? (T)0.5 * (v10 + v11) : v10;
-  return oz ? (T)0.5 * (y0 + y1) : y0;
-}
-
 }  // namespace s16
 
-// ------------------------------------------------------------------ 16^3 stencil SpMV (finest level)
-// 256 threads: thread = one 2x2 (x, y) quad column over 4 z planes (64 quads x 4 z segments).
-// Natural tile with a one-node halo; local x sits at offset x + 1 so that the pairs (x0-1, x0)
-// and (x0+1, x0+2) a quad's row needs are 8-byte (FP32) / 16-byte (FP64) aligned, and the row
-// stride of 24 puts the two quad rows of a half-warp on disjoint banks.  The planes are swept
-// in z once: each plane's in-plane sums go to the output row of the plane itself (centre,
-// in-plane edges) and to the rows above and below (edges and corners), so a thread keeps two
-// accumulators per node instead of three planes of sums.
+// ------------------------------------------------------------------ 16^3 stencil rows
 namespace n16 {
-// ZT: z planes per thread (2, 4 or 8); the CTA has 1024 / ZT threads (64 quad columns x 16 / ZT
-// z segments).  The arithmetic of a node, and every per-block sum, is the same for every ZT.
-constexpr int N = 4096;
-template <int ZT>
-struct Zt {
-  static constexpr int NT = 1024 / ZT;
-};
-constexpr int RS = 24, PS = 18 * RS + 4, TILE = 18 * PS;
-__device__ __forceinline__ int nat(int ux, int uy, int uz) { return uz * PS + uy * RS + ux; }  // u = local + 1
-
-template <typename T>
-struct Pair;
-template <>
-struct Pair<float> {
-  typedef float2 type;
-};
-template <>
-struct Pair<double> {
-  typedef double2 type;
-};
-
-// the 4 x 4 patch (rows y0-1..y0+2, columns x0-1..x0+2) of tile plane uz around quad (x0, y0)
-template <typename T, int RSX>
-__device__ __forceinline__ void patch(const T* tile, int off, T r[4][4]) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const typename Pair<T>::type l = *reinterpret_cast<const typename Pair<T>::type*>(tile + off + j * RSX);
-    const typename Pair<T>::type h = *reinterpret_cast<const typename Pair<T>::type*>(tile + off + j * RSX + 2);
-    r[j][0] = l.x;
-    r[j][1] = l.y;
-    r[j][2] = h.x;
-    r[j][3] = h.y;
-  }
-}
-
 // in-plane sums of the quad's 4 nodes: tz = ce*faces + cc*diagonals (for the rows z-1, z+1),
 // own = c0*centre + ce*diagonals (for row z)
 template <typename T>
@@ -827,17 +627,468 @@ __device__ __forceinline__ void plane_sums(const T r[4][4], T f[4], T d[4], T ct
     }
 }
 
+}  // namespace n16
+
+// ------------------------------------------------------------------ the z-run tile of the 16^3 block kernels
+// A 16^3 block with its one-node halo.  Column (x, y), x and y in -1..16, holds its 8 even planes, then
+// its 8 odd ones, in consecutive words; the halo planes z = -1 and 16 are two small planes of their own.
+// Thread = one 2x2 (x, y) quad column over ZT planes of one parity (ZT = 2 or 4), one 8- or 16-byte
+// access of a column; the 16 / ZT segments of a quad column sit on neighbouring lanes, and the in-plane
+// sums of the planes below and above come from those lanes by shuffle: only the block's first and last
+// plane read the halo planes.  The parity is the lowest lane bit and the quads follow in Morton order, so
+// that for each of its planes a warp loads (and stores) whole 128-byte lines, four 16-byte quads of two
+// planes each.  (Segments of consecutive planes touched four times the lines, a quarter of each, and the
+// L1's look-ups bounded the kernel; one 32-byte load per lane and two planes, one sector a cycle, too.)
+// Bank conflicts: eight lanes of a 16-byte column access (ZT = 4: four segments of two quads 48 words
+// apart) fill the 32 banks once; the halo planes' rows are 20 words and the planes 368 words apart, which
+// puts the 16 lanes of a halo access on the 16 even banks.
+// What bounds the kernels is the L1's data pipe (84% busy in the post-smoothing sweep: its own columns,
+// 5 neighbouring ones per phase, shuffles, and the halo's sectors).  At depth 9 in FP32, against the
+// plane-by-plane tile with one quad per lane and plane before: post-smoothing 753 -> 537 us (floor by
+// HBM bytes 260), CG update and pre-smoothing 750 -> 556 (583), residual and restriction 560 -> 482
+// (177), first sweep 277 -> 184 (167), plain SpMV 338 -> 311 (167), with d = z + beta d 454 -> 462 (333).
+// Every value and every sum is the same for every ZT.
+namespace z16 {
+constexpr int kCS = 24, kRY = 18 * kCS + 4, kHR = 20, kHP = 368, TILE = 18 * kRY + 2 * kHP;
+// word of column (x, y); of plane z in it
+__device__ __forceinline__ int at(int x, int y) { return (y + 1) * kRY + (x + 1) * kCS; }
+__device__ __forceinline__ int zw(int z) { return ((z & 1) << 3) | (z >> 1); }
+// word of (x, y) on the halo plane z = -1 (hi 0) or 16 (hi 1)
+__device__ __forceinline__ int halo_at(int hi, int x, int y) { return 18 * kRY + hi * kHP + (y + 1) * kHR + x + 1; }
+// node (x, y) of plane z, -1..16, with its strides in x and y
+template <typename T>
+struct PlaneRef {
+  const T* p;
+  int sx, sy;
+  __device__ __forceinline__ T operator()(int dx, int dy) const { return p[dx * sx + dy * sy]; }
+};
+template <typename T>
+__device__ __forceinline__ PlaneRef<T> plane_ref(const T* tile, int x, int y, int z) {
+  if (z < 0 || z > 15) return {tile + halo_at(z > 15, x, y), 1, kHR};
+  return {tile + at(x, y) + zw(z), kCS, kRY};
+}
+// quad coordinates of quad qm (Morton order)
+__device__ __forceinline__ void quad_of(int qm, int& qx, int& qy) {
+  qx = (qm & 1) | ((qm >> 1) & 2) | ((qm >> 2) & 4);
+  qy = ((qm >> 1) & 1) | ((qm >> 2) & 2) | ((qm >> 3) & 4);
+}
+template <typename T>
+__device__ __forceinline__ void ld4q(const T* p, T (&o)[4]) {
+  const typename s16::Vec4<T>::type v = s16::ld4(p);
+  o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+}
+template <typename T>
+__device__ __forceinline__ void st4q(T* p, const T (&o)[4]) {
+  typename s16::Vec4<T>::type v;
+  v.x = o[0]; v.y = o[1]; v.z = o[2]; v.w = o[3];
+  s16::st4(p, v);
+}
+template <int ZT>
+struct Zt {
+  static constexpr int SEG = 16 / ZT;       // z segments of a column
+  static constexpr int NT = 64 * SEG;       // threads
+  static constexpr int NSIDE = 36 * SEG;    // halo quad columns beside the block, a segment per thread
+  static constexpr int NZF = NT - NSIDE;    // the other threads take the 2 x 100 quads of the z halo planes
+  static constexpr int ZN = (200 + NZF - 1) / NZF;
+  static constexpr int HV = ZT > ZN ? ZT : ZN;
+};
+// a segment: its parity, first plane, first word in a column, and place among the column's segments
+template <int ZT>
+struct Seg {
+  int p, z0, w0, s;
+  __device__ __forceinline__ explicit Seg(int lane) {
+    s = lane % Zt<ZT>::SEG;
+    p = s & 1;
+    z0 = 2 * ZT * (s >> 1) + p;
+    w0 = 8 * p + ZT * (s >> 1);
+  }
+  __device__ __forceinline__ int z(int k) const { return z0 + 2 * k; }
+  __device__ __forceinline__ bool first() const { return s == 0; }                // holds plane 0 (k = 0)
+  __device__ __forceinline__ bool last() const { return s == Zt<ZT>::SEG - 1; }  // holds plane 15 (k = ZT - 1)
+};
+// Values of the planes next to the segment's: y[k] those of plane z(k) + 1 (parity 0) or - 1 (parity 1),
+// o[k] those of the other side; end: what lies beyond the block for its first and last plane.  Every lane
+// of the warp takes part.
+template <int ZT, typename T>
+__device__ __forceinline__ void beside(const Seg<ZT>& g, const T (&x)[ZT], T end, T (&y)[ZT], T (&o)[ZT]) {
+#pragma unroll
+  for (int k = 0; k < ZT; ++k) y[k] = __shfl_xor_sync(0xffffffffu, x[k], 1);
+  const int lane = threadIdx.x & 31;
+  T w = __shfl_sync(0xffffffffu, g.p ? x[ZT - 1] : x[0], g.p ? lane + 1 : lane - 1);
+  if (g.first() || g.last()) w = end;
+#pragma unroll
+  for (int k = 0; k < ZT; ++k) o[k] = g.p ? (k < ZT - 1 ? y[k < ZT - 1 ? k + 1 : k] : w) : (k > 0 ? y[k > 0 ? k - 1 : 0] : w);
+}
+template <int ZT>
+__device__ __forceinline__ void ldz(const float* p, float (&o)[ZT]) {
+  if constexpr (ZT == 2) {
+    const float2 a = *reinterpret_cast<const float2*>(p);
+    o[0] = a.x; o[1] = a.y;
+  } else {
+#pragma unroll
+    for (int k = 0; k < ZT; k += 4) {
+      const float4 a = *reinterpret_cast<const float4*>(p + k);
+      o[k] = a.x; o[k + 1] = a.y; o[k + 2] = a.z; o[k + 3] = a.w;
+    }
+  }
+}
+template <int ZT>
+__device__ __forceinline__ void ldz(const double* p, double (&o)[ZT]) {
+#pragma unroll
+  for (int k = 0; k < ZT; k += 2) {
+    const double2 a = *reinterpret_cast<const double2*>(p + k);
+    o[k] = a.x; o[k + 1] = a.y;
+  }
+}
+template <int ZT>
+__device__ __forceinline__ void stz(float* p, const float (&o)[ZT]) {
+  if constexpr (ZT == 2) {
+    *reinterpret_cast<float2*>(p) = make_float2(o[0], o[1]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < ZT; k += 4) *reinterpret_cast<float4*>(p + k) = make_float4(o[k], o[k + 1], o[k + 2], o[k + 3]);
+  }
+}
+template <int ZT>
+__device__ __forceinline__ void stz(double* p, const double (&o)[ZT]) {
+#pragma unroll
+  for (int k = 0; k < ZT; k += 2) *reinterpret_cast<double2*>(p + k) = make_double2(o[k], o[k + 1]);
+}
+// the quad's four columns of ZT planes
+template <int ZT, typename T>
+__device__ __forceinline__ void store_quad(T* tile, int x0, int y0, const Seg<ZT>& g, const T (&v)[ZT][4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    T c[ZT];
+#pragma unroll
+    for (int k = 0; k < ZT; ++k) c[k] = v[k][e];
+    stz<ZT>(tile + at(x0 + (e & 1), y0 + (e >> 1)) + g.w0, c);
+  }
+}
+// The coarse tile of the prolongation: coarse nodes -1..8 per axis, plane cz of column (cx, cy) at word
+// cz + 4 of its kCC.  (Quads beside the block's last column read a column past it.)
+constexpr int kCC = 20, kCX = 11, kCTile = kCX * kCX * kCC;
+__device__ __forceinline__ int coarse_at(int cx, int cy) { return ((cy + 1) * kCX + cx + 1) * kCC + 4; }
+// P ec on quad (qx, qy) (block-local, -1..8) from its four coarse columns on one coarse plane
+template <typename T>
+__device__ __forceinline__ void prolong_plane(T c00, T c10, T c01, T c11, T (&pl)[4]) {
+  pl[0] = c00;
+  pl[1] = (T)0.5 * (c00 + c10);
+  pl[2] = (T)0.5 * (c00 + c01);
+  pl[3] = (T)0.25 * ((c00 + c10) + (c01 + c11));
+}
+// v += P ec on the quad's segment (even planes lie on a coarse plane, odd ones halfway between two)
+template <int ZT, typename T, int M>
+__device__ __forceinline__ void prolong_quads(const T* ctile, int qx, int qy, const Seg<ZT>& g, T (&v)[M][4]) {
+  const T* c = ctile + coarse_at(qx, qy) + (g.z0 >> 1);
+  T q[4][ZT + 1];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    T a[ZT];
+    const T* ci = c + (i & 1) * kCC + (i >> 1) * kCX * kCC;
+    ldz<ZT>(ci, a);
+#pragma unroll
+    for (int k = 0; k < ZT; ++k) q[i][k] = a[k];
+    q[i][ZT] = ci[ZT];
+  }
+  T lo[4], hi[4];
+  prolong_plane<T>(q[0][0], q[1][0], q[2][0], q[3][0], lo);
+#pragma unroll
+  for (int k = 0; k < ZT; ++k) {
+    prolong_plane<T>(q[0][k + 1], q[1][k + 1], q[2][k + 1], q[3][k + 1], hi);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      v[k][e] += g.p ? (T)0.5 * (lo[e] + hi[e]) : lo[e];
+      lo[e] = hi[e];
+    }
+  }
+}
+
+// The halo in two steps, so that its loads are in flight with the block's own: halo quad columns beside
+// the block (threads 0 .. NSIDE - 1) and the quads of the planes z = -1 and 16 (the others).
+// quad(m, o): the four values of the quad at Morton index m of the vector.
+__device__ __forceinline__ void side_quad(int h, int& qx, int& qy) {
+  if (h < 20) {
+    qy = h < 10 ? -1 : 8;
+    qx = (h < 10 ? h : h - 10) - 1;
+  } else {
+    qy = (h - 20) >> 1;
+    qx = (h & 1) ? 8 : -1;
+  }
+}
+__device__ __forceinline__ void face_quad(int i, int& qx, int& qy) {  // the 64 of the block first
+  if (i < 64) quad_of(i, qx, qy);
+  else side_quad(i - 64, qx, qy);
+}
+__device__ __forceinline__ int side_of(int q) { return q < 0 ? -1 : (q > 7 ? 1 : 0); }
+template <int ZT, typename T, typename Quad>
+__device__ __forceinline__ void load_halo(const uint32_t* nb, Quad quad, T (&hv)[Zt<ZT>::HV][4]) {
+  typedef Zt<ZT> Z;
+  const int t = threadIdx.x;
+  if (t < Z::NSIDE) {
+    int qx, qy;
+    side_quad(t / Z::SEG, qx, qy);
+    const Seg<ZT> g(t);
+    const uint32_t base = nb[13 + side_of(qx) + 3 * side_of(qy)];
+    const uint32_t mq = s16::sp4(2 * (qx & 7)) | (s16::sp4(2 * (qy & 7)) << 1);
+#pragma unroll
+    for (int k = 0; k < ZT; ++k) {
+      hv[k][0] = hv[k][1] = hv[k][2] = hv[k][3] = (T)0;
+      if (base != ~0u) quad(base + (mq | (s16::sp4(g.z(k)) << 2)), hv[k]);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < Z::ZN; ++j) {
+      const int i = t - Z::NSIDE + Z::NZF * j;
+      if (i >= 200) break;
+      const int hi = i >= 100;
+      int qx, qy;
+      face_quad(i - 100 * hi, qx, qy);
+      const uint32_t base = nb[13 + side_of(qx) + 3 * side_of(qy) + (hi ? 9 : -9)];
+      const uint32_t m = s16::sp4(2 * (qx & 7)) | (s16::sp4(2 * (qy & 7)) << 1) | (hi ? 0u : 0x249u << 2);
+      hv[j][0] = hv[j][1] = hv[j][2] = hv[j][3] = (T)0;
+      if (base != ~0u) quad(base + m, hv[j]);
+    }
+  }
+}
+// ctile (nullable): the coarse tile whose prolongation is added at nodes inside the domain
+template <int ZT, bool PROLONG, typename T>
+__device__ __forceinline__ void store_halo(T* tile, const uint32_t* nb, const T* ctile, T (&hv)[Zt<ZT>::HV][4]) {
+  typedef Zt<ZT> Z;
+  const int t = threadIdx.x;
+  if (t < Z::NSIDE) {
+    int qx, qy;
+    side_quad(t / Z::SEG, qx, qy);
+    const Seg<ZT> g(t);
+    if (PROLONG && nb[13 + side_of(qx) + 3 * side_of(qy)] != ~0u) prolong_quads<ZT>(ctile, qx, qy, g, hv);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int x = 2 * qx + (e & 1), y = 2 * qy + (e >> 1);
+      if (x < -1 || x > 16 || y < -1 || y > 16) continue;
+      T c[ZT];
+#pragma unroll
+      for (int k = 0; k < ZT; ++k) c[k] = hv[k][e];
+      stz<ZT>(tile + at(x, y) + g.w0, c);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < Z::ZN; ++j) {
+      const int i = t - Z::NSIDE + Z::NZF * j;
+      if (i >= 200) break;
+      const int hi = i >= 100;
+      int qx, qy;
+      face_quad(i - 100 * hi, qx, qy);
+      if (PROLONG && nb[13 + side_of(qx) + 3 * side_of(qy) + (hi ? 9 : -9)] != ~0u) {
+        const T* c = ctile + coarse_at(qx, qy) + (hi ? 8 : -1);
+        T lo[4], up[4];
+        prolong_plane<T>(c[0], c[kCC], c[kCX * kCC], c[kCX * kCC + kCC], lo);
+        if (!hi) prolong_plane<T>(c[1], c[kCC + 1], c[kCX * kCC + 1], c[kCX * kCC + kCC + 1], up);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) hv[j][e] += hi ? lo[e] : (T)0.5 * (lo[e] + up[e]);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int x = 2 * qx + (e & 1), y = 2 * qy + (e >> 1);
+        if (x >= -1 && x <= 16 && y >= -1 && y <= 16) tile[halo_at(hi, x, y)] = hv[j][e];
+      }
+    }
+  }
+}
+// a zero halo (a sweep from zero reads no halo plane, only the columns beside the block)
+template <int ZT, typename T>
+__device__ __forceinline__ void zero_side_halo(T* tile) {
+  const T zero[ZT] = {};
+  for (int i = threadIdx.x; i < 68 * Zt<ZT>::SEG; i += Zt<ZT>::NT) {
+    const int h = i / Zt<ZT>::SEG, z0 = ZT * (i % Zt<ZT>::SEG);  // (words)
+    const int x = h < 36 ? (h < 18 ? h : h - 18) - 1 : ((h & 1) ? 16 : -1);
+    const int y = h < 36 ? (h < 18 ? -1 : 16) : (h - 36) >> 1;
+    stz<ZT>(tile + at(x, y) + z0, zero);
+  }
+}
+
+// loads the coarse tile by quads: the block's 128 coarse ones in memory order, then the 232 around them
+template <int NT, typename T>
+__device__ __forceinline__ void load_coarse_tile(T* ctile, const T* __restrict__ ec, const uint32_t* nb) {
+  for (int i = threadIdx.x; i < 360; i += NT) {
+    int qx, qy, cz;
+    if (i < 128) {
+      qx = ((i >> 1) & 1) | ((i >> 3) & 2);
+      qy = ((i >> 2) & 1) | ((i >> 4) & 2);
+      cz = (i & 1) | ((i >> 2) & 2) | ((i >> 4) & 4);
+    } else if (i < 200) {  // the planes below and above
+      const int r = (i - 128) % 36;
+      qx = r % 6 - 1;
+      qy = r / 6 - 1;
+      cz = i < 164 ? -1 : 8;
+    } else {  // beside the block
+      const int r = (i - 200) % 20;
+      cz = (i - 200) / 20;
+      if (r < 12) {
+        qx = r % 6 - 1;
+        qy = r < 6 ? -1 : 4;
+      } else {
+        qx = (r & 1) ? 4 : -1;
+        qy = (r - 12) >> 1;
+      }
+    }
+    const int dx = qx < 0 ? -1 : (qx > 3 ? 1 : 0), dy = qy < 0 ? -1 : (qy > 3 ? 1 : 0),
+              dz = cz < 0 ? -1 : (cz > 7 ? 1 : 0);
+    const uint32_t b = nb[13 + dx + 3 * dy + 9 * dz];
+    T o[4] = {0, 0, 0, 0};
+    if (b != ~0u) ld4q(ec + (b >> 3) + (s16::sp4(2 * (qx & 3)) | (s16::sp4(2 * (qy & 3)) << 1) | (s16::sp4(cz & 7) << 2)), o);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int cx = 2 * qx + (e & 1), cy = 2 * qy + (e >> 1);
+      if (cx >= -1 && cx <= 8 && cy >= -1 && cy <= 8) ctile[coarse_at(cx, cy) + cz] = o[e];
+    }
+  }
+}
+
+// The sum over the block of one value per (quad column q, plane z), in an order fixed by the block: each
+// column's planes in z order, then the 64 column sums by a fixed tree.  red: 64 x 18 doubles of shared
+// memory, the value of (q, z) at red_at(q, z), written after a barrier that ends every other use of that
+// memory.  Every thread calls this (it has barriers); thread 0 returns the sum.
+__device__ __forceinline__ int red_at(int qx, int qy, int z) {  // columns in Morton order, as the writing lanes
+  return 18 * (int)(s16::sp2(qx) | s16::sp2(qy) << 1) + z;
+}
+__device__ __forceinline__ double block_sum_fixed(double* red) {
+  __syncthreads();
+  const int t = threadIdx.x;
+  double s = 0.0;
+  if (t < 64) {
+#pragma unroll
+    for (int z = 0; z < 16; ++z) s += red[red_at(t & 7, t >> 3, z)];
+  }
+  __syncthreads();
+  if (t < 64) red[t] = s;
+  __syncthreads();
+  if (t < 32) {
+    s = red[t] + red[t + 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  }
+  return s;
+}
+
+// the 4 x 4 patch around quad (x0, y0) on a halo plane
+template <typename T>
+__device__ __forceinline__ void halo_patch(const T* tile, int hi, int x0, int y0, T (&r)[4][4]) {
+  const T* p = tile + halo_at(hi, x0, y0);
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[j][i] = p[(j - 1) * kHR + i - 1];
+}
+// the 4 x 4 columns around the quad over the thread's planes, the quad's own from v
+template <int ZT, typename T>
+__device__ __forceinline__ void load_columns(const T* tile, int x0, int y0, const Seg<ZT>& g, const T (&v)[ZT][4],
+                                             T (&col)[4][4][ZT]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if ((i == 1 || i == 2) && (j == 1 || j == 2)) {
+#pragma unroll
+        for (int k = 0; k < ZT; ++k) col[j][i][k] = v[k][2 * (j - 1) + i - 1];
+      } else {
+        ldz<ZT>(tile + at(x0 - 1 + i, y0 - 1 + j) + g.w0, col[j][i]);
+      }
+    }
+}
+// Stencil rows y = A v of the quad column's ZT planes (v: its own values, also in the tile): per plane the
+// in-plane sums tz (for the planes above and below) and own; a row is (tz(z - 1) + own(z)) + tz(z + 1).
+template <int ZT, typename T>
+__device__ __forceinline__ void stencil_rows(const T* tile, int x0, int y0, const Seg<ZT>& g, const T (&v)[ZT][4],
+                                             T c0, T ce, T cc, T (&y)[ZT][4]) {
+  T tz[ZT][4];
+  {
+    T col[4][4][ZT];
+    load_columns<ZT, T>(tile, x0, y0, g, v, col);
+#pragma unroll
+    for (int k = 0; k < ZT; ++k) {
+      T r[4][4], ctr[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[j][i] = col[j][i][k];
+      n16::plane_terms<T>(r, c0, ce, cc, tz[k], y[k], ctr);
+    }
+  }
+  T te[4] = {0, 0, 0, 0};  // tz of the halo plane at the block's end
+  if (g.first() || g.last()) {
+    T r[4][4], own[4], ctr[4];
+    halo_patch<T>(tile, g.last(), x0, y0, r);
+    n16::plane_terms<T>(r, c0, ce, cc, te, own, ctr);
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    T x[ZT], nx[ZT], ox[ZT];
+#pragma unroll
+    for (int k = 0; k < ZT; ++k) x[k] = tz[k][e];
+    beside<ZT>(g, x, te[e], nx, ox);
+#pragma unroll
+    for (int k = 0; k < ZT; ++k) y[k][e] = ((g.p ? nx[k] : ox[k]) + y[k][e]) + (g.p ? ox[k] : nx[k]);
+  }
+}
+// The same rows with a node's edge and corner neighbours summed before they meet their coefficients.
+template <int ZT, typename T>
+__device__ __forceinline__ void stencil_rows_summed(const T* tile, int x0, int y0, const Seg<ZT>& g,
+                                                    const T (&v)[ZT][4], T c0, T ce, T cc, T (&y)[ZT][4]) {
+  T fk[ZT][4], dk[ZT][4], ctr[4];
+  {
+    T col[4][4][ZT];
+    load_columns<ZT, T>(tile, x0, y0, g, v, col);
+#pragma unroll
+    for (int k = 0; k < ZT; ++k) {
+      T r[4][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[j][i] = col[j][i][k];
+      n16::plane_sums<T>(r, fk[k], dk[k], ctr);
+    }
+  }
+  T fe[4] = {0, 0, 0, 0}, de[4] = {0, 0, 0, 0};
+  if (g.first() || g.last()) {
+    T r[4][4];
+    halo_patch<T>(tile, g.last(), x0, y0, r);
+    n16::plane_sums<T>(r, fe, de, ctr);
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    T f[ZT], d[ZT], fn[ZT], fo[ZT], dn[ZT], dO[ZT];
+#pragma unroll
+    for (int k = 0; k < ZT; ++k) {
+      f[k] = fk[k][e];
+      d[k] = dk[k][e];
+    }
+    beside<ZT>(g, f, fe[e], fn, fo);
+    beside<ZT>(g, d, de[e], dn, dO);
+#pragma unroll
+    for (int k = 0; k < ZT; ++k) y[k][e] = c0 * v[k][e] + ce * (d[k] + (fn[k] + fo[k])) + cc * (dn[k] + dO[k]);
+  }
+}
+}  // namespace z16
+
+// ------------------------------------------------------------------ 16^3 stencil SpMV (finest level)
+namespace n16 {
+template <int ZT>
+using Zt = z16::Zt<ZT>;
+// CTAs per SM that the register budget is set for: the loads of a quad column's 12 neighbouring columns
+// are in flight together (about 80 registers in FP32 at 4 planes)
+template <typename T, int ZT>
+constexpr int kCtas = sizeof(T) == 4 ? (ZT == 2 ? 2 : 4) : 1;
+
 // KIND 0: q = A a, part = a.q;  1: an = bvec + beta a, q = A an, part = an.q;
 // 3: q = A a for a caller's vector: a node's 12 edge and 8 corner neighbours are summed before they
 // meet their coefficients, as in the per-node stencil, which rounds less than the solver's order;
 // 2: an = a + beta bvec (FP64 solution + correction of type E; a null: zero), q = rhs - A an.
 // beta_dev (packed launches): the cloud's beta, in place of the beta argument.
 template <typename T, int KIND, typename E, int ZT>
-__global__ void __launch_bounds__(Zt<ZT>::NT, (sizeof(T) == 4 ? 5 : 3) * ZT / 4)
+__global__ void __launch_bounds__(Zt<ZT>::NT, kCtas<T, ZT>)
     k_spmv16(uint32_t D, const T* __restrict__ a, const E* __restrict__ bvec, T* __restrict__ an, T beta,
              T* __restrict__ q, T c0, T ce, T cc, const T* __restrict__ rhs, double* __restrict__ part,
              const double* __restrict__ beta_dev) {
-  constexpr int NT = Zt<ZT>::NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* tile = reinterpret_cast<T*>(smem_raw);
   __shared__ uint32_t nb[27];
@@ -852,139 +1103,95 @@ __global__ void __launch_bounds__(Zt<ZT>::NT, (sizeof(T) == 4 ? 5 : 3) * ZT / 4)
     part = cloud_slice(part, gridDim.x);
     if (beta_dev) beta = (T)beta_dev[blockIdx.y];
   }
-  const uint32_t blk = blockIdx.x;
-  const uint64_t base = (uint64_t)blk * N;
+  const uint32_t blk = blockIdx.x, base = blk << 12;
   uint32_t bx, by, bz;
   unmorton3(blk, bx, by, bz);
   const int t = threadIdx.x;
-  s16::neighbour_bases(nb, bx, by, bz, res >> 4);
-  auto val = [&](uint32_t m) -> T {
-    if (KIND == 0 || KIND == 3) return __ldg(a + m);
-    if (KIND == 1) return (T)__ldg(bvec + m) + beta * __ldg(a + m);
-    // KIND 2 with beta 0: a cloud of a packed launch that has stopped keeps its solution
-    const T av = a ? __ldg(a + m) : (T)0;
-    return beta == (T)0 ? av : av + beta * (T)__ldg(bvec + m);
-  };
-#pragma unroll
-  for (int r = 0; r < ZT; ++r) {
-    const int qd = t + NT * r;
-    int lx, ly, lz;
-    s16::quad_coords(qd, lx, ly, lz);
-    const uint64_t m = base + 4 * qd;
-    typename s16::Vec4<T>::type v;
-    if (KIND != 2 || a) v = s16::ld4(a + m);
-    else v.x = v.y = v.z = v.w = (T)0;
-    if (KIND == 1 || KIND == 2) {
-      const typename s16::Vec4<E>::type bv = s16::ld4(bvec + m);
-      if (KIND == 1) {
-        v.x = (T)bv.x + beta * v.x; v.y = (T)bv.y + beta * v.y; v.z = (T)bv.z + beta * v.z; v.w = (T)bv.w + beta * v.w;
-      } else if (beta != (T)0) {
-        v.x += beta * (T)bv.x; v.y += beta * (T)bv.y; v.z += beta * (T)bv.z; v.w += beta * (T)bv.w;
-      }
-      s16::st4(an + m, v);
-    }
-    T* p0 = tile + nat(lx + 1, ly + 1, lz + 1);
-    p0[0] = v.x;
-    p0[1] = v.y;
-    p0[RS] = v.z;
-    p0[RS + 1] = v.w;
-  }
-  __syncthreads();  // nb
-  s16::load_halo<NT>(tile, a, nb, [](int ux, int uy, int uz) { return nat(ux, uy, uz); }, val);
-  __syncthreads();
-  const int qi = t & 63, zs = t >> 6;
-  const int x0 = 2 * (qi & 7), y0 = 2 * (qi >> 3), z0 = ZT * zs;
+  const z16::Seg<ZT> g(t);
+  int qx, qy;
+  z16::quad_of(t / Zt<ZT>::SEG, qx, qy);
+  const int x0 = 2 * qx, y0 = 2 * qy;
   const uint32_t mq = s16::sp4(x0) | (s16::sp4(y0) << 1);
-  if constexpr (KIND == 3) {
-    T fm[4], dm[4], f0[4], d0[4], c0v[4], fp[4], dp[4], cp[4];  // planes p - 2, p - 1 and p
+  s16::neighbour_bases(nb, bx, by, bz, res >> 4);
+  auto add = [&](T (&o)[4], const E (&bv)[4]) {
 #pragma unroll
-    for (int p = 0; p < ZT + 2; ++p) {  // tile plane z0 + p = local z0 + p - 1
-      T r[4][4];
-      patch<T, RS>(tile, nat(x0, y0, z0 + p), r);
-      plane_sums<T>(r, fp, dp, cp);
-      if (p >= 2) {
-        T y[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) y[e] = c0 * c0v[e] + ce * (d0[e] + (fm[e] + fp[e])) + cc * (dm[e] + dp[e]);
-        typename s16::Vec4<T>::type o;
-        o.x = y[0]; o.y = y[1]; o.z = y[2]; o.w = y[3];
-        s16::st4(q + base + (mq | (s16::sp4(z0 + p - 2) << 2)), o);
-      }
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        fm[e] = f0[e];
-        dm[e] = d0[e];
-        f0[e] = fp[e];
-        d0[e] = dp[e];
-        c0v[e] = cp[e];
-      }
+    for (int i = 0; i < 4; ++i) {
+      if (KIND == 1) o[i] = (T)bv[i] + beta * o[i];
+      else if (beta != (T)0) o[i] += beta * (T)bv[i];  // beta 0: a cloud that has stopped keeps its solution
     }
-    return;
+  };
+  auto quad = [&](uint32_t m, T (&o)[4]) {
+    if (KIND != 2 || a) z16::ld4q(a + m, o);
+    else o[0] = o[1] = o[2] = o[3] = (T)0;
+    if (KIND == 1 || KIND == 2) {
+      E bv[4];
+      z16::ld4q(bvec + m, bv);
+      add(o, bv);
+    }
+  };
+  T v[ZT][4];
+#pragma unroll
+  for (int k = 0; k < ZT; ++k) quad(base + (mq | (s16::sp4(g.z(k)) << 2)), v[k]);
+  __syncthreads();  // nb
+  {
+    T hv[Zt<ZT>::HV][4];
+    z16::load_halo<ZT, T>(nb, quad, hv);
+    z16::store_quad<ZT>(tile, x0, y0, g, v);
+    if (KIND == 1 || KIND == 2) {
+#pragma unroll
+      for (int k = 0; k < ZT; ++k) z16::st4q(an + (base + (mq | (s16::sp4(g.z(k)) << 2))), v[k]);
+    }
+    z16::store_halo<ZT, false, T>(tile, nb, nullptr, hv);
   }
-  T cur[4] = {0, 0, 0, 0}, nxt[4] = {0, 0, 0, 0}, cprev[4] = {0, 0, 0, 0};
+  __syncthreads();
+  T y[ZT][4];
+  if constexpr (KIND == 3) z16::stencil_rows_summed<ZT, T>(tile, x0, y0, g, v, c0, ce, cc, y);
+  else z16::stencil_rows<ZT, T>(tile, x0, y0, g, v, c0, ce, cc, y);
   double pv[ZT];  // per plane: the quad's four products of the dot
 #pragma unroll
-  for (int p = 0; p < ZT + 2; ++p) {  // tile plane z0 + p = local z0 + p - 1
-    T r[4][4], tz[4], own[4], ctr[4];
-    patch<T, RS>(tile, nat(x0, y0, z0 + p), r);
-    plane_terms<T>(r, c0, ce, cc, tz, own, ctr);
+  for (int k = 0; k < ZT; ++k) {
+    const uint32_t m = base + (mq | (s16::sp4(g.z(k)) << 2));
+    if (KIND == 2) {
+      T rv[4];
+      z16::ld4q(rhs + m, rv);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      cur[e] += tz[e];
-      nxt[e] += own[e];
-    }
-    if (p >= 2) {  // row of local z0 + p - 2 is complete
-      const uint64_t m = base + (mq | (s16::sp4(z0 + p - 2) << 2));
-      typename s16::Vec4<T>::type o;
-      if (KIND == 2) {
-        const typename s16::Vec4<T>::type rv = s16::ld4(rhs + m);
-        o.x = rv.x - cur[0]; o.y = rv.y - cur[1]; o.z = rv.z - cur[2]; o.w = rv.w - cur[3];
-      } else {
-        o.x = cur[0]; o.y = cur[1]; o.z = cur[2]; o.w = cur[3];
-        double a4 = 0.0;
+      for (int e = 0; e < 4; ++e) y[k][e] = rv[e] - y[k][e];
+    } else {
+      double a4 = 0.0;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) a4 += (double)cprev[e] * (double)cur[e];
-        pv[p - 2] = a4;
-      }
-      s16::st4(q + m, o);
+      for (int e = 0; e < 4; ++e) a4 += (double)v[k][e] * (double)y[k][e];
+      pv[k] = a4;
     }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      cur[e] = nxt[e];
-      nxt[e] = tz[e];
-      cprev[e] = ctr[e];
-    }
+    z16::st4q(q + m, y[k]);
   }
   if (KIND < 2) {
     __syncthreads();  // the tile's last reads: its memory takes the per-plane sums
     double* red = reinterpret_cast<double*>(smem_raw);
 #pragma unroll
-    for (int k = 0; k < ZT; ++k) red[(z0 + k) * 64 + qi] = pv[k];
-    const double sdot = s16::block_sum_fixed(red);
+    for (int k = 0; k < ZT; ++k) red[z16::red_at(qx, qy, g.z(k))] = pv[k];
+    const double sdot = z16::block_sum_fixed(red);
     if (t == 0) part[blk] = sdot;
   }
 }
 template <typename T>
 constexpr size_t smem_bytes() {
-  return sizeof(T) * TILE;
+  return sizeof(T) * z16::TILE;
 }
 }  // namespace n16
 
 // ------------------------------------------------------------------ 16^3 residual + restriction
 // Two launches, no redundant work.  k_resid16: r = f - A e on the block's 16^3 nodes (the
-// SpMV's tile and quad columns), then (a) the part of the restriction to the block's 8^3 coarse
-// nodes that comes from its own fine nodes, and (b) the restriction partials its high faces
-// (local 15) owe the coarse nodes of its high neighbours: per face the sum over the face's other
-// two axes (8 x 8), per edge over the remaining axis (8), and the corner (1), into a face buffer
-// of 224 values per block.  k_restrict_faces adds to the coarse nodes on each block's low faces
-// these partials of its low neighbours, scaled by 1/2 per crossed axis.  Restriction: coarse c
-// gathers fine 2c-1, 2c, 2c+1 per axis with weights 1/2, 1, 1/2.
+// SpMV's tile and quad columns; r then takes e's place in the tile), then (a) the part of the
+// restriction to the block's 8^3 coarse nodes that comes from its own fine nodes, and (b) the
+// restriction partials its high faces (local 15) owe the coarse nodes of its high neighbours: per
+// face the sum over the face's other two axes (8 x 8), per edge over the remaining axis (8), and
+// the corner (1), into a face buffer of 224 values per block.  k_restrict_faces adds to the coarse
+// nodes on each block's low faces these partials of its low neighbours, scaled by 1/2 per crossed
+// axis.  Restriction: coarse c gathers fine 2c-1, 2c, 2c+1 per axis with weights 1/2, 1, 1/2.
 namespace r16 {
-constexpr int N = 4096, FACE = 224;  // ZT, NT: as n16 (the residual is the same for every ZT)
+constexpr int FACE = 224;
 // face buffer layout: [0,64) x face (cy + 8 cz), [64,128) y face (cx + 8 cz), [128,192) z face
 // (cx + 8 cy), [192,200) xy edge (cz), [200,208) xz edge (cy), [208,216) yz edge (cx), 216 corner
-constexpr int RSR = 20, PSR = 16 * RSR + 8, RTILE = 16 * PSR;  // half-warps of the restriction on disjoint banks
-__device__ __forceinline__ int ridx(int x, int y, int z) { return z * PSR + y * RSR + x; }  // local coordinates
 
 // What the low-face row `cm` of a node changes in its residual: (interior row - face row) of A e, with
 // at(dx, dy, dz) the node's neighbours.
@@ -1004,38 +1211,63 @@ __device__ __forceinline__ T face_change(At at, const T* cm, T c0, T ce, T cc) {
   return yi - yf;
 }
 
-// restriction of the block's residual tile to its coarse node ci (Morton) from its own fine nodes
+// r += what the low-face rows change at the quad column's nodes on a low domain face
+template <int ZT, typename T>
+__device__ __forceinline__ void face_residual(const T* tile, const T* table, int ox, int oy, int oz, int x0, int y0,
+                                              const z16::Seg<ZT>& g, T c0, T ce, T cc, T (&r)[ZT][4]) {
+#pragma unroll 1
+  for (int i = 0; i < 4 * ZT; ++i) {
+    const int x = x0 + (i & 1), y = y0 + ((i >> 1) & 1), z = g.z(i >> 2);
+    const int mask = ((ox + x) == 0) | (((oy + y) == 0) << 1) | (((oz + z) == 0) << 2);
+    if (!mask) continue;
+    const z16::PlaneRef<T> pl[3] = {z16::plane_ref(tile, x, y, z - 1), z16::plane_ref(tile, x, y, z),
+                                    z16::plane_ref(tile, x, y, z + 1)};
+    const T dr = face_change<T>([&](int dx, int dy, int dz) { return pl[dz + 1](dx, dy); }, table + 27 * mask, c0, ce,
+                                cc);
+#pragma unroll
+    for (int k = 0; k < ZT; ++k)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (4 * k + e == i) r[k][e] += dr;
+  }
+}
+
+// restriction of the block's residual tile to its coarse node (cx, cy, cz) from its own fine nodes
 template <typename T>
-__device__ __forceinline__ T restrict_own(const T* rt, uint32_t ci) {
-  uint32_t cx, cy, cz;
-  unmorton3(ci, cx, cy, cz);
+__device__ __forceinline__ T restrict_own(const T* tile, int cx, int cy, int cz) {
+  T c[3][3][3];  // fine planes 2cz - 1, 2cz, 2cz + 1 of columns x, then y, 2c - 1 .. 2c + 1
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const T* p = tile + z16::at(2 * cx + i - 1, 2 * cy + j - 1) + cz;  // plane 2 cz; plane 2 cz + 1 at p[8]
+      c[0][j][i] = cz > 0 ? p[7] : (T)0;
+      c[1][j][i] = p[0];
+      c[2][j][i] = p[8];
+    }
   T s = 0;
 #pragma unroll
   for (int dz = -1; dz <= 1; ++dz) {
-    const int fz = 2 * (int)cz + dz;
-    if (fz < 0) continue;
+    if (dz < 0 && cz == 0) continue;
 #pragma unroll
     for (int dy = -1; dy <= 1; ++dy) {
-      const int fy = 2 * (int)cy + dy;
-      if (fy < 0) continue;
+      if (dy < 0 && cy == 0) continue;
       const T wyz = (T)((dy == 0 ? 1.0 : 0.5) * (dz == 0 ? 1.0 : 0.5));
-      const T* row = rt + ridx(2 * cx, fy, fz);
-      const typename n16::Pair<T>::type pr = *reinterpret_cast<const typename n16::Pair<T>::type*>(row);
-      const T left = cx > 0 ? row[-1] : (T)0;
-      s += wyz * (pr.x + (T)0.5 * (pr.y + left));
+      const T* r = c[dz + 1][dy + 1];
+      const T left = cx > 0 ? r[0] : (T)0;
+      s += wyz * (r[1] + (T)0.5 * (r[2] + left));
     }
   }
   return s;
 }
 
 template <typename T, bool FACES, int ZT>
-__global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT / 4)
+__global__ void __launch_bounds__(n16::Zt<ZT>::NT, n16::kCtas<T, ZT>)
     k_resid16(uint32_t D, const T* __restrict__ e, const T* __restrict__ f, T* __restrict__ fc,
               T* __restrict__ face, T c0, T ce, T cc, const T* __restrict__ table) {
   constexpr int NT = n16::Zt<ZT>::NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* et = reinterpret_cast<T*>(smem_raw);  // n16::TILE
-  T* rt = et + n16::TILE;                  // RTILE
+  T* tile = reinterpret_cast<T*>(smem_raw);
   __shared__ uint32_t nb[27];
   const int res = 1 << D;
   {
@@ -1045,79 +1277,49 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
     fc = cloud_slice(fc, nl / 8);
     face = cloud_slice(face, (uint64_t)gridDim.x * FACE);
   }
-  const uint32_t blk = blockIdx.x;
-  const uint64_t base = (uint64_t)blk * N;
+  const uint32_t blk = blockIdx.x, base = blk << 12;
   uint32_t bx, by, bz;
   unmorton3(blk, bx, by, bz);
   const int ox = (int)bx * 16, oy = (int)by * 16, oz = (int)bz * 16;
   const int t = threadIdx.x;
+  const z16::Seg<ZT> g(t);
+  int qx, qy;
+  z16::quad_of(t / n16::Zt<ZT>::SEG, qx, qy);
+  const int x0 = 2 * qx, y0 = 2 * qy;
+  const uint32_t mq = s16::sp4(x0) | (s16::sp4(y0) << 1);
   s16::neighbour_bases(nb, bx, by, bz, res >> 4);
+  T r[ZT][4];
+  {
+    T v[ZT][4];
 #pragma unroll
-  for (int r = 0; r < ZT; ++r) {
-    const int qd = t + NT * r;
-    int lx, ly, lz;
-    s16::quad_coords(qd, lx, ly, lz);
-    const typename s16::Vec4<T>::type ev = s16::ld4(e + base + 4 * qd);
-    T* p0 = et + n16::nat(lx + 1, ly + 1, lz + 1);
-    p0[0] = ev.x;
-    p0[1] = ev.y;
-    p0[n16::RS] = ev.z;
-    p0[n16::RS + 1] = ev.w;
-  }
-  __syncthreads();  // nb
-  s16::load_halo<NT>(et, e, nb, [](int ux, int uy, int uz) { return n16::nat(ux, uy, uz); },
-                    [&](uint32_t m) { return __ldg(e + m); });
-  __syncthreads();
-  {  // r = f - A e on quad columns, z swept once
-    const int qi = t & 63, zs = t >> 6;
-    const int x0 = 2 * (qi & 7), y0 = 2 * (qi >> 3), z0 = ZT * zs;
-    const uint32_t mq = s16::sp4(x0) | (s16::sp4(y0) << 1);
-    T cur[4] = {0, 0, 0, 0}, nxt[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (int p = 0; p < ZT + 2; ++p) {  // local plane z0 + p - 1
-      T r[4][4], tz[4], own[4], ctr[4];
-      n16::patch<T, n16::RS>(et, n16::nat(x0, y0, z0 + p), r);
-      n16::plane_terms<T>(r, c0, ce, cc, tz, own, ctr);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        cur[k] += tz[k];
-        nxt[k] += own[k];
-      }
-      if (p >= 2) {
-        const int lz = z0 + p - 2;
-        const typename s16::Vec4<T>::type fv = s16::ld4(f + base + (mq | (s16::sp4(lz) << 2)));
-        T* q0 = rt + ridx(x0, y0, lz);
-        q0[0] = fv.x - cur[0];
-        q0[1] = fv.y - cur[1];
-        q0[RSR] = fv.z - cur[2];
-        q0[RSR + 1] = fv.w - cur[3];
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        cur[k] = nxt[k];
-        nxt[k] = tz[k];
-      }
-    }
-  }
-  __syncthreads();
-  if (FACES && (ox == 0 || oy == 0 || oz == 0)) {
-    // nodes on a low domain face: replace the interior row by the face row
-    for (int i = t; i < N; i += NT) {
-      uint32_t lx, ly, lz;
-      unmorton3((uint32_t)i, lx, ly, lz);
-      const int mask = ((ox + (int)lx) == 0) | (((oy + (int)ly) == 0) << 1) | (((oz + (int)lz) == 0) << 2);
-      if (!mask) continue;
-      const int ei = n16::nat(lx + 1, ly + 1, lz + 1);
-      rt[ridx(lx, ly, lz)] += face_change<T>([&](int dx, int dy, int dz) { return et[ei + dx + n16::RS * dy + n16::PS * dz]; },
-                                             table + 27 * mask, c0, ce, cc);
+    for (int k = 0; k < ZT; ++k) z16::ld4q(e + (base + (mq | (s16::sp4(g.z(k)) << 2))), v[k]);
+    __syncthreads();  // nb
+    {
+      T hv[n16::Zt<ZT>::HV][4];
+      z16::load_halo<ZT, T>(nb, [&](uint32_t m, T (&o)[4]) { z16::ld4q(e + m, o); }, hv);
+      z16::store_quad<ZT>(tile, x0, y0, g, v);
+      z16::store_halo<ZT, false, T>(tile, nb, nullptr, hv);
     }
     __syncthreads();
+    z16::stencil_rows<ZT, T>(tile, x0, y0, g, v, c0, ce, cc, r);
   }
-  // own part of the restriction
+#pragma unroll
+  for (int k = 0; k < ZT; ++k) {
+    T fq[4];
+    z16::ld4q(f + (base + (mq | (s16::sp4(g.z(k)) << 2))), fq);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[k][i] = fq[i] - r[k][i];
+  }
+  if (FACES && (ox == 0 || oy == 0 || oz == 0)) face_residual<ZT>(tile, table, ox, oy, oz, x0, y0, g, c0, ce, cc, r);
+  __syncthreads();  // e is read
+  z16::store_quad<ZT>(tile, x0, y0, g, r);
+  __syncthreads();
+  // own part of the restriction (lanes: eight coarse planes of a 2 x 2 of columns)
   const uint64_t cbase = (uint64_t)blk * 512;
 #pragma unroll
-  for (int ci = t; ci < 512; ci += NT) {
-    fc[cbase + ci] = restrict_own<T>(rt, (uint32_t)ci);
+  for (int i = t; i < 512; i += NT) {
+    const int cz = i & 7, cx = ((i >> 3) & 1) | ((i >> 5) & 3) << 1, cy = ((i >> 4) & 1) | ((i >> 7) & 3) << 1;
+    fc[cbase + (s16::sp4(cx) | (s16::sp4(cy) << 1) | (s16::sp4(cz) << 2))] = restrict_own<T>(tile, cx, cy, cz);
   }
   // restriction partials of the high faces, edges and corner
   {
@@ -1136,7 +1338,7 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
             const int fi = 2 * i + di;
             if (fi < 0) continue;
             const int x = axis == 0 ? 15 : fi, y = axis == 1 ? 15 : (axis == 0 ? fi : fj), z = axis == 2 ? 15 : fj;
-            acc += w(di) * w(dj) * rt[ridx(x, y, z)];
+            acc += w(di) * w(dj) * tile[z16::at(x, y) + z16::zw(z)];
           }
         }
         fb[u] = acc;
@@ -1148,11 +1350,11 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
           const int fi = 2 * i + di;
           if (fi < 0) continue;
           const int x = e == 2 ? fi : 15, y = e == 1 ? fi : 15, z = e == 0 ? fi : 15;
-          acc += w(di) * rt[ridx(x, y, z)];
+          acc += w(di) * tile[z16::at(x, y) + z16::zw(z)];
         }
         fb[u] = acc;
       } else {
-        fb[216] = rt[ridx(15, 15, 15)];
+        fb[216] = tile[z16::at(15, 15) + 15];
       }
     }
   }
@@ -1203,7 +1405,7 @@ __global__ void __launch_bounds__(768) k_restrict_faces(uint32_t D, const T* __r
 }
 template <typename T>
 constexpr size_t smem_bytes() {
-  return sizeof(T) * (n16::TILE + RTILE);
+  return sizeof(T) * z16::TILE;
 }
 }  // namespace r16
 
@@ -1225,25 +1427,21 @@ constexpr size_t smem_bytes() {
 // of the levels 16^3 to 64^3 took 29-31 us (115 us at 8 planes per thread); a depth-7 reconstruction
 // of 20,011 points went from 4.65 to 3.22 ms and a depth-9 one of 317,003 from 33.0 to 29.9 ms.
 namespace g16 {
-constexpr int CW = s16::CW;  // ZT, NT: as n16 (a node's relaxation is the same for every ZT)
-// Parity-split tile (u = local + 1 in 0..17 per axis): each row holds its even columns (u even)
-// first, then its odd ones, HS words each, so the columns of one class that a warp relaxes
-// (x0 = 0, 2, .., 14: stride 2 in x) are consecutive words, and its four quad rows (y two apart,
-// 2 RS = 40 words = 8 banks apart) fill the 32 banks once: every tile access of a phase is free
-// of bank conflicts for FP32, and per half-warp for FP64.
-constexpr int HS = 10, RS = 2 * HS, PS = 18 * RS + 4, TILE = 18 * PS;
-__device__ __forceinline__ int col(int ux) { return (ux & 1) * HS + (ux >> 1); }
-__device__ __forceinline__ int nat(int ux, int uy, int uz) { return uz * PS + uy * RS + col(ux); }
+// CTAs per SM that the register budget is set for: four, three where the face rows would spill
+template <typename T, bool FACES, int ZT>
+constexpr int kCtas = sizeof(T) == 8 ? 2 : (ZT == 2 ? 2 : (FACES ? 3 : 4));
 
 // One phase: new values of the class-CLS column of the thread's quad (planes z0..z0+ZT-1).
-// On the thread's own planes the ring members inside its quad come from registers (v), the
-// other five from the tile; the two halo planes read all eight.
+// The ring members inside the thread's quad come from registers (v), the other five columns from the
+// tile; the in-plane sums of the planes below and above from the neighbouring lanes, at the block's ends
+// from the halo planes (zero there for a sweep from zero).
 // ZERO: a forward sweep from zero, in which the classes after CLS are still zero everywhere
 // (their loads are skipped; phase 0 needs none).
-template <typename T, int CLS, bool ZERO, int ZT>
-__device__ __forceinline__ void relax_column(const T* tile, int x0, int y0, int z0, const T (&fv)[ZT][4],
-                                             const T (&v)[ZT][4], T ce, T cc, T c0inv, T (&nv)[ZT]) {
-  constexpr int CX = CLS & 1, CY = CLS >> 1;
+template <typename T, int CLS, bool FROM_ZERO, bool ZERO, int ZT>
+__device__ __forceinline__ void relax_column(const T* tile, int x0, int y0, const z16::Seg<ZT>& g,
+                                             const T (&fv)[ZT][4], const T (&v)[ZT][4], T ce, T cc, T c0inv,
+                                             T (&nv)[ZT]) {
+  constexpr int CX = CLS & 1, CY = CLS >> 1, CS = z16::kCS, RY = z16::kRY;
   constexpr int EDX = CX == 0 ? -1 : 1, EDY = CY == 0 ? -1 : 1;  // direction of the external ring side
   constexpr int EFX = (CX ^ 1) | (CY << 1), EFY = CX | ((CY ^ 1) << 1), ED = (CX ^ 1) | ((CY ^ 1) << 1);
   // classes updated before CLS in a forward sweep are 0..CLS-1
@@ -1253,44 +1451,41 @@ __device__ __forceinline__ void relax_column(const T* tile, int x0, int y0, int 
     for (int k = 0; k < ZT; ++k) nv[k] = fv[k][CLS] * c0inv;
     return;
   }
-  // the ring's columns x-1, x, x+1 (x = x0 + CX, tile column x + 1; x0 even): their row offsets
-  const int xh = x0 >> 1;
-  const int cm = CX * HS + xh, cz = (1 - CX) * HS + xh + CX, cp = CX * HS + xh + 1;
-  const int cxe = EDX < 0 ? cm : cp;  // the external column x + EDX
-  const T* rbase = tile + (y0 + CY) * RS;  // ring row y-1 of tile plane 0
-  T Dm = 0, Fm = 0, D0 = 0, F0 = 0;
+  const T* c = tile + z16::at(x0 + CX, y0 + CY) + g.w0;
+  T q0[ZT], q1[ZT], q2[ZT], ed[ZT], ex[ZT], Dk[ZT], Fk[ZT];
+  if (ND) {
+    z16::ldz<ZT>(c + EDY * RY - CS, q0);
+    z16::ldz<ZT>(c + EDY * RY + CS, q2);
+    z16::ldz<ZT>(c - EDY * RY + EDX * CS, ed);
+  }
+  if (NFY) z16::ldz<ZT>(c + EDY * RY, q1);
+  if (NFX) z16::ldz<ZT>(c + EDX * CS, ex);
 #pragma unroll
-  for (int p = 0; p < ZT + 2; ++p) {  // local plane z0 + p - 1
-    const T* r0 = rbase + (z0 + p) * PS;
-    T Dp = 0, Fp = 0;
-    if (p >= 1 && p <= ZT) {  // own plane: (x', y), (x, y'), (x', y') from registers
-      const int k = p - 1;
-      const T* rr = r0 + (EDY + 1) * RS;  // external row: columns x-1, x, x+1
-      T q0 = 0, q1 = 0, q2 = 0;
-      if (ND) {
-        q0 = rr[cm];
-        q2 = rr[cp];
-      }
-      if (NFY) q1 = rr[cz];
-      // the same pairing as a halo plane's (row y-1 pair + row y+1 pair), so that a node's sums
-      // do not depend on which of its planes are a thread's own
-      if (ND) Dp = (q0 + q2) + (r0[(1 - EDY) * RS + cxe] + v[k][ED]);
-      if (NFY) Fp += q1 + v[k][EFY];
-      if (NFX) Fp += r0[RS + cxe] + v[k][EFX];
-    } else {  // halo plane: the whole ring from the tile
-      const T a0 = r0[cm], a1 = r0[cz], a2 = r0[cp];
-      const T c0v = r0[2 * RS + cm], c1 = r0[2 * RS + cz], c2 = r0[2 * RS + cp];
-      Dp = (a0 + a2) + (c0v + c2);
-      Fp = (a1 + c1) + (r0[RS + cm] + r0[RS + cp]);
-    }
-    if (p >= 2) {  // node at local z0 + p - 2: edges D0 + Fm + Fp, corners Dm + Dp
-      const int k = p - 2;
-      nv[k] = (fv[k][CLS] - ce * (D0 + Fm + Fp) - cc * (Dm + Dp)) * c0inv;
-    }
-    Dm = D0;
-    Fm = F0;
-    D0 = Dp;
-    F0 = Fp;
+  for (int k = 0; k < ZT; ++k) {
+    Dk[k] = Fk[k] = 0;
+    if (ND) Dk[k] = (q0[k] + q2[k]) + (ed[k] + v[k][ED]);
+    if (NFY) Fk[k] += q1[k] + v[k][EFY];
+    if (NFX) Fk[k] += ex[k] + v[k][EFX];
+  }
+  T De = 0, Fe = 0;
+  if (!FROM_ZERO && (g.first() || g.last())) {  // the halo plane: the whole ring from the tile
+    const T* h = tile + z16::halo_at(g.last(), x0 + CX, y0 + CY);
+    constexpr int HR = z16::kHR;
+    De = (h[-HR - 1] + h[-HR + 1]) + (h[HR - 1] + h[HR + 1]);
+    Fe = (h[-HR] + h[HR]) + (h[-1] + h[1]);
+  }
+  T Dn[ZT], Do[ZT], Fn[ZT], Fo[ZT];
+  if (ND) {
+    z16::beside<ZT>(g, Dk, De, Dn, Do);
+  } else {
+#pragma unroll
+    for (int k = 0; k < ZT; ++k) Dn[k] = Do[k] = 0;
+  }
+  z16::beside<ZT>(g, Fk, Fe, Fn, Fo);
+#pragma unroll
+  for (int k = 0; k < ZT; ++k) {  // edges D(z) + F(z-1) + F(z+1), corners D(z-1) + D(z+1)
+    const T fm = g.p ? Fn[k] : Fo[k], fp = g.p ? Fo[k] : Fn[k];
+    nv[k] = (fv[k][CLS] - ce * (Dk[k] + fm + fp) - cc * (Dn[k] + Do[k])) * c0inv;
   }
 }
 
@@ -1298,34 +1493,35 @@ __device__ __forceinline__ void relax_column(const T* tile, int x0, int y0, int 
 // low domain face (uniform in the block), whose rows are in ftab.
 template <typename T, bool FWD, bool FROM_ZERO, bool FACES, int ZT>
 __device__ __forceinline__ void sweep(T* tile, const T* ftab, bool faces, int ox, int oy, int oz, int x0, int y0,
-                                      int z0, const T (&fv)[ZT][4], T (&v)[ZT][4], T ce, T cc, T c0inv) {
+                                      const z16::Seg<ZT>& g, const T (&fv)[ZT][4], T (&v)[ZT][4], T ce, T cc,
+                                      T c0inv) {
 #pragma unroll
   for (int ph = 0; ph < 4; ++ph) {
     const int cls = FWD ? ph : 3 - ph;
-    const int cx = cls & 1, cy = cls >> 1;
-    const int x = x0 + cx, y = y0 + cy;
+    const int x = x0 + (cls & 1), y = y0 + (cls >> 1);
     T nv[ZT];
     constexpr bool ZERO = FROM_ZERO && FWD;
     switch (cls) {
-      case 0: relax_column<T, 0, ZERO, ZT>(tile, x0, y0, z0, fv, v, ce, cc, c0inv, nv); break;
-      case 1: relax_column<T, 1, ZERO, ZT>(tile, x0, y0, z0, fv, v, ce, cc, c0inv, nv); break;
-      case 2: relax_column<T, 2, ZERO, ZT>(tile, x0, y0, z0, fv, v, ce, cc, c0inv, nv); break;
-      default: relax_column<T, 3, ZERO, ZT>(tile, x0, y0, z0, fv, v, ce, cc, c0inv, nv); break;
+      case 0: relax_column<T, 0, FROM_ZERO, ZERO, ZT>(tile, x0, y0, g, fv, v, ce, cc, c0inv, nv); break;
+      case 1: relax_column<T, 1, FROM_ZERO, ZERO, ZT>(tile, x0, y0, g, fv, v, ce, cc, c0inv, nv); break;
+      case 2: relax_column<T, 2, FROM_ZERO, ZERO, ZT>(tile, x0, y0, g, fv, v, ce, cc, c0inv, nv); break;
+      default: relax_column<T, 3, FROM_ZERO, ZERO, ZT>(tile, x0, y0, g, fv, v, ce, cc, c0inv, nv); break;
     }
+    T* self = tile + z16::at(x, y) + g.w0;
     if (faces) {  // low-domain-face nodes of this column: their table rows, neighbours from the tile
-      const int cl = col(x), cm1 = col(x + 1), cr = col(x + 2);  // tile columns x-1, x, x+1
 #pragma unroll 1
       for (int k = 0; k < ZT; ++k) {
-        const int z = z0 + k;
-        const int mask = ((ox + x) == 0) | (((oy + y) == 0) << 1) | (((oz + z) == 0) << 2);
+        const int mask = ((ox + x) == 0) | (((oy + y) == 0) << 1) | (((oz + g.z(k)) == 0) << 2);
         if (!mask) continue;
         const T* cm = ftab + 27 * mask;
-        const T* tb = tile + z * PS + y * RS;  // tile row y-1 of tile plane z-1
+        const int z = g.z(k);
+        const z16::PlaneRef<T> pl[3] = {z16::plane_ref<T>(tile, x, y, z - 1), z16::plane_ref<T>(tile, x, y, z),
+                                        z16::plane_ref<T>(tile, x, y, z + 1)};
         T off = 0;
 #pragma unroll
         for (int o = 0; o < 27; ++o) {
           if (o == 13) continue;
-          off += cm[o] * tb[(o / 9) * PS + ((o / 3) % 3) * RS + (o % 3 == 0 ? cl : (o % 3 == 1 ? cm1 : cr))];
+          off += cm[o] * pl[o / 9](o % 3 - 1, (o / 3) % 3 - 1);
         }
         T fk = fv[0][cls];
 #pragma unroll
@@ -1339,33 +1535,10 @@ __device__ __forceinline__ void sweep(T* tile, const T* ftab, bool faces, int ox
       __syncthreads();  // same-class column neighbours were read with their old values
     }
 #pragma unroll
-    for (int k = 0; k < ZT; ++k) {
-      v[k][cls] = nv[k];
-      tile[nat(x + 1, y + 1, z0 + k + 1)] = nv[k];
-    }
+    for (int k = 0; k < ZT; ++k) v[k][cls] = nv[k];
+    z16::stz<ZT>(self, nv);
     __syncthreads();
   }
-}
-
-// v += P ec on the quad column: coarse (cx, cx+1) x (cy, cy+1) at the coarse planes z0/2 .. z0/2+ZT/2
-// (z0 even: planes z0, z0+2 lie on a coarse plane, z0+1, z0+3 halfway between two)
-template <typename T, int ZT>
-__device__ __forceinline__ void prolong_quads(const T* ctile, int x0, int y0, int z0, T (&v)[ZT][4]) {
-  const int ax = x0 / 2 + 1, ay = y0 / 2 + 1, az = z0 / 2 + 1;
-  T pl[ZT / 2 + 1][4];
-#pragma unroll
-  for (int w = 0; w <= ZT / 2; ++w) {
-    const T* c = ctile + ((az + w) * CW + ay) * CW + ax;
-    const T c00 = c[0], c10 = c[1], c01 = c[CW], c11 = c[CW + 1];
-    pl[w][0] = c00;
-    pl[w][1] = (T)0.5 * (c00 + c10);
-    pl[w][2] = (T)0.5 * (c00 + c01);
-    pl[w][3] = (T)0.25 * ((c00 + c10) + (c01 + c11));
-  }
-#pragma unroll
-  for (int k = 0; k < ZT; ++k)  // even planes on a coarse plane, odd halfway between two
-#pragma unroll
-    for (int e = 0; e < 4; ++e) v[k][e] += (k & 1) ? (T)0.5 * (pl[k / 2][e] + pl[k / 2 + 1][e]) : pl[k / 2][e];
 }
 
 // MODE 0: xo = sweep(xi); 1: xo = sweep(0); 2: xo = sweep(xi + P ec).  DOT: part = f.xo
@@ -1373,16 +1546,17 @@ __device__ __forceinline__ void prolong_quads(const T* ctile, int x0, int y0, in
 // (pointwise), then xo = sweep(0) with f = the new r; part = per-block sums of r^2.  A sweep
 // from zero reads no halo, so updating r in place is race-free.
 template <typename T, int MODE, bool DOT, bool FWD, bool FACES, int ZT>
-__global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT / 4)
+__global__ void __launch_bounds__(n16::Zt<ZT>::NT, kCtas<T, FACES, ZT>)
     k_smooth16(uint32_t D, const T* __restrict__ xi, T* __restrict__ xo, const T* __restrict__ f,
                const T* __restrict__ ec, T c0inv, T ce, T cc, const T* __restrict__ table,
                double* __restrict__ part, CgFuse<T> cg) {
   static_assert(MODE != 3 || (FWD && !FACES), "the fused CG update is a forward sweep on the finest level");
   constexpr int NT = n16::Zt<ZT>::NT;
+  constexpr bool FROM_ZERO = MODE == 1 || MODE == 3;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* tile = reinterpret_cast<T*>(smem_raw);  // TILE
-  T* ctile = tile + TILE;                    // CW^3 (MODE 2)
-  __shared__ uint32_t nb[27], cnb[27];
+  T* tile = reinterpret_cast<T*>(smem_raw);  // z16::TILE
+  T* ctile = tile + z16::TILE;               // z16::kCTile (MODE 2)
+  __shared__ uint32_t nb[27];
   __shared__ T ftab[FACES ? 216 : 1];  // the face rows
   const int res = 1 << D;
   {
@@ -1401,86 +1575,84 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
       if (cg.alpha_dev) cg.alpha = (T)cg.alpha_dev[blockIdx.y];
     }
   }
-  const uint32_t blk = blockIdx.x;
-  const uint64_t base = (uint64_t)blk * 4096;
+  const uint32_t blk = blockIdx.x, base = blk << 12;
   uint32_t bx, by, bz;
   unmorton3(blk, bx, by, bz);
   const int ox = (int)bx * 16, oy = (int)by * 16, oz = (int)bz * 16;
   const int t = threadIdx.x;
+  const z16::Seg<ZT> g(t);
+  int qx, qy;
+  z16::quad_of(t / n16::Zt<ZT>::SEG, qx, qy);
+  const int x0 = 2 * qx, y0 = 2 * qy;
+  const uint32_t mq = s16::sp4(x0) | (s16::sp4(y0) << 1);
   const bool faces = FACES && (ox == 0 || oy == 0 || oz == 0);  // uniform in the block
   if (faces)
     for (int i = t; i < 216; i += NT) ftab[i] = table[i];  // read after the barriers below
-  constexpr bool FROM_ZERO = MODE == 1 || MODE == 3;
   if (!FROM_ZERO) s16::neighbour_bases(nb, bx, by, bz, res >> 4);
-  else if (t < 27) nb[t] = ~0u;  // zero halo
-  if (MODE == 2) s16::load_coarse_tile<NT>(ctile, ec, blk, bx, by, bz, res >> 4, cnb);  // ends with a barrier
-  else __syncthreads();                                                                 // nb
-  const int qi = t & 63, zs = t >> 6;
-  const int x0 = 2 * (qi & 7), y0 = 2 * (qi >> 3), z0 = ZT * zs;
-  const uint32_t mq = s16::sp4(x0) | (s16::sp4(y0) << 1);
   T fv[ZT][4], v[ZT][4];
   double rr[ZT];  // MODE 3: per plane, the quad's r^2
 #pragma unroll
   for (int k = 0; k < ZT; ++k) {
-    const uint64_t m = base + (mq | (s16::sp4(z0 + k) << 2));
-    typename s16::Vec4<T>::type fq;
+    const uint32_t m = base + (mq | (s16::sp4(g.z(k)) << 2));
     if (MODE == 3) {  // the CG update of this quad (plain loads: x and r are written here)
       typedef typename s16::Vec4<T>::type V4;
-      fq = cg.rin ? s16::ld4(cg.rin + m) : *reinterpret_cast<const V4*>(cg.r + m);
+      const V4 rq = *reinterpret_cast<const V4*>((cg.rin ? cg.rin : cg.r) + m);
+      fv[k][0] = rq.x; fv[k][1] = rq.y; fv[k][2] = rq.z; fv[k][3] = rq.w;
       if (cg.alpha != (T)0 || cg.rin) {  // alpha 0: a cloud that has stopped keeps x and r
-        V4 xq;
-        if (cg.rin) xq.x = xq.y = xq.z = xq.w = (T)0;
-        else xq = *reinterpret_cast<const V4*>(cg.x + m);
-        if (cg.alpha != (T)0) {
-          const V4 dq = s16::ld4(cg.d + m), qq = s16::ld4(cg.q + m);
-          xq.x += cg.alpha * dq.x; xq.y += cg.alpha * dq.y; xq.z += cg.alpha * dq.z; xq.w += cg.alpha * dq.w;
-          fq.x -= cg.alpha * qq.x; fq.y -= cg.alpha * qq.y; fq.z -= cg.alpha * qq.z; fq.w -= cg.alpha * qq.w;
+        T xq[4] = {};
+        if (!cg.rin) {
+          const V4 xv = *reinterpret_cast<const V4*>(cg.x + m);
+          xq[0] = xv.x; xq[1] = xv.y; xq[2] = xv.z; xq[3] = xv.w;
         }
-        s16::st4(cg.x + m, xq);
-        s16::st4(cg.r + m, fq);
-      }
-      rr[k] = (double)fq.x * fq.x + (double)fq.y * fq.y + (double)fq.z * fq.z + (double)fq.w * fq.w;
-    } else {
-      fq = s16::ld4(f + m);
-    }
-    fv[k][0] = fq.x; fv[k][1] = fq.y; fv[k][2] = fq.z; fv[k][3] = fq.w;
-    if (FROM_ZERO) {
-      v[k][0] = v[k][1] = v[k][2] = v[k][3] = (T)0;
-    } else {
-      const typename s16::Vec4<T>::type xq = s16::ld4(xi + m);
-      v[k][0] = xq.x; v[k][1] = xq.y; v[k][2] = xq.z; v[k][3] = xq.w;
-    }
-  }
-  if (MODE == 2) prolong_quads<T, ZT>(ctile, x0, y0, z0, v);
+        if (cg.alpha != (T)0) {
+          T dq[4], qq[4];
+          z16::ld4q(cg.d + m, dq);
+          z16::ld4q(cg.q + m, qq);
 #pragma unroll
-  for (int k = 0; k < ZT; ++k) {
-    T* p0 = tile + nat(0, y0 + 1, z0 + k + 1);
-    p0[col(x0 + 1)] = v[k][0];
-    p0[col(x0 + 2)] = v[k][1];
-    p0[RS + col(x0 + 1)] = v[k][2];
-    p0[RS + col(x0 + 2)] = v[k][3];
-  }
-  s16::load_halo<NT>(tile, xi, nb, [](int ux, int uy, int uz) { return nat(ux, uy, uz); },
-                    [&](uint32_t m) -> T { return FROM_ZERO ? (T)0 : __ldg(xi + m); });
-  __syncthreads();
-  if (MODE == 2) {  // add P ec on the halo shell (in-domain positions only)
-    for (int i = t; i < 1736; i += NT) {
-      int ux, uy, uz;
-      halo_u<16>(i, ux, uy, uz);
-      const int gx = ox - 1 + ux, gy = oy - 1 + uy, gz = oz - 1 + uz;
-      if (gx < 0 || gy < 0 || gz < 0 || gx >= res || gy >= res || gz >= res) continue;
-      tile[nat(ux, uy, uz)] += s16::prolong_at<T>(ctile, ux, uy, uz);
+          for (int e = 0; e < 4; ++e) {
+            xq[e] += cg.alpha * dq[e];
+            fv[k][e] -= cg.alpha * qq[e];
+          }
+        }
+        z16::st4q(cg.x + m, xq);
+        z16::st4q(cg.r + m, fv[k]);
+      }
+      rr[k] = (double)fv[k][0] * fv[k][0] + (double)fv[k][1] * fv[k][1] + (double)fv[k][2] * fv[k][2] +
+              (double)fv[k][3] * fv[k][3];
+    } else if (FROM_ZERO) {
+      z16::ld4q(f + m, fv[k]);
     }
-    __syncthreads();
+    if (FROM_ZERO) v[k][0] = v[k][1] = v[k][2] = v[k][3] = (T)0;
+    else z16::ld4q(xi + m, v[k]);
   }
-  sweep<T, FWD, FROM_ZERO, FACES, ZT>(tile, ftab, faces, ox, oy, oz, x0, y0, z0, fv, v, ce, cc, c0inv);
+  if (FROM_ZERO) {
+    z16::zero_side_halo<ZT, T>(tile);
+    if (faces) {  // face rows read the planes above and below, and every class
+      for (int i = t; i < z16::TILE; i += NT) tile[i] = 0;
+    } else if (!FWD) {
+      z16::store_quad<ZT>(tile, x0, y0, g, v);
+    }
+  } else {
+    T hv[n16::Zt<ZT>::HV][4];
+    __syncthreads();  // nb
+    z16::load_halo<ZT, T>(nb, [&](uint32_t m, T (&o)[4]) { z16::ld4q(xi + m, o); }, hv);
+    if (MODE == 2) {
+      z16::load_coarse_tile<NT>(ctile, ec, nb);
+      __syncthreads();  // ctile
+      z16::prolong_quads<ZT>(ctile, qx, qy, g, v);
+    }
+#pragma unroll
+    for (int k = 0; k < ZT; ++k) z16::ld4q(f + (base + (mq | (s16::sp4(g.z(k)) << 2))), fv[k]);
+    z16::store_quad<ZT>(tile, x0, y0, g, v);
+    z16::store_halo<ZT, MODE == 2, T>(tile, nb, ctile, hv);
+  }
+  __syncthreads();
+  sweep<T, FWD, FROM_ZERO, FACES, ZT>(tile, ftab, faces, ox, oy, oz, x0, y0, g, fv, v, ce, cc, c0inv);
   double acc[ZT];  // DOT: per plane, the quad's f.x
 #pragma unroll
+  for (int k = 0; k < ZT; ++k) z16::st4q(xo + (base + (mq | (s16::sp4(g.z(k)) << 2))), v[k]);
+#pragma unroll
   for (int k = 0; k < ZT; ++k) {
-    const uint64_t m = base + (mq | (s16::sp4(z0 + k) << 2));
-    typename s16::Vec4<T>::type o;
-    o.x = v[k][0]; o.y = v[k][1]; o.z = v[k][2]; o.w = v[k][3];
-    s16::st4(xo + m, o);
     acc[k] = 0.0;
     if (DOT)
 #pragma unroll
@@ -1490,14 +1662,14 @@ __global__ void __launch_bounds__(n16::Zt<ZT>::NT, (sizeof(T) == 4 ? 4 : 2) * ZT
     // the last phase ended with a barrier: the tile's memory takes the per-plane sums
     double* red = reinterpret_cast<double*>(smem_raw);
 #pragma unroll
-    for (int k = 0; k < ZT; ++k) red[(z0 + k) * 64 + qi] = MODE == 3 ? rr[k] : acc[k];
-    const double sum = s16::block_sum_fixed(red);
+    for (int k = 0; k < ZT; ++k) red[z16::red_at(qx, qy, g.z(k))] = MODE == 3 ? rr[k] : acc[k];
+    const double sum = z16::block_sum_fixed(red);
     if (t == 0) part[blk] = sum;
   }
 }
 template <typename T>
 constexpr size_t smem_bytes(int mode) {
-  return sizeof(T) * (TILE + (mode == 2 ? CW * CW * CW : 0));
+  return sizeof(T) * (z16::TILE + (mode == 2 ? z16::kCTile : 0));
 }
 }  // namespace g16
 
@@ -1520,7 +1692,7 @@ struct Coefs {  // of the 16^3 and the 8^3 level
   const T *table4, *table3;  // face rows, 216 each
   const T* inv;              // 64 x 64
 };
-constexpr int kWords = g16::TILE + r16::RTILE + 1000 + 1000 + 512 + WE * WE * WE + WR * WR * WR + 64 +
+constexpr int kWords = z16::TILE + z16::kCTile + 1000 + 512 + WE * WE * WE + WR * WR * WR + 64 +
                        CW3 * CW3 * CW3 + 64 * kInvStride + 432;
 
 // the 8 colours of an 8^3 sweep by threads 0..63 (two warps, their own barrier)
@@ -1545,10 +1717,9 @@ __device__ __forceinline__ void sweep8(T* tile, const T* fs, const T* ftab, T c0
 template <typename T>
 __global__ void __launch_bounds__(NT, 1) k_coarse_tail(const T* __restrict__ f, T* __restrict__ e, Coefs<T> k) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* tile = reinterpret_cast<T*>(smem_raw);  // 16^3 level: parity-split tile
-  T* rt = tile + g16::TILE;                  // its residual
-  T* ctile = rt + r16::RTILE;                // the 8^3 level with a one-node border, natural
-  T* tile3 = ctile + 1000;                   // 8^3 level: parity-split tile
+  T* tile = reinterpret_cast<T*>(smem_raw);  // 16^3 level: its tile, then its residual
+  T* ctile = tile + z16::TILE;               // the 8^3 level with a one-node border, natural
+  T* tile3 = ctile + z16::kCTile;            // 8^3 level: parity-split tile
   T* fs3 = tile3 + 1000;                     // its right-hand side, colour-major
   T* et3 = fs3 + 512;                        // natural tiles of its residual
   T* rt3 = et3 + WE * WE * WE;
@@ -1560,13 +1731,15 @@ __global__ void __launch_bounds__(NT, 1) k_coarse_tail(const T* __restrict__ f, 
   f = cloud_slice(f, 4096);
   e = cloud_slice(e, 4096);
   const int t = threadIdx.x;
-  const int qi = t & 63, zs = t >> 6;
-  const int x0 = 2 * (qi & 7), y0 = 2 * (qi >> 3), z0 = ZT * zs;
+  const z16::Seg<ZT> g(t);
+  int qx, qy;
+  z16::quad_of(t / z16::Zt<ZT>::SEG, qx, qy);
+  const int x0 = 2 * qx, y0 = 2 * qy;
   const uint32_t mq = s16::sp4(x0) | (s16::sp4(y0) << 1);
   T fv[ZT][4], v[ZT][4];
 #pragma unroll
   for (int p = 0; p < ZT; ++p) {
-    const typename s16::Vec4<T>::type q = s16::ld4(f + (mq | (s16::sp4(z0 + p) << 2)));
+    const typename s16::Vec4<T>::type q = s16::ld4(f + (mq | (s16::sp4(g.z(p)) << 2)));
     fv[p][0] = q.x; fv[p][1] = q.y; fv[p][2] = q.z; fv[p][3] = q.w;
     v[p][0] = v[p][1] = v[p][2] = v[p][3] = (T)0;
   }
@@ -1576,65 +1749,33 @@ __global__ void __launch_bounds__(NT, 1) k_coarse_tail(const T* __restrict__ f, 
     tab3[i] = k.table3[i];
   }
   // everything outside the domain is zero, and the sweeps start from zero
-  for (int i = t; i < g16::TILE; i += NT) tile[i] = 0;
-  for (int i = t; i < 1000; i += NT) ctile[i] = tile3[i] = 0;
+  for (int i = t; i < z16::TILE; i += NT) tile[i] = 0;
+  for (int i = t; i < z16::kCTile; i += NT) ctile[i] = 0;
+  for (int i = t; i < 1000; i += NT) tile3[i] = 0;
   for (int i = t; i < WE * WE * WE; i += NT) et3[i] = 0;
   for (int i = t; i < WR * WR * WR; i += NT) rt3[i] = 0;
   for (int i = t; i < CW3 * CW3 * CW3; i += NT) ctile3[i] = 0;
   __syncthreads();
 
   // 16^3: pre-smoothing from zero
-  g16::sweep<T, true, true, true, ZT>(tile, tab4, true, 0, 0, 0, x0, y0, z0, fv, v, k.ce4, k.cc4, k.c0inv4);
-  {  // r = f - A a on quad columns
-    T cur[4] = {0, 0, 0, 0}, nxt[4] = {0, 0, 0, 0};
+  g16::sweep<T, true, true, true, ZT>(tile, tab4, true, 0, 0, 0, x0, y0, g, fv, v, k.ce4, k.cc4, k.c0inv4);
+  {  // r = f - A a takes a's place in the tile (the threads keep a)
+    T r[ZT][4];
+    z16::stencil_rows<ZT, T>(tile, x0, y0, g, v, k.c04, k.ce4, k.cc4, r);
 #pragma unroll
-    for (int p = 0; p < ZT + 2; ++p) {  // local plane z0 + p - 1
-      T r[4][4], tz[4], own[4], ctr[4];
+    for (int p = 0; p < ZT; ++p)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const T* row = tile + (z0 + p) * g16::PS + (y0 + j) * g16::RS + (x0 >> 1);
-        r[j][0] = row[0];
-        r[j][1] = row[g16::HS];
-        r[j][2] = row[1];
-        r[j][3] = row[g16::HS + 1];
-      }
-      n16::plane_terms<T>(r, k.c04, k.ce4, k.cc4, tz, own, ctr);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        cur[i] += tz[i];
-        nxt[i] += own[i];
-      }
-      if (p >= 2) {
-        T* q0 = rt + r16::ridx(x0, y0, z0 + p - 2);
-        q0[0] = fv[p - 2][0] - cur[0];
-        q0[1] = fv[p - 2][1] - cur[1];
-        q0[r16::RSR] = fv[p - 2][2] - cur[2];
-        q0[r16::RSR + 1] = fv[p - 2][3] - cur[3];
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        cur[i] = nxt[i];
-        nxt[i] = tz[i];
-      }
-    }
-  }
-  __syncthreads();
-  for (int i = t; i < 721; i += NT) {  // the low-face nodes: x = 0, then y = 0 < x, then z = 0 < x, y
-    int lx, ly, lz;
-    if (i < 256) { lx = 0; ly = i & 15; lz = i >> 4; }
-    else if (i < 496) { lx = 1 + (i - 256) % 15; ly = 0; lz = (i - 256) / 15; }
-    else { lx = 1 + (i - 496) % 15; ly = 1 + (i - 496) / 15; lz = 0; }
-    const int mask = (lx == 0) | ((ly == 0) << 1) | ((lz == 0) << 2);
-    rt[r16::ridx(lx, ly, lz)] += r16::face_change<T>(
-        [&](int dx, int dy, int dz) { return tile[g16::nat(lx + 1 + dx, ly + 1 + dy, lz + 1 + dz)]; },
-        tab4 + 27 * mask, k.c04, k.ce4, k.cc4);
+      for (int i = 0; i < 4; ++i) r[p][i] = fv[p][i] - r[p][i];
+    r16::face_residual<ZT>(tile, tab4, 0, 0, 0, x0, y0, g, k.c04, k.ce4, k.cc4, r);
+    __syncthreads();
+    z16::store_quad<ZT>(tile, x0, y0, g, r);
   }
   __syncthreads();
   uint32_t nx, ny, nz;  // this thread's 8^3 node (Morton t)
   unmorton3((uint32_t)t, nx, ny, nz);
   const int ux = (int)nx + 1, uy = (int)ny + 1, uz = (int)nz + 1;
   {
-    const T s = r16::restrict_own<T>(rt, (uint32_t)t);
+    const T s = r16::restrict_own<T>(tile, (int)nx, (int)ny, (int)nz);
     const int col = (nx & 1) | ((ny & 1) << 1) | ((nz & 1) << 2);
     fs3[col * 64 + ((nx >> 1) | ((ny >> 1) << 2) | ((nz >> 1) << 4))] = s;
     rt3[(uz * WR + uy) * WR + ux] = s;  // f first, r = f - A a below
@@ -1679,26 +1820,19 @@ __global__ void __launch_bounds__(NT, 1) k_coarse_tail(const T* __restrict__ f, 
   __syncthreads();
   if (t < 64) sweep8<T, false>(tile3, fs3, tab3, k.c03, k.ce3, k.cc3, t);
   __syncthreads();
-  ctile[(uz * s16::CW + uy) * s16::CW + ux] = tile3[self3];
+  ctile[z16::coarse_at((int)nx, (int)ny) + (int)nz] = tile3[self3];
   __syncthreads();
 
   // 16^3: post-smoothing on a + P e
-  g16::prolong_quads<T, ZT>(ctile, x0, y0, z0, v);
-#pragma unroll
-  for (int p = 0; p < ZT; ++p) {
-    T* p0 = tile + g16::nat(0, y0 + 1, z0 + p + 1);
-    p0[g16::col(x0 + 1)] = v[p][0];
-    p0[g16::col(x0 + 2)] = v[p][1];
-    p0[g16::RS + g16::col(x0 + 1)] = v[p][2];
-    p0[g16::RS + g16::col(x0 + 2)] = v[p][3];
-  }
+  z16::prolong_quads<ZT>(ctile, qx, qy, g, v);
+  z16::store_quad<ZT>(tile, x0, y0, g, v);
   __syncthreads();
-  g16::sweep<T, false, false, true, ZT>(tile, tab4, true, 0, 0, 0, x0, y0, z0, fv, v, k.ce4, k.cc4, k.c0inv4);
+  g16::sweep<T, false, false, true, ZT>(tile, tab4, true, 0, 0, 0, x0, y0, g, fv, v, k.ce4, k.cc4, k.c0inv4);
 #pragma unroll
   for (int p = 0; p < ZT; ++p) {
     typename s16::Vec4<T>::type o;
     o.x = v[p][0]; o.y = v[p][1]; o.z = v[p][2]; o.w = v[p][3];
-    s16::st4(e + (mq | (s16::sp4(z0 + p) << 2)), o);
+    s16::st4(e + (mq | (s16::sp4(g.z(p)) << 2)), o);
   }
 }
 }  // namespace t4
@@ -1755,15 +1889,16 @@ void smooth_dispatch(cudaStream_t s, uint32_t D, const T* xi, T* xo, const T* f,
 }
 
 // ------------------------------------------------------------------ the z-segment autotuner
-// The 16^3 block kernels (SpMV, residual + restriction, smoother) run with ZT = 2, 4 or 8 z planes
-// per thread, i.e. 512, 256 or 128 threads per 16^3 brick: more planes per thread read fewer halo
-// planes from shared memory per node but leave fewer threads to hide latency.  Every ZT computes
-// the same values (per-block sums in a fixed order), so the choice is free and made by timing: the
-// first FP32 launch of a (kernel family, level, launch size, with or without face rows: the same
-// level is one solve's finest and another's coarse) key times each ZT (one warm-up and
-// three timed launches on the launch's own buffers; every candidate writes what the real launch
-// then overwrites) and keeps the fastest for the process.  FP64 launches and launches inside a
-// stream capture use ZT = 4.  PR_AUTOTUNE=0 fixes ZT = 4; PR_ZT=2|4|8 forces one.
+// The 16^3 block kernels (SpMV, residual + restriction, smoother) run with ZT = 2 or 4 planes per
+// thread, i.e. 512 or 256 threads per 16^3 brick: 4 planes move a column in 16-byte accesses (faster
+// on large levels by 20-30%), 2 put twice the warps on a level of few bricks.  Both compute the same
+// values (per-block sums in a fixed order), so the choice is free and made by timing: the first FP32
+// launch of a (kernel family, level, launch size, with or without face rows: the same level is one
+// solve's finest and another's coarse) key times both (one warm-up and three timed launches on the
+// launch's own buffers; every candidate writes what the real launch then overwrites) and keeps the
+// faster for the process.  Launches inside a stream capture use ZT = 4; FP64 launches 2 planes for the
+// SpMV and the residual, whose 12 columns in flight do not fit the registers of 4, and 4 for the
+// smoother.  PR_AUTOTUNE=0 fixes ZT = 4; PR_ZT=2|4 forces one (8, an earlier shape, means 4).
 enum TuneFamily { kTuneSpmv = 0, kTuneResid = 1, kTuneSmooth = 2, kTuneSmoothPost = 3 };
 struct TuneTable {
   std::mutex mu;
@@ -1780,12 +1915,15 @@ const char* family_name(int f) {
 // PR_ZT_<FAMILY> (e.g. PR_ZT_SPMV16), else PR_ZT, forces a choice; read at every launch, so that a
 // process may switch
 int forced_zt(int family) {
-  auto valid = [](const char* v) { return v && (std::atoi(v) == 2 || std::atoi(v) == 4 || std::atoi(v) == 8); };
+  auto choice = [](const char* v) {
+    const int z = v ? std::atoi(v) : 0;
+    return z == 8 ? 4 : (z == 2 || z == 4 ? z : 0);
+  };
   char name[32];
   std::snprintf(name, sizeof(name), "PR_ZT_%s", family == kTuneSpmv ? "SPMV16" : (family == kTuneResid ? "RESID16" : "SMOOTH16"));
   // (both smoother families answer to PR_ZT_SMOOTH16)
-  if (valid(std::getenv(name))) return std::atoi(std::getenv(name));
-  if (valid(std::getenv("PR_ZT"))) return std::atoi(std::getenv("PR_ZT"));
+  if (const int z = choice(std::getenv(name))) return z;
+  if (const int z = choice(std::getenv("PR_ZT"))) return z;
   const char* a = std::getenv("PR_AUTOTUNE");
   return (a && std::atoi(a) == 0) ? 4 : 0;
 }
@@ -1824,9 +1962,9 @@ void tuned_launch(cudaStream_t s, int family, uint32_t level, uint64_t blocks, b
   cudaEvent_t e0, e1;
   PR_CUDA(cudaEventCreate(&e0));
   PR_CUDA(cudaEventCreate(&e1));
-  const int cand[3] = {2, 4, 8};
-  float ms[3];
-  for (int k = 0; k < 3; ++k) {
+  const int cand[2] = {2, 4};
+  float ms[2];
+  for (int k = 0; k < 2; ++k) {
     launch(cand[k]);
     PR_CUDA(cudaEventRecord(e0, s));
     for (int r = 0; r < 3; ++r) launch(cand[k]);
@@ -1836,15 +1974,13 @@ void tuned_launch(cudaStream_t s, int family, uint32_t level, uint64_t blocks, b
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  int best = 1;  // ZT = 4 unless another is faster
-  for (int k = 0; k < 3; ++k)
-    if (ms[k] < ms[best]) best = k;
+  const int best = ms[0] < ms[1] ? 0 : 1;
   {
     std::lock_guard<std::mutex> g(tt.mu);
     tt.zt[key] = cand[best];
     char line[200];
-    std::snprintf(line, sizeof(line), "%s level %u%s blocks 2^%d: ZT 2/4/8 = %.4f/%.4f/%.4f ms -> ZT %d\n",
-                  family_name(family), level, faces ? " (faces)" : "", bin, ms[0] / 3, ms[1] / 3, ms[2] / 3, cand[best]);
+    std::snprintf(line, sizeof(line), "%s level %u%s blocks 2^%d: ZT 2/4 = %.4f/%.4f ms -> ZT %d\n",
+                  family_name(family), level, faces ? " (faces)" : "", bin, ms[0] / 3, ms[1] / 3, cand[best]);
     tt.log += line;
   }
   launch(cand[best]);
@@ -1865,7 +2001,6 @@ void launch_s16(cudaStream_t s, uint32_t D, const T* xi, T* xo, const T* f, cons
   tuned_launch(s, MODE == 2 ? kTuneSmoothPost : kTuneSmooth, D, (uint64_t)grid.x * grid.y, FACES, kTunable, [&](int zt) {
     if constexpr (kTunable) {
       if (zt == 2) return go(std::integral_constant<int, 2>());
-      if (zt == 8) return go(std::integral_constant<int, 8>());
     }
     go(std::integral_constant<int, 4>());
   });
@@ -1981,7 +2116,6 @@ void mg_cg_update_presmooth(cudaStream_t s, const LevelCoef& L, const T* table, 
   const int zt = std::is_same<T, float>::value && forced_zt(kTuneSmooth) ? forced_zt(kTuneSmooth) : 4;
   if constexpr (std::is_same<T, float>::value) {
     if (zt == 2) go(std::integral_constant<int, 2>());
-    else if (zt == 8) go(std::integral_constant<int, 8>());
     else go(std::integral_constant<int, 4>());
   } else {
     go(std::integral_constant<int, 4>());
@@ -2012,9 +2146,8 @@ void mg_resid_restrict(cudaStream_t s, const LevelCoef& L, const T* table, const
     tuned_launch(s, kTuneResid, D, (uint64_t)nb * clouds, L.has_faces, kTunable, [&](int zt) {
       if constexpr (kTunable) {
         if (zt == 2) return go_f(std::integral_constant<int, 2>());
-        if (zt == 8) return go_f(std::integral_constant<int, 8>());
       }
-      go_f(std::integral_constant<int, 4>());
+      go_f(std::integral_constant<int, kTunable ? 4 : 2>());
     });
     PR_CHECK_LAUNCH();
     r16::k_restrict_faces<T><<<dim3((nb + 3) / 4, clouds), 768, 0, s>>>(D, face, fc, nb);
@@ -2075,9 +2208,8 @@ void mg_spmv(cudaStream_t s, const LevelCoef& L, const T* table, const T* z, con
     tuned_launch(s, kTuneSpmv, D, (uint64_t)g.x * g.y, false, kTunable, [&](int zt) {
       if constexpr (kTunable) {
         if (zt == 2) return go(std::integral_constant<int, 2>());
-        if (zt == 8) return go(std::integral_constant<int, 8>());
       }
-      go(std::integral_constant<int, 4>());
+      go(std::integral_constant<int, kTunable ? 4 : 2>());
     });
   } else {
     if (clouds != 1 || beta_dev) throw Error(PR_ERR_INTERNAL, "packed SpMV needs depth >= 4");
@@ -2094,8 +2226,9 @@ void mg_apply(cudaStream_t s, const LevelCoef& L, const T* x, T* y) {
   const uint32_t D = L.depth;
   if (D < 4 || L.has_faces) throw Error(PR_ERR_INTERNAL, "mg_apply needs the finest level, depth >= 4");
   const size_t sm = n16::smem_bytes<T>();
-  allow_smem(n16::k_spmv16<T, 3, T, 4>, sm);
-  n16::k_spmv16<T, 3, T, 4><<<1u << (3 * (D - 4)), n16::Zt<4>::NT, sm, s>>>(
+  constexpr int ZT = sizeof(T) == 4 ? 4 : 2;
+  allow_smem(n16::k_spmv16<T, 3, T, ZT>, sm);
+  n16::k_spmv16<T, 3, T, ZT><<<1u << (3 * (D - 4)), n16::Zt<ZT>::NT, sm, s>>>(
       D, x, nullptr, nullptr, (T)0, y, (T)L.c0, (T)L.ce, (T)L.cc, nullptr, nullptr, nullptr);
   PR_CHECK_LAUNCH();
 }
@@ -2106,8 +2239,8 @@ void mg_resid_update(cudaStream_t s, const LevelCoef& L, const double* x, const 
   const uint32_t D = L.depth;
   if (D < 4 || L.has_faces) throw Error(PR_ERR_INTERNAL, "mg_resid_update needs the finest level, depth >= 4");
   const size_t sm = n16::smem_bytes<double>();
-  allow_smem(n16::k_spmv16<double, 2, E, 4>, sm);
-  n16::k_spmv16<double, 2, E, 4><<<dim3(1u << (3 * (D - 4)), clouds), n16::Zt<4>::NT, sm, s>>>(
+  allow_smem(n16::k_spmv16<double, 2, E, 2>, sm);
+  n16::k_spmv16<double, 2, E, 2><<<dim3(1u << (3 * (D - 4)), clouds), n16::Zt<2>::NT, sm, s>>>(
       D, x, e, xn, scale, r, L.c0, L.ce, L.cc, b, nullptr, scale_dev);
   PR_CHECK_LAUNCH();
 }
