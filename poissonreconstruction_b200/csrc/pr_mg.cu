@@ -1074,10 +1074,10 @@ __device__ __forceinline__ void stencil_rows_summed(const T* tile, int x0, int y
 namespace n16 {
 template <int ZT>
 using Zt = z16::Zt<ZT>;
-// CTAs per SM that the register budget is set for: the loads of a quad column's 12 neighbouring columns
-// are in flight together (about 80 registers in FP32 at 4 planes)
+// CTAs per SM that the register budget is set for; FP64 at depth 9, 4 planes: two CTAs 749 us for the
+// plain SpMV, one 926, three (spilling) 1246
 template <typename T, int ZT>
-constexpr int kCtas = sizeof(T) == 4 ? (ZT == 2 ? 2 : 4) : 1;
+constexpr int kCtas = sizeof(T) == 4 && ZT == 4 ? 4 : 2;
 
 // KIND 0: q = A a, part = a.q;  1: an = bvec + beta a, q = A an, part = an.q;
 // 3: q = A a for a caller's vector: a node's 12 edge and 8 corner neighbours are summed before they
@@ -1896,9 +1896,7 @@ void smooth_dispatch(cudaStream_t s, uint32_t D, const T* xi, T* xo, const T* f,
 // launch of a (kernel family, level, launch size, with or without face rows: the same level is one
 // solve's finest and another's coarse) key times both (one warm-up and three timed launches on the
 // launch's own buffers; every candidate writes what the real launch then overwrites) and keeps the
-// faster for the process.  Launches inside a stream capture use ZT = 4; FP64 launches 2 planes for the
-// SpMV and the residual, whose 12 columns in flight do not fit the registers of 4, and 4 for the
-// smoother.  PR_AUTOTUNE=0 fixes ZT = 4; PR_ZT=2|4 forces one (8, an earlier shape, means 4).
+// faster for the process.  FP64 launches and launches inside a stream capture use ZT = 4.  PR_AUTOTUNE=0 fixes ZT = 4; PR_ZT=2|4 forces one (8, an earlier shape, means 4).
 enum TuneFamily { kTuneSpmv = 0, kTuneResid = 1, kTuneSmooth = 2, kTuneSmoothPost = 3 };
 struct TuneTable {
   std::mutex mu;
@@ -2147,7 +2145,7 @@ void mg_resid_restrict(cudaStream_t s, const LevelCoef& L, const T* table, const
       if constexpr (kTunable) {
         if (zt == 2) return go_f(std::integral_constant<int, 2>());
       }
-      go_f(std::integral_constant<int, kTunable ? 4 : 2>());
+      go_f(std::integral_constant<int, 4>());
     });
     PR_CHECK_LAUNCH();
     r16::k_restrict_faces<T><<<dim3((nb + 3) / 4, clouds), 768, 0, s>>>(D, face, fc, nb);
@@ -2209,7 +2207,7 @@ void mg_spmv(cudaStream_t s, const LevelCoef& L, const T* table, const T* z, con
       if constexpr (kTunable) {
         if (zt == 2) return go(std::integral_constant<int, 2>());
       }
-      go(std::integral_constant<int, kTunable ? 4 : 2>());
+      go(std::integral_constant<int, 4>());
     });
   } else {
     if (clouds != 1 || beta_dev) throw Error(PR_ERR_INTERNAL, "packed SpMV needs depth >= 4");
@@ -2226,7 +2224,7 @@ void mg_apply(cudaStream_t s, const LevelCoef& L, const T* x, T* y) {
   const uint32_t D = L.depth;
   if (D < 4 || L.has_faces) throw Error(PR_ERR_INTERNAL, "mg_apply needs the finest level, depth >= 4");
   const size_t sm = n16::smem_bytes<T>();
-  constexpr int ZT = sizeof(T) == 4 ? 4 : 2;
+  constexpr int ZT = 4;
   allow_smem(n16::k_spmv16<T, 3, T, ZT>, sm);
   n16::k_spmv16<T, 3, T, ZT><<<1u << (3 * (D - 4)), n16::Zt<ZT>::NT, sm, s>>>(
       D, x, nullptr, nullptr, (T)0, y, (T)L.c0, (T)L.ce, (T)L.cc, nullptr, nullptr, nullptr);
@@ -2239,8 +2237,8 @@ void mg_resid_update(cudaStream_t s, const LevelCoef& L, const double* x, const 
   const uint32_t D = L.depth;
   if (D < 4 || L.has_faces) throw Error(PR_ERR_INTERNAL, "mg_resid_update needs the finest level, depth >= 4");
   const size_t sm = n16::smem_bytes<double>();
-  allow_smem(n16::k_spmv16<double, 2, E, 2>, sm);
-  n16::k_spmv16<double, 2, E, 2><<<dim3(1u << (3 * (D - 4)), clouds), n16::Zt<2>::NT, sm, s>>>(
+  allow_smem(n16::k_spmv16<double, 2, E, 4>, sm);
+  n16::k_spmv16<double, 2, E, 4><<<dim3(1u << (3 * (D - 4)), clouds), n16::Zt<4>::NT, sm, s>>>(
       D, x, e, xn, scale, r, L.c0, L.ce, L.cc, b, nullptr, scale_dev);
   PR_CHECK_LAUNCH();
 }
