@@ -177,6 +177,9 @@ struct pr_context {
     PR_CUDA(cudaMemcpyAsync(dst, h_ring + h_ring_used, bytes, cudaMemcpyHostToDevice, stream));
     h_ring_used += need;
   }
+  // pinned slots and events of the copies between pageable host memory and the device (pr_abi.cu)
+  unsigned char* h_slots = nullptr;
+  std::vector<cudaEvent_t> slot_events;
   int* h_flag = nullptr;  // pinned: the status of the last spd_inverse (pr_operator.cu)
   // pinned staging for device->host mesh copies (grown on demand)
   unsigned char* h_stage = nullptr;

@@ -61,3 +61,18 @@ def test_degree2_short_plane_runs(ctx, depth, precision):
     t = oracle.Tree2(depth, unit, 4.0)
     b = t.rhs()
     assert np.linalg.norm(b - t.apply(ctx.coefficients())) <= 1e-9 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("depth,n", [(5, 700_001), (6, 50_000), (7, 20_000)])
+def test_staged_host_copies(ctx, depth, n):
+    """Copies to and from pageable memory on either side of the staging thresholds (32 MiB in; 1 and 8
+    MiB out) give the same bytes as copies to and from pinned memory, which are not staged."""
+    import torch
+    pts = synthetic.sphere(n, seed=70 + depth)
+    params = prb.ReconstructParams(depth=depth, point_weight=4.0)
+    ctx.solve(pts, params)
+    x = ctx.coefficients()
+    ctx.solve(torch.from_numpy(pts).pin_memory().numpy(), params)
+    y = torch.empty(8 ** depth, dtype=torch.float64).pin_memory().numpy()
+    prb._check(prb.lib().pr_ctx_get_coefficients(ctx._h, prb._ptr(y)))
+    assert np.array_equal(x, y)
