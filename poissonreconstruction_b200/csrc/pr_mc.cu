@@ -12,8 +12,8 @@
 //   1. per cell: case index; per block of cells: active-cell count      (k_mc_count)
 //   2. exclusive scan; active cells written in Morton order             (k_mc_compact)
 //   3. per active cell: vertex slots (cell order, then edge order) with position and key
-//   4. stable sort of slots by key; the first slot of each key run is its vertex; vertex
-//      ids = rank of first slots in slot order (= the crate's first-appearance numbering)
+//   4. a hash table of the keys holds the first slot of each, which is its vertex; vertex ids =
+//      rank of first slots in slot order (= the crate's first-appearance numbering)
 //   5. triangles from the packed table, vertices back-transformed to model space.
 // Corner values at integer grid positions reduce to a shifted gather (the evaluation is
 // offset by one cell, src/fem_tree.rs:645-649): node k-1 per axis, none at k = 0 and the
@@ -240,14 +240,22 @@ __global__ void k_iso_partial(const double* __restrict__ x, uint32_t D, const do
   }
 }
 
-__global__ void k_iso_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
-  if (threadIdx.x != 0) return;
+// the partials in order, one chain (thread 0); staged through shared memory, from which the chain reads
+// ahead (from global memory it waited for every load): 90 -> 40 us at 1M points, 30 -> 15 at 100k
+__global__ void __launch_bounds__(kThreads) k_iso_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
+  __shared__ double s[2 * kThreads];
   Neu t{0.0, 0.0};
-  for (int i = 0; i < nb; ++i) {
-    t = neu_add(t, part[2 * i]);
-    t = neu_add(t, part[2 * i + 1]);
+  for (int b = 0; b < nb; b += kThreads) {
+    const int m = min(kThreads, nb - b);
+    for (int i = threadIdx.x; i < 2 * m; i += kThreads) s[i] = part[2 * b + i];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll 8
+      for (int i = 0; i < 2 * m; ++i) t = neu_add(t, s[i]);
+    }
+    __syncthreads();
   }
-  out[0] = t.s + t.c;
+  if (threadIdx.x == 0) out[0] = t.s + t.c;
 }
 
 // ------------------------------------------------------------------ marching cubes
@@ -297,8 +305,8 @@ __global__ void k_mc_compact(const double* __restrict__ x, uint32_t D, double is
 template <int DEG>
 __global__ void k_mc_vertices(const double* __restrict__ x, uint32_t D, double iso, const uint32_t* __restrict__ acell,
                               uint64_t A, const uint32_t* __restrict__ eoff, double* __restrict__ pos,
-                              uint64_t* __restrict__ k1, uint32_t* __restrict__ k2, uint32_t* __restrict__ slot_id,
-                              uint64_t E, int* __restrict__ err) {
+                              uint64_t* __restrict__ k1, uint32_t* __restrict__ k2, uint64_t E,
+                              int* __restrict__ err) {
   const int res = 1 << D;
   const double w = 1.0 / (double)res;  // (max_res >> d) as f64 / max_res as f64
   for (uint64_t a = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; a < A; a += (uint64_t)gridDim.x * blockDim.x) {
@@ -327,28 +335,42 @@ __global__ void k_mc_vertices(const double* __restrict__ x, uint32_t D, double i
       if (key[0] >= (1ull << 30) || key[1] >= (1ull << 30) || key[2] >= (1ull << 30)) atomicOr(err, 1);
       k1[sl] = (key[0] << 30) | (key[1] & ((1ull << 30) - 1));
       k2[sl] = (uint32_t)(key[2] & ((1u << 30) - 1));
-      slot_id[sl] = sl;
       ++sl;
     }
   }
 }
 
-// head[i] = sorted position i starts a run of equal keys
-__global__ void k_mc_heads(const uint64_t* __restrict__ k1s, const uint32_t* __restrict__ k2s,
-                           const uint32_t* __restrict__ slots, uint64_t E, uint32_t* __restrict__ repflag,
-                           uint32_t* __restrict__ headpos) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < E; i += (uint64_t)gridDim.x * blockDim.x) {
-    bool head = (i == 0) || k1s[i] != k1s[i - 1] || k2s[i] != k2s[i - 1];
-    repflag[slots[i]] = head ? 1u : 0u;
-    headpos[i] = head ? (uint32_t)i : 0u;
+// Vertices are slots with equal keys.  An open-addressing table (a power of two, 2 E entries or more)
+// takes each key once; its entry ends as the smallest slot of that key, whatever the order of the
+// insertions.  home[s] = the entry of slot s's key.  Scattered reads and atomics in L2 bound it: 46 us for
+// the mesh of depth 9, k_mc_first 15, and k_mc_emit_tris 24 more than with ids in slot order.  An LSD radix
+// sort of the 90-bit keys, two gathers and two passes over the runs, which stood here, took about 0.5 ms,
+// and 35 launches more at depth 5, where the mesh as a whole went from 1.62 to 1.48 ms.
+constexpr uint32_t kNoSlot = 0xffffffffu;
+__global__ void k_mc_hash(const uint64_t* __restrict__ k1, const uint32_t* __restrict__ k2, uint64_t E, uint32_t mask,
+                          uint32_t* __restrict__ table, uint32_t* __restrict__ home) {
+  for (uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s < E; s += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t a = k1[s];
+    const uint32_t b = k2[s];
+    uint64_t h = (a ^ ((uint64_t)b << 29)) * 0x9e3779b97f4a7c15ull;
+    h ^= h >> 32;
+    uint32_t e = (uint32_t)(h * 0xd6e8feb86659fd93ull >> 32) & mask;
+    for (uint32_t probe = 0; probe < mask; ++probe, e = (e + 1) & mask) {  // ends early: entries stay free
+      const uint32_t old = atomicCAS(table + e, kNoSlot, (uint32_t)s);
+      if (old == kNoSlot) break;
+      if (k1[old] == a && k2[old] == b) {
+        if ((uint32_t)s < old) atomicMin(table + e, (uint32_t)s);
+        break;
+      }
+    }
+    home[s] = e;
   }
 }
-
-// after an inclusive max-scan, headpos[i] = start of i's run
-__global__ void k_mc_assign(const uint32_t* __restrict__ slots, const uint32_t* __restrict__ headpos, uint64_t E,
-                            const uint32_t* __restrict__ vid_rep, uint32_t* __restrict__ vid) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < E; i += (uint64_t)gridDim.x * blockDim.x)
-    vid[slots[i]] = vid_rep[slots[headpos[i]]];
+// first[s] = slot s is the first of its key
+__global__ void k_mc_first(const uint32_t* __restrict__ table, const uint32_t* __restrict__ home, uint64_t E,
+                           uint32_t* __restrict__ first) {
+  for (uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s < E; s += (uint64_t)gridDim.x * blockDim.x)
+    first[s] = table[home[s]] == (uint32_t)s ? 1u : 0u;
 }
 
 struct Mat16 {
@@ -376,7 +398,8 @@ __global__ void k_mc_emit_vertices(const double* __restrict__ pos, uint64_t E, c
 }
 
 __global__ void k_mc_emit_tris(const uint8_t* __restrict__ acase, uint64_t A, const uint32_t* __restrict__ eoff,
-                               const uint32_t* __restrict__ toff, const uint32_t* __restrict__ vid,
+                               const uint32_t* __restrict__ toff, const uint32_t* __restrict__ table,
+                               const uint32_t* __restrict__ home, const uint32_t* __restrict__ vid_rep,
                                uint64_t* __restrict__ tris) {
   for (uint64_t a = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; a < A; a += (uint64_t)gridDim.x * blockDim.x) {
     uint32_t mc = acase[a];
@@ -388,7 +411,7 @@ __global__ void k_mc_emit_tris(const uint8_t* __restrict__ acase, uint64_t A, co
     for (uint32_t i = 0; i < 3 * nt; ++i) {
       uint32_t e = (uint32_t)((packed >> (4 * i)) & 15ull);
       uint32_t rank = __popc(em & ((1u << e) - 1u));
-      tris[3 * t0 + i] = vid[e0 + rank];
+      tris[3 * t0 + i] = vid_rep[table[home[e0 + rank]]];
     }
   }
 }
@@ -624,31 +647,6 @@ __global__ void k_scatter_ids(const uint32_t* __restrict__ flag, const uint32_t*
 }
 
 // ====================================================================== host stages
-namespace {
-__global__ void k_gather_u64(const uint64_t* __restrict__ v, const uint32_t* __restrict__ perm, uint64_t E,
-                             uint64_t* __restrict__ out) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < E; i += (uint64_t)gridDim.x * blockDim.x)
-    out[i] = v[perm[i]];
-}
-__global__ void k_gather_u32(const uint32_t* __restrict__ v, const uint32_t* __restrict__ perm, uint64_t E,
-                             uint32_t* __restrict__ out) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < E; i += (uint64_t)gridDim.x * blockDim.x)
-    out[i] = v[perm[i]];
-}
-}  // namespace
-
-void mc_gather_u64(cudaStream_t s, const uint64_t* v, const uint32_t* perm, uint64_t E, uint64_t* out) {
-  k_gather_u64<<<grid_for(E), kThreads, 0, s>>>(v, perm, E, out);
-  PR_CHECK_LAUNCH();
-}
-void mc_gather_u32(cudaStream_t s, const uint32_t* v, const uint32_t* perm, uint64_t E, uint32_t* out) {
-  k_gather_u32<<<grid_for(E), kThreads, 0, s>>>(v, perm, E, out);
-  PR_CHECK_LAUNCH();
-}
-
-struct MaxOp {
-  __device__ __forceinline__ uint32_t operator()(uint32_t a, uint32_t b) const { return a > b ? a : b; }
-};
 void evaluate_points(pr_context* c, uint32_t D, const double* d_x64, const double* d_pts, uint64_t stride,
                      uint64_t n, double* d_out, int degree) {
   if (n == 0) return;
@@ -669,7 +667,7 @@ double stage_iso(pr_context* c, const double* d_x64, bool natural) {
   else if (c->degree == 2) k_iso_partial<2><<<nb, kThreads, 0, c->stream>>>(d_x64, c->D, up, P, part);
   else k_iso_partial<1><<<nb, kThreads, 0, c->stream>>>(d_x64, c->D, up, P, part);
   PR_CHECK_LAUNCH();
-  k_iso_final<<<1, 32, 0, c->stream>>>(part, nb, out);
+  k_iso_final<<<1, kThreads, 0, c->stream>>>(part, nb, out);
   PR_CHECK_LAUNCH();
   double sum = 0.0;
   PR_CUDA(cudaMemcpyAsync(&sum, out, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -774,55 +772,32 @@ void stage_extract(pr_context* c, uint32_t D, const double* x, double iso, bool 
   double* pos = c->buf<double>("mc_pos", 3 * E);
   uint64_t* k1 = c->buf<uint64_t>("mc_k1", E);
   uint32_t* k2 = c->buf<uint32_t>("mc_k2", E);
-  uint32_t* sid = c->buf<uint32_t>("mc_sid", E);
-  uint64_t* k1b = c->buf<uint64_t>("mc_k1b", E);
-  uint32_t* k2b = c->buf<uint32_t>("mc_k2b", E);
-  uint32_t* sidb = c->buf<uint32_t>("mc_sidb", E);
   int* err = c->buf<int>("mc_err", 1);
   PR_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
   if (degree == 2 && natural)
-    k_mc_vertices<3><<<grid_for(A), kThreads, 0, s>>>(x, D, iso, acell, A, eoff, pos, k1, k2, sid, E, err);
+    k_mc_vertices<3><<<grid_for(A), kThreads, 0, s>>>(x, D, iso, acell, A, eoff, pos, k1, k2, E, err);
   else if (degree == 2)
-    k_mc_vertices<2><<<grid_for(A), kThreads, 0, s>>>(x, D, iso, acell, A, eoff, pos, k1, k2, sid, E, err);
-  else k_mc_vertices<1><<<grid_for(A), kThreads, 0, s>>>(x, D, iso, acell, A, eoff, pos, k1, k2, sid, E, err);
+    k_mc_vertices<2><<<grid_for(A), kThreads, 0, s>>>(x, D, iso, acell, A, eoff, pos, k1, k2, E, err);
+  else k_mc_vertices<1><<<grid_for(A), kThreads, 0, s>>>(x, D, iso, acell, A, eoff, pos, k1, k2, E, err);
   PR_CHECK_LAUNCH();
 
-  // stable LSD sort: by k2 (z key), then by k1 (x,y key); ties keep slot order
-  size_t b1 = 0, b2 = 0;
-  PR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, b1, k2, k2b, sid, sidb, (int64_t)E, 0, 30, s));
-  PR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, b2, k1, k1b, sidb, sid, (int64_t)E, 0, 60, s));
-  tb = std::max(b1, b2);
-  tmp = c->buf<char>("cub_tmp", tb);
-  PR_COUNT_PRIMITIVE();
-  PR_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, k2, k2b, sid, sidb, (int64_t)E, 0, 30, s));
-  // k1 in the order of the first sort
-  uint64_t* k1g = c->buf<uint64_t>("mc_k1g", E);
-  mc_gather_u64(s, k1, sidb, E, k1g);
-  PR_COUNT_PRIMITIVE();
-  PR_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, k1g, k1b, sidb, sid, (int64_t)E, 0, 60, s));
-  // sorted: k1b (x,y keys), sid (slots); need the z keys in the same order
-  uint32_t* k2s = c->buf<uint32_t>("mc_k2s", E);
-  mc_gather_u32(s, k2, sid, E, k2s);
-
-  uint32_t* repflag = c->buf<uint32_t>("mc_rep", E + 1);
-  uint32_t* headpos = c->buf<uint32_t>("mc_head", E);
+  uint64_t cap = 1024;  // E < 2^32 - 1, so 2^32 entries always have room
+  while (cap < 2 * E && cap < (1ull << 32)) cap *= 2;
+  uint32_t* table = c->buf<uint32_t>("mc_table", cap);
+  uint32_t* home = c->buf<uint32_t>("mc_home", E);
+  uint32_t* first = c->buf<uint32_t>("mc_first", E + 1);
   uint32_t* vid_rep = c->buf<uint32_t>("mc_vidrep", E + 1);
-  uint32_t* vid = c->buf<uint32_t>("mc_vid", E);
-  k_mc_heads<<<grid_for(E), kThreads, 0, s>>>(k1b, k2s, sid, E, repflag, headpos);
+  PR_CUDA(cudaMemsetAsync(table, 0xff, cap * sizeof(uint32_t), s));
+  k_mc_hash<<<grid_for(E), kThreads, 0, s>>>(k1, k2, E, (uint32_t)(cap - 1), table, home);
   PR_CHECK_LAUNCH();
-  PR_CUDA(cudaMemsetAsync(repflag + E, 0, sizeof(uint32_t), s));
-  size_t b3 = 0, b4 = 0;
-  PR_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b3, repflag, vid_rep, (int64_t)E + 1, s));
-  uint32_t* headrun = c->buf<uint32_t>("mc_headrun", E);
-  PR_CUDA(cub::DeviceScan::InclusiveScan(nullptr, b4, headpos, headrun, MaxOp(), (int64_t)E, s));
-  tb = std::max(b3, b4);
+  k_mc_first<<<grid_for(E), kThreads, 0, s>>>(table, home, E, first);
+  PR_CHECK_LAUNCH();
+  PR_CUDA(cudaMemsetAsync(first + E, 0, sizeof(uint32_t), s));
+  tb = 0;
+  PR_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, first, vid_rep, (int64_t)E + 1, s));
   tmp = c->buf<char>("cub_tmp", tb);
   PR_COUNT_PRIMITIVE();
-  PR_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, repflag, vid_rep, (int64_t)E + 1, s));
-  PR_COUNT_PRIMITIVE();
-  PR_CUDA(cub::DeviceScan::InclusiveScan(tmp, tb, headpos, headrun, MaxOp(), (int64_t)E, s));
-  k_mc_assign<<<grid_for(E), kThreads, 0, s>>>(sid, headrun, E, vid_rep, vid);
-  PR_CHECK_LAUNCH();
+  PR_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, first, vid_rep, (int64_t)E + 1, s));
   uint32_t hNV = 0;
   int herr = 0;
   PR_CUDA(cudaMemcpyAsync(&hNV, vid_rep + E, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -834,9 +809,9 @@ void stage_extract(pr_context* c, uint32_t D, const double* x, double iso, bool 
   uint64_t* tris = c->buf<uint64_t>("mesh_t", 3 * NT);
   Mat16 mi;
   for (int k = 0; k < 16; ++k) mi.m[k] = c->Minv[k];
-  k_mc_emit_vertices<<<grid_for(E), kThreads, 0, s>>>(pos, E, repflag, vid_rep, back_transform ? 1 : 0, mi, verts);
+  k_mc_emit_vertices<<<grid_for(E), kThreads, 0, s>>>(pos, E, first, vid_rep, back_transform ? 1 : 0, mi, verts);
   PR_CHECK_LAUNCH();
-  k_mc_emit_tris<<<grid_for(A), kThreads, 0, s>>>(acase, A, eoff, toff, vid, tris);
+  k_mc_emit_tris<<<grid_for(A), kThreads, 0, s>>>(acase, A, eoff, toff, table, home, vid_rep, tris);
   PR_CHECK_LAUNCH();
   c->nv = NV;
   c->nt = NT;

@@ -76,3 +76,19 @@ def test_staged_host_copies(ctx, depth, n):
     y = torch.empty(8 ** depth, dtype=torch.float64).pin_memory().numpy()
     prb._check(prb.lib().pr_ctx_get_coefficients(ctx._h, prb._ptr(y)))
     assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("side,low", [(0, 0.0), (1, 0.0), (2, 0.0), (4, 0.0), (5, 0.0), (8, 0.0), (4, 0.5)])
+def test_vertex_table(ctx, side, low):
+    """Cubes of raised coefficients in a level field: no slot, a few, slots on both sides of the smallest
+    table (1,024 entries for 512 slots, four to a vertex), and the level at the iso value, where vertices
+    fall on corners and share keys."""
+    depth = 4
+    xyz = np.stack(np.meshgrid(*[np.arange(16)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    code = sum(((xyz[:, a] >> b) & 1) << (3 * b + a) for a in range(3) for b in range(depth))
+    field = np.empty(16 ** 3)
+    field[code] = np.where(((xyz >= 4) & (xyz < 4 + side)).all(1), 2.0, low)
+    mesh = ctx.extract(field, 0.5, depth=depth)
+    v_ref, t_ref = oracle.extract_surface(depth, field, 0.5)
+    assert np.array_equal(mesh.vertices, v_ref)
+    assert np.array_equal(mesh.triangles, t_ref)
