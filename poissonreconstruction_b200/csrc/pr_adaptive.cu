@@ -369,175 +369,276 @@ __global__ void __launch_bounds__(kThreads) k_ab_rhs(const uint32_t* __restrict_
 // ------------------------------------------------------------------ the band operator
 // One brick per CTA iteration, kOpThreads threads.  The brick and its 2-node halo (a 12^3 tile,
 // gathered from the 27 neighbouring bricks, zero outside the band) go to shared memory; the
-// stencil h (S M M + M S M + M M S) + wg then runs as three register passes: a thread per (x, y)
-// column filters z (M and S), a thread per (x, z) column filters y, a thread per (y, z) row filters
-// x and writes its 8 outputs as two 16-byte stores.
+// stencil h (S M M + M S M + M M S) + wg then runs as three register passes: a thread per pair of
+// (x, y) columns filters z (M and S), a thread per pair of (x, z) columns filters y, a thread per
+// (y, z) row filters x and writes its 8 outputs as two 16-byte stores.
 //   kBandApply: y = A x          kBandResid: y = f - A x
-//   kBandDir:   the CG direction step: d = z + beta dold (dold = x, z = f; x unread when beta = 0)
+//   kBandDir:   the CG direction step: d = z + beta dold (dold = x, z = f; x unread on the first pass)
 //               formed while gathering, written to dout (a buffer other than x: neighbouring CTAs
-//               still gather dold) for the brick, and y = A d with per-CTA partials of d . y
+//               still gather dold) for the brick, and y = A d with per-CTA partials of d . y; e += alpha
+//               dold, the last iteration's step (e null on the first pass), rides on the same loads
 // GSRC (kBandResid, FP64): the tile is the prolonged coarse function on every node (x unused):
 // y = f - (K + wg I) g on the band.
-constexpr int kOpThreads = 160;
-constexpr int kWS = 13;  // row stride of the y-filtered planes (conflict-free x pass)
+// Bound by the latency of the gather and the L1 / shared-memory pipe.  So: the next brick's gather is in
+// flight while the y and x passes work on this one; a tile plane holds its 12 rows' 8 own values, then
+// their 4 side values (x = -2, -1, 8, 9), so that the gather is 16-byte copies by consecutive lanes
+// (cp.async) and 8-byte loads (through registers: cheaper there than as 8-byte copies); planes are padded against bank conflicts; the z and y passes work on pairs
+// (64-bit shared accesses, two FP32 FMAs to an instruction).  FP32 at 245M nodes (depth 11): operator and
+// update pass 3.04 -> 2.61 ms an iteration (1.76 + 1.29 -> 1.84 + 0.77; the traffic of the two vectors
+// formed here takes 0.91 of the 1.84), with 75 % of the shared-memory pipe's cycles used.
+constexpr int kOpThreads = 96;
+constexpr int kOpCtas = 8;       // per SM (shared memory, registers); the grid is one wave of them
+constexpr int kTP = 144;         // tile plane: [y 12][8], then [y 12][4]
+constexpr int kFO = 104;         // z-filtered plane, own columns [y 12][8]
+constexpr int kFS = 52;          // side columns [y 12][4]
+constexpr int kFW = 8 * (kFO + kFS);
+constexpr int kWP = 8 * 12 + 8;  // y-filtered plane: [y 8][12]; the y pass puts them over the z pass's
+static_assert(8 * kWP <= kFW, "y-filtered planes fit the z-filtered ones");
 enum { kBandApply = 0, kBandResid = 1, kBandDir = 2 };
 
 template <typename T>
-constexpr size_t band_op_smem(bool gsrc) {
-  return (size_t)(kOT3 + 2 * 8 * kOT * kOT + 2 * 8 * 8 * kWS) * sizeof(T) +
+constexpr size_t band_op_smem(int mode, bool gsrc) {
+  return (size_t)((mode == kBandDir ? 2 : 1) * kOT * kTP + 2 * kFW + kBN) * sizeof(T) +
          (gsrc ? (size_t)(kProlongScratch(kOT) + kOT3) * sizeof(double) : 0);
 }
 
-// 12 values of a tile row from the band vector v: brick sl[0] at x = 6, 7, sl[1] at x = 0..7,
-// sl[2] at x = 0, 1 of the row at offset rowoff; zero for kSent
-template <typename T>
-__device__ __forceinline__ void ab_load_row(const T* __restrict__ v, const uint32_t* sl, int rowoff, T* out) {
-#pragma unroll
-  for (int k = 0; k < kOT; ++k) out[k] = T(0);
-  if (sl[0] != kSent) {
-    const T* p = v + (uint64_t)sl[0] * kBN + rowoff + 6;
-    out[0] = p[0];
-    out[1] = p[1];
-  }
-  if (sl[1] != kSent) {
-    const T* p = v + (uint64_t)sl[1] * kBN + rowoff;
-    if (sizeof(T) == 4) {
-      const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
-      out[2] = (T)a.x; out[3] = (T)a.y; out[4] = (T)a.z; out[5] = (T)a.w;
-      out[6] = (T)b.x; out[7] = (T)b.y; out[8] = (T)b.z; out[9] = (T)b.w;
-    } else {
-#pragma unroll
-      for (int k = 0; k < 8; k += 2) {
-        const double2 a = *reinterpret_cast<const double2*>(p + k);
-        out[2 + k] = (T)a.x;
-        out[3 + k] = (T)a.y;
-      }
-    }
-  }
-  if (sl[2] != kSent) {
-    const T* p = v + (uint64_t)sl[2] * kBN + rowoff;
-    out[10] = p[0];
-    out[11] = p[1];
-  }
+// asynchronous copy of 16 bytes to shared memory; zeros where !ok (p is not read then)
+__device__ __forceinline__ void ab_copy16(void* to, const void* p, bool ok) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(to), n = ok ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a), "l"(p), "r"(n) : "memory");
 }
+
+// two values to an instruction where the unit has it (FP32)
 template <typename T>
-__device__ __forceinline__ void ab_store8(T* __restrict__ p, const T* v) {
-  if (sizeof(T) == 4) {
-    *reinterpret_cast<float4*>(p) = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
-    *reinterpret_cast<float4*>(p + 4) = make_float4((float)v[4], (float)v[5], (float)v[6], (float)v[7]);
-  } else {
-#pragma unroll
-    for (int k = 0; k < 8; k += 2) *reinterpret_cast<double2*>(p + k) = make_double2((double)v[k], (double)v[k + 1]);
+struct Two;
+template <>
+struct Two<float> {
+  typedef float2 V;
+  typedef unsigned long long K;
+  static __device__ __forceinline__ K dup(float k) {
+    K r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(k));
+    return r;
   }
+  static __device__ __forceinline__ V fma(K k, V v, V acc) {
+    unsigned long long d, a, b;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(v.x), "f"(v.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(acc.x), "f"(acc.y));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(k), "l"(a), "l"(b));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(acc.x), "=f"(acc.y) : "l"(d));
+    return acc;
+  }
+};
+template <>
+struct Two<double> {
+  typedef double2 V;
+  typedef double K;
+  static __device__ __forceinline__ K dup(double k) { return k; }
+  static __device__ __forceinline__ V fma(K k, V v, V acc) {
+    return make_double2(::fma(k, v.x, acc.x), ::fma(k, v.y, acc.y));
+  }
+};
+
+__device__ __forceinline__ void ab_load4(const float* p, float* v) {
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
 }
-template <typename T>
-__device__ __forceinline__ void ab_store_tile_row(T* p, const T* v) {
-  if (sizeof(T) == 4) {
-#pragma unroll
-    for (int k = 0; k < kOT; k += 4)
-      *reinterpret_cast<float4*>(p + k) = make_float4((float)v[k], (float)v[k + 1], (float)v[k + 2], (float)v[k + 3]);
-  } else {
-#pragma unroll
-    for (int k = 0; k < kOT; k += 2) *reinterpret_cast<double2*>(p + k) = make_double2((double)v[k], (double)v[k + 1]);
-  }
+__device__ __forceinline__ void ab_load4(const double* p, double* v) {
+  const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void ab_store4(float* p, const float* v) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void ab_store4(double* p, const double* v) {
+  *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+  *reinterpret_cast<double2*>(p + 2) = make_double2(v[2], v[3]);
 }
 
 template <typename T, int MODE, bool GSRC>
-__global__ void __launch_bounds__(kOpThreads) k_ab_op(const T* __restrict__ x, const T* __restrict__ f,
-                                                      T* __restrict__ y, T* __restrict__ dout, double beta,
-                                                      const uint32_t* __restrict__ nbr,
-                                                      const uint32_t* __restrict__ bkey, uint64_t NB, BandCoef<T> K,
-                                                      const double* __restrict__ xc, Prolong W, int res,
-                                                      double* __restrict__ part) {
+__global__ void __launch_bounds__(kOpThreads, sizeof(T) == 4 ? kOpCtas : 4)
+    k_ab_op(const T* __restrict__ x, const T* __restrict__ f, T* __restrict__ y, T* __restrict__ dout, double beta,
+            double alpha, T* __restrict__ e, const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ bkey,
+            uint64_t NB, BandCoef<T> K, const double* __restrict__ xc, Prolong W, int res, double* __restrict__ part) {
+  typedef Two<T> T2;
+  typedef typename T2::V V;
+  typedef typename T2::K KK;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* tile = reinterpret_cast<T*>(smem_raw);   // [z][y][x], 12^3
-  T* um = tile + kOT3;                         // [z 8][y 12][x 12]
-  T* us = um + 8 * kOT * kOT;
-  T* w1 = us + 8 * kOT * kOT;                  // [z 8][y 8][x kWS]
-  T* w23 = w1 + 8 * 8 * kWS;
-  double* gs = reinterpret_cast<double*>(w23 + 8 * 8 * kWS);  // GSRC: prolongation scratch, then the tile
+  T* tile = reinterpret_cast<T*>(smem_raw);                 // [z 12][kTP]
+  T* told = tile + kOT * kTP;                                // kBandDir: dold, own values
+  T* um = MODE == kBandDir ? told + kOT * kTP : told;        // M z-filtered: [z 8][kFO], [z 8][kFS]
+  T* us = um + kFW;                                          // S z-filtered
+  T *w1 = um, *w23 = us;                                     // [z 8][kWP]
+  T* ctr = us + kFW;                                         // the brick's own values
+  double* gs = reinterpret_cast<double*>(ctr + kBN);         // GSRC: prolongation scratch, then the tile
   __shared__ uint32_t nb[27];
   __shared__ double red[kOpThreads / 32 + 1];
   const int t = threadIdx.x;
-  const T tb = (T)beta;
+  const T tb = (T)beta, ta = (T)alpha;
+  const bool old = MODE == kBandDir && (beta != 0.0 || e);
   double dacc = 0.0;
-  for (uint64_t slot = blockIdx.x; slot < NB; slot += gridDim.x) {
-    if (t < 27) nb[t] = nbr[27 * slot + t];
+  // the gather: rows (y, z) of the tile, two items (halves, sides) to a row; a thread's three rows lie
+  // four planes apart
+  const int gy = (t >> 1) % kOT, gz = (t >> 1) / kOT, gh = t & 1;
+  const int ly = gy - 2, oy = ly < 0 ? -1 : (ly >= 8 ? 1 : 0);
+  V sv[3], sw[3];
+  auto gather = [&]() {
+    const T* src = MODE == kBandDir ? f : x;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const int lz = gz + 4 * r - 2, oz = lz < 0 ? -1 : (lz >= 8 ? 1 : 0);
+      const int rowoff = ((lz - 8 * oz) << 6) | ((ly - 8 * oy) << 3), kb = (oz + 1) * 9 + (oy + 1) * 3;
+      const uint32_t bc = nb[kb + 1], bs = nb[kb + 2 * gh];
+      const uint64_t oc = bc == kSent ? 0 : (uint64_t)bc * kBN + rowoff + 4 * gh;
+      const uint64_t os = bs == kSent ? 0 : (uint64_t)bs * kBN + rowoff + (gh ? 0 : 6);
+      const int tc = (gz + 4 * r) * kTP + 8 * gy + 4 * gh;
+      sv[r].x = sv[r].y = sw[r].x = sw[r].y = T(0);
+#pragma unroll
+      for (int k = 0; k < 4; k += 16 / sizeof(T)) ab_copy16(tile + tc + k, src + oc + k, bc != kSent);
+      if (bs != kSent) sv[r] = *reinterpret_cast<const V*>(src + os);
+      if (old) {
+#pragma unroll
+        for (int k = 0; k < 4; k += 16 / sizeof(T)) ab_copy16(told + tc + k, x + oc + k, bc != kSent);
+        if (bs != kSent) sw[r] = *reinterpret_cast<const V*>(x + os);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (!GSRC && blockIdx.x < NB) {
+    if (t < 27) nb[t] = nbr[27 * (uint64_t)blockIdx.x + t];
     __syncthreads();
+    gather();
+  }
+  for (uint64_t slot = blockIdx.x; slot < NB; slot += gridDim.x) {
+    const bool more = slot + gridDim.x < NB;
+    uint32_t next = kSent;
+    V ev[8];
+    // own columns of the brick's own rows: y = t / 4 - 2, x = 2 (t % 4)
+    const bool mine = t >= 8 && t < 40;
+    const uint64_t g1 = slot * kBN + (uint64_t)(2 * (t - 8));
     if (GSRC) {
       uint32_t bx, by, bz;
       unmorton3(bkey[slot], bx, by, bz);
       double* gt = gs + kProlongScratch(kOT);
       prolong_tile<kOT>(xc, W, res, 8 * (int)bx - 2, 8 * (int)by - 2, 8 * (int)bz - 2, gs, gt);
-      for (int i = t; i < kOT3; i += kOpThreads) tile[i] = (T)gt[i];
-    } else if (t < kOT * kOT) {
-      // a thread per tile row (y, z): 2 values of the left neighbour brick (its x = 6, 7), 8 of the
-      // centre one, 2 of the right one (x = 0, 1), as vector loads
-      const int ly = t % kOT - 2, lz = t / kOT - 2;
-      const int oy = ly < 0 ? -1 : (ly >= 8 ? 1 : 0), oz = lz < 0 ? -1 : (lz >= 8 ? 1 : 0);
-      const int rowoff = ((lz - 8 * oz) << 6) | ((ly - 8 * oy) << 3);
-      const int kb = (oz + 1) * 9 + (oy + 1) * 3;
-      const uint32_t sl[3] = {nb[kb], nb[kb + 1], nb[kb + 2]};
-      T v[kOT];
-      ab_load_row<T>(MODE == kBandDir ? f : x, sl, rowoff, v);
-      if (MODE == kBandDir) {
-        if (beta != 0.0) {
-          T w[kOT];
-          ab_load_row<T>(x, sl, rowoff, w);
-#pragma unroll
-          for (int k = 0; k < kOT; ++k) v[k] += tb * w[k];
-        }
-        if (oy == 0 && oz == 0) ab_store8<T>(dout + slot * kBN + rowoff, v + 2);
+      for (int i = t; i < kOT3; i += kOpThreads) {
+        const int ix = i % kOT - 2, iy = (i / kOT) % kOT, iz = i / (kOT * kOT);
+        const int w = ix >= 0 && ix < 8 ? 8 * iy + ix : 96 + 4 * iy + (ix < 0 ? ix + 2 : ix - 6);
+        tile[iz * kTP + w] = (T)gt[i];
       }
-      ab_store_tile_row<T>(tile + t * kOT, v);
-    }    __syncthreads();
-    if (t < kOT * kOT) {  // z filter of column (x, y)
-      T v[kOT];
+    } else {
+      if (t < 27 && more) next = nbr[27 * (slot + gridDim.x) + t];
+      if (MODE == kBandDir && e && mine) {
 #pragma unroll
-      for (int z = 0; z < kOT; ++z) v[z] = tile[z * kOT * kOT + t];
-#pragma unroll
-      for (int z = 0; z < 8; ++z) {
-        T am = T(0), as = T(0);
-#pragma unroll
-        for (int c = 0; c < 5; ++c) {
-          am += K.m[c] * v[z + c];
-          as += K.s[c] * v[z + c];
-        }
-        um[z * kOT * kOT + t] = am;
-        us[z * kOT * kOT + t] = as;
+        for (int z = 0; z < 8; ++z) ev[z] = *reinterpret_cast<const V*>(e + g1 + 64 * z);
       }
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        if (MODE == kBandDir && beta != 0.0) {
+          sv[r].x += tb * sw[r].x;
+          sv[r].y += tb * sw[r].y;
+        }
+        *reinterpret_cast<V*>(tile + (gz + 4 * r) * kTP + 96 + 4 * gy + 2 * gh) = sv[r];
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
     }
     __syncthreads();
-    if (t < 8 * kOT) {  // y filter of column (x, z)
-      const int xx = t % kOT, z = t / kOT;
-      T a[kOT], b[kOT];
+    KK km[5], ks[5];
 #pragma unroll
-      for (int yy = 0; yy < kOT; ++yy) {
-        a[yy] = um[(z * kOT + yy) * kOT + xx];
-        b[yy] = us[(z * kOT + yy) * kOT + xx];
+    for (int k = 0; k < 5; ++k) {
+      km[k] = T2::dup(K.m[k]);
+      ks[k] = T2::dup(K.s[k]);
+    }
+    if (t < kTP / 2) {  // z filter of a pair of columns (x, y)
+      V v[kOT];
+#pragma unroll
+      for (int z = 0; z < kOT; ++z) v[z] = *reinterpret_cast<const V*>(tile + z * kTP + 2 * t);
+      if (MODE == kBandDir && old && t < 48) {  // own columns (the sides are formed already)
+#pragma unroll
+        for (int z = 0; z < kOT; ++z) {
+          const V w = *reinterpret_cast<const V*>(told + z * kTP + 2 * t);
+          if (beta != 0.0) {
+            v[z].x += tb * w.x;
+            v[z].y += tb * w.y;
+          }
+          if (e && mine && z >= 2 && z < 10) {
+            ev[z - 2].x += ta * w.x;
+            ev[z - 2].y += ta * w.y;
+            *reinterpret_cast<V*>(e + g1 + 64 * (z - 2)) = ev[z - 2];
+          }
+        }
       }
+      if (mine) {
+#pragma unroll
+        for (int z = 0; z < 8; ++z) {
+          *reinterpret_cast<V*>(ctr + 64 * z + 2 * (t - 8)) = v[z + 2];
+          if (MODE == kBandDir) *reinterpret_cast<V*>(dout + g1 + 64 * z) = v[z + 2];
+        }
+      }
+      const int to = t < 48 ? 2 * t : 8 * kFO + 2 * (t - 48), step = t < 48 ? kFO : kFS;
+#pragma unroll
+      for (int z = 0; z < 8; ++z) {
+        V am = {T(0), T(0)}, as = {T(0), T(0)};
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+          am = T2::fma(km[k], v[z + k], am);
+          as = T2::fma(ks[k], v[z + k], as);
+        }
+        *reinterpret_cast<V*>(um + to + z * step) = am;
+        *reinterpret_cast<V*>(us + to + z * step) = as;
+      }
+    }
+    if (!GSRC && t < 27) nb[t] = next;
+    __syncthreads();
+    if (!GSRC && more) gather();  // the tiles are free
+    {  // y filter of a pair of columns (x, z), half of the outputs: two warps for the own columns, one for the sides
+      const bool own = t < 64;
+      const int u = own ? t & 31 : (t - 64) & 15, half = own ? t >> 5 : (t - 64) >> 4;
+      const int z = own ? u >> 2 : u >> 1, xp = own ? u & 3 : u & 1, step = own ? 8 : 4;
+      const int from = (own ? z * kFO : 8 * kFO + z * kFS) + 2 * xp + 4 * half * step;
+      const int to = z * kWP + (own ? 2 * xp : 8 + 2 * xp) + 48 * half;
+      V a[8], b[8], o1[4], o2[4];
 #pragma unroll
       for (int yy = 0; yy < 8; ++yy) {
-        T a1 = T(0), a2 = T(0), a3 = T(0);
+        a[yy] = *reinterpret_cast<const V*>(um + from + yy * step);
+        b[yy] = *reinterpret_cast<const V*>(us + from + yy * step);
+      }
 #pragma unroll
-        for (int c = 0; c < 5; ++c) {
-          a1 += K.m[c] * a[yy + c];
-          a2 += K.s[c] * a[yy + c];
-          a3 += K.m[c] * b[yy + c];
+      for (int yy = 0; yy < 4; ++yy) {
+        V a1 = {T(0), T(0)}, a2 = {T(0), T(0)}, a3 = {T(0), T(0)};
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+          a1 = T2::fma(km[k], a[yy + k], a1);
+          a2 = T2::fma(ks[k], a[yy + k], a2);
+          a3 = T2::fma(km[k], b[yy + k], a3);
         }
-        w1[(z * 8 + yy) * kWS + xx] = a1;
-        w23[(z * 8 + yy) * kWS + xx] = a2 + a3;
+        o1[yy] = a1;
+        o2[yy].x = a2.x + a3.x;
+        o2[yy].y = a2.y + a3.y;
+      }
+      __syncthreads();  // all columns are read
+#pragma unroll
+      for (int yy = 0; yy < 4; ++yy) {
+        *reinterpret_cast<V*>(w1 + to + yy * 12) = o1[yy];
+        *reinterpret_cast<V*>(w23 + to + yy * 12) = o2[yy];
       }
     }
     __syncthreads();
     if (t < 64) {  // x filter of row (y, z), 8 outputs
       const int yy = t % 8, z = t / 8;
-      T p[kOT], q[kOT], o[8];
-#pragma unroll
-      for (int xx = 0; xx < kOT; ++xx) {
-        p[xx] = w1[(z * 8 + yy) * kWS + xx];
-        q[xx] = w23[(z * 8 + yy) * kWS + xx];
-      }
+      T p[kOT], q[kOT], g[8], o[8];  // p, q: x = -2 .. 9
+      const T *r1 = w1 + z * kWP + yy * 12, *r2 = w23 + z * kWP + yy * 12, *rc = ctr + z * 64 + yy * 8;
+      T sd[4];
+      ab_load4(r1, p + 2);
+      ab_load4(r1 + 4, p + 6);
+      ab_load4(r1 + 8, sd);
+      p[0] = sd[0]; p[1] = sd[1]; p[10] = sd[2]; p[11] = sd[3];
+      ab_load4(r2, q + 2);
+      ab_load4(r2 + 4, q + 6);
+      ab_load4(r2 + 8, sd);
+      q[0] = sd[0]; q[1] = sd[1]; q[10] = sd[2]; q[11] = sd[3];
+      ab_load4(rc, g);
+      ab_load4(rc + 4, g + 4);
       const uint64_t g0 = slot * kBN + (uint64_t)(z * 64 + yy * 8);
       T dpart = T(0);  // this row's share of d . q (at most 8 terms, then accumulated in FP64)
 #pragma unroll
@@ -545,15 +646,15 @@ __global__ void __launch_bounds__(kOpThreads) k_ab_op(const T* __restrict__ x, c
         T acc = T(0);
 #pragma unroll
         for (int c = 0; c < 5; ++c) acc += K.s[c] * p[xx + c] + K.m[c] * q[xx + c];
-        const T ctr = tile[((z + 2) * kOT + yy + 2) * kOT + xx + 2];
-        o[xx] = K.H * acc + K.wg * ctr;
+        o[xx] = K.H * acc + K.wg * g[xx];
         if (MODE == kBandResid) o[xx] = f[g0 + xx] - o[xx];
-        if (MODE == kBandDir) dpart += ctr * o[xx];
+        if (MODE == kBandDir) dpart += g[xx] * o[xx];
       }
       if (MODE == kBandDir) dacc += (double)dpart;
-      ab_store8<T>(y + g0, o);
+      ab_store4(y + g0, o);
+      ab_store4(y + g0 + 4, o + 4);
     }
-    __syncthreads();
+    if (GSRC) __syncthreads();
   }
   if (MODE == kBandDir && part) {
 #pragma unroll
@@ -616,16 +717,21 @@ __global__ void k_ab_dinv_screen(const uint32_t* __restrict__ run_key, const dou
   for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < T_runs; r += (uint64_t)gridDim.x * blockDim.x)
     dinv[run_key[r]] = (T)(1.0 / (diag + wh3 * sphi2[r]));
 }
-// the CG update with the Jacobi step: x += alpha d, r -= alpha q, z = dinv r; per-block sums of
-// r . r (part[2 b]) and r . z (part[2 b + 1]) in FP64
+// x += alpha d: the last iteration's step (the others ride on the next operator pass)
 template <typename T>
-__global__ void k_ab_update(uint64_t n, double alpha, const T* __restrict__ d, const T* __restrict__ q,
-                            T* __restrict__ x, T* __restrict__ r, const T* __restrict__ dinv, T* __restrict__ z,
-                            double* __restrict__ part) {
+__global__ void k_ab_step(uint64_t n, double alpha, const T* __restrict__ d, T* __restrict__ x) {
+  const T a = (T)alpha;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    x[i] += a * d[i];
+}
+// the CG update with the Jacobi step: r -= alpha q, z = dinv r; per-block sums of r . r (part[2 b]) and
+// r . z (part[2 b + 1]) in FP64
+template <typename T>
+__global__ void k_ab_update(uint64_t n, double alpha, const T* __restrict__ q, T* __restrict__ r,
+                            const T* __restrict__ dinv, T* __restrict__ z, double* __restrict__ part) {
   const T a = (T)alpha;
   double rr = 0.0, rz = 0.0;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    x[i] += a * d[i];
     const T ri = r[i] - a * q[i];
     r[i] = ri;
     const T zi = dinv[i] * ri;
@@ -1014,19 +1120,19 @@ struct Band {
   // y = A_BB x (kBandApply) or y = f - A_BB x (kBandResid), screening included
   template <typename T, int MODE>
   void op(const T* x, const T* f, T* y) {
-    launch_op<T, MODE, false>(x, f, y, nullptr, 0.0, nullptr);
+    launch_op<T, MODE, false>(x, f, y, nullptr, 0.0, 0.0, nullptr, nullptr);
     bytes += 2.0 * n * sizeof(T) + (MODE == kBandResid ? n * sizeof(T) : 0.0);
     screen<T>(x, y, MODE == kBandApply ? 1.0 : -1.0, nullptr);
   }
   template <typename T, int MODE, bool GSRC>
-  void launch_op(const T* x, const T* f, T* y, T* dout, double beta, double* part) {
-    const size_t sm = band_op_smem<T>(GSRC);
+  void launch_op(const T* x, const T* f, T* y, T* dout, double beta, double alpha, T* e, double* part) {
+    const size_t sm = band_op_smem<T>(MODE, GSRC);
     allow_smem(k_ab_op<T, MODE, GSRC>, sm);
-    k_ab_op<T, MODE, GSRC><<<grid_op(), kOpThreads, sm, c->stream>>>(x, f, y, dout, beta, nbr, bkey, NB,
+    k_ab_op<T, MODE, GSRC><<<grid_op(), kOpThreads, sm, c->stream>>>(x, f, y, dout, beta, alpha, e, nbr, bkey, NB,
                                                                      band_coef<T>(c->D, c->pw), xc, W, res, part);
     PR_CHECK_LAUNCH();
   }
-  unsigned grid_op() const { return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(NB, 148 * 16)); }
+  unsigned grid_op() const { return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(NB, 148 * kOpCtas)); }
   // y += sign wh3 Phi Phi^T x; sq: per-block sums of proj^2 (returns their count)
   template <typename T>
   int screen(const T* x, T* y, double sign, double* sq) {
@@ -1064,8 +1170,9 @@ void release_prefix(pr_context* c, const std::string& prefix);
 
 // Jacobi-preconditioned CG on A_BB x = r from x = 0 until ||r|| <= tol; r is overwritten with
 // the residual; returns the iterations.  Per iteration: one operator pass that forms the direction
-// d = z + beta dold and q = A d with d . q (plus the screening pass), and one update pass x, r, z
-// with r . r and r . z; every sum is a fixed-order FP64 sum of per-block partials.
+// d = z + beta dold and q = A d with d . q and takes the last iteration's step in x (plus the screening
+// pass), and one update pass r, z with r . r and r . z; every sum is a fixed-order FP64 sum of per-block
+// partials.
 template <typename T>
 int band_pcg(Band& B, T* r, T* x, double tol, int maxit) {
   pr_context* c = B.c;
@@ -1089,13 +1196,16 @@ int band_pcg(Band& B, T* r, T* x, double tol, int maxit) {
   PR_CHECK_LAUNCH();
   PR_CUDA(cudaMemcpyAsync(h, sums, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
   c->sync();
-  double rr = h[0], rz = h[1], beta = 0.0;
+  double rr = h[0], rz = h[1], beta = 0.0, alpha = 0.0;
+  bool step = false;  // x lacks alpha d
   B.bytes += 3.0 * n * sizeof(T);
   int it = 0;
   while (std::sqrt(rr) > tol && it < maxit) {
     // dn = z + beta d, q = A dn (beta = 0 on the first pass: d is not read)
     const int nop = (int)B.grid_op();
-    B.launch_op<T, kBandDir, false>(d, z, q, dn, beta, part);
+    B.launch_op<T, kBandDir, false>(d, z, q, dn, beta, alpha, step ? x : nullptr, part);
+    B.bytes += (step ? 6.0 : 4.0) * n * sizeof(T);
+    step = false;
     std::swap(d, dn);
     const int nsq = B.screen<T>(d, q, 1.0, part2);
     k_ab_sum_parts<<<1, 32, 0, s>>>(part, nop, 1, 1.0, sums);
@@ -1107,20 +1217,25 @@ int band_pcg(Band& B, T* r, T* x, double tol, int maxit) {
     PR_CUDA(cudaMemcpyAsync(h, sums, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
     c->sync();
     const double dq = h[0] + (nsq ? h[2] : 0.0);
-    B.bytes += 4.0 * n * sizeof(T);
     if (!(dq > 0.0)) break;
-    const double alpha = rz / dq;
-    k_ab_update<T><<<nbk, kThreads, 0, s>>>(n, alpha, d, q, x, r, dv, z, part);
+    alpha = rz / dq;
+    step = true;
+    k_ab_update<T><<<nbk, kThreads, 0, s>>>(n, alpha, q, r, dv, z, part);
     PR_CHECK_LAUNCH();
     k_ab_sum_parts<<<2, 32, 0, s>>>(part, nbk, 2, 1.0, sums);
     PR_CHECK_LAUNCH();
     PR_CUDA(cudaMemcpyAsync(h, sums, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
     c->sync();
-    B.bytes += 8.0 * n * sizeof(T);
+    B.bytes += 5.0 * n * sizeof(T);
     ++it;
     rr = h[0];
     beta = h[1] / rz;
     rz = h[1];
+  }
+  if (step) {
+    k_ab_step<T><<<nbk, kThreads, 0, s>>>(n, alpha, d, x);
+    PR_CHECK_LAUNCH();
+    B.bytes += 3.0 * n * sizeof(T);
   }
   return it;
 }
@@ -1387,7 +1502,7 @@ void stage_adaptive(pr_context* c, const pr_params& p, pr_stats& st, bool extrac
     double* e64 = c->buf<double>("ab_e64", n);
     k_ab_prolong_band<<<brick_grid(B.NB), kThreads, 0, s>>>(B.bkey, B.NB, B.xc, B.W, B.res, gB);
     PR_CHECK_LAUNCH();
-    B.launch_op<double, kBandResid, true>(nullptr, b, r0, nullptr, 0.0, nullptr);  // r0 = b - (K + wg) g
+    B.launch_op<double, kBandResid, true>(nullptr, b, r0, nullptr, 0.0, 0.0, nullptr, nullptr);  // r0 = b - (K + wg) g
     B.screen<double>(gB, r0, -1.0, nullptr);
     bn = std::sqrt(dot<double>(c, b, b, n));
     used = band_solve(B, r0, bn, e64, p, rn, st.refinement_steps);
