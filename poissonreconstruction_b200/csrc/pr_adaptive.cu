@@ -91,11 +91,22 @@ __device__ __forceinline__ int floor_div(int a, int b) { return a >= 0 ? a / b :
 // The coarse function's depth-D coefficients on a TT^3 tile of fine nodes starting at (ox, oy, oz)
 // (zero outside the grid), by the whole CTA: the coarse coefficients that reach the tile (at most
 // 9 per axis), then the separable sums over x, y and z, every one in increasing coarse index, so
-// a node gets the same bits in any tile.  scratch: 729 + 81 TT + 9 TT^2 doubles.
-__host__ __device__ constexpr int kProlongScratch(int tt) { return 729 + 81 * tt + 9 * tt * tt; }
+// a node gets the same bits in any tile.  scratch: 729 + 81 TT + 9 TT^2 doubles and the taps.
+// A fine node has at most 3 taps per axis (3 2^L - 2 of them, 2^L apart): they are looked up once per tile
+// and axis.  (Tried one by one over the coarse range for every node, with the weights read from constant
+// memory at an index of each lane's own: k_ab_mc_count 6.6 -> 5.2 ms at 428,000 bricks, the first residual
+// 12.0 -> 9.9.)
+struct Taps {
+  double w[3];
+  int first, n;  // coarse index (from the tile's first), taps
+};
+__host__ __device__ constexpr int kProlongScratch(int tt) {
+  return 729 + 81 * tt + 9 * tt * tt + (int)(sizeof(Taps) / sizeof(double)) * 3 * tt;
+}
 template <int TT>
 __device__ void prolong_tile(const double* __restrict__ xc, const Prolong& W, int res, int ox, int oy, int oz,
                              double* scratch, double* out) {
+  static_assert(sizeof(Taps) % sizeof(double) == 0, "taps lie in the scratch");
   const int step = 1 << W.L;
   const int o[3] = {ox, oy, oz};
   int lo[3], cnt[3];
@@ -108,47 +119,49 @@ __device__ void prolong_tile(const double* __restrict__ xc, const Prolong& W, in
   double* c = scratch;        // [cz][cy][cx]
   double* ax = c + 729;       // [cz][cy][TT]
   double* ay = ax + 81 * TT;  // [cz][TT][TT]
+  Taps* taps = reinterpret_cast<Taps*>(ay + 9 * TT * TT);  // [axis][TT]
   const int t = threadIdx.x, nt = blockDim.x;
   for (int i = t; i < cnt[0] * cnt[1] * cnt[2]; i += nt) {
     const int ix = i % cnt[0], iy = (i / cnt[0]) % cnt[1], iz = i / (cnt[0] * cnt[1]);
     c[i] = xc[(int64_t)(lo[0] + ix) + (int64_t)W.resc * ((lo[1] + iy) + (int64_t)W.resc * (lo[2] + iz))];
   }
-  __syncthreads();
-  for (int i = t; i < cnt[2] * cnt[1] * TT; i += nt) {
-    const int tx = i % TT, r = i / TT;  // r = iz cnt1 + iy
-    const int f = ox + tx;
-    double v = 0.0;
+  for (int i = t; i < 3 * TT; i += nt) {
+    const int a = i / TT, f = (a == 0 ? ox : a == 1 ? oy : oz) + i % TT;
+    const int l = a == 0 ? lo[0] : a == 1 ? lo[1] : lo[2], m = a == 0 ? cnt[0] : a == 1 ? cnt[1] : cnt[2];
+    Taps p = {{0.0, 0.0, 0.0}, 0, 0};
     if (f >= 0 && f < res)
-      for (int ix = 0; ix < cnt[0]; ++ix) {
-        const int k = f - step * (lo[0] + ix) - W.kmin;
-        if (k >= 0 && k <= W.kmax - W.kmin) v += W.w[k] * c[r * cnt[0] + ix];
+      for (int j = 0; j < m; ++j) {
+        const int k = f - step * (l + j) - W.kmin;
+        if (k < 0 || k > W.kmax - W.kmin) continue;
+        if (p.n == 0) p.first = j;
+        const double w = W.w[k];
+        if (p.n == 0) p.w[0] = w;
+        else if (p.n == 1) p.w[1] = w;
+        else p.w[2] = w;
+        ++p.n;
       }
-    ax[i] = v;
+    taps[i] = p;
+  }
+  __syncthreads();
+  auto sum = [](const Taps& p, const double* v, int stride) {
+    double s = 0.0;
+    v += p.first * stride;
+    if (p.n > 0) s += p.w[0] * v[0];
+    if (p.n > 1) s += p.w[1] * v[stride];
+    if (p.n > 2) s += p.w[2] * v[2 * stride];
+    return s;
+  };
+  for (int i = t; i < cnt[2] * cnt[1] * TT; i += nt) {
+    const int r = i / TT;  // iz cnt1 + iy
+    ax[i] = sum(taps[i % TT], c + r * cnt[0], 1);
   }
   __syncthreads();
   for (int i = t; i < cnt[2] * TT * TT; i += nt) {
     const int tx = i % TT, ty = (i / TT) % TT, iz = i / (TT * TT);
-    const int f = oy + ty;
-    double v = 0.0;
-    if (f >= 0 && f < res)
-      for (int iy = 0; iy < cnt[1]; ++iy) {
-        const int k = f - step * (lo[1] + iy) - W.kmin;
-        if (k >= 0 && k <= W.kmax - W.kmin) v += W.w[k] * ax[(iz * cnt[1] + iy) * TT + tx];
-      }
-    ay[i] = v;
+    ay[i] = sum(taps[TT + ty], ax + iz * cnt[1] * TT + tx, TT);
   }
   __syncthreads();
-  for (int i = t; i < TT * TT * TT; i += nt) {
-    const int yx = i % (TT * TT), tz = i / (TT * TT);
-    const int f = oz + tz;
-    double v = 0.0;
-    if (f >= 0 && f < res)
-      for (int iz = 0; iz < cnt[2]; ++iz) {
-        const int k = f - step * (lo[2] + iz) - W.kmin;
-        if (k >= 0 && k <= W.kmax - W.kmin) v += W.w[k] * ay[iz * TT * TT + yx];
-      }
-    out[i] = v;
-  }
+  for (int i = t; i < TT * TT * TT; i += nt) out[i] = sum(taps[2 * TT + i / (TT * TT)], ay + i % (TT * TT), TT * TT);
   __syncthreads();
 }
 
@@ -299,30 +312,42 @@ __global__ void __launch_bounds__(kThreads) k_ab_rhs(const uint32_t* __restrict_
   double* tz = nf + 3 * kOT3;       // [8][12][12]
   double* ty = tz + 8 * kOT * kOT;  // [8][8][12]
   double* ob = ty + 8 * 8 * kOT;    // [512]
-  __shared__ uint32_t nb[27];
+  __shared__ uint32_t first[27], before[28];  // a neighbour's first run, the runs of those before it
   const int t = threadIdx.x;
   const double gg[5] = {g0, g1, 0.0, g3, g4};
   for (uint64_t slot = blockIdx.x; slot < NB; slot += gridDim.x) {
-    if (t < 27) nb[t] = nbr[27 * slot + t];
+    if (t < 32) {
+      const uint32_t s2 = t < 27 ? nbr[27 * slot + t] : kSent;
+      const uint32_t r0 = s2 != kSent ? brun[s2] : 0, m = s2 != kSent ? brun[s2 + 1] - r0 : 0;
+      uint32_t upto = m;
+#pragma unroll
+      for (int k = 1; k < 32; k *= 2) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, upto, k);
+        if (t >= k) upto += v;
+      }
+      if (t < 27) first[t] = r0;
+      if (t < 28) before[t] = upto - m;
+    }
     for (int i = t; i < 3 * kOT3; i += kThreads) nf[i] = 0.0;
     __syncthreads();
-    for (int k = 0; k < 27; ++k) {
-      const uint32_t s2 = nb[k];
-      if (s2 == kSent) continue;
+    // the neighbours' runs as one list (brick by brick each waited for its loads: 14.6 -> 9.3 ms at 428,000 bricks)
+    int k = 0;
+    for (uint32_t i = t; i < before[27]; i += kThreads) {
+      while (i >= before[k + 1]) ++k;
+      const uint32_t r = first[k] + (i - before[k]);
       const int ox = k % 3 - 1, oy = (k / 3) % 3 - 1, oz = k / 9 - 1;
-      for (uint32_t r = brun[s2] + t; r < brun[s2 + 1]; r += kThreads) {
-        const uint32_t local = run_key[r] - s2 * (uint32_t)kBN;
-        const int tx = (int)(local & 7) + 8 * ox + 2, ty_ = (int)((local >> 3) & 7) + 8 * oy + 2,
-                  tz_ = (int)(local >> 6) + 8 * oz + 2;
-        if (tx < 0 || ty_ < 0 || tz_ < 0 || tx >= kOT || ty_ >= kOT || tz_ >= kOT) continue;
-        const int o = (tz_ * kOT + ty_) * kOT + tx;
-        nf[o] = nfc[3 * (uint64_t)r];
-        nf[kOT3 + o] = nfc[3 * (uint64_t)r + 1];
-        nf[2 * kOT3 + o] = nfc[3 * (uint64_t)r + 2];
-      }
+      const uint32_t local = run_key[r] % (uint32_t)kBN;
+      const int tx = (int)(local & 7) + 8 * ox + 2, ty_ = (int)((local >> 3) & 7) + 8 * oy + 2,
+                tz_ = (int)(local >> 6) + 8 * oz + 2;
+      if (tx < 0 || ty_ < 0 || tz_ < 0 || tx >= kOT || ty_ >= kOT || tz_ >= kOT) continue;
+      const int o = (tz_ * kOT + ty_) * kOT + tx;
+      nf[o] = nfc[3 * (uint64_t)r];
+      nf[kOT3 + o] = nfc[3 * (uint64_t)r + 1];
+      nf[2 * kOT3 + o] = nfc[3 * (uint64_t)r + 2];
     }
     __syncthreads();
     double acc[2] = {0.0, 0.0};
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
       const double* fz = a == 2 ? gg : K.m;
       const double* fy = a == 1 ? gg : K.m;
@@ -383,9 +408,9 @@ __global__ void __launch_bounds__(kThreads) k_ab_rhs(const uint32_t* __restrict_
 // flight while the y and x passes work on this one; a tile plane holds its 12 rows' 8 own values, then
 // their 4 side values (x = -2, -1, 8, 9), so that the gather is 16-byte copies by consecutive lanes
 // (cp.async) and 8-byte loads (through registers: cheaper there than as 8-byte copies); planes are padded against bank conflicts; the z and y passes work on pairs
-// (64-bit shared accesses, two FP32 FMAs to an instruction).  FP32 at 245M nodes (depth 11): operator and
-// update pass 3.04 -> 2.61 ms an iteration (1.76 + 1.29 -> 1.84 + 0.77; the traffic of the two vectors
-// formed here takes 0.91 of the 1.84), with 75 % of the shared-memory pipe's cycles used.
+// (64-bit shared accesses, two FP32 FMAs to an instruction).  FP32 at 219M nodes (depth 11): operator and
+// update pass 3.04 -> 2.61 ms an iteration (1.76 + 1.29 -> 1.84 + 0.77); at the copy rate the two would
+// take 0.82 + 0.68.  The shared-memory pipe is busy for about 75 % of the operator's cycles (29M nodes).
 constexpr int kOpThreads = 96;
 constexpr int kOpCtas = 8;       // per SM (shared memory, registers); the grid is one wave of them
 constexpr int kTP = 144;         // tile plane: [y 12][8], then [y 12][4]
@@ -853,9 +878,9 @@ __device__ __forceinline__ uint32_t ab_edge_mask(uint32_t mc) {
 }
 
 // The brick's 9^3 corner values at grid positions 8b + q (q = 0..8 per axis): node tile 10^3
-// (nodes 8b - 1 .. 8b + 8; f on the band, g elsewhere), each corner the in-order sum over the
-// nodes p - 1, p per axis inside the grid of ((x / 2) / 2) / 2 (the dense path's grid-position
-// evaluation).
+// (nodes 8b - 1 .. 8b + 8; f on the band, g elsewhere, zero outside the grid), each corner the in-order
+// sum over the nodes p - 1, p per axis of ((x / 2) / 2) / 2 (the dense path's grid-position evaluation;
+// the zeros add nothing).
 __device__ void ab_corner_values(uint64_t slot, const uint32_t* nb, const double* __restrict__ f,
                                  const uint32_t* __restrict__ bkey, const double* __restrict__ xc, const Prolong& W,
                                  int res, double* node, double* cv, double* scratch) {
@@ -869,41 +894,36 @@ __device__ void ab_corner_values(uint64_t slot, const uint32_t* nb, const double
     const int ox = lx < 0 ? -1 : (lx >= 8 ? 1 : 0), oy = ly < 0 ? -1 : (ly >= 8 ? 1 : 0),
               oz = lz < 0 ? -1 : (lz >= 8 ? 1 : 0);
     const uint32_t s2 = nb[(oz + 1) * 9 + (oy + 1) * 3 + (ox + 1)];
-    if (s2 != kSent) node[i] = f[(uint64_t)s2 * kBN + (((lz - 8 * oz) << 6) | ((ly - 8 * oy) << 3) | (lx - 8 * ox))];
+    const double v =
+        s2 != kSent ? f[(uint64_t)s2 * kBN + (((lz - 8 * oz) << 6) | ((ly - 8 * oy) << 3) | (lx - 8 * ox))] : node[i];
+    node[i] = xmul(xmul(xmul(v, 0.5), 0.5), 0.5);
   }
   __syncthreads();
   for (int i = t; i < 9 * 9 * 9; i += kThreads) {
     const int qz = i / 81, qy = (i / 9) % 9, qx = i % 9;
+    const double* p = node + (qz * kMT + qy) * kMT + qx;
     double v = 0.0;
-    for (int dz = -1; dz <= 0; ++dz) {
-      const int z = org[2] + qz + dz;
-      if (z < 0 || z >= res) continue;
-      for (int dy = -1; dy <= 0; ++dy) {
-        const int y = org[1] + qy + dy;
-        if (y < 0 || y >= res) continue;
-        for (int dx = -1; dx <= 0; ++dx) {
-          const int x = org[0] + qx + dx;
-          if (x < 0 || x >= res) continue;
-          const double nv = node[((qz + dz + 1) * kMT + qy + dy + 1) * kMT + qx + dx + 1];
-          v = xadd(v, xmul(xmul(xmul(nv, 0.5), 0.5), 0.5));
-        }
-      }
-    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v = xadd(v, p[((k >> 2) * kMT + ((k >> 1) & 1)) * kMT + (k & 1)]);
     cv[i] = v;
   }
   __syncthreads();
 }
 
-// key of edge e of a cell: its lower grid position and axis, ((z (res+1) + y) (res+1) + x) 3 + axis
-__device__ __forceinline__ uint64_t ab_edge_key(const int* cell, int e, uint64_t R1) {
-  const int ia = c_abev[e][0], ib = c_abev[e][1];
-  int st[3], axis = 0;
+// the corners of edge e as bits x, y, z: from ev & 7 to ev >> 3
+__device__ __forceinline__ uint32_t ab_edge_ends(int e) {
+  uint32_t v = 0;
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    st[a] = cell[a] + min(c_abco[ia][a], c_abco[ib][a]);
-    if (c_abco[ia][a] != c_abco[ib][a]) axis = a;
-  }
-  return (((uint64_t)st[2] * R1 + (uint64_t)st[1]) * R1 + (uint64_t)st[0]) * 3 + (uint64_t)axis;
+  for (int k = 0; k < 2; ++k)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) v |= (uint32_t)c_abco[c_abev[e][k]][a] << (3 * k + a);
+  return v;
+}
+// key of an edge of a cell: its lower grid position and axis, ((z (res+1) + y) (res+1) + x) 3 + axis
+__device__ __forceinline__ uint64_t ab_edge_key(int x, int y, int z, uint32_t ends, uint64_t R1) {
+  const uint32_t low = ends & (ends >> 3) & 7u, dir = (ends ^ (ends >> 3)) & 7u;
+  return (((uint64_t)(z + (int)(low >> 2)) * R1 + (uint64_t)(y + (int)((low >> 1) & 1u))) * R1 +
+          (uint64_t)(x + (int)(low & 1u))) * 3 + (dir >> 1);
 }
 
 __device__ __forceinline__ uint32_t ab_cell_case(const double* cv, int o, double iso) {
@@ -947,26 +967,37 @@ __global__ void __launch_bounds__(kThreads) k_ab_mc_count(const double* __restri
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 2) k_ab_mc_emit(const double* __restrict__ f, const uint32_t* __restrict__ nbr,
+// Few cells of a brick are cut: its cut edges and its triangles' corners are listed in shared memory (a
+// cell and an edge each, over the tile that the corner values came from), then a thread per entry works and
+// writes next to its neighbours.  With a cell to a thread most of them idled: 15.2 ms at 428,000 bricks
+// (depth 11), now 5.2 (k_ab_mc_count, without an output, the same).
+constexpr int kEmitTile = kMT * kMT * kMT + kProlongScratch(kMT);  // doubles
+static_assert(kEmitTile * sizeof(double) >= 512 * (12 + 15) * sizeof(uint16_t), "the lists fit the tile");
+__global__ void __launch_bounds__(kThreads, 4) k_ab_mc_emit(const double* __restrict__ f, const uint32_t* __restrict__ nbr,
                                                          const uint32_t* __restrict__ bkey, uint64_t NB,
                                                          const double* __restrict__ xc, Prolong W, int res, double iso,
                                                          const uint64_t* __restrict__ toff, const uint64_t* __restrict__ eoff,
                                                          uint64_t* __restrict__ tri_key, uint64_t* __restrict__ edge_key,
                                                          double* __restrict__ epos) {
-  __shared__ double node[kMT * kMT * kMT], cv[729], scratch[kProlongScratch(kMT)];
-  __shared__ uint32_t nb[27];
+  __shared__ double node[kEmitTile], cv[729];
+  __shared__ uint32_t nb[27], ends[12];
   typedef cub::BlockScan<uint32_t, kThreads> BS;
   __shared__ typename BS::TempStorage tmp;
+  uint16_t *elist = reinterpret_cast<uint16_t*>(node), *tlist = elist + 512 * 12;
   const int t = threadIdx.x;
   const double w = 1.0 / (double)res;
   const uint64_t R1 = (uint64_t)res + 1;
+  if (t < 12) ends[t] = ab_edge_ends(t);
   for (uint64_t slot = blockIdx.x; slot < NB; slot += gridDim.x) {
+    const uint64_t e0 = eoff[slot], t0 = toff[slot];
+    const int ne = (int)(eoff[slot + 1] - e0), ntc = 3 * (int)(toff[slot + 1] - t0);
+    if (ne == 0) continue;  // no cell is cut (every triangle has cut edges)
     if (t < 27) nb[t] = nbr[27 * slot + t];
     __syncthreads();
-    ab_corner_values(slot, nb, f, bkey, xc, W, res, node, cv, scratch);
+    ab_corner_values(slot, nb, f, bkey, xc, W, res, node, cv, node + kMT * kMT * kMT);
     uint32_t bx, by, bz;
     unmorton3(bkey[slot], bx, by, bz);
-    const int org[3] = {8 * (int)bx, 8 * (int)by, 8 * (int)bz};
+    const int ox = 8 * (int)bx, oy = 8 * (int)by, oz = 8 * (int)bz;
     uint32_t mc[2], ct = 0, ce = 0;
     for (int j = 0; j < 2; ++j) {
       mc[j] = ab_cell_case(cv, 2 * t + j, iso);
@@ -977,31 +1008,36 @@ __global__ void __launch_bounds__(kThreads, 2) k_ab_mc_emit(const double* __rest
     BS(tmp).ExclusiveSum(ct, pt);
     __syncthreads();
     BS(tmp).ExclusiveSum(ce, pe);
-    uint64_t to = toff[slot] + pt, eo = eoff[slot] + pe;
+    pt *= 3;
     for (int j = 0; j < 2; ++j) {
-      const int o = 2 * t + j, cz = o >> 6, cy = (o >> 3) & 7, cx = o & 7;
-      const int cell[3] = {org[0] + cx, org[1] + cy, org[2] + cz};
-      const uint32_t em = ab_edge_mask(mc[j]);
-      for (int e = 0; e < 12; ++e) {
-        if (!((em >> e) & 1u)) continue;
-        const int ia = c_abev[e][0], ib = c_abev[e][1];
-        const double va = cv[((cz + c_abco[ia][2]) * 9 + cy + c_abco[ia][1]) * 9 + cx + c_abco[ia][0]];
-        const double vb = cv[((cz + c_abco[ib][2]) * 9 + cy + c_abco[ib][1]) * 9 + cx + c_abco[ib][0]];
-        const double dv = xsub(vb, va);
-        const double tt = fabs(dv) < 1e-15 ? 0.5 : xdiv(xsub(iso, va), dv);
+      const uint32_t o = (uint32_t)(2 * t + j) << 4;
+      for (uint32_t em = ab_edge_mask(mc[j]); em; em &= em - 1) elist[pe++] = (uint16_t)(o | (uint32_t)(__ffs(em) - 1));
+      uint64_t packed = PR_MC_TRIS[mc[j]];
+      for (uint32_t i = 3 * PR_MC_NTRI[mc[j]]; i; --i, packed >>= 4) tlist[pt++] = (uint16_t)(o | (packed & 15u));
+    }
+    __syncthreads();
+    for (int i = t; i < ne; i += kThreads) {
+      const uint32_t v = elist[i], en = ends[v & 15u], a = en & 7u, b = en >> 3;
+      const int cx = (v >> 4) & 7, cy = (v >> 7) & 7, cz = v >> 10;
+      const double* at = cv + (cz * 9 + cy) * 9 + cx;
+      const double va = at[((a >> 2) * 9 + ((a >> 1) & 1u)) * 9 + (a & 1u)];
+      const double vb = at[((b >> 2) * 9 + ((b >> 1) & 1u)) * 9 + (b & 1u)];
+      const double dv = xsub(vb, va);
+      const double tt = fabs(dv) < 1e-15 ? 0.5 : xdiv(xsub(iso, va), dv);
+      const int cell[3] = {ox + cx, oy + cy, oz + cz};
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          const double base = xmul((double)(cell[a] + c_abco[ia][a]), w);
-          const double d = (double)(c_abco[ib][a] - c_abco[ia][a]);
-          epos[3 * eo + a] = xadd(base, xmul(xmul(tt, d), w));
-        }
-        edge_key[eo] = ab_edge_key(cell, e, R1);
-        ++eo;
+      for (int k = 0; k < 3; ++k) {
+        const int ak = (int)((a >> k) & 1u);
+        const double base = xmul((double)(cell[k] + ak), w);
+        const double d = (double)((int)((b >> k) & 1u) - ak);
+        epos[3 * (e0 + i) + k] = xadd(base, xmul(xmul(tt, d), w));
       }
-      const uint64_t packed = PR_MC_TRIS[mc[j]];
-      const uint32_t ntr = PR_MC_NTRI[mc[j]];
-      for (uint32_t i = 0; i < 3 * ntr; ++i) tri_key[3 * to + i] = ab_edge_key(cell, (int)((packed >> (4 * i)) & 15u), R1);
-      to += ntr;
+      edge_key[e0 + i] = ab_edge_key(cell[0], cell[1], cell[2], en, R1);
+    }
+    for (int i = t; i < ntc; i += kThreads) {
+      const uint32_t v = tlist[i];
+      tri_key[3 * t0 + i] = ab_edge_key(ox + (int)((v >> 4) & 7u), oy + (int)((v >> 7) & 7u), oz + (int)(v >> 10),
+                                        ends[v & 15u], R1);
     }
     __syncthreads();
   }

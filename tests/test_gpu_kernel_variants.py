@@ -5,6 +5,7 @@ import pytest
 import oracle
 import poissonreconstruction_b200 as prb
 from poissonreconstruction_b200 import synthetic
+from tests.test_gpu_adaptive import _morton_to_natural_vec, _prolong
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +93,24 @@ def test_vertex_table(ctx, side, low):
     v_ref, t_ref = oracle.extract_surface(depth, field, 0.5)
     assert np.array_equal(mesh.vertices, v_ref)
     assert np.array_equal(mesh.triangles, t_ref)
+
+
+@pytest.mark.parametrize("depth", [4, 5, 6, 7])
+@pytest.mark.parametrize("flags", [0, prb.PR_BAND_FULL])
+def test_band_coarse_function(ctx, depth, flags):
+    """One to four levels above the coarse one (two taps per axis, then two or three), with bricks at the
+    faces of the grid or without: the fixed coarse function is the subdivision of the coarse solution (its
+    sums of at most 27 terms to 1e-13), and the mesh uses each of its vertices."""
+    coarse = 3
+    pts = synthetic.torus(4000, seed=80 + depth)
+    ctx.solve(pts, prb.ReconstructParams(depth=coarse, degree=2, point_weight=4.0))
+    xc = _morton_to_natural_vec(ctx.coefficients(), coarse)
+    mesh, st = ctx.reconstruct(pts, prb.ReconstructParams(depth=depth, coarse_depth=coarse, degree=2, point_weight=4.0,
+                                                          band_flags=flags))
+    assert st.converged == 1 and len(mesh.triangles) > 0
+    _, _, codes = ctx.band_info()
+    g_all = _prolong(xc, coarse, depth)
+    g = ctx.band_vector(2)
+    assert np.max(np.abs(g - g_all[prb.band_natural_index(codes, depth)])) <= 1e-13 * np.max(np.abs(g_all))
+    t = mesh.triangles.astype(np.int64)
+    assert t.max() + 1 == len(mesh.vertices) == len(np.unique(t))
