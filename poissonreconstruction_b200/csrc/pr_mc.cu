@@ -419,64 +419,95 @@ __global__ void k_mc_emit_tris(const uint8_t* __restrict__ acase, uint64_t A, co
 }  // namespace
 
 // ------------------------------------------------------------------ block-tiled classification (depth >= 4)
-// A CTA classifies the 16^3 cells of one Morton block.  Cell c has corners at grid
-// positions c + co[k]; the corner value is node (position - 1) per axis, so the CTA needs
-// nodes [-1, 15]^3 of its block: the block's own 16^3 nodes plus the low layer from the
-// neighbour blocks (zeros outside the domain, matching the crate's empty evaluation at 0).
-constexpr int MCW = 17;  // node tile width, tile coordinate = node local + 1
+// A CTA classifies the 16^3 cells of one Morton block.  Cell c has corners at grid positions c + co[k].
+// The inside/outside bits of the block's 17^3 corner positions are one 17-bit word per (y, z) row: bit tx
+// of row (ty, tz) is (corner value < iso) for grid position (o + t); a cell reads 4 words.
+constexpr int MCW = 17;
 
 __device__ __forceinline__ uint32_t sp4(uint32_t v) {
   return (v & 1u) | ((v & 2u) << 2) | ((v & 4u) << 4) | ((v & 8u) << 6);
 }
 
-__device__ void mc_load_tile(double* tile, const double* __restrict__ x, uint32_t blk, int res) {
-  const int t = threadIdx.x;
+// Degree 1: the corner value at a position is node (position - 1) per axis, so the bits are those of the
+// block's own 16^3 nodes and of the low layer from the neighbour blocks (zeros outside the domain,
+// matching the crate's empty evaluation at 0).  The value at a grid position equal to res on k axes is the
+// node value added 2^k times in sequence, like the crate's evaluate() at the top boundary.  The values go
+// from a coalesced 16-byte load (two nodes of a row) straight to bits: a lane's bits of one (y, z) row and
+// its neighbour's (x bit 1 is lane bit 2) make the row.
+__device__ void mc_masks1(uint32_t* mask, uint8_t* xbit, const double* __restrict__ x, uint32_t blk, int res,
+                          double iso) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   uint32_t bx, by, bz;
   unmorton3(blk, bx, by, bz);
-  const uint64_t base = (uint64_t)blk << 12;
-  for (int i = t; i < 4096; i += blockDim.x) {
-    uint32_t lx, ly, lz;
-    unmorton3((uint32_t)i, lx, ly, lz);
-    tile[((lz + 1) * MCW + (ly + 1)) * MCW + (lx + 1)] = __ldg(x + base + i);
-  }
-  // low layer: positions with a local coordinate -1 (817 of them)
-  const int nba = res >> 4;
-  for (int i = t; i < 817; i += blockDim.x) {
-    int lx, ly, lz;
-    if (i < 289) { lx = -1; ly = i % 17 - 1; lz = i / 17 - 1; }
-    else if (i < 561) { const int u = i - 289; lx = u % 16; ly = -1; lz = u / 16 - 1; }
-    else { const int u = i - 561; lx = u % 16; ly = u / 16; lz = -1; }
-    const int nx = (int)bx + (lx < 0 ? -1 : 0), ny = (int)by + (ly < 0 ? -1 : 0), nz = (int)bz + (lz < 0 ? -1 : 0);
-    double v = 0.0;
-    if (nx >= 0 && ny >= 0 && nz >= 0 && nx < nba && ny < nba && nz < nba) {
-      const uint32_t nb = morton3((uint32_t)nx, (uint32_t)ny, (uint32_t)nz) << 12;
-      v = __ldg(x + nb + (sp4((uint32_t)(lx & 15)) | (sp4((uint32_t)(ly & 15)) << 1) | (sp4((uint32_t)(lz & 15)) << 2)));
-    }
-    tile[((lz + 1) * MCW + (ly + 1)) * MCW + (lx + 1)] = v;
-  }
-}
-
-// Inside/outside bits of the tile's 17^3 corner positions, one 17-bit word per (y, z) row:
-// bit tx of row (ty, tz) is (corner value < iso) for grid position (o + t).  The value at a grid
-// position equal to res on k axes is the node value added 2^k times in sequence, like the crate's
-// evaluate() at the top boundary.  Every cell then reads 4 words instead of 8 doubles.
-__device__ __forceinline__ void mc_build_masks(const double* tile, uint32_t* mask, int ox, int oy, int oz, int res,
-                                               double iso) {
-  for (int r = threadIdx.x; r < MCW * MCW; r += blockDim.x) {
-    const int ty = r % MCW, tz = r / MCW;
-    const int myz = ((oy + ty == res) ? 2 : 1) * ((oz + tz == res) ? 2 : 1);
-    const double* row = tile + (tz * MCW + ty) * MCW;
-    uint32_t m = 0;
+  const uint32_t last = (uint32_t)(res >> 4) - 1;
+  const auto top = [](bool at_top, int l) { return at_top && l == 15 ? 2 : 1; };
+  const bool tx = bx == last, ty = by == last, tz = bz == last;
+  const auto bit = [iso](double s, int mult) {
+    double v = s;
+    for (int i = 1; i < mult; ++i) v = xadd(v, s);
+    return (uint32_t)(v < iso);
+  };
+  const auto load2 = [x](uint64_t i) { return __ldg(reinterpret_cast<const double2*>(x + i)); };  // i even
+  // node (lx, ly, lz) of the block dx, dy, dz below; ok: it lies in the domain
+  const auto at = [&](int dx, int dy, int dz, int lx, int ly, int lz) {
+    return ((uint64_t)morton3(bx - dx, by - dy, bz - dz) << 12) +
+           (sp4((uint32_t)lx) | (sp4((uint32_t)ly) << 1) | (sp4((uint32_t)lz) << 2));
+  };
+  const bool okx = bx > 0, oky = by > 0, okz = bz > 0;
+  double2 own[8];
 #pragma unroll
-    for (int tx = 0; tx < MCW; ++tx) {
-      const double s = row[tx];
-      const int mult = myz * ((ox + tx == res) ? 2 : 1);
-      double v = s;
-      for (int i = 1; i < mult; ++i) v = xadd(v, s);
-      m |= (uint32_t)(v < iso) << tx;
-    }
-    mask[r] = m;
+  for (int k = 0; k < 8; ++k) {  // pair bits: y0 z0 x1 y1 z1 (lane), x2 (k) y2 z2 (warp, k), x3 (k) y3 z3 (warp)
+    const uint32_t combo = 2 * warp + (k >> 2);
+    const uint32_t q = lane | (k & 1) << 5 | (combo & 3u) << 6 | ((k >> 1) & 1) << 8 | (combo >> 2) << 9;
+    own[k] = load2(((uint64_t)blk << 12) + 2 * q);
   }
+  const int u = t & 127, xp = u & 7, yz = u >> 3;  // the low y layer (t < 128), the low z layer
+  const bool on_y = t < 128;
+  double2 low = make_double2(0.0, 0.0), edge = make_double2(0.0, 0.0);
+  if (on_y ? oky : okz) low = load2(on_y ? at(0, 1, 0, 2 * xp, 15, yz) : at(0, 0, 1, 2 * xp, yz, 15));
+  if (t < 32 && oky && okz) edge = load2(at(0, 1, 1, 2 * (t & 7), 15, 15));
+  double side = 0.0, side2 = 0.0;  // the low x layer: row (t & 15, t >> 4), and its rows in the other low layers
+  if (okx) side = __ldg(x + at(1, 0, 0, 15, t & 15, t >> 4));
+  if (okx && t < 33) {
+    if (t < 16) { if (oky) side2 = __ldg(x + at(1, 1, 0, 15, 15, t)); }
+    else if (t < 32) { if (okz) side2 = __ldg(x + at(1, 0, 1, 15, t - 16, 15)); }
+    else if (oky && okz) side2 = __ldg(x + at(1, 1, 1, 15, 15, 15));
+  }
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const int combo = 2 * warp + c;
+    const int y = (lane & 1) | ((lane >> 3) & 1) << 1 | (combo & 1) << 2 | ((combo >> 2) & 1) << 3;
+    const int z = ((lane >> 1) & 1) | ((lane >> 4) & 1) << 1 | ((combo >> 1) & 1) << 2 | ((combo >> 3) & 1) << 3;
+    const int m = top(ty, y) * top(tz, z), x1 = (lane >> 2) & 1;
+    uint32_t bits = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int lx = 2 * x1 + 4 * (k & 1) + 8 * (k >> 1);
+      bits |= bit(own[4 * c + k].x, m) << lx | bit(own[4 * c + k].y, m * top(tx, lx + 1)) << (lx + 1);
+    }
+    bits |= __shfl_xor_sync(0xffffffffu, bits, 4);
+    if (!x1) mask[(z + 1) * MCW + y + 1] = bits << 1;
+  }
+  {
+    const int m = on_y ? top(tz, yz) : top(ty, yz);
+    uint32_t bits = bit(low.x, m) << (2 * xp) | bit(low.y, m * top(tx, 2 * xp + 1)) << (2 * xp + 1);
+#pragma unroll
+    for (int k = 1; k < 8; k *= 2) bits |= __shfl_xor_sync(0xffffffffu, bits, k);
+    if (xp == 0) mask[on_y ? (yz + 1) * MCW : yz + 1] = bits << 1;
+  }
+  if (t < 32) {
+    const int p = 2 * (t & 7);
+    uint32_t bits = bit(edge.x, 1) << p | bit(edge.y, top(tx, p + 1)) << (p + 1);
+#pragma unroll
+    for (int k = 1; k < 8; k *= 2) bits |= __shfl_xor_sync(0xffffffffu, bits, k);
+    if (t == 0) mask[0] = bits << 1;
+  }
+  xbit[((t >> 4) + 1) * MCW + (t & 15) + 1] = (uint8_t)bit(side, top(ty, t & 15) * top(tz, t >> 4));
+  if (t < 16) xbit[(t + 1) * MCW] = (uint8_t)bit(side2, top(tz, t));
+  else if (t < 32) xbit[t - 16 + 1] = (uint8_t)bit(side2, top(ty, t - 16));
+  else if (t == 32) xbit[0] = (uint8_t)bit(side2, 1);
+  __syncthreads();
+  for (int r = t; r < MCW * MCW; r += blockDim.x) mask[r] |= xbit[r];
 }
 // Degree 2: the corner value at grid position p is the sum over the nodes p-1, p per axis of
 // ((x 1/2) 1/2) 1/2, z-major, then y, then x (corner_value2).  The CTA stages the terms
@@ -486,54 +517,85 @@ constexpr int MCW2 = 18;  // node tile width, tile coordinate = node local + 1
 
 __device__ __forceinline__ double mc_term2(double v) { return xmul(xmul(xmul(v, 0.5), 0.5), 0.5); }
 
+// entry i of the 18^3 tile: its coordinates.  Natural order: row by row.  Morton order: the block's own
+// nodes as they lie in memory, then the shell: the z faces (2 x 18 x 18), the y faces of the inner z range
+// (2 x 16 x 18), the x faces of the inner y and z ranges (2 x 16 x 16)
 template <bool NAT>
-__device__ void mc_load_tile2(double* tile, const double* __restrict__ x, uint32_t blk, int res) {
-  uint32_t bx, by, bz;
-  unmorton3(blk, bx, by, bz);
-  if (NAT) {  // natural order: the tile's rows are contiguous in memory (18 values per row)
-    const uint32_t D = 31 - __clz(res);
-    for (int i = threadIdx.x; i < MCW2 * MCW2 * MCW2; i += blockDim.x) {
-      const int tx = i % MCW2, ty = (i / MCW2) % MCW2, tz = i / (MCW2 * MCW2);
-      const int gx = (int)bx * 16 + tx - 1, gy = (int)by * 16 + ty - 1, gz = (int)bz * 16 + tz - 1;
-      double v = 0.0;
-      if (gx >= 0 && gy >= 0 && gz >= 0 && gx < res && gy < res && gz < res)
-        v = mc_term2(__ldg(x + node_index<true>((uint32_t)gx, (uint32_t)gy, (uint32_t)gz, D)));
-      tile[i] = v;
-    }
-    return;
-  }
-  const uint64_t base = (uint64_t)blk << 12;
-  for (int i = threadIdx.x; i < 4096; i += blockDim.x) {
+__device__ __forceinline__ void mc_tile2_entry(int i, int& tx, int& ty, int& tz) {
+  if (NAT) {
+    tx = i % MCW2;
+    ty = (i / MCW2) % MCW2;
+    tz = i / (MCW2 * MCW2);
+  } else if (i < 4096) {
     uint32_t lx, ly, lz;
     unmorton3((uint32_t)i, lx, ly, lz);
-    tile[((lz + 1) * MCW2 + (ly + 1)) * MCW2 + (lx + 1)] = mc_term2(__ldg(x + base + i));
+    tx = (int)lx + 1;
+    ty = (int)ly + 1;
+    tz = (int)lz + 1;
+  } else if (i < 4096 + 648) {
+    const int r = (i - 4096) % 324;
+    tz = i < 4096 + 324 ? 0 : 17;
+    ty = r / 18;
+    tx = r % 18;
+  } else if (i < 4096 + 1224) {
+    const int j = i - 4096 - 648, r = j % 288;
+    ty = j < 288 ? 0 : 17;
+    tz = 1 + r / 18;
+    tx = r % 18;
+  } else {
+    const int j = i - 4096 - 1224, r = j % 256;
+    tx = j < 256 ? 0 : 17;
+    tz = 1 + r / 16;
+    ty = 1 + r % 16;
   }
-  // the shell, 18^3 - 16^3 = 1736 entries: the z faces (2 x 18 x 18), then the y faces of the
-  // inner z range (2 x 16 x 18), then the x faces of the inner y and z ranges (2 x 16 x 16)
-  for (int i = threadIdx.x; i < 1736; i += blockDim.x) {
+}
+// Fills the tile, unless no cell can be cut: rounded addition is monotone, so where eight times the
+// smallest term, added up like a corner value, is not below iso, no corner is, and likewise where eight
+// times the largest is below it (both only without NaN).  Returns whether the tile is filled; all threads agree.
+template <bool NAT>
+__device__ bool mc_load_tile2(double* tile, const double* __restrict__ x, uint32_t blk, int res, double iso) {
+  constexpr int kN = MCW2 * MCW2 * MCW2, kPer = (kN + 255) / 256;
+  uint32_t bx, by, bz;
+  unmorton3(blk, bx, by, bz);
+  const uint32_t D = 31 - __clz(res);
+  double v[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int i = threadIdx.x + 256 * k;
     int tx, ty, tz;
-    if (i < 648) {
-      const int r = i % 324;
-      tz = i < 324 ? 0 : 17;
-      ty = r / 18;
-      tx = r % 18;
-    } else if (i < 1224) {
-      const int j = i - 648, r = j % 288;
-      ty = j < 288 ? 0 : 17;
-      tz = 1 + r / 18;
-      tx = r % 18;
-    } else {
-      const int j = i - 1224, r = j % 256;
-      tx = j < 256 ? 0 : 17;
-      tz = 1 + r / 16;
-      ty = 1 + r % 16;
-    }
+    mc_tile2_entry<NAT>(i, tx, ty, tz);
     const int gx = (int)bx * 16 + tx - 1, gy = (int)by * 16 + ty - 1, gz = (int)bz * 16 + tz - 1;
-    double v = 0.0;
-    if (gx >= 0 && gy >= 0 && gz >= 0 && gx < res && gy < res && gz < res)
-      v = mc_term2(__ldg(x + morton3((uint32_t)gx, (uint32_t)gy, (uint32_t)gz)));
-    tile[(tz * MCW2 + ty) * MCW2 + tx] = v;
+    v[k] = 0.0;
+    if (i < kN && gx >= 0 && gy >= 0 && gz >= 0 && gx < res && gy < res && gz < res)
+      v[k] = __ldg(x + node_index<NAT>((uint32_t)gx, (uint32_t)gy, (uint32_t)gz, D));
   }
+  double lo = INFINITY, hi = -INFINITY;
+  bool number = true;
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    v[k] = mc_term2(v[k]);
+    if (threadIdx.x + 256 * k < kN) {
+      lo = fmin(lo, v[k]);
+      hi = fmax(hi, v[k]);
+      number = number && v[k] == v[k];
+    }
+  }
+  double slo = 0.0, shi = 0.0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    slo = xadd(slo, lo);
+    shi = xadd(shi, hi);
+  }
+  const bool above = __syncthreads_and(number && slo >= iso), below = __syncthreads_and(number && shi < iso);
+  if (above || below) return false;
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int i = threadIdx.x + 256 * k;
+    int tx, ty, tz;
+    mc_tile2_entry<NAT>(i, tx, ty, tz);
+    if (i < kN) tile[NAT ? i : (tz * MCW2 + ty) * MCW2 + tx] = v[k];
+  }
+  return true;
 }
 
 __device__ __forceinline__ void mc_build_masks2(const double* tile, uint32_t* mask, double iso) {
@@ -555,19 +617,24 @@ __device__ __forceinline__ void mc_build_masks2(const double* tile, uint32_t* ma
 }
 
 template <int DEG>
-__device__ __forceinline__ void mc_block_masks(double* tile, uint32_t* mask, const double* __restrict__ x,
-                                               uint32_t blk, int res, double iso) {
-  uint32_t bx, by, bz;
-  unmorton3(blk, bx, by, bz);
+struct McShared {
+  double tile[DEG >= 2 ? MCW2 * MCW2 * MCW2 : 1];
+  uint32_t mask[MCW * MCW];
+  uint8_t xbit[DEG >= 2 ? 1 : MCW * MCW];
+};
+// fills s.mask, unless no cell of the block is cut (degree 2; false then)
+template <int DEG>
+__device__ __forceinline__ bool mc_block_masks(McShared<DEG>& s, const double* __restrict__ x, uint32_t blk, int res,
+                                               double iso) {
   if (DEG >= 2) {
-    mc_load_tile2<DEG == 3>(tile, x, blk, res);
+    if (!mc_load_tile2<DEG == 3>(s.tile, x, blk, res, iso)) return false;
     __syncthreads();
-    mc_build_masks2(tile, mask, iso);
+    mc_build_masks2(s.tile, s.mask, iso);
   } else {
-    mc_load_tile(tile, x, blk, res);
-    __syncthreads();
-    mc_build_masks(tile, mask, bx * 16, by * 16, bz * 16, res, iso);
+    mc_masks1(s.mask, s.xbit, x, blk, res, iso);
   }
+  __syncthreads();
+  return true;
 }
 
 // case of local cell (lx, ly, lz) from the row masks (corner order of c_co)
@@ -578,22 +645,21 @@ __device__ __forceinline__ uint32_t mc_mask_case(const uint32_t* mask, int lx, i
          ((m01 >> 1) & 1u) << 5 | ((m11 >> 1) & 1u) << 6 | (m11 & 1u) << 7;
 }
 
+// Reading the values bounds it: 8.6 GB at depth 10, 1.33 ms at the copy rate.  Degree 1: 3.82 -> 1.62 ms
+// (before, through a tile in shared memory, read back by a thread per row); degree 2: 6.66 -> 4.11 (before,
+// every block's corners were formed; rows of 128 bytes, and the index arithmetic of the 18^3 tile, hold it).
 template <int DEG>
 __global__ void __launch_bounds__(256) k_mc_block_count(const double* __restrict__ x, uint32_t D, double iso,
                                                         uint32_t* __restrict__ blockcnt) {
-  __shared__ double tile[DEG >= 2 ? MCW2 * MCW2 * MCW2 : MCW * MCW * MCW];
-  __shared__ uint32_t mask[MCW * MCW];
+  __shared__ McShared<DEG> s;
   const int res = 1 << D;
   const uint32_t blk = blockIdx.x;
-  mc_block_masks<DEG>(tile, mask, x, blk, res, iso);
-  __syncthreads();
-  // thread = one x row of 16 cells
-  const int ly = threadIdx.x & 15, lz = threadIdx.x >> 4;
   int cnt = 0;
-#pragma unroll 4
-  for (int lx = 0; lx < 16; ++lx) {
-    const uint32_t mc = mc_mask_case(mask, lx, ly, lz);
-    cnt += (mc != 0u && mc != 255u);
+  if (mc_block_masks<DEG>(s, x, blk, res, iso)) {
+    // thread = one x row of 16 cells; a cell is cut when its corners' bits differ
+    const uint32_t* m = s.mask + (threadIdx.x >> 4) * MCW + (threadIdx.x & 15);
+    const uint32_t any = m[0] | m[1] | m[MCW] | m[MCW + 1], all = m[0] & m[1] & m[MCW] & m[MCW + 1];
+    cnt = __popc((any | any >> 1) & ~(all & all >> 1) & 0xffffu);
   }
   typedef cub::BlockReduce<int, 256> BR;
   __shared__ typename BR::TempStorage tmp;
@@ -601,39 +667,40 @@ __global__ void __launch_bounds__(256) k_mc_block_count(const double* __restrict
   if (threadIdx.x == 0) blockcnt[blk] = (uint32_t)tot;
 }
 
-// active blocks only (list from a compaction of blockcnt > 0); cells written in Morton order
+// active blocks only (list from a compaction of blockcnt > 0); cells written in Morton order, 16 to a
+// thread (one scan of the block)
 template <int DEG>
 __global__ void __launch_bounds__(256) k_mc_block_emit(const double* __restrict__ x, uint32_t D, double iso,
                                                        const uint32_t* __restrict__ ablk,
                                                        const uint32_t* __restrict__ blockoff,
                                                        uint32_t* __restrict__ acell, uint8_t* __restrict__ acase,
                                                        uint32_t* __restrict__ nedge, uint32_t* __restrict__ ntri) {
-  __shared__ double tile[DEG >= 2 ? MCW2 * MCW2 * MCW2 : MCW * MCW * MCW];
-  __shared__ uint32_t mask[MCW * MCW];
+  __shared__ McShared<DEG> s;
   const int res = 1 << D;
   const uint32_t blk = ablk[blockIdx.x];
-  mc_block_masks<DEG>(tile, mask, x, blk, res, iso);
-  __syncthreads();
+  if (!mc_block_masks<DEG>(s, x, blk, res, iso)) return;
   typedef cub::BlockScan<int, 256> BS;
   __shared__ typename BS::TempStorage tmp;
-  uint32_t running = blockoff[blk];
-  for (int chunk = 0; chunk < 16; ++chunk) {
-    const int i = chunk * 256 + threadIdx.x;  // Morton-local cell index
-    uint32_t lx, ly, lz;
-    unmorton3((uint32_t)i, lx, ly, lz);
-    const uint32_t mc = mc_mask_case(mask, (int)lx, (int)ly, (int)lz);
-    const int active = (mc != 0u && mc != 255u);
-    int off, tot;
-    BS(tmp).ExclusiveSum(active, off, tot);
-    if (active) {
-      const uint32_t a = running + (uint32_t)off;
-      acell[a] = (blk << 12) | (uint32_t)i;
-      acase[a] = (uint8_t)mc;
-      nedge[a] = __popc(edge_mask(mc));
-      ntri[a] = PR_MC_NTRI[mc];
-    }
-    running += (uint32_t)tot;
-    __syncthreads();  // temp storage reuse
+  const uint32_t i0 = 16 * threadIdx.x;  // Morton-local cell index
+  uint32_t lx, ly, lz, active = 0;
+  unmorton3(i0, lx, ly, lz);
+  const auto cell_of = [&](int k) {  // 4 x 2 x 2 cells
+    return mc_mask_case(s.mask, (int)lx + ((k & 1) | (k >> 2 & 2)), (int)ly + (k >> 1 & 1), (int)lz + (k >> 2 & 1));
+  };
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    const uint32_t mc = cell_of(k);
+    active |= (uint32_t)(mc != 0u && mc != 255u) << k;
+  }
+  int off;
+  BS(tmp).ExclusiveSum(__popc(active), off);
+  for (uint32_t a = blockoff[blk] + (uint32_t)off; active; active &= active - 1, ++a) {
+    const int k = __ffs(active) - 1;
+    const uint32_t mc = cell_of(k);
+    acell[a] = (blk << 12) | (i0 + (uint32_t)k);
+    acase[a] = (uint8_t)mc;
+    nedge[a] = __popc(edge_mask(mc));
+    ntri[a] = PR_MC_NTRI[mc];
   }
 }
 

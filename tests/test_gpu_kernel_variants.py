@@ -114,3 +114,25 @@ def test_band_coarse_function(ctx, depth, flags):
     assert np.max(np.abs(g - g_all[prb.band_natural_index(codes, depth)])) <= 1e-13 * np.max(np.abs(g_all))
     t = mesh.triangles.astype(np.int64)
     assert t.max() + 1 == len(mesh.vertices) == len(np.unique(t))
+
+
+@pytest.mark.parametrize("degree", [1, 2])
+@pytest.mark.parametrize("depth", [4, 5])
+@pytest.mark.parametrize("lo,hi", [((0, 0, 0), (3, 5, 4)), ((11, 0, 16), (16, 16, 17)), ((0, 15, 0), (99, 99, 99)),
+                                   ((13, 14, 15), (99, 99, 99)), ((0, 0, 0), (99, 99, 99))])
+def test_block_classification(ctx, degree, depth, lo, hi):
+    """Boxes of raised coefficients at the low and the top faces of the grid and across the 16^3 blocks, in
+    a level field: the blocks that are told from their extremes
+    and those whose corners are formed give the oracle's mesh, with the iso value between the two levels and
+    at each of them."""
+    res = 1 << depth
+    xyz = np.stack(np.meshgrid(*[np.arange(res)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    code = sum(((xyz[:, a] >> b) & 1) << (3 * b + a) for a in range(3) for b in range(depth))
+    field = np.empty(res ** 3)
+    field[code] = np.where(((xyz >= lo) & (xyz < hi)).all(1), 1.0, -0.5)
+    ctx.solve(synthetic.sphere(2000, seed=90), prb.ReconstructParams(depth=depth, degree=degree, point_weight=4.0))
+    for iso in (0.25, 1.0, -0.5, 0.0, 2.0):
+        mesh = ctx.extract(field, iso)
+        v_ref, t_ref = (oracle.extract_surface if degree == 1 else oracle.extract_surface2)(depth, field, iso)
+        assert np.array_equal(mesh.vertices, v_ref)
+        assert np.array_equal(mesh.triangles, t_ref)
