@@ -509,20 +509,22 @@ __global__ void k_dense_solve(uint32_t nc, const T* __restrict__ inv, const T* _
   }
 }
 
-// A = L L^T, then A^-1 = L^-T L^-1, each entry with the products subtracted one by one in ascending
-// order.  The factorisation and Y = L^-1 advance together: step k finishes column k of L and row k
-// of Y and subtracts their products from the rest (a thread owns 8 of the 64 x 64 entries, of L right
-// of column k and of Y up to it).  The back substitution is a thread per column, whose chain of
-// 64 * 63 / 2 subtractions bounds the kernel (about 30 us in all; on the host, where it was a chain of
-// half a million dependent operations, 0.4 ms of every solve with the GPU idle).
+// A = L D L^T (L unit lower), Y = L^-1, A^-1 = Y^T D^-1 Y.  The factorisation and Y advance together: step k
+// subtracts the products of column k of L D and of row k of Y from what is left of both (a thread owns one
+// column j, 8 of its 64 entries: of L D while k < j, of Y from then on), so a step is one reciprocal, one
+// round of multiply-adds and one barrier, and the chain of the 64 steps bounds the kernel: 43 us.  The
+// product is 64 independent multiply-adds per entry.  (With the roots and quotients of L L^T, three
+// barriers a step, and back substitutions, a chain of 64 * 63 / 2 subtractions per column: 84 us.  On the
+// host it was 0.4 ms of every solve.)
 constexpr int kInvN = 64, kInvStride = kInvN + 1;
 template <typename T>
 __global__ void __launch_bounds__(512) k_spd_inverse(int n, const double* __restrict__ A, T* __restrict__ inv,
                                                      int* __restrict__ bad) {
   extern __shared__ double spd_smem[];
-  double* L = spd_smem;                     // lower triangle
+  double* L = spd_smem;  // L D below the diagonal, D on it
   double* Y = spd_smem + kInvN * kInvStride;
-  const int t = threadIdx.x;
+  __shared__ double dinv[kInvN];
+  const int t = threadIdx.x, j = t & 63;
   for (int i = t; i < n * n; i += 512) {
     const int r = i / n, q = i % n;
     L[r * kInvStride + q] = A[i];
@@ -533,35 +535,26 @@ __global__ void __launch_bounds__(512) k_spd_inverse(int n, const double* __rest
   for (int k = 0; k < n; ++k) {
     const double p = L[k * kInvStride + k];
     if (!(p > 0.0)) failed = 1;
-    const double d = __dsqrt_rn(p);
-    __syncthreads();  // every thread has read the pivot
-    if (t < n) {
-      if (t == k) L[k * kInvStride + k] = d;
-      else if (t > k) L[t * kInvStride + k] = xdiv(L[t * kInvStride + k], d);
-    } else if (t >= kInvN && t - kInvN <= k) {
-      Y[k * kInvStride + t - kInvN] = xdiv(Y[k * kInvStride + t - kInvN], d);
-    }
-    __syncthreads();
+    const double inverse = xdiv(1.0, p);
+    if (t == 0) dinv[k] = inverse;
+    if (j < n) {
+      double* M = j > k ? L : Y;
+      const double f = (j > k ? L[j * kInvStride + k] : Y[k * kInvStride + j]) * inverse;
 #pragma unroll
-    for (int u = 0; u < kInvN * kInvN / 512; ++u) {
-      const int i = (u * 512 + t) >> 6, j = t & 63;
-      if (i <= k || i >= n || j > i) continue;
-      double* e = (j > k ? L : Y) + i * kInvStride + j;
-      const double f = j > k ? L[j * kInvStride + k] : Y[k * kInvStride + j];
-      *e = xsub(*e, xmul(L[i * kInvStride + k], f));
+      for (int u = 0; u < kInvN * kInvN / 512; ++u) {
+        const int i = 8 * u + (t >> 6);
+        if (i > k && i < n && j <= i) M[i * kInvStride + j] -= L[i * kInvStride + k] * f;
+      }
     }
     __syncthreads();
   }
-  if (t < n) {
-    for (int i = n - 1; i >= 0; --i) {
-      double s = Y[i * kInvStride + t];
+  for (int i = t; i < n * n; i += 512) {
+    const int r = i / n, q = i % n, low = min(r, q), high = max(r, q);  // the same bits at (r, q) and (q, r)
+    double s = 0.0;
 #pragma unroll 8
-      for (int k = i + 1; k < n; ++k) s = xsub(s, xmul(L[k * kInvStride + i], Y[k * kInvStride + t]));
-      Y[i * kInvStride + t] = xdiv(s, L[i * kInvStride + i]);
-    }
+    for (int k = high; k < n; ++k) s += Y[k * kInvStride + low] * (Y[k * kInvStride + high] * dinv[k]);
+    inv[i] = (T)s;
   }
-  __syncthreads();
-  for (int i = t; i < n * n; i += 512) inv[i] = (T)Y[(i / n) * kInvStride + i % n];
   if (t == 0) *bad = failed;
 }
 
