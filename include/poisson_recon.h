@@ -305,7 +305,7 @@ int pr_ply_write_mesh(const char* path, const pr_mesh* mesh, int format);
 uint64_t pr_kernel_launches(uint64_t* primitive_calls);
 
 /* The z-segment choices of the degree-1 block kernels made so far in this process: the first
- * FP32 launch of a (kernel family, level, launch size) times 2, 4 and 8 z planes per thread
+ * FP32 launch of a (kernel family, level, launch size) times 2 and 4 z planes per thread
  * (identical results) and keeps the fastest; one line per choice with its timings.  Library
  * memory, valid until the next call. */
 const char* pr_autotune_log(void);

@@ -1896,7 +1896,8 @@ void smooth_dispatch(cudaStream_t s, uint32_t D, const T* xi, T* xo, const T* f,
 // launch of a (kernel family, level, launch size, with or without face rows: the same level is one
 // solve's finest and another's coarse) key times both (one warm-up and three timed launches on the
 // launch's own buffers; every candidate writes what the real launch then overwrites) and keeps the
-// faster for the process.  FP64 launches and launches inside a stream capture use ZT = 4.  PR_AUTOTUNE=0 fixes ZT = 4; PR_ZT=2|4 forces one (8, an earlier shape, means 4).
+// faster for the process.  FP64 launches and launches inside a stream capture use ZT = 4.
+// PR_AUTOTUNE=0 fixes ZT = 4; PR_ZT=2|4 forces one (8, an earlier shape, means 4).
 enum TuneFamily { kTuneSpmv = 0, kTuneResid = 1, kTuneSmooth = 2, kTuneSmoothPost = 3 };
 struct TuneTable {
   std::mutex mu;

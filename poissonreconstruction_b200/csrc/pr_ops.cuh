@@ -118,7 +118,7 @@ template <typename T>
 void dense_solve(cudaStream_t s, uint32_t nc, const T* inv, const T* f, T* e, uint32_t clouds = 1);
 
 // inv = A^-1 of a symmetric positive definite matrix of order n <= 64 (A: host, row-major, FP64), by
-// Cholesky in FP64 on the device.  Whether A was positive definite is known after the stream's next
+// L D L^T in FP64 on the device.  Whether A was positive definite is known after the stream's next
 // synchronisation: spd_check throws if it was not.
 template <typename T>
 void spd_inverse(pr_context* c, int n, const double* A, T* inv);
