@@ -180,20 +180,13 @@ void* alloc_host_out(size_t bytes) {
   return p;
 }
 
-// Large copies between pageable host memory and the device.  The driver's own path is one thread that
-// stages through a pinned buffer; out of the device it also faults in the pages of a fresh destination.
-// Here host threads copy 1 MiB pieces to and from eight pinned slots (8 MiB per context) while the DMAs of
-// other slots run.  The calling thread issues every DMA; the helpers call no CUDA function, since a stream
-// handle can name another stream in another thread (cudaStreamPerThread).  Beside helpers the calling
-// thread copies nothing itself: they would wait for it.  A call returns when the host side is done with: the source may be reused
-// (copy_to_device: the last DMAs may still run on the context's stream) or the destination is complete.
-// Measured (ms, the driver's path and this one): out 2 MB 0.34 and 0.23 with one thread, 17 MB 2.1 and 1.5 with
-// two, 134 MB 27 and 9.9 with four; in, what a solve takes longer from pageable points than from pinned ones,
-// 48 MB 3.6 and 1.0 with four, while 19 MB and less gain nothing.  Pinned caller memory, small copies and the
-// batch engine's threads (many copies at once) keep the plain path.
+// Large copies between pageable host memory and the device go through pinned slots (pr_staged_copy.h, 8 MiB
+// per context).  Measured (ms, the driver's path and this one): out 2 MB 0.34 and 0.23 with one thread, 17 MB
+// 2.1 and 1.5 with two, 134 MB 27 and 9.9 with four; in, what a solve takes longer from pageable points than
+// from pinned ones, 48 MB 3.6 and 1.0 with four, while 19 MB and less gain nothing.  Pinned caller memory,
+// small copies, the batch engine's threads (many copies at once) and a host without pinned memory for the
+// slots keep the driver's path.
 thread_local bool t_in_batch = false;
-constexpr size_t kSlot = size_t(1) << 20;
-constexpr int kStageThreads = 4, kSlots = 2 * kStageThreads;
 
 // threads that copy pieces, one: the calling thread by itself; 0: the plain path
 int stage_threads(const void* host, size_t bytes, bool out) {
@@ -204,126 +197,29 @@ int stage_threads(const void* host, size_t bytes, bool out) {
     return 0;
   }
   if (a.type != cudaMemoryTypeUnregistered) return 0;
-  const int nt = bytes < size_t(8) << 20 ? 1 : (bytes < size_t(32) << 20 ? 2 : kStageThreads);
+  const int nt = bytes < size_t(8) << 20 ? 1 : (bytes < size_t(32) << 20 ? 2 : pr::kStageThreads);
   return std::max(1, std::min<int>(nt, (int)std::thread::hardware_concurrency()));
 }
-
-// The pieces of one copy between host memory and the slots (piece k in slot k mod kSlots), shared by the
-// copying threads: pieces [0, avail) may be moved, next is the first that no thread has taken.
-struct StagedPieces {
-  const size_t pieces;
-  std::atomic<size_t> avail{0}, next{0};
-  std::atomic<bool> stop{false};
-  std::unique_ptr<std::atomic<bool>[]> moved;
-  explicit StagedPieces(size_t n) : pieces(n), moved(new std::atomic<bool>[n]) {
-    for (size_t k = 0; k < n; ++k) moved[k].store(false, std::memory_order_relaxed);
-  }
-  // takes a piece and moves it; false if there is none for now
-  template <typename F>
-  bool move_one(F move) {
-    size_t k = next.load(std::memory_order_relaxed);
-    do {
-      if (k >= avail.load(std::memory_order_acquire)) return false;
-    } while (!next.compare_exchange_weak(k, k + 1, std::memory_order_relaxed));
-    move(k);
-    moved[k].store(true, std::memory_order_release);
-    return true;
-  }
-  bool is_moved(size_t k) const { return moved[k].load(std::memory_order_acquire); }
-  // a helper thread's work
-  template <typename F>
-  void help(F move) {
-    while (!stop.load(std::memory_order_relaxed) && next.load(std::memory_order_relaxed) < pieces)
-      if (!move_one(move)) std::this_thread::yield();
-  }
-};
-
-// Runs drive(whether this thread is alone) in this thread, beside nt helpers that move pieces (none for one).
-template <typename Drive, typename Move>
-cudaError_t with_helpers(StagedPieces& q, int nt, Drive drive, Move move) {
-  std::vector<std::thread> th;
-  try {
-    for (int i = 0; nt > 1 && i < nt; ++i) th.emplace_back([&q, move] { q.help(move); });
-  } catch (...) {  // no more threads: those that there are share the pieces
-  }
-  const cudaError_t e = drive(th.empty());
-  q.stop = true;
-  for (auto& t : th) t.join();
-  return e;
-}
-
-// Copies in pieces through the slots.  `out`: device to host.
-void staged_copy(pr_context* c, unsigned char* dev, unsigned char* host, size_t bytes, int nt, bool out) {
-  if (!c->h_slots) PR_CUDA(cudaMallocHost(&c->h_slots, kSlots * kSlot));
-  while (c->slot_events.size() < kSlots) {
-    cudaEvent_t e = nullptr;
-    PR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    c->slot_events.push_back(e);
-  }
-  StagedPieces q((bytes + kSlot - 1) / kSlot);
-  unsigned char* const slots = c->h_slots;
-  auto length = [bytes](size_t k) { return std::min(kSlot, bytes - k * kSlot); };
-  auto slot = [slots](size_t k) { return slots + (k % kSlots) * kSlot; };
-  auto move = [=](size_t k) {
-    if (out) std::memcpy(host + k * kSlot, slot(k), length(k));
-    else std::memcpy(slot(k), host + k * kSlot, length(k));
-  };
-  auto drive = [&](bool alone) -> cudaError_t {
-    size_t issued = 0;  // pieces whose DMA was issued
-    size_t done = 0;    // out: pieces whose DMA has arrived; in: pieces whose slot is free of earlier DMAs
-    for (;;) {
-      const bool can_issue = issued < q.pieces && (out ? issued < kSlots || q.is_moved(issued - kSlots) : q.is_moved(issued));
-      if (can_issue) {
-        const size_t k = issued % kSlots;
-        cudaError_t e = cudaSuccess;
-        if (out && issued < kSlots) e = cudaEventSynchronize(c->slot_events[k]);  // an earlier copy's DMA from the slot
-        if (e == cudaSuccess)
-          e = out ? cudaMemcpyAsync(slot(issued), dev + issued * kSlot, length(issued), cudaMemcpyDeviceToHost, c->stream)
-                  : cudaMemcpyAsync(dev + issued * kSlot, slot(issued), length(issued), cudaMemcpyHostToDevice, c->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(c->slot_events[k], c->stream);
-        if (e != cudaSuccess) return e;
-        ++issued;
-        continue;
-      }
-      if (out ? done < issued : done < q.pieces && done < issued + kSlots) {
-        const cudaError_t e = cudaEventQuery(c->slot_events[done % kSlots]);
-        if (e == cudaSuccess) {
-          q.avail.store(++done, std::memory_order_release);
-          continue;
-        }
-        if (e != cudaErrorNotReady) return e;
-        cudaGetLastError();
-      }
-      if (alone && q.move_one(move)) continue;
-      if (!out && issued == q.pieces) return cudaSuccess;
-      if (out && done == q.pieces) {
-        size_t k = q.pieces > kSlots ? q.pieces - kSlots : 0;  // the earlier ones' slots were reused
-        while (k < q.pieces && q.is_moved(k)) ++k;
-        if (k == q.pieces) return cudaSuccess;
-      }
-      std::this_thread::yield();
-    }
-  };
-  const cudaError_t e = with_helpers(q, nt, drive, move);
+bool copy_staged(pr_context* c, void* dev, void* host, size_t bytes, bool out) {
+  const int nt = stage_threads(host, bytes, out);
+  if (nt == 0 || !c->slots.make()) return false;
+  const cudaError_t e = pr::staged_copy(c->stream, c->slots, static_cast<unsigned char*>(dev),
+                                        static_cast<unsigned char*>(host), bytes, nt, out);
   if (e != cudaSuccess) {
     cudaStreamSynchronize(c->stream);
     throw pr::Error(PR_ERR_CUDA, std::string("host copy failed: ") + cudaGetErrorString(e));
   }
+  return true;
 }
 void copy_to_device(pr_context* c, void* d, const void* h, size_t bytes) {
-  const int nt = stage_threads(h, bytes, false);
-  if (nt == 0) PR_CUDA(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, c->stream));
-  else staged_copy(c, static_cast<unsigned char*>(d), static_cast<unsigned char*>(const_cast<void*>(h)), bytes, nt, false);
+  if (copy_staged(c, d, const_cast<void*>(h), bytes, false)) return;
+  PR_CUDA(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, c->stream));
 }
 // complete on return
 void copy_to_host(pr_context* c, void* h, const void* d, size_t bytes) {
-  const int nt = stage_threads(h, bytes, true);
-  if (nt == 0) {
-    PR_CUDA(cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, c->stream));
-    c->sync();
-  } else {
-    staged_copy(c, static_cast<unsigned char*>(const_cast<void*>(d)), static_cast<unsigned char*>(h), bytes, nt, true);
-  }
+  if (copy_staged(c, const_cast<void*>(d), h, bytes, true)) return;
+  PR_CUDA(cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, c->stream));
+  c->sync();
 }
 
 // Device mesh -> caller memory: D2H copies of 8 MiB chunks into the context's pinned staging,
@@ -1003,9 +899,7 @@ int pr_context_destroy(pr_context* c) {
     if (c->h_scalars) cudaFreeHost(c->h_scalars);
     if (c->h_pack) cudaFreeHost(c->h_pack);
     if (c->h_ring) cudaFreeHost(c->h_ring);
-    if (c->h_slots) cudaFreeHost(c->h_slots);
-    for (cudaEvent_t e : c->slot_events)
-      if (e) cudaEventDestroy(e);
+    c->slots.free();
     if (c->h_flag) cudaFreeHost(c->h_flag);
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->own_stream) cudaStreamDestroy(c->stream);

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "../../include/poisson_recon.h"
+#include "pr_staged_copy.h"
 
 namespace pr {
 
@@ -177,9 +178,7 @@ struct pr_context {
     PR_CUDA(cudaMemcpyAsync(dst, h_ring + h_ring_used, bytes, cudaMemcpyHostToDevice, stream));
     h_ring_used += need;
   }
-  // pinned slots and events of the copies between pageable host memory and the device (pr_abi.cu)
-  unsigned char* h_slots = nullptr;
-  std::vector<cudaEvent_t> slot_events;
+  pr::StageSlots slots;  // of the copies between pageable host memory and the device (pr_abi.cu)
   int* h_flag = nullptr;  // pinned: the status of the last spd_inverse (pr_operator.cu)
   // pinned staging for device->host mesh copies (grown on demand)
   unsigned char* h_stage = nullptr;
