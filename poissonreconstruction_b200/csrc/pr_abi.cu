@@ -890,6 +890,7 @@ int pr_context_destroy(pr_context* c) {
     c->copy_events.clear();
     for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second.exec);
     c->graphs.clear();
+    if (c->capture) cudaStreamDestroy(c->capture);
     if (c->side) {
       cudaStreamSynchronize(c->side);
       cudaStreamDestroy(c->side);

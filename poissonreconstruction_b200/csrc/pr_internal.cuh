@@ -227,7 +227,7 @@ struct pr_context {
     return side;
   }
   pr_params params{};             // parameters of the last reconstruction
-  // Instantiated CUDA graphs of repeated launch sequences on `stream` (the solver's V-cycle),
+  // Instantiated CUDA graphs of repeated launch sequences on `stream` (the solver's iterations),
   // keyed by everything they were captured with (sizes, coefficients, buffer addresses); kept for
   // reuse, with the kernel launches they hold (counted again at every replay).
   struct Graph {
@@ -237,7 +237,27 @@ struct pr_context {
     int parts = 0;       // and the partial sums that they leave
   };
   std::map<std::string, Graph> graphs;
-  // Runs body() through the graph of `key`, capturing it on first use.
+  // Graphs are captured on a stream of the context's own, of the priority of `stream`, and launched on
+  // `stream`: the legacy stream cannot be captured, and while a caller's stream that orders with it is
+  // being captured no thread of the process may use the legacy stream.
+  cudaStream_t capture = nullptr;
+  struct CaptureStream {  // `stream` is the capture stream for the life of this object
+    pr_context& c;
+    cudaStream_t const launch;
+    explicit CaptureStream(pr_context& ctx) : c(ctx), launch(ctx.stream) {
+      if (!c.capture) {
+        int priority = 0;
+        PR_CUDA(cudaStreamGetPriority(launch, &priority));
+        PR_CUDA(cudaStreamCreateWithPriority(&c.capture, cudaStreamNonBlocking, priority));
+      }
+      c.stream = c.capture;
+    }
+    ~CaptureStream() { c.stream = launch; }
+    CaptureStream(const CaptureStream&) = delete;
+    CaptureStream& operator=(const CaptureStream&) = delete;
+  };
+  // Runs body() through the graph of `key`, capturing it on first use.  body() takes the stream to launch
+  // on from `stream`, when it runs.
   template <typename F>
   Graph& run_graph(const std::string& key, F body) {
     auto it = graphs.find(key);
@@ -249,16 +269,19 @@ struct pr_context {
       }
       cudaGraph_t g = nullptr;
       const uint64_t l0 = pr::thread_launch_count(0), p0 = pr::thread_launch_count(1);
-      PR_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-      try {
-        body();
-      } catch (...) {
-        cudaStreamEndCapture(stream, &g);
-        if (g) cudaGraphDestroy(g);
-        cudaGetLastError();
-        throw;
+      {
+        const CaptureStream on(*this);
+        PR_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+        try {
+          body();
+        } catch (...) {
+          cudaStreamEndCapture(stream, &g);
+          if (g) cudaGraphDestroy(g);
+          cudaGetLastError();
+          throw;
+        }
+        PR_CUDA(cudaStreamEndCapture(stream, &g));
       }
-      PR_CUDA(cudaStreamEndCapture(stream, &g));
       const uint64_t l1 = pr::thread_launch_count(0), p1 = pr::thread_launch_count(1);
       Graph gr;
       const cudaError_t e = cudaGraphInstantiate(&gr.exec, g, 0);

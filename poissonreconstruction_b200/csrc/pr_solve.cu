@@ -462,7 +462,7 @@ PcgResult pcg(Pack& pk, CgOperator<T>& A, Multigrid<T>& M, const T* b, T* x, con
     M.apply(sc, kCgRz0, b, z0, false);
     A.apply_dot(sc, z0, z0, nullptr, false, q);
     M.cg_update_presmooth(sc, z0, q, x, r, b);
-    PR_CUDA(cudaMemcpyAsync(h, sc.rr, back, cudaMemcpyDeviceToHost, s));
+    PR_CUDA(cudaMemcpyAsync(h, sc.rr, back, cudaMemcpyDeviceToHost, c->stream));
   };
   if (graphs && (M.checked || c->graphs.count(base + "/f"))) c->run_graph(base + "/f", first);
   else first();
@@ -478,7 +478,7 @@ PcgResult pcg(Pack& pk, CgOperator<T>& A, Multigrid<T>& M, const T* b, T* x, con
       M.apply(sc, kCgRz, r, z, true);
       A.apply_dot(sc, z, d, dn, true, q);
       M.cg_update_presmooth(sc, dn, q, x, r, nullptr);
-      PR_CUDA(cudaMemcpyAsync(h, sc.rr, back, cudaMemcpyDeviceToHost, s));
+      PR_CUDA(cudaMemcpyAsync(h, sc.rr, back, cudaMemcpyDeviceToHost, c->stream));
     };
     if (graphs) c->run_graph(base + (dn == dA ? "/a" : "/z"), body);
     else body();
