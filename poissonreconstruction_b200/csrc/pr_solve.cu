@@ -738,14 +738,14 @@ void solve_packed(pr_context* sc, const std::vector<pr_context*>& cl, const pr_p
 namespace {
 // y = A x for a caller's vectors.  From depth 4 on the solver's tiled SpMV, whose rows read each node
 // once from memory and are shared between a 2x2 column's nodes: at depth 9 in FP32 the per-node
-// stencil, 21 gathers a node, took 1.75 ms, the tiles 0.34.  It needs 32-byte aligned vectors; other
-// pointers, and smaller grids, take the per-node stencil.
+// stencil, 21 gathers a node, takes 1.67 ms, the tiles 0.33.  They access 16 bytes at a time; vectors
+// that are not aligned so, and smaller grids, take the per-node stencil.
 template <typename T>
 void apply_operator(pr_context* c, const T* d_x, T* d_y) {
   const double h = 1.0 / (double)(1u << c->D);
   const double wg = c->pw > 0.0 ? (c->pw * (h * h * h) / 1.5) * 0.005 : 0.0;
   const FineOp<T> op = make_fine_op<T>(c, wg);
-  const bool aligned = ((reinterpret_cast<uintptr_t>(d_x) | reinterpret_cast<uintptr_t>(d_y)) & 31u) == 0;
+  const bool aligned = ((reinterpret_cast<uintptr_t>(d_x) | reinterpret_cast<uintptr_t>(d_y)) & 15u) == 0;
   if (c->D < 4 || !aligned) {
     op.apply(c->stream, d_x, d_y);
     return;

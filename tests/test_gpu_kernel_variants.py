@@ -50,6 +50,29 @@ def test_operator_on_device_vectors(ctx, depth, offset, precision):
 
 
 @pytest.mark.parametrize("precision", [prb.PR_PRECISION_FP64, prb.PR_PRECISION_MIXED])
+def test_operator_takes_the_tiles_from_16_bytes_on(ctx, precision):
+    """Vectors that are aligned to 16 bytes and no further take the kernel of the aligned ones: the same
+    bits, where the per-node stencil adds in another order."""
+    import torch
+    depth = 5
+    ctx.solve(synthetic.sphere(2500, seed=55), prb.ReconstructParams(depth=depth, point_weight=4.0))
+    dtype = torch.float64 if precision == prb.PR_PRECISION_FP64 else torch.float32
+    x0 = torch.randn(8 ** depth, dtype=dtype, generator=torch.Generator().manual_seed(5))
+    got = {}
+    for nbytes in (0, x0.element_size(), 16):
+        k = nbytes // x0.element_size()
+        x, y = (torch.zeros(8 ** depth + k, dtype=dtype, device="cuda")[k:] for _ in range(2))
+        assert x.data_ptr() % 32 == nbytes and y.data_ptr() % 32 == nbytes
+        x.copy_(x0)
+        torch.cuda.synchronize()
+        ctx.apply_operator_device(x.data_ptr(), y.data_ptr(), precision)
+        ctx.synchronize()
+        got[nbytes] = y.cpu().numpy()
+    assert np.array_equal(got[0], got[16])
+    assert not np.array_equal(got[0], got[x0.element_size()])
+
+
+@pytest.mark.parametrize("precision", [prb.PR_PRECISION_FP64, prb.PR_PRECISION_MIXED])
 @pytest.mark.parametrize("depth", [5, 6, 7])
 def test_degree2_short_plane_runs(ctx, depth, precision):
     """The levels up to 128^3 run in short runs of planes: the solution satisfies the oracle's equations
