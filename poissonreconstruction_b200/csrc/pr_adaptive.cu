@@ -755,15 +755,15 @@ __global__ void k_ab_step(uint64_t n, const CgBand* __restrict__ cg, const T* __
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
     x[i] += a * d[i];
 }
-// the CG update with the Jacobi step: r -= alpha q, z = dinv r; per-block sums of r . r (part[2 b]) and
-// r . z (part[2 b + 1]) in FP64
+// the CG update with the Jacobi step: r -= alpha q (alpha 0, after a breakdown: r stays, whatever q holds),
+// z = dinv r; per-block sums of r . r (part[2 b]) and r . z (part[2 b + 1]) in FP64
 template <typename T>
 __global__ void k_ab_update(uint64_t n, const CgBand* __restrict__ cg, const T* __restrict__ q, T* __restrict__ r,
                             const T* __restrict__ dinv, T* __restrict__ z, double* __restrict__ part) {
   const T a = (T)cg->alpha;
   double rr = 0.0, rz = 0.0;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const T ri = r[i] - a * q[i];
+    const T ri = a != T(0) ? r[i] - a * q[i] : r[i];
     r[i] = ri;
     const T zi = dinv[i] * ri;
     z[i] = zi;

@@ -159,3 +159,22 @@ def test_block_classification(ctx, degree, depth, lo, hi):
         v_ref, t_ref = (oracle.extract_surface if degree == 1 else oracle.extract_surface2)(depth, field, iso)
         assert np.array_equal(mesh.vertices, v_ref)
         assert np.array_equal(mesh.triangles, t_ref)
+
+
+@pytest.mark.parametrize("degree,depth,coarse", [(1, 3, 0), (1, 5, 0), (2, 4, 0), (2, 6, 0), (2, 6, 4)])
+def test_breakdown_of_conjugate_gradients(ctx, degree, depth, coarse):
+    """A screening weight beyond FP32 makes the FP32 operator infinite: the first direction's product with
+    it is not a positive number, the iteration stops there with its solution, zero (on a band the coarse
+    function).  The same weight in FP64 is solved."""
+    pts = synthetic.torus(2000, seed=1)
+    params = dict(depth=depth, degree=degree, coarse_depth=coarse, point_weight=1e150)
+
+    def solution():
+        return ctx.band_vector(1) if coarse else ctx.coefficients()
+
+    st = ctx.solve(pts, prb.ReconstructParams(precision=prb.PR_PRECISION_MIXED, **params))
+    assert (st.converged, st.pcg_iterations) == (0, 0), st
+    start = ctx.band_vector(2) if coarse else np.zeros(8 ** depth)
+    assert np.isfinite(start).all() and np.array_equal(solution(), start)
+    st = ctx.solve(pts, prb.ReconstructParams(precision=prb.PR_PRECISION_FP64, **params))
+    assert st.converged == 1 and np.isfinite(solution()).all(), st
