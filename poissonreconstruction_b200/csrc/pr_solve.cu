@@ -162,6 +162,10 @@ struct Multigrid {
   }
   const T* table(uint32_t l) const { return tables + (size_t)l * 216; }
 
+  static bool coarse_tail() {
+    const char* v = std::getenv("PR_COARSE_TAIL");
+    return !(v && std::atoi(v) == 0);
+  }
   // el = V(fl); at the finest level `part` (nullable) receives per-block fl.el partials.
   // presmoothed: the first pre-smoothing sweep of this level is already in a_l.
   void vcycle(uint32_t l, const T* fl, T* el, double* part, bool presmoothed = false) {
@@ -170,8 +174,9 @@ struct Multigrid {
       dense_solve<T>(s, nc, inv, fl, el, clouds);
       return;
     }
-    // the coarse levels that fit one block; with more sweeps, and on grids up to 16^3, level by level
-    if (l == 4 && l < D && sweeps == 1) {
+    // the coarse levels that fit one block; with more sweeps, on grids up to 16^3, and with
+    // PR_COARSE_TAIL=0 (the same values), level by level
+    if (l == 4 && l < D && sweeps == 1 && coarse_tail()) {
       mg_coarse_tail<T>(s, L[4], L[3], table(4), table(3), inv, fl, el, clouds);
       return;
     }
@@ -236,7 +241,7 @@ struct Multigrid {
   }
   bool checked = false;
   // everything that captured launches of this hierarchy depend on besides the caller's vectors:
-  // sizes, the shift (kernel arguments), every buffer, the z-segment switches
+  // sizes, the shift (kernel arguments), every buffer, the switches between kernels
   std::string graph_base() {
     char b[96];
     std::snprintf(b, sizeof(b), "cg/%s/%u/%u/%d/%a", tname<T>(), D, clouds, sweeps, pk->wg);
@@ -255,7 +260,7 @@ struct Multigrid {
       add(t[l]);
       add(face[l]);
     }
-    for (const char* v : {"PR_ZT", "PR_AUTOTUNE", "PR_ZT_SPMV16", "PR_ZT_RESID16", "PR_ZT_SMOOTH16"}) {
+    for (const char* v : {"PR_ZT", "PR_AUTOTUNE", "PR_ZT_SPMV16", "PR_ZT_RESID16", "PR_ZT_SMOOTH16", "PR_COARSE_TAIL"}) {
       const char* x = std::getenv(v);
       k += "/";
       k += x ? x : "-";

@@ -26,6 +26,35 @@ def test_coarse_levels_of_the_degree1_vcycle(ctx, depth, sweeps, precision):
     assert np.linalg.norm(x - x_ref) <= 1e-6 * np.linalg.norm(x_ref)
 
 
+def _solution(c, pts, params):
+    st = c.solve(pts, params)
+    return (st.pcg_iterations, st.refinement_steps, st.rel_residual), c.coefficients()
+
+
+def _same(a, b):
+    return a[0] == b[0] and np.array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("precision", [prb.PR_PRECISION_FP64, prb.PR_PRECISION_MIXED])
+@pytest.mark.parametrize("depth,pw", [(5, 4.0), (6, 0.0), (7, 4.0)])
+def test_coarse_levels_in_one_launch_and_level_by_level(ctx, depth, pw, precision, monkeypatch):
+    """The kernel of the levels 16^3, 8^3 and 4^3 does the arithmetic of their own kernels: every bit of a
+    solve, and of a packed batch's meshes, is the same with and without it."""
+    params = prb.ReconstructParams(depth=depth, point_weight=pw, precision=precision)
+    clouds = [synthetic.torus(2000 + 500 * k, seed=30 + k) for k in range(3)]
+    runs = []
+    for value in ("1", "0"):
+        monkeypatch.setenv("PR_COARSE_TAIL", value)
+        before = prb.kernel_launches()[0]
+        one = _solution(ctx, clouds[0], params)
+        runs.append((prb.kernel_launches()[0] - before, one, prb.reconstruct_batch(clouds, [params] * 3)))
+    (n1, one1, batch1), (n0, one0, batch0) = runs
+    assert n0 > n1 and _same(one1, one0)
+    for (m1, s1), (m0, s0) in zip(batch1, batch0):
+        assert s1.pcg_iterations == s0.pcg_iterations and s1.iso_value == s0.iso_value
+        assert np.array_equal(m1.vertices, m0.vertices) and np.array_equal(m1.triangles, m0.triangles)
+
+
 @pytest.mark.parametrize("precision", [prb.PR_PRECISION_FP64, prb.PR_PRECISION_MIXED])
 @pytest.mark.parametrize("depth,offset", [(3, 0), (4, 0), (4, 1), (5, 0), (5, 1), (5, 2)])
 def test_operator_on_device_vectors(ctx, depth, offset, precision):
