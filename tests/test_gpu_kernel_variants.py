@@ -55,6 +55,40 @@ def test_coarse_levels_in_one_launch_and_level_by_level(ctx, depth, pw, precisio
         assert np.array_equal(m1.vertices, m0.vertices) and np.array_equal(m1.triangles, m0.triangles)
 
 
+def test_replayed_and_plain_launches(monkeypatch):
+    """One context takes clouds of several sizes, weights, sweeps, depths, precisions and both degrees until
+    it has dropped its 64 graphs, comes back to the first of them again and again, and gives what another
+    context gives without graphs."""
+    configs = []
+    for k in range(60):  # two or three graphs of degree 1, one of degree 2 each
+        configs.append((1000 + 700 * (k % 5), prb.ReconstructParams(
+            depth=5 + k % 2, degree=1 + (k // 2) % 2, point_weight=0.0 if k % 9 == 5 else 1.0 + 0.5 * k,
+            smooth_sweeps=1 + (k % 7 == 4),
+            precision=prb.PR_PRECISION_FP64 if k % 3 == 2 else prb.PR_PRECISION_MIXED)))
+    order = [i for k in range(len(configs)) for i in (k, 0)] + list(range(len(configs)))
+    with prb.Context(0) as replayed, prb.Context(0) as plain:
+        expected = {}
+        for i in order:
+            n, params = configs[i]
+            pts = synthetic.torus(n, seed=i)
+            if i not in expected:
+                monkeypatch.setenv("PR_GRAPHS", "0")
+                expected[i] = _solution(plain, pts, params)
+                monkeypatch.delenv("PR_GRAPHS")
+            assert _same(_solution(replayed, pts, params), expected[i]), (i, configs[i])
+
+
+@pytest.mark.parametrize("spmv,resid,smooth", [(2, 4, 4), (4, 2, 4), (4, 4, 2), (2, 2, 4), (4, 2, 2), (2, 4, 2)])
+def test_plane_counts_of_the_kernel_families_mix(ctx, spmv, resid, smooth, monkeypatch):
+    """Two or four planes per thread, by kernel family: the same bits in any mixture."""
+    pts, params = synthetic.torus(3000, seed=33), prb.ReconstructParams(depth=6, point_weight=4.0)
+    monkeypatch.setenv("PR_ZT", "4")
+    expected = _solution(ctx, pts, params)
+    for family, value in (("SPMV16", spmv), ("RESID16", resid), ("SMOOTH16", smooth)):
+        monkeypatch.setenv("PR_ZT_" + family, str(value))
+    assert _same(_solution(ctx, pts, params), expected)
+
+
 @pytest.mark.parametrize("precision", [prb.PR_PRECISION_FP64, prb.PR_PRECISION_MIXED])
 @pytest.mark.parametrize("depth,offset", [(3, 0), (4, 0), (4, 1), (5, 0), (5, 1), (5, 2)])
 def test_operator_on_device_vectors(ctx, depth, offset, precision):
