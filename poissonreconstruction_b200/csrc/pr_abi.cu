@@ -180,12 +180,14 @@ void* alloc_host_out(size_t bytes) {
   return p;
 }
 
-// Large copies between pageable host memory and the device go through pinned slots (pr_staged_copy.h, 8 MiB
-// per context).  Measured (ms, the driver's path and this one): out 2 MB 0.34 and 0.23 with one thread, 17 MB
-// 2.1 and 1.5 with two, 134 MB 27 and 9.9 with four; in, what a solve takes longer from pageable points than
-// from pinned ones, 48 MB 3.6 and 1.0 with four, while 19 MB and less gain nothing.  Pinned caller memory,
-// small copies, the batch engine's threads (many copies at once) and a host without pinned memory for the
-// slots keep the driver's path.
+// Large copies between pageable host memory and the device go through pinned slots (pr_staged_copy.h): four of
+// 192 KiB in memory that every context has (out of the device only), or eight of 1 MiB, which are faster but take
+// 6 ms to allocate.  A context makes those when its copies of 8 MiB and more come to kSlotsFrom bytes, about as
+// many as save that.  Measured (ms; the driver's path, 192 KiB, 1 MiB; destinations in huge pages): out 2 MB
+// 0.42, 0.21, 0.20 with one thread, 24 MB 4.8, 2.0, 1.7 with two, 134 MB 26, 15.6, 8.1 with four; in 48 MB 3.1,
+// 2.6, 1.6 with four, 17 MB 0.87, 0.96, 0.72 with two.  Pinned caller memory, small copies, the batch engine's
+// threads (many copies at once) and a host without pinned memory for the slots keep the driver's path.
+constexpr size_t kSlotsFrom = size_t(112) << 20;
 thread_local bool t_in_batch = false;
 
 // threads that copy pieces, one: the calling thread by itself; 0: the plain path
@@ -200,10 +202,21 @@ int stage_threads(const void* host, size_t bytes, bool out) {
   const int nt = bytes < size_t(8) << 20 ? 1 : (bytes < size_t(32) << 20 ? 2 : pr::kStageThreads);
   return std::max(1, std::min<int>(nt, (int)std::thread::hardware_concurrency()));
 }
+// the slots of a copy; null: it takes the driver's path
+pr::StageSlots* staged_slots(pr_context* c, size_t bytes, bool out) {
+  if (bytes >= size_t(8) << 20) {
+    c->staged += bytes;
+    if (c->staged >= kSlotsFrom && c->slots.make()) return &c->slots;
+  }
+  if (!out || !c->make_block()) return nullptr;
+  constexpr size_t n = 4;
+  return c->block_slots.lend(c->h_block + c->kRing, (c->kBlock - c->kRing) / n, n) ? &c->block_slots : nullptr;
+}
 bool copy_staged(pr_context* c, void* dev, void* host, size_t bytes, bool out) {
   const int nt = stage_threads(host, bytes, out);
-  if (nt == 0 || !c->slots.make()) return false;
-  const cudaError_t e = pr::staged_copy(c->stream, c->slots, static_cast<unsigned char*>(dev),
+  pr::StageSlots* const slots = nt ? staged_slots(c, bytes, out) : nullptr;
+  if (!slots) return false;
+  const cudaError_t e = pr::staged_copy(c->stream, *slots, static_cast<unsigned char*>(dev),
                                         static_cast<unsigned char*>(host), bytes, nt, out);
   if (e != cudaSuccess) {
     cudaStreamSynchronize(c->stream);
@@ -862,8 +875,8 @@ int pr_context_create(int device, void* stream, pr_context** out_ctx) {
       PR_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
       c->own_stream = true;
     }
-    PR_CUDA(cudaMallocHost(&c->h_scalars, 64 * sizeof(double)));
-    PR_CUDA(cudaMallocHost(&c->h_flag, sizeof(int)));
+    PR_CUDA(cudaMallocHost(&c->h_scalars, 65 * sizeof(double)));
+    c->h_flag = reinterpret_cast<int*>(c->h_scalars + 64);
     {
       std::lock_guard<std::mutex> g(pr::spare_mutex());
       pr::context_registry().insert(c.get());
@@ -899,9 +912,10 @@ int pr_context_destroy(pr_context* c) {
     }
     if (c->h_scalars) cudaFreeHost(c->h_scalars);
     if (c->h_pack) cudaFreeHost(c->h_pack);
-    if (c->h_ring) cudaFreeHost(c->h_ring);
+    c->block_slots.free();
     c->slots.free();
-    if (c->h_flag) cudaFreeHost(c->h_flag);
+    if (c->h_ring && c->h_ring != c->h_block) cudaFreeHost(c->h_ring);
+    if (c->h_block) cudaFreeHost(c->h_block);
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;

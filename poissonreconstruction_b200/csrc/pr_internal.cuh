@@ -154,6 +154,17 @@ struct pr_context {
     }
     return h_pack;
   }
+  // 1 MiB of pinned memory, made by the first call that needs some of it: a ring for `upload`, then the
+  // slots of `block_slots`.  (Pinning 1 MiB takes 0.8 ms, 2 MiB 2, 8 MiB 6.)
+  static constexpr size_t kBlock = size_t(1) << 20, kRing = size_t(256) << 10;
+  unsigned char* h_block = nullptr;
+  bool make_block() {
+    if (h_block) return true;
+    if (cudaMallocHost(&h_block, kBlock) == cudaSuccess) return true;
+    cudaGetLastError();
+    h_block = nullptr;
+    return false;
+  }
   // Pinned ring for small host -> device tables: the bytes are copied into it and from there to the
   // device on `stream`, so the caller's buffer is free at once and the host does not wait.  When the
   // ring is full the stream is waited for, after which none of it is in flight.
@@ -162,24 +173,28 @@ struct pr_context {
   void upload(void* dst, const void* src, size_t bytes) {
     if (bytes == 0) return;
     const size_t need = (bytes + 255) & ~size_t(255);
+    if (!h_ring && make_block()) {
+      h_ring = h_block;
+      h_ring_cap = kRing;
+    }
     if (h_ring_used + need > h_ring_cap) {
-      PR_CUDA(cudaStreamSynchronize(stream));
-      h_ring_used = 0;
+      sync();
       if (need > h_ring_cap) {
-        if (h_ring) PR_CUDA(cudaFreeHost(h_ring));
+        if (h_ring && h_ring != h_block) PR_CUDA(cudaFreeHost(h_ring));
         h_ring = nullptr;
         h_ring_cap = 0;
-        const size_t cap = need > (size_t(1) << 20) ? need : (size_t(1) << 20);
-        PR_CUDA(cudaMallocHost(&h_ring, cap));
-        h_ring_cap = cap;
+        PR_CUDA(cudaMallocHost(&h_ring, need));
+        h_ring_cap = need;
       }
     }
     std::memcpy(h_ring + h_ring_used, src, bytes);
     PR_CUDA(cudaMemcpyAsync(dst, h_ring + h_ring_used, bytes, cudaMemcpyHostToDevice, stream));
     h_ring_used += need;
   }
-  pr::StageSlots slots;  // of the copies between pageable host memory and the device (pr_abi.cu)
-  int* h_flag = nullptr;  // pinned: the status of the last spd_inverse (pr_operator.cu)
+  // slots of the large copies between pageable host memory and the device (pr_abi.cu)
+  pr::StageSlots block_slots, slots;
+  size_t staged = 0;      // bytes of those copies so far
+  int* h_flag = nullptr;  // pinned, behind h_scalars: the status of the last spd_inverse (pr_operator.cu)
   // pinned staging for device->host mesh copies (grown on demand)
   unsigned char* h_stage = nullptr;
   size_t h_stage_cap = 0;
@@ -376,7 +391,10 @@ struct pr_context {
     spare_bytes += it->second.cap;
     bufs.erase(it);
   }
-  void sync() { PR_CUDA(cudaStreamSynchronize(stream)); }
+  void sync() {
+    PR_CUDA(cudaStreamSynchronize(stream));
+    h_ring_used = 0;  // nothing of it is in flight
+  }
 };
 
 namespace pr {
