@@ -93,9 +93,8 @@ __device__ __forceinline__ int floor_div(int a, int b) { return a >= 0 ? a / b :
 // 9 per axis), then the separable sums over x, y and z, every one in increasing coarse index, so
 // a node gets the same bits in any tile.  scratch: 729 + 81 TT + 9 TT^2 doubles and the taps.
 // A fine node has at most 3 taps per axis (3 2^L - 2 of them, 2^L apart): they are looked up once per tile
-// and axis.  (Tried one by one over the coarse range for every node, with the weights read from constant
-// memory at an index of each lane's own: k_ab_mc_count 6.6 -> 5.2 ms at 428,000 bricks, the first residual
-// 12.0 -> 9.9.)
+// and axis: k_ab_mc_count 5.2 ms at 428,000 bricks, the first residual 9.9.  (6.6 and 12.0 where every node
+// tries the coarse range one by one, its weights from constant memory at an index of each lane's own.)
 struct Taps {
   double w[3];
   int first, n;  // coarse index (from the tile's first), taps
@@ -330,7 +329,7 @@ __global__ void __launch_bounds__(kThreads) k_ab_rhs(const uint32_t* __restrict_
     }
     for (int i = t; i < 3 * kOT3; i += kThreads) nf[i] = 0.0;
     __syncthreads();
-    // the neighbours' runs as one list (brick by brick each waited for its loads: 14.6 -> 9.3 ms at 428,000 bricks)
+    // the neighbours' runs as one list: 9.3 ms at 428,000 bricks (14.6 brick by brick, each waiting for its loads)
     int k = 0;
     for (uint32_t i = t; i < before[27]; i += kThreads) {
       while (i >= before[k + 1]) ++k;
@@ -408,11 +407,12 @@ __global__ void __launch_bounds__(kThreads) k_ab_rhs(const uint32_t* __restrict_
 // flight while the y and x passes work on this one; a tile plane holds its 12 rows' 8 own values, then
 // their 4 side values (x = -2, -1, 8, 9), so that the gather is 16-byte copies by consecutive lanes
 // (cp.async) and 8-byte loads (through registers: cheaper there than as 8-byte copies); planes are padded against bank conflicts; the z and y passes work on pairs
-// (64-bit shared accesses, two FP32 FMAs to an instruction).  FP32 at 219M nodes (depth 11): operator and
-// update pass 3.04 -> 2.61 ms an iteration (1.76 + 1.29 -> 1.84 + 0.77); at the copy rate the two would
-// take 0.82 + 0.68.  The shared-memory pipe is busy for about 75 % of the operator's cycles (29M nodes).
+// (64-bit shared accesses, two FP32 FMAs to an instruction).  FP32 at 219M nodes (depth 11): operator 1.84 ms
+// and update pass 0.77 (1.76 and 1.29 with a plain 12^3 tile, a column to a thread and x's step in the
+// update); at the copy rate the two would take 0.82 and 0.68.  The shared-memory pipe is busy for about 75 %
+// of the operator's cycles (29M nodes).
 constexpr int kOpThreads = 96;
-constexpr int kOpCtas = 8;       // per SM (shared memory, registers); the grid is one wave of them
+constexpr int kOpCtas = 8;       // FP32 CTAs per SM (shared memory, registers); the grid is one wave of them, two in FP64
 constexpr int kTP = 144;         // tile plane: [y 12][8], then [y 12][4]
 constexpr int kFO = 104;         // z-filtered plane, own columns [y 12][8]
 constexpr int kFS = 52;          // side columns [y 12][4]
@@ -421,7 +421,7 @@ constexpr int kWP = 8 * 12 + 8;  // y-filtered plane: [y 8][12]; the y pass puts
 static_assert(8 * kWP <= kFW, "y-filtered planes fit the z-filtered ones");
 enum { kBandApply = 0, kBandResid = 1, kBandDir = 2 };
 // the scalars of a CG solve, on the device: one host read an iteration instead of two, and two sum
-// launches instead of three (depth 9 over 7, 50 iterations: 11.6 -> 11.0 ms)
+// launches instead of three (depth 9 over 7, 50 iterations: 11.0 ms instead of 11.6)
 struct CgBand {
   double rr, rz, dq, alpha, beta;
 };

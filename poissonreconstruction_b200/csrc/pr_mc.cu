@@ -241,7 +241,7 @@ __global__ void k_iso_partial(const double* __restrict__ x, uint32_t D, const do
 }
 
 // the partials in order, one chain (thread 0); staged through shared memory, from which the chain reads
-// ahead (from global memory it waited for every load): 90 -> 40 us at 1M points, 30 -> 15 at 100k
+// ahead (from global memory it waits for every load): 40 us instead of 90 at 1M points, 15 instead of 30 at 100k
 __global__ void __launch_bounds__(kThreads) k_iso_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
   __shared__ double s[2 * kThreads];
   Neu t{0.0, 0.0};
@@ -343,9 +343,9 @@ __global__ void k_mc_vertices(const double* __restrict__ x, uint32_t D, double i
 // Vertices are slots with equal keys.  An open-addressing table (a power of two, 2 E entries or more)
 // takes each key once; its entry ends as the smallest slot of that key, whatever the order of the
 // insertions.  home[s] = the entry of slot s's key.  Scattered reads and atomics in L2 bound it: 46 us for
-// the mesh of depth 9, k_mc_first 15, and k_mc_emit_tris 24 more than with ids in slot order.  An LSD radix
-// sort of the 90-bit keys, two gathers and two passes over the runs, which stood here, took about 0.5 ms,
-// and 35 launches more at depth 5, where the mesh as a whole went from 1.62 to 1.48 ms.
+// the mesh of depth 9, k_mc_first 15, and k_mc_emit_tris 24 more than with ids in slot order.  By an LSD radix
+// sort of the 90-bit keys, two gathers and two passes over the runs it is about 0.5 ms, and at depth 5 35
+// launches more.
 constexpr uint32_t kNoSlot = 0xffffffffu;
 __global__ void k_mc_hash(const uint64_t* __restrict__ k1, const uint32_t* __restrict__ k2, uint64_t E, uint32_t mask,
                           uint32_t* __restrict__ table, uint32_t* __restrict__ home) {
@@ -645,9 +645,9 @@ __device__ __forceinline__ uint32_t mc_mask_case(const uint32_t* mask, int lx, i
          ((m01 >> 1) & 1u) << 5 | ((m11 >> 1) & 1u) << 6 | (m11 & 1u) << 7;
 }
 
-// Reading the values bounds it: 8.6 GB at depth 10, 1.33 ms at the copy rate.  Degree 1: 3.82 -> 1.62 ms
-// (before, through a tile in shared memory, read back by a thread per row); degree 2: 6.66 -> 4.11 (before,
-// every block's corners were formed; rows of 128 bytes, and the index arithmetic of the 18^3 tile, hold it).
+// Reading the values bounds it: 8.6 GB at depth 10, 1.33 ms at the copy rate.  Degree 1: 1.62 ms (3.82
+// through a tile in shared memory that a thread per row reads back); degree 2: 4.11 (6.66 where every
+// block's corners are formed; rows of 128 bytes, and the index arithmetic of the 18^3 tile, hold it).
 template <int DEG>
 __global__ void __launch_bounds__(256) k_mc_block_count(const double* __restrict__ x, uint32_t D, double iso,
                                                         uint32_t* __restrict__ blockcnt) {

@@ -643,10 +643,11 @@ __device__ __forceinline__ void plane_sums(const T r[4][4], T f[4], T d[4], T ct
 // apart) fill the 32 banks once; the halo planes' rows are 20 words and the planes 368 words apart, which
 // puts the 16 lanes of a halo access on the 16 even banks.
 // What bounds the kernels is the L1's data pipe (84% busy in the post-smoothing sweep: its own columns,
-// 5 neighbouring ones per phase, shuffles, and the halo's sectors).  At depth 9 in FP32, against the
-// plane-by-plane tile with one quad per lane and plane before: post-smoothing 753 -> 537 us (floor by
-// HBM bytes 260), CG update and pre-smoothing 750 -> 556 (583), residual and restriction 560 -> 482
-// (177), first sweep 277 -> 184 (167), plain SpMV 338 -> 311 (167), with d = z + beta d 454 -> 462 (333).
+// 5 neighbouring ones per phase, shuffles, and the halo's sectors).  At depth 9 in FP32, in us, with the
+// floor by HBM bytes and the time on a plane-by-plane tile with one quad per lane and plane:
+//   post-smoothing 537 (floor 260; 753 plane by plane), CG update and pre-smoothing 556 (583; 750),
+//   residual and restriction 482 (177; 560), first sweep 184 (167; 277), plain SpMV 311 (167; 338),
+//   with d = z + beta d 462 (333; 454).
 // Every value and every sum is the same for every ZT.
 namespace z16 {
 constexpr int kCS = 24, kRY = 18 * kCS + 4, kHR = 20, kHP = 368, TILE = 18 * kRY + 2 * kHP;
@@ -1423,9 +1424,8 @@ constexpr size_t smem_bytes() {
 // values are written after a barrier), a Jacobi step along the column for those rows only.  On the
 // coarse levels these rows are a phase's critical path (few blocks, most of them on a face), so a
 // row is unrolled: its 26 tile and table loads (the table in shared memory) are in flight together
-// before the chain of its multiply-adds.  In a rolled loop with the table in global memory a launch
-// of the levels 16^3 to 64^3 took 29-31 us (115 us at 8 planes per thread); a depth-7 reconstruction
-// of 20,011 points went from 4.65 to 3.22 ms and a depth-9 one of 317,003 from 33.0 to 29.9 ms.
+// before the chain of its multiply-adds: post-smoothing on 32^3 and 64^3 in FP32 8.1 us, the first sweep
+// 6.1 (29 to 31 us in a rolled loop with the table in global memory).
 namespace g16 {
 // CTAs per SM that the register budget is set for: four, three where the face rows would spill
 template <typename T, bool FACES, int ZT>
